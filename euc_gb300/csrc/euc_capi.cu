@@ -479,6 +479,19 @@ void dispatch_resolve_ordered(uint32_t shader, const SceneDev *sc, const uint64_
     }
 }
 
+// Four-texel words need every source row aligned to the word (four texels'
+// bytes up to a 4-byte word for RGB8's three) and every target row to 16 bytes.
+template <uint32_t FMT>
+void launch_ingest(const uint8_t *src, uint64_t spitch, uint8_t *dst, uint64_t dpitch, uint32_t W, uint32_t H,
+                   cudaStream_t st) {
+    const uint64_t word = src_bpp(FMT) == 3 ? 4 : 4 * src_bpp(FMT);
+    const bool vec = ((uintptr_t)src | spitch) % word == 0 && ((uintptr_t)dst | dpitch) % 16 == 0;
+    const dim3 grid((unsigned)(((uint64_t)W + 4 * kIngestQuads - 1) / (4 * kIngestQuads)),
+                    (unsigned)std::min<uint64_t>(((uint64_t)H + 8 * kIngestRows - 1) / (8 * kIngestRows), 65535u));
+    if (vec) k_ingest<FMT, true><<<grid, dim3(32, 8), 0, st>>>(src, spitch, dst, dpitch, W, H);
+    else k_ingest<FMT, false><<<grid, dim3(32, 8), 0, st>>>(src, spitch, dst, dpitch, W, H);
+}
+
 // Runs a batch of scenes.  All pointers inside `scenes` are device pointers.
 // Staging supplied by a CUDA graph instead of the context's ring.  With
 // `dry` the batch is planned and the scratch buffers are sized, nothing is
@@ -1345,8 +1358,14 @@ int euc_texture_ingest(euc_ctx *ctx, const void *src, uint32_t width, uint32_t h
         from = (const uint8_t *)ctx->h_tex[0].p;
         pitch = srow;
     }
-    const dim3 grid((unsigned)((width + 31) / 32), (unsigned)std::min<uint32_t>(height, 65535u));
-    k_ingest<<<grid, dim3(32, 8), 0, st>>>(from, pitch, src_format, (uint8_t *)dst, dst_pitch, width, height);
+    switch (src_format) {
+    case EUC_SRC_RGBA8: launch_ingest<EUC_SRC_RGBA8>(from, pitch, (uint8_t *)dst, dst_pitch, width, height, st); break;
+    case EUC_SRC_BGRA8: launch_ingest<EUC_SRC_BGRA8>(from, pitch, (uint8_t *)dst, dst_pitch, width, height, st); break;
+    case EUC_SRC_RGB8: launch_ingest<EUC_SRC_RGB8>(from, pitch, (uint8_t *)dst, dst_pitch, width, height, st); break;
+    case EUC_SRC_LUMA8: launch_ingest<EUC_SRC_LUMA8>(from, pitch, (uint8_t *)dst, dst_pitch, width, height, st); break;
+    case EUC_SRC_R32F: launch_ingest<EUC_SRC_R32F>(from, pitch, (uint8_t *)dst, dst_pitch, width, height, st); break;
+    default: launch_ingest<EUC_SRC_LUMA_ALPHA8>(from, pitch, (uint8_t *)dst, dst_pitch, width, height, st); break;
+    }
     ctx->launches += 1;
     CUDA_TRY(cudaGetLastError());
     if (!on_device) CUDA_TRY(cudaStreamSynchronize(st));  // the staging is reused by the next call

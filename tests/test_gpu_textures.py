@@ -79,3 +79,40 @@ def test_texture_ingest_matches_oracle(fmt, ch, dtype, where):
         del keep
     finally:
         ctx.close()
+
+
+@pytest.mark.parametrize("fmt,ch,dtype", [(abi.SRC_RGBA8, 4, np.uint8), (abi.SRC_BGRA8, 4, np.uint8),
+                                          (abi.SRC_RGB8, 3, np.uint8), (abi.SRC_LUMA8, 1, np.uint8),
+                                          (abi.SRC_LUMA_ALPHA8, 2, np.uint8), (abi.SRC_R32F, 1, np.float32)])
+@pytest.mark.parametrize("w,h,pad,off", [(1, 1, 0, 0), (4, 17, 0, 0), (128, 16, 0, 0), (130, 33, 6, 0), (256, 9, 0, 1),
+                                         (127, 15, 1, 3), (515, 40, 13, 0)])
+def test_texture_ingest_tile_edges(fmt, ch, dtype, w, h, pad, off):
+    """Edges of the 128x16 tiles, aligned and unaligned source rows (`pad`
+    bytes a row, `off` bytes ahead of the first)."""
+    import torch
+    rng = np.random.default_rng(w * 7 + h + fmt)
+    if dtype == np.float32:  # its rows must stay 4-byte aligned
+        pad, off = 4 * pad, 4 * off
+        img = rng.standard_normal((h, w)).astype(np.float32)
+    else:
+        img = rng.integers(0, 256, (h, w, ch), dtype=np.uint8)
+        if ch == 1:
+            img = img[..., 0]
+    want = oracle.texture_ingest(img, fmt)
+    row = w * ch * img.itemsize
+    raw = np.zeros(off + h * (row + pad), dtype=np.uint8)
+    for y in range(h):
+        at = off + y * (row + pad)
+        raw[at:at + row] = np.ascontiguousarray(img[y]).view(np.uint8).reshape(-1)
+    src = torch.from_numpy(raw).cuda()
+    ctx = capi.Context(0)
+    try:
+        dst = torch.zeros((h, w + 4, 4), dtype=torch.uint8, device="cuda")
+        rc = capi.lib().euc_texture_ingest(ctx.handle, src.data_ptr() + off, w, h, row + pad, fmt, dst.data_ptr(),
+                                           dst.stride(0), _stream())
+        assert rc == abi.OK
+        torch.cuda.synchronize()
+        assert np.array_equal(dst.cpu().numpy()[:, :w], want)
+        assert (dst.cpu().numpy()[:, w:] == 0).all()
+    finally:
+        ctx.close()
