@@ -663,12 +663,10 @@ int run_batch(euc_ctx *ctx, const euc_scene *scenes, size_t n, cudaStream_t st, 
     prep.err = (int *)ctx->err.p;
     prep.stats = (SceneStats *)ctx->stats.p;
     prep.cov = (uint4 *)ctx->cov.p;
-    prep.chunk_sums = (uint2 *)ctx->chunk_sums.p;
     prep.strip_cnt = (uint32_t *)ctx->strip_cnt.p;
     prep.strip_fill = (uint32_t *)ctx->strip_fill.p;
     prep.totals = (unsigned long long *)ctx->totals.p;
-    prep.nchunks = nchunks;
-    prep.n = std::max<uint64_t>(std::max<uint64_t>((uint64_t)ns, nchunks), std::max<uint64_t>(nstrips, 2));
+    prep.n = std::max<uint64_t>((uint64_t)ns, std::max<uint64_t>(nstrips, 2));
     prep.nsc = (uint32_t)ns;
     prep.nstrips = (uint32_t)nstrips;
     // vertex stage, one launch per shader kind; the first also does the clears
@@ -1861,10 +1859,8 @@ extern "C" int euc_render_noalloc(const euc_pipeline_desc *desc, const void *uni
     prep.err = (int *)(a + kNaOffErr);
     prep.stats = (SceneStats *)(a + kNaOffStats);
     prep.cov = (uint4 *)(a + kNaOffCov);
-    prep.chunk_sums = (uint2 *)(a + kNaOffChunks);
     prep.totals = (unsigned long long *)(a + kNaOffTotals);
-    prep.nchunks = tri / kBlock;
-    prep.n = std::max<uint64_t>(prep.nchunks, 2);
+    prep.n = 2;
     prep.nsc = 1;
     k_prep<<<(unsigned)((prep.n + kBlock - 1) / kBlock), kBlock, 0, st>>>(prep);
     t_na_nsm = nsm;

@@ -8,8 +8,8 @@
 //                 (index.rs:52-54), flip, perspective divide, winding, cull /
 //                 reverse, weight matrix, screen bbox, per-pixel weight deltas,
 //                 vertices by y, z-clip class (triangles.rs:55-199)
-//   k_prep        per batch: clears the error, statistics, covered-rectangle
-//                 and setup-sum entries (done by the first k_vertex launch
+//   k_prep        per batch: clears the error, statistics and
+//                 covered-rectangle entries (done by the first k_vertex launch
 //                 when the batch has one)
 //   k_scan_plan   exclusive scan of per-primitive row counts, compaction of the
 //                 primitives that cover at least one row; one more block
@@ -255,10 +255,9 @@ EUC_DEV T block_excl_scan(T v, T *smem /* >= kBlock/32 + 1 */, T *total) {
 
 // ---------------------------------------------------------------------------
 // The per-batch clears before k_setup: each scene's error, statistics and
-// covered rectangle, the setup-chunk sums, the strip counts and the strip
-// path's counters (totals[6]: entries taken, totals[7]: k_strip's work
-// counter).  Entry i of the n = max(scenes, chunks, strips, 2) covers index i
-// of each.  The first vertex launch of a batch does them (nothing it reads or
+// covered rectangle, the strip counts and the strip path's counters
+// (totals[6]: entries taken, totals[7]: k_strip's work counter).  Entry i of
+// the n = max(scenes, strips, 2) covers index i of each.  The first vertex launch of a batch does them (nothing it reads or
 // writes is cleared), which saves a launch; k_prep does them when a batch has
 // no vertex launch, and on the no-allocation path.
 // ---------------------------------------------------------------------------
@@ -266,10 +265,9 @@ struct PrepArgs {
     int *err;
     SceneStats *stats;
     uint4 *cov;
-    uint2 *chunk_sums;
     uint32_t *strip_cnt, *strip_fill;
     unsigned long long *totals;
-    uint64_t nchunks, n;  // n = 0: nothing to clear
+    uint64_t n;  // n = 0: nothing to clear
     uint32_t nsc, nstrips;
 };
 
@@ -279,7 +277,6 @@ EUC_DEV void prep_clear(const PrepArgs &a, uint64_t i) {
         a.stats[i] = SceneStats{};
         a.cov[i] = make_uint4(0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu);
     }
-    if (i < a.nchunks) a.chunk_sums[i] = make_uint2(0u, 0u);
     if (i < a.nstrips) {
         a.strip_cnt[i] = 0;
         a.strip_fill[i] = 0;
@@ -616,7 +613,7 @@ __host__ __device__ inline uint32_t width_bucket(uint32_t w) {
 // k_setup: triangles.rs:55-199, once per primitive (euc repeats it per band;
 // only the bbox clamp depends on the band and that is applied per row).
 // Block b sets up primitives [b * kBlock, (b + 1) * kBlock), all of scene
-// chunk_scene[b] (null: scene 0); chunk_sums must be zero at launch.  bbox
+// chunk_scene[b] (null: scene 0).  bbox
 // (null when the batch has no strips) receives the bbox of every triangle
 // with rows: the binning reads those 16 bytes instead of the record's line.
 // ---------------------------------------------------------------------------
@@ -631,6 +628,8 @@ __global__ void __launch_bounds__(kBlock) k_setup(const SceneDev *__restrict__ s
     // 16-byte word k of lane l's record sits at l * 8 + (k ^ (l & 7)), which
     // keeps both the staging and the copy-out at the minimum four wavefronts
     __shared__ uint4 s_rec[kBlock / 32][32 * 8];
+    __shared__ uint4 s_cov[kBlock / 32], s_sum[kBlock / 32];
+    __shared__ unsigned long long s_walk[kBlock / 32];
     const int lane = threadIdx.x & 31;
     uint4 *stage = s_rec[threadIdx.x >> 5];
     bool staged = false;
@@ -840,29 +839,46 @@ __global__ void __launch_bounds__(kBlock) k_setup(const SceneDev *__restrict__ s
         }
     }
     rows[t] = nrows;
-    // the scene's covered rectangle: min of (x0, y0, ~x1, ~y1) over its primitives
-    {
-        const uint32_t m0 = __reduce_min_sync(0xFFFFFFFFu, cx0), m1 = __reduce_min_sync(0xFFFFFFFFu, cy0);
-        const uint32_t m2 = __reduce_min_sync(0xFFFFFFFFu, ~cx1), m3 = __reduce_min_sync(0xFFFFFFFFu, ~cy1);
-        if ((threadIdx.x & 31) == 0 && m0 != 0xFFFFFFFFu) {
-            atomicMin(&cov[si].x, m0);
-            atomicMin(&cov[si].y, m1);
-            atomicMin(&cov[si].z, m2);
-            atomicMin(&cov[si].w, m3);
-        }
+    // The block's sums, one atomic each: the scene's covered rectangle (min of
+    // (x0, y0, ~x1, ~y1) over its primitives), its culled count and, for the
+    // strip path's routing, the pixels its rows may walk; the scan's per-chunk
+    // sums are this block's alone.  One set of atomics a block, not a warp: all
+    // of a scene's meet in two L2 sectors, where nine a warp (15.6 k warps of a
+    // 500 k triangle mesh) bounded this kernel.
+    const uint32_t m0 = __reduce_min_sync(0xFFFFFFFFu, cx0), m1 = __reduce_min_sync(0xFFFFFFFFu, cy0);
+    const uint32_t m2 = __reduce_min_sync(0xFFFFFFFFu, ~cx1), m3 = __reduce_min_sync(0xFFFFFFFFu, ~cy1);
+    const uint32_t wl = __popc(__ballot_sync(0xFFFFFFFFu, nrows != 0)), wr = __reduce_add_sync(0xFFFFFFFFu, nrows);
+    const uint32_t wc = __popc(__ballot_sync(0xFFFFFFFFu, culled != 0));
+    const unsigned long long ww = bbox ? warp_sum(nrows ? (unsigned long long)frag_est : 0ull) : 0ull;
+    if (lane == 0) {
+        const int w = threadIdx.x >> 5;
+        s_cov[w] = make_uint4(m0, m1, m2, m3);
+        s_sum[w] = make_uint4(wl, wr, wc, 0u);
+        s_walk[w] = ww;
     }
-    // per-block sums for the scan (zeroed before the launch; each warp adds
-    // its own, no block barrier), the culled count of this scene, and the
-    // pixels its rows may walk (the strip path's routing)
-    const uint32_t live = nrows ? 1u : 0u;
-    uint32_t wl = warp_sum(live), wr = warp_sum(nrows), wc = warp_sum(culled);
-    const unsigned long long ww = warp_sum(nrows ? (unsigned long long)frag_est : 0ull);
-    if ((threadIdx.x & 31) == 0) {
-        if (wl) atomicAdd(&chunk_sums[blockIdx.x].x, wl);
-        if (wr) atomicAdd(&chunk_sums[blockIdx.x].y, wr);
-        if (wc) atomicAdd(&stats[si].culled, (unsigned long long)wc);
-        if (ww) atomicAdd(&stats[si].walked, ww);
-        if (wl) atomicAdd(&stats[si].live, (unsigned long long)wl);
+    __syncthreads();
+    if (threadIdx.x < kBlock / 32) {
+        constexpr uint32_t kMask = (1u << (kBlock / 32)) - 1u;
+        const uint4 c = s_cov[threadIdx.x], q = s_sum[threadIdx.x];
+        unsigned long long bw = s_walk[threadIdx.x];
+        const uint32_t b0 = __reduce_min_sync(kMask, c.x), b1 = __reduce_min_sync(kMask, c.y);
+        const uint32_t b2 = __reduce_min_sync(kMask, c.z), b3 = __reduce_min_sync(kMask, c.w);
+        const uint32_t bl = __reduce_add_sync(kMask, q.x), br = __reduce_add_sync(kMask, q.y);
+        const uint32_t bc = __reduce_add_sync(kMask, q.z);
+#pragma unroll
+        for (int d = kBlock / 64; d > 0; d >>= 1) bw += __shfl_xor_sync(kMask, bw, d);
+        if (threadIdx.x == 0) {
+            chunk_sums[blockIdx.x] = make_uint2(bl, br);
+            if (b0 != 0xFFFFFFFFu) {
+                atomicMin(&cov[si].x, b0);
+                atomicMin(&cov[si].y, b1);
+                atomicMin(&cov[si].z, b2);
+                atomicMin(&cov[si].w, b3);
+            }
+            if (bc) atomicAdd(&stats[si].culled, (unsigned long long)bc);
+            if (bw) atomicAdd(&stats[si].walked, bw);
+            if (bbox && bl) atomicAdd(&stats[si].live, (unsigned long long)bl);
+        }
     }
 }
 
