@@ -48,7 +48,9 @@ struct euc_ctx {
     int device = 0;
     int nsm = 0;
     DevBuf clip, vdata, recs, rows, chunk_sums, live_tri, live_rowoff, totals, vbuf, err, stats, cov;
-    DevBuf obsum, frags;  // ordered path: pixel-scan block sums, fragment lists
+    DevBuf frags;         // ordered path: fragment lists
+    unsigned long long *h_total = nullptr;  // ... and their number, written by k_oscan (page-locked)
+    cudaEvent_t total_ready = nullptr;
     DevBuf plan;          // plan_chunks: k_init and k_resolve chunk bases (2 x (scenes + 1))
     DevBuf galive;        // geometry stage: 1 per output slot that holds a triangle
     // strip path: per-strip entry counts, fill cursors, list offsets, unit
@@ -459,23 +461,25 @@ void dispatch_resolve(uint32_t shader, const SceneDev *sc, const uint64_t *rbase
 
 template <class F>
 void launch_resolve_ordered(const SceneDev *sc, const uint64_t *pb, int s0, int s1, uint64_t blk0, uint64_t nblk,
-                            euc_ctx *ctx, cudaStream_t st) {
+                            uint64_t cap, euc_ctx *ctx, cudaStream_t st) {
     if (nblk)
         k_resolve_ordered<F><<<(unsigned)nblk, kBlock, 0, st>>>(sc, pb, s0, s1, blk0, (const TriRec *)ctx->recs.p,
                                                                 (const float *)ctx->vdata.p,
                                                                 (const unsigned long long *)ctx->vbuf.p,
-                                                                (const uint2 *)ctx->frags.p, (const uint4 *)ctx->cov.p);
+                                                                (const uint2 *)ctx->frags.p, cap,
+                                                                (const unsigned long long *)ctx->totals.p,
+                                                                (const uint4 *)ctx->cov.p);
 }
 
 void dispatch_resolve_ordered(uint32_t shader, const SceneDev *sc, const uint64_t *pb, int s0, int s1, uint64_t blk0,
-                              uint64_t nblk, euc_ctx *ctx, cudaStream_t st) {
+                              uint64_t nblk, uint64_t cap, euc_ctx *ctx, cudaStream_t st) {
     switch (shader) {
-    case EUC_SHADER_FLAT: launch_resolve_ordered<FlatFn>(sc, pb, s0, s1, blk0, nblk, ctx, st); break;
-    case EUC_SHADER_VCOLOR: launch_resolve_ordered<VColorFn>(sc, pb, s0, s1, blk0, nblk, ctx, st); break;
-    case EUC_SHADER_GOURAUD: launch_resolve_ordered<GouraudFn>(sc, pb, s0, s1, blk0, nblk, ctx, st); break;
-    case EUC_SHADER_TEXTURED: launch_resolve_ordered<TexturedFn>(sc, pb, s0, s1, blk0, nblk, ctx, st); break;
-    case EUC_SHADER_PHONG: launch_resolve_ordered<PhongFn>(sc, pb, s0, s1, blk0, nblk, ctx, st); break;
-    case EUC_SHADER_SHADOW: launch_resolve_ordered<ShadowFn>(sc, pb, s0, s1, blk0, nblk, ctx, st); break;
+    case EUC_SHADER_FLAT: launch_resolve_ordered<FlatFn>(sc, pb, s0, s1, blk0, nblk, cap, ctx, st); break;
+    case EUC_SHADER_VCOLOR: launch_resolve_ordered<VColorFn>(sc, pb, s0, s1, blk0, nblk, cap, ctx, st); break;
+    case EUC_SHADER_GOURAUD: launch_resolve_ordered<GouraudFn>(sc, pb, s0, s1, blk0, nblk, cap, ctx, st); break;
+    case EUC_SHADER_TEXTURED: launch_resolve_ordered<TexturedFn>(sc, pb, s0, s1, blk0, nblk, cap, ctx, st); break;
+    case EUC_SHADER_PHONG: launch_resolve_ordered<PhongFn>(sc, pb, s0, s1, blk0, nblk, cap, ctx, st); break;
+    case EUC_SHADER_SHADOW: launch_resolve_ordered<ShadowFn>(sc, pb, s0, s1, blk0, nblk, cap, ctx, st); break;
     }
 }
 
@@ -757,42 +761,55 @@ int run_batch(euc_ctx *ctx, const euc_scene *scenes, size_t n, cudaStream_t st, 
     k_raster<<<rgrid, kBlock, 0, st>>>(dsc, (const TriRec *)ctx->recs.p, (const uint32_t *)ctx->live_tri.p,
                                        (const uint64_t *)ctx->live_rowoff.p, (unsigned long long *)ctx->totals.p,
                                        (const int *)ctx->err.p, (unsigned long long *)ctx->vbuf.p,
-                                       (SceneStats *)ctx->stats.p, 0, nullptr, witems, probe);
+                                       (SceneStats *)ctx->stats.p, 0, nullptr, 0, witems, probe);
     ctx->launches += 4;
-    // ordered scenes: scan the per-pixel counts, size the fragment buffer
-    // (one stream synchronisation), fill the lists in a second raster pass
+    // ordered scenes: the per-pixel counts become list offsets, then the lists
+    // are filled in a second raster pass and resolved.  Both passes are
+    // enqueued against the fragment buffer as it is, and do nothing when the
+    // lists do not fit it; the host waits for the number of fragments alone
+    // (while they run), and enqueues them again after growing the buffer.
     int first_ordered = ns;
     while (first_ordered > 0 && plans[first_ordered - 1].d.keytype == KEY_ORDERED) --first_ordered;
     if (first_ordered < ns) {
         const uint64_t p0 = plans[first_ordered].d.pix_base, p1 = pix;
         const uint64_t nb = (p1 - p0 + kOScanBlock - 1) / kOScanBlock;
-        if ((rc = grow(ctx->obsum, nb * sizeof(unsigned long long)))) return rc;
+        if (!ctx->h_total) CUDA_TRY(cudaMallocHost((void **)&ctx->h_total, sizeof(unsigned long long)));
+        if (!ctx->total_ready) CUDA_TRY(cudaEventCreateWithFlags(&ctx->total_ready, cudaEventDisableTiming));
+        // a first guess: four fragments a pixel, 512 MB at most
+        if ((rc = grow(ctx->frags, std::min<uint64_t>(4 * pix, 1ull << 26) * sizeof(uint2)))) return rc;
         unsigned long long *totals = (unsigned long long *)ctx->totals.p;
-        k_oscan_reduce<<<(unsigned)nb, kBlock, 0, st>>>((const unsigned long long *)ctx->vbuf.p, p0, p1,
-                                                        (unsigned long long *)ctx->obsum.p);
-        k_oscan_apply<<<(unsigned)nb, kBlock, 0, st>>>((unsigned long long *)ctx->vbuf.p, p0, p1,
-                                                       (const unsigned long long *)ctx->obsum.p, totals + 4);
-        unsigned long long nfrag = 0;
-        CUDA_TRY(cudaMemcpyAsync(&nfrag, totals + 4, sizeof(nfrag), cudaMemcpyDeviceToHost, st));
-        CUDA_TRY(cudaStreamSynchronize(st));
-        if (nfrag >= 0xFFFFFFFFull) return EUC_ERR_CAPACITY;  // list offsets are 32-bit
-        if ((rc = grow(ctx->frags, std::max<uint64_t>(nfrag, 1) * sizeof(uint2)))) return rc;
-        k_raster<<<rgrid, kBlock, 0, st>>>(dsc, (const TriRec *)ctx->recs.p, (const uint32_t *)ctx->live_tri.p,
-                                           (const uint64_t *)ctx->live_rowoff.p, (unsigned long long *)ctx->totals.p,
-                                           (const int *)ctx->err.p, (unsigned long long *)ctx->vbuf.p,
-                                           (SceneStats *)ctx->stats.p, 1, (uint2 *)ctx->frags.p, witems, probe);
-        ctx->launches += 3;
+        k_oscan<<<(unsigned)nb, kBlock, 0, st>>>((unsigned long long *)ctx->vbuf.p, p0, p1, totals, ctx->h_total);
+        CUDA_TRY(cudaEventRecord(ctx->total_ready, st));
+        ctx->launches += 1;
+        for (;;) {
+            const uint64_t cap = std::min<uint64_t>(ctx->frags.cap / sizeof(uint2), 0xFFFFFFFEull);
+            k_raster<<<rgrid, kBlock, 0, st>>>(dsc, (const TriRec *)ctx->recs.p, (const uint32_t *)ctx->live_tri.p,
+                                               (const uint64_t *)ctx->live_rowoff.p, totals, (const int *)ctx->err.p,
+                                               (unsigned long long *)ctx->vbuf.p, (SceneStats *)ctx->stats.p, 1,
+                                               (uint2 *)ctx->frags.p, cap, witems, probe);
+            ctx->launches += 1;
+            for (int a = first_ordered; a < ns;) {
+                int b = a;
+                while (b < ns && group_of(plans[b]) == group_of(plans[a])) ++b;
+                const uint64_t blk0 = res_base[a], blk1 = b < ns ? res_base[b] : res;
+                dispatch_resolve_ordered(plans[a].d.shader, dsc, drb, a, b, blk0, blk1 - blk0, cap, ctx, st);
+                ctx->launches += blk1 > blk0;
+                a = b;
+            }
+            CUDA_TRY(cudaEventSynchronize(ctx->total_ready));
+            const unsigned long long nfrag = *(volatile unsigned long long *)ctx->h_total;
+            if (nfrag <= cap) break;
+            if (nfrag >= 0xFFFFFFFFull) return EUC_ERR_CAPACITY;  // list offsets are 32-bit
+            if ((rc = grow(ctx->frags, nfrag * sizeof(uint2)))) return rc;  // (waits for the passes above)
+        }
     }
     cudaEvent_t e5 = prof_event(ctx, st);
-    for (int a = 0; a < ns;) {
+    for (int a = 0; a < first_ordered;) {  // the ordered scenes are done
         int b = a;
-        while (b < ns && group_of(plans[b]) == group_of(plans[a])) ++b;
+        while (b < first_ordered && group_of(plans[b]) == group_of(plans[a])) ++b;
         const uint64_t blk0 = res_base[a];
         const uint64_t blk1 = b < ns ? res_base[b] : res;
-        if (plans[a].d.keytype == KEY_ORDERED)
-            dispatch_resolve_ordered(plans[a].d.shader, dsc, drb, a, b, blk0, blk1 - blk0, ctx, st);
-        else
-            dispatch_resolve(plans[a].d.shader, dsc, rbase, a, b, blk1 - blk0, ctx, st);
+        dispatch_resolve(plans[a].d.shader, dsc, rbase, a, b, blk1 - blk0, ctx, st);
         ctx->launches += blk1 > blk0;
         a = b;
     }
@@ -873,12 +890,14 @@ int euc_ctx_destroy(euc_ctx *ctx) {
     cudaDeviceSynchronize();
     free_shapes(ctx);
     DevBuf *bufs[] = {&ctx->clip, &ctx->vdata, &ctx->recs, &ctx->rows, &ctx->chunk_sums, &ctx->live_tri, &ctx->live_rowoff,
-                      &ctx->totals, &ctx->vbuf, &ctx->err, &ctx->stats, &ctx->cov, &ctx->obsum, &ctx->frags,
+                      &ctx->totals, &ctx->vbuf, &ctx->err, &ctx->stats, &ctx->cov, &ctx->frags,
                       &ctx->plan, &ctx->galive, &ctx->h_arena, &ctx->h_tex[0], &ctx->strip_cnt, &ctx->strip_fill,
                       &ctx->strip_off, &ctx->strip_uoff, &ctx->entries, &ctx->unit_strip, &ctx->bbox};
     for (DevBuf *b : bufs)
         if (b->p) cudaFree(b->p);
     if (ctx->h_pinned.p) cudaFreeHost(ctx->h_pinned.p);
+    if (ctx->h_total) cudaFreeHost(ctx->h_total);
+    if (ctx->total_ready) cudaEventDestroy(ctx->total_ready);
     for (cudaEvent_t e : ctx->ev_pool) cudaEventDestroy(e);
     for (auto &s : ctx->slots) {
         if (s.host) cudaFreeHost(s.host);
@@ -1884,7 +1903,7 @@ extern "C" int euc_render_noalloc(const euc_pipeline_desc *desc, const void *uni
     k_raster<<<(unsigned)(nsm * raster_blocks_per_sm()), kBlock, 0, st>>>(
         dsc, (const TriRec *)(a + kNaOffRecs), (const uint32_t *)(a + kNaOffLiveTri), (const uint64_t *)(a + kNaOffLiveOff),
         (unsigned long long *)(a + kNaOffTotals), (const int *)(a + kNaOffErr),
-        (unsigned long long *)(a + kNaOffVbuf), (SceneStats *)(a + kNaOffStats), 0, nullptr, kWarpItems, false);
+        (unsigned long long *)(a + kNaOffVbuf), (SceneStats *)(a + kNaOffStats), 0, nullptr, 0, kWarpItems, false);
     na_dispatch(false, d.shader, dsc, rbase, resolve_blocks(d), a, st);
     if (device_status)
         CUDA_TRY(cudaMemcpyAsync(device_status, a + kNaOffErr, sizeof(int), cudaMemcpyDeviceToDevice, st));

@@ -294,3 +294,39 @@ def test_index_out_of_bounds_draws_nothing(gpu_ctx, strip_ctx, strips):
     clean = make().alloc_host_targets()
     for k in clean:
         assert np.array_equal(got[k], clean[k])
+
+
+def _layers(n, w=37, h=19, seed=60, **desc):
+    """n full-target triangles over each other with random depths, in a
+    shuffled order, blended src-over: every pixel's list has n fragments."""
+    def make():
+        rng = np.random.default_rng(seed + n)
+        tri = np.array([[-1.5, -1.5], [4.0, -1.5], [-1.5, 4.0]], dtype=np.float32)
+        clip = np.zeros((n, 3, 4), dtype=np.float32)
+        clip[:, :, :2] = tri
+        clip[:, :, 2] = rng.uniform(0.05, 0.95, (n, 1))
+        clip[:, :, 3] = 1.0
+        col = rng.integers(0, 256, (n * 3, 4), dtype=np.uint8)
+        kw = dict(blend=abi.BLEND_ALPHA)
+        kw.update(desc)
+        return scenes.clip_triangles_frame(clip.reshape(-1, 4), col, w, h, **kw)
+    return make
+
+
+@pytest.mark.parametrize("test,write", [(abi.TEST_LESS, 1), (abi.TEST_NONE, 0), (abi.TEST_GREATER, 0)])
+@pytest.mark.parametrize("n", [1, 7, 8, 9, 16, 17, 41])
+def test_ordered_lists_at_the_window_edges(gpu_ctx, n, test, write):
+    """Lists of one window, exactly full, one over and several windows, and a
+    fragment buffer that has to grow (more than four fragments a pixel)."""
+    make = _layers(n, depth_test=test, depth_write=write, depth_clear=0.5 if test == abi.TEST_GREATER else 1.0)
+    ref, ref_stats = run_oracle(make())
+    got, got_stats = run_gpu(gpu_ctx, make())
+    assert [s[1] for s in got_stats] == [s[1] for s in ref_stats]
+    assert_targets_match(make(), ref, got)
+    from euc_gb300 import capi
+    fresh = capi.Context(0)  # its buffer starts at four fragments a pixel
+    try:
+        got, _ = run_gpu(fresh, make())
+    finally:
+        fresh.close()
+    assert_targets_match(make(), ref, got)
