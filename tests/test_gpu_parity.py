@@ -330,3 +330,32 @@ def test_ordered_lists_at_the_window_edges(gpu_ctx, n, test, write):
     finally:
         fresh.close()
     assert_targets_match(make(), ref, got)
+
+
+@pytest.mark.parametrize("clear", [1.0, 0.0, -0.0, float("inf"), float("nan")])
+@pytest.mark.parametrize("z", [0.0, -0.0, 1.0, 0.5])
+def test_depths_at_the_edges_of_the_positive_class(gpu_ctx, strip_ctx, z, clear):
+    """Triangles whose vertex depths are at or above +0 take a shorter key:
+    zeros of both signs, the clip limits, and targets that hold infinity or a
+    NaN, on both raster paths; one triangle's w is tiny (weights near the f32
+    limit), one mixes the zeros."""
+    def make():
+        rng = np.random.default_rng(71)
+        clip = np.zeros((9, 3, 4), dtype=np.float32)
+        clip[:, :, :2] = rng.uniform(-1.3, 1.3, (9, 3, 2))
+        clip[:, :, 2] = np.float32(z)
+        clip[1:4, :, 2] = rng.uniform(0.0, 1.0, (3, 3))
+        clip[4, 1, 2] = -0.0
+        clip[5, 2, 2] = 0.0
+        clip[:, :, 3] = 1.0
+        clip[6] *= np.float32(1e-30)
+        clip[7] *= np.float32(1e30)
+        col = rng.integers(0, 256, (27, 4), dtype=np.uint8)
+        return scenes.clip_triangles_frame(clip.reshape(-1, 4), col, 61, 43, depth_clear=clear)
+    ref, ref_stats = run_oracle(make())
+    for ctx in (gpu_ctx, strip_ctx):
+        got, got_stats = run_gpu(ctx, make())
+        assert [s[1] for s in got_stats] == [s[1] for s in ref_stats]
+        a, b = ref["depth"].view(np.uint32), got["depth"].view(np.uint32)
+        assert np.array_equal(a, b)
+        assert np.array_equal(ref["color"], got["color"])
