@@ -218,6 +218,13 @@ EUC_DEV unsigned long long init_key_min(float d0, bool greater) {
     return (unsigned long long)o << 32;
 }
 
+// Programmatic dependent launch: a kernel launched with it in stream order
+// starts once every block of the kernel before it has called launch_next (or
+// ended), and calls wait_previous before it ends, so that what follows it in
+// the stream still comes after both.
+EUC_DEV void launch_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+EUC_DEV void wait_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 template <typename T>
 EUC_DEV T warp_incl_scan(T v) {
     const int lane = threadIdx.x & 31;
@@ -1011,6 +1018,7 @@ __global__ void __launch_bounds__(kBlock) k_init(const SceneDev *__restrict__ sc
                                                  int nsc, const uint4 *__restrict__ cov,
                                                  unsigned long long *__restrict__ vbuf, uint32_t group) {
     __shared__ int s_scene;
+    launch_next();  // k_bin, which reads nothing this kernel writes
     const uint64_t nchunks = ibase[nsc];
     for (uint64_t g = blockIdx.x; g * group < nchunks; g += gridDim.x) {
         const uint64_t c0 = g * group;
@@ -1331,6 +1339,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_raster(const SceneDev *__restrict
                                                    uint2 *__restrict__ frags, uint64_t frag_cap, int witems,
                                                    bool probe) {
     __shared__ uint64_t s_off[kBlock / 32][kWarpItems];
+    launch_next();  // k_strip: its keys and this kernel's meet in order-free reductions
     if (phase == 1 && totals[4] > frag_cap) return;  // the lists do not fit: the host grows them and comes back
     const int lane = threadIdx.x & 31;
     uint64_t *off = s_off[threadIdx.x >> 5];
@@ -1530,6 +1539,7 @@ __global__ void __launch_bounds__(kBlock) k_bin(const SceneDev *__restrict__ sc,
             entries[pos] = make_uint2((uint32_t)t, (ya << 16) | yb);
         }
     }
+    wait_previous();
 }
 
 // Shared-memory 64-bit min reduction (no value returned).
@@ -1824,6 +1834,7 @@ __global__ void __launch_bounds__(kStripThreads, kStripBlocksPerSm) k_strip(cons
         if (lane == 0 && wsum) atomicAdd(&stats[si].candidates, (unsigned long long)wsum);
         __syncthreads();
     }
+    wait_previous();
 }
 
 // ---------------------------------------------------------------------------
