@@ -49,13 +49,17 @@ struct euc_ctx {
     int nsm = 0;
     DevBuf clip, vdata, recs, rows, chunk_sums, live_tri, live_rowoff, totals, vbuf, err, stats, cov;
     DevBuf frags;         // ordered path: fragment lists
-    unsigned long long *h_total = nullptr;  // ... and their number, written by k_oscan (page-locked)
+    // page-locked words that kernels write: the number of fragments (k_oscan),
+    // a host-buffer frame's error (k_frame_raster)
+    unsigned long long *h_words = nullptr;
     cudaEvent_t total_ready = nullptr;
     DevBuf plan;          // plan_chunks: k_init and k_resolve chunk bases (2 x (scenes + 1))
     DevBuf galive;        // geometry stage: 1 per output slot that holds a triangle
     // strip path: per-strip entry counts, fill cursors, list offsets, unit
     // offsets, the entry lists and the strip of each unit
     DevBuf strip_cnt, strip_fill, strip_off, strip_uoff, entries, unit_strip;
+    // frame path: FrontScratch and the scene's staging (fixed sizes)
+    DevBuf front, frame_stage;
     DevBuf bbox;  // strip path: each primitive's bbox (16 B), the binning's only read of it
     int raster_blocks = 0;  // resident k_raster blocks per SM
     bool pageable = false;  // kernels may access pageable host memory (cudaDevAttrPageableMemoryAccess)
@@ -105,6 +109,11 @@ int grow(DevBuf &b, size_t bytes) {
     }
     CUDA_TRY(cudaMalloc(&b.p, ncap));
     b.cap = ncap;
+    return EUC_OK;
+}
+
+int ensure_host_words(euc_ctx *ctx) {
+    if (!ctx->h_words) CUDA_TRY(cudaMallocHost((void **)&ctx->h_words, 2 * sizeof(unsigned long long)));
     return EUC_OK;
 }
 
@@ -424,6 +433,21 @@ void dispatch_geometry(uint32_t shader, const SceneDev *sc, const uint64_t *gb, 
     }
 }
 
+template <class... P, class... A>
+cudaError_t launch_beside(void (*kernel)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t st, A... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+}
+
 template <class F>
 void launch_resolve(const SceneDev *sc, const uint64_t *rbase, int s0, int s1, uint64_t nblk, euc_ctx *ctx,
                     cudaStream_t st) {
@@ -485,21 +509,6 @@ void dispatch_resolve_ordered(uint32_t shader, const SceneDev *sc, const uint64_
 
 // Launches `kernel` so that it may start while the kernel before it in the
 // stream still runs (see launch_next); the kernel before that one has ended.
-template <class... P, class... A>
-cudaError_t launch_beside(void (*kernel)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t st, A... args) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3(block);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
-}
-
 // Four-texel words need every source row aligned to the word (four texels'
 // bytes up to a 4-byte word for RGB8's three) and every target row to 16 bytes.
 template <uint32_t FMT>
@@ -798,12 +807,12 @@ int run_batch(euc_ctx *ctx, const euc_scene *scenes, size_t n, cudaStream_t st, 
     if (first_ordered < ns) {
         const uint64_t p0 = plans[first_ordered].d.pix_base, p1 = pix;
         const uint64_t nb = (p1 - p0 + kOScanBlock - 1) / kOScanBlock;
-        if (!ctx->h_total) CUDA_TRY(cudaMallocHost((void **)&ctx->h_total, sizeof(unsigned long long)));
+        if ((rc = ensure_host_words(ctx))) return rc;
         if (!ctx->total_ready) CUDA_TRY(cudaEventCreateWithFlags(&ctx->total_ready, cudaEventDisableTiming));
         // a first guess: four fragments a pixel, 512 MB at most
         if ((rc = grow(ctx->frags, std::min<uint64_t>(4 * pix, 1ull << 26) * sizeof(uint2)))) return rc;
         unsigned long long *totals = (unsigned long long *)ctx->totals.p;
-        k_oscan<<<(unsigned)nb, kBlock, 0, st>>>((unsigned long long *)ctx->vbuf.p, p0, p1, totals, ctx->h_total);
+        k_oscan<<<(unsigned)nb, kBlock, 0, st>>>((unsigned long long *)ctx->vbuf.p, p0, p1, totals, ctx->h_words);
         CUDA_TRY(cudaEventRecord(ctx->total_ready, st));
         ctx->launches += 1;
         for (;;) {
@@ -822,7 +831,7 @@ int run_batch(euc_ctx *ctx, const euc_scene *scenes, size_t n, cudaStream_t st, 
                 a = b;
             }
             CUDA_TRY(cudaEventSynchronize(ctx->total_ready));
-            const unsigned long long nfrag = *(volatile unsigned long long *)ctx->h_total;
+            const unsigned long long nfrag = *(volatile unsigned long long *)ctx->h_words;
             if (nfrag <= cap) break;
             if (nfrag >= 0xFFFFFFFFull) return EUC_ERR_CAPACITY;  // list offsets are 32-bit
             if ((rc = grow(ctx->frags, nfrag * sizeof(uint2)))) return rc;  // (waits for the passes above)
@@ -851,6 +860,95 @@ int run_batch(euc_ctx *ctx, const euc_scene *scenes, size_t n, cudaStream_t st, 
         slot->pending = true;
     }
     return EUC_OK;
+}
+
+// ---------------------------------------------------------------------------
+// The frame path (k_front, k_frame_raster, k_resolve): scenes small enough
+// that launches, not work, set their time (k_front's comment has the figures).
+// kFramePrims bounds the groups a block scans; kFramePixels bounds the keys that k_front seeds beyond the
+// covered rectangle (12 bytes a pixel: 12.6 MB, some 2 us beside the setup);
+// kFrameVerts keeps a large unindexed buffer on the batch's path.  A batch, a
+// forced strip path and a profiled context take the other kernels.
+// ---------------------------------------------------------------------------
+constexpr uint64_t kFramePixels = 1ull << 20, kFrameVerts = 1ull << 16;
+
+bool frame_path(const euc_ctx *ctx, const Plan &p) {
+    return p.d.keytype != KEY_ORDERED && p.d.geom == EUC_GEOM_NONE && p.d.ngroups >= 1 && p.d.ngroups <= kFramePrims &&
+           p.d.nverts <= kFrameVerts && (uint64_t)p.d.W * p.d.H <= kFramePixels && ctx->tune.strip_path != 2 &&
+           !ctx->profiling;
+}
+
+// Sizes the scratch and fills k_front's parameter for a planned scene.
+int fill_front(euc_ctx *ctx, const Plan &p, FrontArgs &a) {
+    const uint64_t tri = pad_up(p.d.ngroups, kBlock), pix = pad_up((uint64_t)p.d.W * p.d.H, kBlock);
+    int rc;
+    if ((rc = grow(ctx->vdata, std::max<uint64_t>(p.d.nverts * p.nv, 1) * sizeof(float)))) return rc;
+    if ((rc = grow(ctx->recs, tri * sizeof(TriRec)))) return rc;
+    if ((rc = grow(ctx->rows, tri * sizeof(uint32_t)))) return rc;
+    if ((rc = grow(ctx->vbuf, pix * sizeof(unsigned long long)))) return rc;
+    if ((rc = grow(ctx->err, sizeof(int)))) return rc;
+    if ((rc = grow(ctx->stats, sizeof(SceneStats)))) return rc;
+    if ((rc = grow(ctx->cov, sizeof(uint4)))) return rc;
+    if ((rc = grow(ctx->plan, 4 * sizeof(uint64_t)))) return rc;
+    if ((rc = grow(ctx->front, sizeof(FrontScratch)))) return rc;
+    constexpr size_t off_u = (sizeof(SceneDev) + 15) / 16 * 16;
+    static_assert(sizeof(euc_phong_uniforms) <= sizeof(FrontArgs::uni), "uniform copies hold any shader's struct");
+    if ((rc = grow(ctx->frame_stage, off_u + sizeof(FrontArgs::uni)))) return rc;
+    a.d = p.d;
+    a.d.vtx_base = a.d.vd_base = a.d.tri_base = a.d.pix_base = 0;
+    a.stage_scene = (SceneDev *)ctx->frame_stage.p;
+    a.stage_uni = (unsigned char *)ctx->frame_stage.p + off_u;
+    a.d.uniforms = a.stage_uni;
+    std::memcpy(a.uni, p.uniforms, p.usize);
+    a.usize = (uint32_t)pad_up(p.usize, 4);
+    a.nsb = (uint32_t)(tri / kBlock);
+    a.nib = (uint32_t)(((uint64_t)p.d.W * p.d.H + kInitChunk - 1) / kInitChunk);
+    a.vdata = (float *)ctx->vdata.p;
+    a.recs = (TriRec *)ctx->recs.p;
+    a.rows = (uint32_t *)ctx->rows.p;
+    a.front = (FrontScratch *)ctx->front.p;
+    a.vbuf = (unsigned long long *)ctx->vbuf.p;
+    a.stats = (SceneStats *)ctx->stats.p;
+    return EUC_OK;
+}
+
+template <class F>
+void launch_front(const FrontArgs &a, cudaStream_t st) {
+    const uint64_t nvb = (a.d.nverts + kBlock - 1) / kBlock;
+    k_front<F><<<(unsigned)(a.nsb + a.nib + nvb), kBlock, 0, st>>>(a);
+}
+
+// Enqueues a frame whose parameter is filled; host_err (or null): page-locked
+// memory that also receives the scene's error.
+int launch_frame(euc_ctx *ctx, const FrontArgs &a, cudaStream_t st, int *host_err = nullptr) {
+    switch (a.d.shader) {
+    case EUC_SHADER_FLAT: launch_front<FlatFn>(a, st); break;
+    case EUC_SHADER_VCOLOR: launch_front<VColorFn>(a, st); break;
+    case EUC_SHADER_GOURAUD: launch_front<GouraudFn>(a, st); break;
+    case EUC_SHADER_TEXTURED: launch_front<TexturedFn>(a, st); break;
+    case EUC_SHADER_PHONG: launch_front<PhongFn>(a, st); break;
+    case EUC_SHADER_SHADOW: launch_front<ShadowFn>(a, st); break;
+    }
+    // a warp takes 32 items a step; a primitive slot has at most max(W, H) + 2
+    const uint64_t items = (uint64_t)a.d.ngroups * ((uint64_t)std::max(a.d.W, a.d.H) + 2);
+    const uint64_t busy = items / kBlock + a.nsb;
+    const unsigned grid = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(busy, (uint64_t)ctx->nsm * ctx->raster_blocks));
+    CUDA_TRY(launch_beside(k_frame_raster, grid, kBlock, 0, st, (const SceneDev *)a.stage_scene, (const TriRec *)a.recs,
+                           (const uint32_t *)a.rows, (const FrontScratch *)a.front, a.nsb, (int *)ctx->err.p, host_err,
+                           (SceneStats *)ctx->stats.p, (uint4 *)ctx->cov.p, (uint64_t *)ctx->plan.p, a.vbuf,
+                           ctx->tune.raster_probe == 1));
+    dispatch_resolve(a.d.shader, a.stage_scene, (uint64_t *)ctx->plan.p, 0, 1, resolve_blocks(a.d), ctx, st);
+    CUDA_TRY(cudaGetLastError());
+    ctx->launches += 3;
+    return EUC_OK;
+}
+
+// One scene on the frame path, its launches enqueued one by one.
+int run_frame(euc_ctx *ctx, const Plan &p, cudaStream_t st, int *host_err = nullptr) {
+    FrontArgs a;
+    if (int rc = fill_front(ctx, p, a)) return rc;
+    ctx->last_nscenes = 1;
+    return launch_frame(ctx, a, st, host_err);
 }
 
 }  // namespace
@@ -917,11 +1015,11 @@ int euc_ctx_destroy(euc_ctx *ctx) {
     DevBuf *bufs[] = {&ctx->clip, &ctx->vdata, &ctx->recs, &ctx->rows, &ctx->chunk_sums, &ctx->live_tri, &ctx->live_rowoff,
                       &ctx->totals, &ctx->vbuf, &ctx->err, &ctx->stats, &ctx->cov, &ctx->frags,
                       &ctx->plan, &ctx->galive, &ctx->h_arena, &ctx->h_tex[0], &ctx->strip_cnt, &ctx->strip_fill,
-                      &ctx->strip_off, &ctx->strip_uoff, &ctx->entries, &ctx->unit_strip, &ctx->bbox};
+                      &ctx->strip_off, &ctx->strip_uoff, &ctx->entries, &ctx->unit_strip, &ctx->bbox, &ctx->front, &ctx->frame_stage};
     for (DevBuf *b : bufs)
         if (b->p) cudaFree(b->p);
     if (ctx->h_pinned.p) cudaFreeHost(ctx->h_pinned.p);
-    if (ctx->h_total) cudaFreeHost(ctx->h_total);
+    if (ctx->h_words) cudaFreeHost(ctx->h_words);
     if (ctx->total_ready) cudaEventDestroy(ctx->total_ready);
     for (cudaEvent_t e : ctx->ev_pool) cudaEventDestroy(e);
     for (auto &s : ctx->slots) {
@@ -1146,6 +1244,8 @@ __global__ void __launch_bounds__(64) k_stage_param(const __grid_constant__ Stag
 struct ShapeGraph {
     std::vector<unsigned char> key;
     void *scratch[kScratchBufs] = {};
+    bool frame = false;             // recorded on the frame path: `front` is the first node's parameter
+    FrontArgs front;
     StageParam param;               // the next replay's staging
     void *dev = nullptr;            // the staging the graph's kernels read
     size_t need = 0;
@@ -1190,13 +1290,19 @@ std::vector<unsigned char> shape_key(const euc_ctx *ctx, const Plan &p) {
 }
 
 // Records the launches of scene `s` as a new shape; nullptr when it cannot.
-ShapeGraph *shape_record(euc_ctx *ctx, const euc_scene &s, std::vector<unsigned char> key) {
+ShapeGraph *shape_record(euc_ctx *ctx, const euc_scene &s, const Plan &p, std::vector<unsigned char> key) {
     StageOverride so;
     so.dry = true;
-    if (run_batch(ctx, &s, 1, nullptr, &so)) return nullptr;  // validates, sizes the scratch
+    const bool frame = frame_path(ctx, p);
+    if (!frame && run_batch(ctx, &s, 1, nullptr, &so)) return nullptr;  // validates, sizes the scratch
     if (so.need > kStageParamBytes) return nullptr;  // too large for the parameter: plain path
     ShapeGraph *g = new (std::nothrow) ShapeGraph();
     if (!g) return nullptr;
+    if (frame && fill_front(ctx, p, g->front)) {
+        delete g;
+        return nullptr;
+    }
+    g->frame = frame;
     g->key = std::move(key);
     g->need = so.need;
     g->param.n = (uint32_t)so.need;
@@ -1212,20 +1318,20 @@ ShapeGraph *shape_record(euc_ctx *ctx, const euc_scene &s, std::vector<unsigned 
         so.need = g->need;
         ctx->capturing = true;
         const uint64_t l0 = ctx->launches;
-        k_stage_param<<<1, 64, 0, cs>>>(g->param, (unsigned char *)g->dev);
-        const int rc = run_batch(ctx, &s, 1, cs, &so);
-        g->launches = ctx->launches - l0 + 1;
+        if (!frame) k_stage_param<<<1, 64, 0, cs>>>(g->param, (unsigned char *)g->dev);
+        const int rc = frame ? launch_frame(ctx, g->front, cs) : run_batch(ctx, &s, 1, cs, &so);
+        g->launches = ctx->launches - l0 + (frame ? 0 : 1);
         ctx->launches = l0;
         ctx->capturing = false;
         cudaGraph_t graph = nullptr;
         const cudaError_t ec = cudaStreamEndCapture(cs, &graph);
         g->graph = graph;
-        // the staging node is the graph's only root
+        // the staging node (the frame path's first kernel) is the graph's only root
         size_t nroot = 1;
         ok = rc == EUC_OK && ec == cudaSuccess && graph &&
              cudaGraphGetRootNodes(graph, &g->stage_node, &nroot) == cudaSuccess && nroot == 1 &&
              cudaGraphKernelNodeGetParams(g->stage_node, &g->stage_kp) == cudaSuccess &&
-             g->stage_kp.func == (void *)k_stage_param &&
+             (frame || g->stage_kp.func == (void *)k_stage_param) &&
              cudaGraphInstantiate(&g->exec, g->graph, 0) == cudaSuccess;
     } else {
         ok = false;
@@ -1263,7 +1369,8 @@ int render_one(euc_ctx *ctx, const euc_scene &s, cudaStream_t st) {
     }
     if (!g) {
         if (ctx->sightings.size() >= kSightCap) ctx->sightings.clear();
-        if (++ctx->sightings[key] < 2) return run_batch(ctx, &s, 1, st);  // seen once: plain
+        const bool frame = frame_path(ctx, p);
+        if (++ctx->sightings[key] < 2) return frame ? run_frame(ctx, p, st) : run_batch(ctx, &s, 1, st);  // seen once: plain
         if (ctx->shapes.size() >= kShapeCap) {  // make room: the least recently used goes
             size_t lru = 0;
             for (size_t i = 1; i < ctx->shapes.size(); ++i)
@@ -1271,19 +1378,25 @@ int render_one(euc_ctx *ctx, const euc_scene &s, cudaStream_t st) {
             shape_free(ctx->shapes[lru]);
             ctx->shapes.erase(ctx->shapes.begin() + (long)lru);
         }
-        g = shape_record(ctx, s, key);
-        if (!g) return run_batch(ctx, &s, 1, st);
+        g = shape_record(ctx, s, p, key);
+        if (!g) return frame ? run_frame(ctx, p, st) : run_batch(ctx, &s, 1, st);
         ctx->shapes.push_back(g);
     }
     g->last_use = ++ctx->shape_clock;
-    StageOverride so;
-    so.fill = true;
-    so.host = g->param.b;
-    so.dev = g->dev;
-    so.need = g->need;
-    if (int rc = run_batch(ctx, &s, 1, st, &so)) return rc;
-    // the parameter is copied here; replays already enqueued keep theirs
     void *args[2] = {&g->param, &g->dev};
+    if (g->frame) {
+        if (int rc = fill_front(ctx, p, g->front)) return rc;
+        ctx->last_nscenes = 1;
+        args[0] = &g->front;
+    } else {
+        StageOverride so;
+        so.fill = true;
+        so.host = g->param.b;
+        so.dev = g->dev;
+        so.need = g->need;
+        if (int rc = run_batch(ctx, &s, 1, st, &so)) return rc;
+    }
+    // the parameter is copied here; replays already enqueued keep theirs
     cudaKernelNodeParams kp = g->stage_kp;
     kp.kernelParams = args;
     kp.extra = nullptr;
@@ -1602,6 +1715,14 @@ int host_batch(euc_ctx *ctx, const euc_scene *scenes, size_t n, int threads) {
             ctx->launches += 1;
         }
         // the kernels use the caller's buffers: none may still run when this returns
+        Plan p;
+        if (n == 1 && plan_scene(dev[0], p) == EUC_OK && !p.skip && frame_path(ctx, p)) {
+            if ((rc = ensure_host_words(ctx))) return rc;
+            int *host_err = (int *)(ctx->h_words + 1);
+            rc = run_frame(ctx, p, nullptr, host_err);
+            CUDA_TRY(cudaStreamSynchronize(nullptr));
+            return rc ? rc : *(volatile int *)host_err;
+        }
         rc = run_batch(ctx, dev.data(), n, nullptr);
         CUDA_TRY(cudaStreamSynchronize(nullptr));
         return rc ? rc : first_scene_error(ctx);

@@ -449,14 +449,23 @@ EUC_DEV float fclamp(float v, float lo, float hi) { return v < lo ? lo : (v > hi
 EUC_DEV long long wsub(long long a, long long b) { return (long long)((unsigned long long)a - (unsigned long long)b); }
 EUC_DEV long long wabs(long long a) { return a < 0 ? (long long)(0ull - (unsigned long long)a) : a; }
 
+// What the setup of one primitive leaves besides its record.
+struct SetupOut {
+    uint32_t nrows = 0, culled = 0;
+    float frag_est = 0.0f;  // the primitive's screen area in pixels, at most its bbox (the strip routing)
+    // pixels this primitive may touch: x in [cx0, cx1), y in [cy0, cy1)
+    uint32_t cx0 = 0xFFFFFFFFu, cy0 = 0xFFFFFFFFu, cx1 = 0, cy1 = 0;
+    bool bad = false;  // an index out of bounds
+};
+
 // Setup of line slot lt.  The pixels are clipline's: the Bresenham line
 // between the truncated end points, both ends included, inside the window
 // (x in [wx1, wx2), y in [wy1, wy2)) -- see the oracle's bresenham_clipped
 // for the restatement and why the band clamp of the window does not change
 // the pixel set.  Lines with a coordinate beyond 2^30 draw nothing.
-EUC_DEV void setup_line(const SceneDev &s, int si, uint64_t lt, uint64_t t, const float4 *__restrict__ clip,
-                        TriRec *__restrict__ recs, int *__restrict__ err, uint32_t &nrows, uint32_t &cx0,
-                        uint32_t &cy0, uint32_t &cx1, uint32_t &cy1) {
+template <class ClipOf>
+EUC_DEV void setup_line(const SceneDev &s, int si, uint64_t lt, uint64_t t, ClipOf clip_of,
+                        TriRec *__restrict__ recs, SetupOut &out) {
     uint64_t e[2];
     bool ok = true;
     if (s.prim == EUC_PRIM_LINE_LIST) {
@@ -487,14 +496,14 @@ EUC_DEV void setup_line(const SceneDev &s, int si, uint64_t lt, uint64_t t, cons
             mine = false;
         }
     }
-    if (!ok) atomicCAS(err + si, 0, EUC_ERR_INDEX_OOB);
+    if (!ok) out.bad = true;
     if (!ok || !mine || lt >= s.ntris) return;
     const float flip1 = s.yflip ? -1.0f : 1.0f;
     const float size_x = (float)s.W, size_y = (float)s.H;
     float ez[2], sx[2], sy[2];
 #pragma unroll
     for (int k = 0; k < 2; ++k) {
-        const float4 c = clip[s.vtx_base + vid[k]];
+        const float4 c = clip_of(vid[k]);
         const float w = rmax(c.w, 0.0001f);  // lines.rs:45-48
         const float ex = (c.x * 1.0f) / w, ey = (c.y * flip1) / w;
         ez[k] = c.z / w;
@@ -560,11 +569,11 @@ EUC_DEV void setup_line(const SceneDev &s, int si, uint64_t lt, uint64_t t, cons
     float4 *dst = reinterpret_cast<float4 *>(recs + t);
 #pragma unroll
     for (int k = 0; k < 8; ++k) dst[k] = src[k];
-    nrows = r.by1;
-    cx0 = (uint32_t)wx1;
-    cx1 = (uint32_t)wx2;
-    cy0 = (uint32_t)wy1;
-    cy1 = (uint32_t)wy2;
+    out.nrows = r.by1;
+    out.cx0 = (uint32_t)wx1;
+    out.cx1 = (uint32_t)wx2;
+    out.cy0 = (uint32_t)wy1;
+    out.cy1 = (uint32_t)wy2;
 }
 
 // Primitives whose full-row bbox holds at most this many pixels are walked
@@ -621,39 +630,21 @@ __host__ __device__ inline uint32_t width_bucket(uint32_t w) {
 }
 
 // ---------------------------------------------------------------------------
-// k_setup: triangles.rs:55-199, once per primitive (euc repeats it per band;
-// only the bbox clamp depends on the band and that is applied per row).
-// Block b sets up primitives [b * kBlock, (b + 1) * kBlock), all of scene
-// chunk_scene[b] (null: scene 0).  bbox
-// (null when the batch has no strips) receives the bbox of every triangle
+// Primitive setup: triangles.rs:55-199, once per primitive (euc repeats it per
+// band; only the bbox clamp depends on the band and that is applied per row).
+// Primitive t of scene si, by one thread; clip_of(v) is vertex v's clip
+// position.  A triangle's record is staged in the warp's 4 KB (store_records);
+// bbox (null when the batch has no strips) receives the bbox of every triangle
 // with rows: the binning reads those 16 bytes instead of the record's line.
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(kBlock) k_setup(const SceneDev *__restrict__ sc,
-                                                  const uint32_t *__restrict__ chunk_scene,
-                                                  const float4 *__restrict__ clip, TriRec *__restrict__ recs,
-                                                  uint32_t *__restrict__ rows, uint2 *__restrict__ chunk_sums,
-                                                  int *__restrict__ err, SceneStats *__restrict__ stats,
-                                                  uint4 *__restrict__ cov, const uint8_t *__restrict__ galive,
-                                                  uint4 *__restrict__ bbox) {
-    // a warp's 32 records, staged so that they leave as 512-byte stores;
-    // 16-byte word k of lane l's record sits at l * 8 + (k ^ (l & 7)), which
-    // keeps both the staging and the copy-out at the minimum four wavefronts
-    __shared__ uint4 s_rec[kBlock / 32][32 * 8];
-    __shared__ uint4 s_cov[kBlock / 32], s_sum[kBlock / 32];
-    __shared__ unsigned long long s_walk[kBlock / 32];
+template <class ClipOf>
+EUC_DEV void setup_prim(const SceneDev &s, int si, uint64_t t, ClipOf clip_of, TriRec *__restrict__ recs,
+                        const uint8_t *__restrict__ galive, uint4 *__restrict__ bbox, uint4 *stage, bool &staged,
+                        SetupOut &out) {
     const int lane = threadIdx.x & 31;
-    uint4 *stage = s_rec[threadIdx.x >> 5];
-    bool staged = false;
-    const uint64_t t = (uint64_t)blockIdx.x * kBlock + threadIdx.x;
-    const int si = chunk_scene ? (int)chunk_scene[blockIdx.x] : 0;
-    const SceneDev &s = sc[si];
     const uint64_t lt = t - s.tri_base;
-    uint32_t nrows = 0, culled = 0;
-    float frag_est = 0.0f;  // the primitive's screen area in pixels, at most its bbox (the strip routing)
-    // pixels this primitive may touch: x in [cx0, cx1), y in [cy0, cy1)
-    uint32_t cx0 = 0xFFFFFFFFu, cy0 = 0xFFFFFFFFu, cx1 = 0, cy1 = 0;
     if (s.prim != EUC_PRIM_TRIANGLE_LIST) {  // uniform: a block holds one scene
-        if (lt < s.ngroups) setup_line(s, si, lt, t, clip, recs, err, nrows, cx0, cy0, cx1, cy1);
+        if (lt < s.ngroups) setup_line(s, si, lt, t, clip_of, recs, out);
     } else if (lt < s.ngroups) {
         uint32_t vid[3] = {0, 0, 0};
         bool ok = true;
@@ -671,15 +662,14 @@ __global__ void __launch_bounds__(kBlock) k_setup(const SceneDev *__restrict__ s
                     vid[k] = (uint32_t)id;
                 }
             }
-            if (!ok) atomicCAS(err + si, 0, EUC_ERR_INDEX_OOB);
+            if (!ok) out.bad = true;
         }
-        const uint64_t cbase = s.geom ? s.gvtx_base : s.vtx_base;
         if (ok && lt < s.ntris) {
             float h[3][4], e3[3][3];
             const float flip1 = s.yflip ? -1.0f : 1.0f;
 #pragma unroll
             for (int k = 0; k < 3; ++k) {
-                const float4 c = clip[cbase + vid[k]];
+                const float4 c = clip_of(vid[k]);
                 h[k][0] = c.x * 1.0f;
                 h[k][1] = c.y * flip1;
                 h[k][2] = c.z;
@@ -698,7 +688,7 @@ __global__ void __launch_bounds__(kBlock) k_setup(const SceneDev *__restrict__ s
                 cull = winding * dir < 0.0f;
             }
             if (cull) {
-                culled = 1;
+                out.culled = 1;
             } else {
                 if (winding >= 0.0f) {  // reverse vertex order (triangles.rs:78-80)
 #pragma unroll
@@ -802,9 +792,9 @@ __global__ void __launch_bounds__(kBlock) k_setup(const SceneDev *__restrict__ s
                           (one_band ? kTriOneBand : 0u) | (zpos ? kTriZPos : 0u);
 #pragma unroll
                 for (int k = 0; k < 5; ++k) r.pad[k] = 0;
-                nrows = bx1 > bx0 ? by1 - by0 : 0u;
+                out.nrows = bx1 > bx0 ? by1 - by0 : 0u;
                 // NDC area |winding| / 2 is (W / 2) x (H / 2) pixels per unit
-                frag_est = fminf(fabsf(winding) * (size_x * size_y * 0.125f), (float)(bx1 - bx0) * (float)(by1 - by0));
+                out.frag_est = fminf(fabsf(winding) * (size_x * size_y * 0.125f), (float)(bx1 - bx0) * (float)(by1 - by0));
                 if (full_rows && (bx1 - bx0) * (by1 - by0) <= kTinyPixels) {
                     // a tiny primitive: walk its few pixels here exactly as
                     // k_raster would (full-bbox rows, triangles.rs:257-301);
@@ -823,9 +813,9 @@ __global__ void __launch_bounds__(kBlock) k_setup(const SceneDev *__restrict__ s
                             w2 = w2 + dxw[2];
                         }
                     }
-                    if (!any) nrows = 0;
+                    if (!any) out.nrows = 0;
                 }
-                if (nrows) {
+                if (out.nrows) {
                     // only a primitive with rows is ever read again (the scan
                     // keeps exactly those)
                     const uint4 *src = reinterpret_cast<const uint4 *>(&r);
@@ -833,67 +823,114 @@ __global__ void __launch_bounds__(kBlock) k_setup(const SceneDev *__restrict__ s
                     for (int k = 0; k < 8; ++k) stage[lane * 8 + (k ^ (lane & 7))] = src[k];
                     staged = true;
                     if (bbox) bbox[t] = make_uint4(bx0, bx1, by0, by1);  // the binning's copy
-                    cx0 = bx0;
-                    cx1 = bx1;
-                    cy0 = by0;
-                    cy1 = by1;
+                    out.cx0 = bx0;
+                    out.cx1 = bx1;
+                    out.cy0 = by0;
+                    out.cy1 = by1;
                 }
             }
         }
     }
-    {  // the warp's staged records, 16-byte word c of the warp's 4 KB per lane and pass
-        const uint32_t live = __ballot_sync(0xFFFFFFFFu, staged);
-        __syncwarp();
-        if (live) {
-            uint4 *dst = reinterpret_cast<uint4 *>(recs + (t - (uint64_t)lane));
+}
+
+// The records a warp staged, out as 512-byte stores: 16-byte word k of lane
+// l's record sits at l * 8 + (k ^ (l & 7)), which keeps both the staging and
+// the copy-out at the minimum four wavefronts.  warp_recs: lane 0's record.
+EUC_DEV void store_records(const uint4 *stage, bool staged, TriRec *__restrict__ warp_recs) {
+    const int lane = threadIdx.x & 31;
+    const uint32_t live = __ballot_sync(0xFFFFFFFFu, staged);
+    __syncwarp();
+    if (live) {
+        uint4 *dst = reinterpret_cast<uint4 *>(warp_recs);
 #pragma unroll
-            for (int k = 0; k < 8; ++k) {
-                const int c = k * 32 + lane, owner = c >> 3;
-                if ((live >> owner) & 1u) dst[c] = stage[owner * 8 + ((c & 7) ^ (owner & 7))];
-            }
+        for (int k = 0; k < 8; ++k) {
+            const int c = k * 32 + lane, owner = c >> 3;
+            if ((live >> owner) & 1u) dst[c] = stage[owner * 8 + ((c & 7) ^ (owner & 7))];
         }
     }
-    rows[t] = nrows;
-    // The block's sums, one atomic each: the scene's covered rectangle (min of
-    // (x0, y0, ~x1, ~y1) over its primitives), its culled count and, for the
-    // strip path's routing, the pixels its rows may walk; the scan's per-chunk
-    // sums are this block's alone.  One set of atomics a block, not a warp: all
-    // of a scene's meet in two L2 sectors, where nine a warp (15.6 k warps of a
-    // 500 k triangle mesh) bounded this kernel.
-    const uint32_t m0 = __reduce_min_sync(0xFFFFFFFFu, cx0), m1 = __reduce_min_sync(0xFFFFFFFFu, cy0);
-    const uint32_t m2 = __reduce_min_sync(0xFFFFFFFFu, ~cx1), m3 = __reduce_min_sync(0xFFFFFFFFu, ~cy1);
-    const uint32_t wl = __popc(__ballot_sync(0xFFFFFFFFu, nrows != 0)), wr = __reduce_add_sync(0xFFFFFFFFu, nrows);
-    const uint32_t wc = __popc(__ballot_sync(0xFFFFFFFFu, culled != 0));
-    const unsigned long long ww = bbox ? warp_sum(nrows ? (unsigned long long)frag_est : 0ull) : 0ull;
-    if (lane == 0) {
+}
+
+// A block's sums over its primitives, left in thread 0 of the block.
+struct SetupSums {
+    uint32_t x0, y0, nx1, ny1;  // min of (cx0, cy0, ~cx1, ~cy1)
+    uint32_t live, rows, culled;
+    unsigned long long walked;
+};
+template <bool kWalked>
+EUC_DEV SetupSums setup_block_sums(const SetupOut &o) {
+    __shared__ uint4 s_cov[kBlock / 32], s_sum[kBlock / 32];
+    __shared__ unsigned long long s_walk[kBlock / 32];
+    const uint32_t m0 = __reduce_min_sync(0xFFFFFFFFu, o.cx0), m1 = __reduce_min_sync(0xFFFFFFFFu, o.cy0);
+    const uint32_t m2 = __reduce_min_sync(0xFFFFFFFFu, ~o.cx1), m3 = __reduce_min_sync(0xFFFFFFFFu, ~o.cy1);
+    const uint32_t wl = __popc(__ballot_sync(0xFFFFFFFFu, o.nrows != 0)), wr = __reduce_add_sync(0xFFFFFFFFu, o.nrows);
+    const uint32_t wc = __popc(__ballot_sync(0xFFFFFFFFu, o.culled != 0));
+    const unsigned long long ww = kWalked ? warp_sum(o.nrows ? (unsigned long long)o.frag_est : 0ull) : 0ull;
+    if ((threadIdx.x & 31) == 0) {
         const int w = threadIdx.x >> 5;
         s_cov[w] = make_uint4(m0, m1, m2, m3);
         s_sum[w] = make_uint4(wl, wr, wc, 0u);
         s_walk[w] = ww;
     }
     __syncthreads();
+    SetupSums b = {};
     if (threadIdx.x < kBlock / 32) {
         constexpr uint32_t kMask = (1u << (kBlock / 32)) - 1u;
         const uint4 c = s_cov[threadIdx.x], q = s_sum[threadIdx.x];
-        unsigned long long bw = s_walk[threadIdx.x];
-        const uint32_t b0 = __reduce_min_sync(kMask, c.x), b1 = __reduce_min_sync(kMask, c.y);
-        const uint32_t b2 = __reduce_min_sync(kMask, c.z), b3 = __reduce_min_sync(kMask, c.w);
-        const uint32_t bl = __reduce_add_sync(kMask, q.x), br = __reduce_add_sync(kMask, q.y);
-        const uint32_t bc = __reduce_add_sync(kMask, q.z);
+        b.walked = s_walk[threadIdx.x];
+        b.x0 = __reduce_min_sync(kMask, c.x);
+        b.y0 = __reduce_min_sync(kMask, c.y);
+        b.nx1 = __reduce_min_sync(kMask, c.z);
+        b.ny1 = __reduce_min_sync(kMask, c.w);
+        b.live = __reduce_add_sync(kMask, q.x);
+        b.rows = __reduce_add_sync(kMask, q.y);
+        b.culled = __reduce_add_sync(kMask, q.z);
 #pragma unroll
-        for (int d = kBlock / 64; d > 0; d >>= 1) bw += __shfl_xor_sync(kMask, bw, d);
-        if (threadIdx.x == 0) {
-            chunk_sums[blockIdx.x] = make_uint2(bl, br);
-            if (b0 != 0xFFFFFFFFu) {
-                atomicMin(&cov[si].x, b0);
-                atomicMin(&cov[si].y, b1);
-                atomicMin(&cov[si].z, b2);
-                atomicMin(&cov[si].w, b3);
-            }
-            if (bc) atomicAdd(&stats[si].culled, (unsigned long long)bc);
-            if (bw) atomicAdd(&stats[si].walked, bw);
-            if (bbox && bl) atomicAdd(&stats[si].live, (unsigned long long)bl);
+        for (int d = kBlock / 64; d > 0; d >>= 1) b.walked += __shfl_xor_sync(kMask, b.walked, d);
+    }
+    return b;
+}
+
+// ---------------------------------------------------------------------------
+// k_setup: block b sets up primitives [b * kBlock, (b + 1) * kBlock), all of
+// scene chunk_scene[b] (null: scene 0).
+// ---------------------------------------------------------------------------
+__global__ void __launch_bounds__(kBlock) k_setup(const SceneDev *__restrict__ sc,
+                                                  const uint32_t *__restrict__ chunk_scene,
+                                                  const float4 *__restrict__ clip, TriRec *__restrict__ recs,
+                                                  uint32_t *__restrict__ rows, uint2 *__restrict__ chunk_sums,
+                                                  int *__restrict__ err, SceneStats *__restrict__ stats,
+                                                  uint4 *__restrict__ cov, const uint8_t *__restrict__ galive,
+                                                  uint4 *__restrict__ bbox) {
+    __shared__ uint4 s_rec[kBlock / 32][32 * 8];
+    uint4 *stage = s_rec[threadIdx.x >> 5];
+    bool staged = false;
+    const uint64_t t = (uint64_t)blockIdx.x * kBlock + threadIdx.x;
+    const int si = chunk_scene ? (int)chunk_scene[blockIdx.x] : 0;
+    const SceneDev &s = sc[si];
+    const float4 *const positions = clip + (s.geom ? s.gvtx_base : s.vtx_base);
+    SetupOut o;
+    setup_prim(s, si, t, [&](uint32_t v) { return positions[v]; }, recs, galive, bbox, stage, staged, o);
+    if (o.bad) atomicCAS(err + si, 0, EUC_ERR_INDEX_OOB);
+    store_records(stage, staged, recs + (t - (threadIdx.x & 31)));
+    rows[t] = o.nrows;
+    // The block's sums, one atomic each: the scene's covered rectangle, its
+    // culled count and, for the strip path's routing, the pixels its rows may
+    // walk; the scan's per-chunk sums are this block's alone.  One set of
+    // atomics a block, not a warp: all of a scene's meet in two L2 sectors,
+    // where nine a warp (15.6 k warps of a 500 k triangle mesh) bounded this
+    // kernel (63 -> 23 us).
+    const SetupSums b = setup_block_sums<true>(o);
+    if (threadIdx.x == 0) {
+        chunk_sums[blockIdx.x] = make_uint2(b.live, b.rows);
+        if (b.x0 != 0xFFFFFFFFu) {
+            atomicMin(&cov[si].x, b.x0);
+            atomicMin(&cov[si].y, b.y0);
+            atomicMin(&cov[si].z, b.nx1);
+            atomicMin(&cov[si].w, b.ny1);
         }
+        if (b.culled) atomicAdd(&stats[si].culled, (unsigned long long)b.culled);
+        if (bbox && b.walked) atomicAdd(&stats[si].walked, b.walked);
+        if (bbox && b.live) atomicAdd(&stats[si].live, (unsigned long long)b.live);
     }
 }
 
@@ -2336,6 +2373,196 @@ __global__ void __launch_bounds__(kBlock, F::kResolveBlocks) k_resolve(const Sce
             }
         }
     }
+}
+
+// ---------------------------------------------------------------------------
+// The frame path: one small scene (at most kFramePrims primitive slots, no
+// geometry stage, no ordered blend) in three launches instead of seven.  Such a
+// scene is bound by the latency of its dependent launches, not by their work,
+// so the stages that need nothing of each other share one:
+//   k_front<F>      the scene's table and uniforms (its parameter) out to the
+//                   staging that the next two read; the setup of 256
+//                   primitives a block, each corner's clip position computed
+//                   by the vertex functor itself (the same function, so the
+//                   same bits) instead of waiting for a vertex stage; the
+//                   varyings of 256 vertices a block; the keys of
+//                   kInitChunk pixels a block, over the whole target
+//                   (the covered rectangle is not known yet)
+//   k_frame_raster  32 items a warp step, spread evenly over the grid from the
+//                   row sums of the 32-primitive groups, which every block
+//                   scans for itself; block 0 also finishes the scene's
+//                   covered rectangle, error and culled count for
+//   k_resolve<F>    as in a batch
+// Nothing is cleared ahead: the setup blocks store their own sums.  640x480
+// sphere, 4 k triangles, back to back: 28.3 us a call as seven launches, 14.4
+// us as three (k_front 5.5, k_frame_raster 7.2, k_resolve 9.0 us each alone).
+// ---------------------------------------------------------------------------
+constexpr uint32_t kFrameGroups = 1024;                // 32-primitive groups at most
+constexpr uint32_t kFramePrims = 32 * kFrameGroups;
+constexpr uint32_t kFrameBlocks = kFramePrims / kBlock;  // setup blocks at most
+
+struct FrontBlock {  // a setup block's sums
+    uint4 cov;       // min of (cx0, cy0, ~cx1, ~cy1)
+    uint32_t culled, bad;
+};
+struct FrontScratch {
+    uint32_t group_rows[kFrameGroups];
+    FrontBlock blk[kFrameBlocks];
+};
+
+struct FrontArgs {
+    SceneDev d;  // bases 0; uniforms: their place in the staging
+    alignas(16) unsigned char uni[512];
+    SceneDev *stage_scene;
+    unsigned char *stage_uni;
+    uint32_t usize;       // bytes of uni, a multiple of 4
+    uint32_t nsb, nib;    // setup blocks, key blocks (the others: vertices)
+    float *vdata;
+    TriRec *recs;
+    uint32_t *rows;
+    FrontScratch *front;
+    unsigned long long *vbuf;
+    SceneStats *stats;
+};
+
+template <class F>
+__global__ void __launch_bounds__(kBlock) k_front(const __grid_constant__ FrontArgs a) {
+    __shared__ uint4 s_rec[kBlock / 32][32 * 8];
+    launch_next();  // k_frame_raster, which waits for this kernel before its first read
+    const SceneDev &s = a.d;
+    const typename F::U &u = *reinterpret_cast<const typename F::U *>(a.uni);
+    const uint32_t b = blockIdx.x;
+    if (b < a.nsb) {
+        uint4 *stage = s_rec[threadIdx.x >> 5];
+        bool staged = false;
+        const uint32_t t = b * kBlock + threadIdx.x;
+        SetupOut o;
+        setup_prim(s, 0, t,
+                   [&](uint32_t v) {
+                       float c[4], vd[F::NV];
+                       F::vertex(u, s.lay, s.verts + (uint64_t)v * s.lay.stride, c, vd);
+                       return make_float4(c[0], c[1], c[2], c[3]);
+                   },
+                   a.recs, nullptr, nullptr, stage, staged, o);
+        store_records(stage, staged, a.recs + (t - (threadIdx.x & 31)));
+        a.rows[t] = o.nrows;
+        const uint32_t wr = __reduce_add_sync(0xFFFFFFFFu, o.nrows);
+        if ((threadIdx.x & 31) == 0) a.front->group_rows[t >> 5] = wr;
+        const int bad = __syncthreads_or(o.bad);
+        const SetupSums q = setup_block_sums<false>(o);
+        if (threadIdx.x == 0) {
+            a.front->blk[b].cov = make_uint4(q.x0, q.y0, q.nx1, q.ny1);
+            a.front->blk[b].culled = q.culled;
+            a.front->blk[b].bad = bad ? 1u : 0u;
+        }
+        if (b == 0) {  // (a scene has at least one setup block)
+            const uint32_t *src = reinterpret_cast<const uint32_t *>(&a.d);
+            for (uint32_t i = threadIdx.x; i < sizeof(SceneDev) / 4; i += kBlock)
+                reinterpret_cast<uint32_t *>(a.stage_scene)[i] = src[i];
+            for (uint32_t i = threadIdx.x; i < a.usize / 4; i += kBlock)
+                reinterpret_cast<uint32_t *>(a.stage_uni)[i] = reinterpret_cast<const uint32_t *>(a.uni)[i];
+            if (threadIdx.x == 0) *a.stats = SceneStats{};
+        }
+    } else if (b < a.nsb + a.nib) {
+        const uint32_t area = s.W * s.H, i0 = (b - a.nsb) * kInitChunk + threadIdx.x;
+        RectWalk rk(i0, s.W);
+        float d[kInitPer];
+#pragma unroll
+        for (int k = 0; k < kInitPer; ++k, rk.next())
+            d[k] = (i0 + k * kBlock < area && s.keytype == KEY_MIN)
+                       ? *reinterpret_cast<const float *>(s.depth + (uint64_t)rk.ry * s.dpitch + 4ull * rk.rx)
+                       : 0.0f;
+#pragma unroll
+        for (int k = 0; k < kInitPer; ++k)
+            if (i0 + k * kBlock < area)
+                a.vbuf[i0 + k * kBlock] =
+                    s.keytype == KEY_MIN ? init_key_min(d[k], s.depth_test == EUC_TEST_GREATER) : ~0ull;
+    } else {
+        const uint64_t v = (uint64_t)(b - a.nsb - a.nib) * kBlock + threadIdx.x;
+        if (v >= s.nverts) return;
+        float c[4], vd[F::NV];
+        F::vertex(u, s.lay, s.verts + v * s.lay.stride, c, vd);
+        store_vd<F>(a.vdata + v * vd_stride(F::NV), vd);
+    }
+}
+
+__global__ void __launch_bounds__(kBlock, 4) k_frame_raster(const SceneDev *__restrict__ sc,
+                                                           const TriRec *__restrict__ recs,
+                                                           const uint32_t *__restrict__ rows,
+                                                           const FrontScratch *__restrict__ front, uint32_t nsb,
+                                                           int *__restrict__ err, volatile int *__restrict__ host_err,
+                                                           SceneStats *__restrict__ stats, uint4 *__restrict__ cov,
+                                                           uint64_t *__restrict__ rbase,
+                                                           unsigned long long *__restrict__ vbuf, bool probe) {
+    __shared__ uint32_t s_a[kBlock / 32 + 1];
+    __shared__ __align__(16) uint32_t s_pref[kFrameGroups];
+    wait_previous();
+    const SceneDev &s = sc[0];
+    const int lane = threadIdx.x & 31;
+    const uint32_t ngroups = (s.ngroups + 31u) >> 5;
+    // four consecutive groups a thread: their steps of 32 items
+    static_assert(kFrameGroups == 4 * kBlock && kFrameBlocks <= kBlock, "four groups a thread, one setup block a thread");
+    const uint4 gr = *reinterpret_cast<const uint4 *>(front->group_rows + 4 * threadIdx.x);
+    uint32_t steps[4] = {gr.x, gr.y, gr.z, gr.w};
+#pragma unroll
+    for (uint32_t k = 0; k < 4; ++k) steps[k] = 4 * threadIdx.x + k < ngroups ? (steps[k] + 31u) >> 5 : 0u;
+    const int bad = __syncthreads_or(threadIdx.x < nsb && front->blk[threadIdx.x].bad);
+    if (blockIdx.x == 0 && threadIdx.x < 32) {
+        FrontBlock q;
+        q.cov = make_uint4(0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu);
+        q.culled = 0;
+        for (uint32_t b = threadIdx.x; b < nsb; b += 32) {
+            const FrontBlock f = front->blk[b];
+            q.cov = make_uint4(min(q.cov.x, f.cov.x), min(q.cov.y, f.cov.y), min(q.cov.z, f.cov.z), min(q.cov.w, f.cov.w));
+            q.culled += f.culled;
+        }
+        q.cov.x = __reduce_min_sync(0xFFFFFFFFu, q.cov.x);
+        q.cov.y = __reduce_min_sync(0xFFFFFFFFu, q.cov.y);
+        q.cov.z = __reduce_min_sync(0xFFFFFFFFu, q.cov.z);
+        q.cov.w = __reduce_min_sync(0xFFFFFFFFu, q.cov.w);
+        q.culled = __reduce_add_sync(0xFFFFFFFFu, q.culled);
+        if (threadIdx.x == 0) {
+            cov[0] = q.cov;
+            err[0] = bad ? EUC_ERR_INDEX_OOB : EUC_OK;
+            if (host_err) {
+                *host_err = bad ? EUC_ERR_INDEX_OOB : EUC_OK;
+                __threadfence_system();
+            }
+            stats[0].culled = q.culled;
+            rbase[0] = 0;
+            rbase[1] = bad ? 0ull : resolve_chunks(s, q.cov);  // a scene with a bad index draws nothing
+        }
+    }
+    if (bad) return;
+    uint32_t total;
+    const uint32_t pre = block_excl_scan<uint32_t>((steps[0] + steps[1]) + (steps[2] + steps[3]), s_a, &total);
+    *reinterpret_cast<uint4 *>(s_pref + 4 * threadIdx.x) =
+        make_uint4(pre, pre + steps[0], pre + steps[0] + steps[1], pre + steps[0] + steps[1] + steps[2]);
+    __syncthreads();
+    const uint32_t nwarps = gridDim.x * (kBlock / 32);
+    uint32_t cnt = 0;
+    for (uint32_t st = blockIdx.x * (kBlock / 32) + (threadIdx.x >> 5); st < total; st += nwarps) {
+        // the last group whose steps start at or before st (one without steps
+        // starts where the next one does)
+        // (groups beyond the scene's start at `total`)
+        static_assert(kFrameGroups == 32 * 32, "a two-level search, 32 ways each");
+        const uint32_t g32 = 32u * (uint32_t)(__popc(__ballot_sync(0xFFFFFFFFu, s_pref[32 * lane] <= st)) - 1);
+        const uint32_t g = g32 + (uint32_t)__popc(__ballot_sync(0xFFFFFFFFu, s_pref[g32 + lane] <= st)) - 1u;
+        const uint32_t i = (st - s_pref[g]) * 32 + lane;  // this lane's item in the group
+        const uint32_t nr = rows[g * 32 + lane], incl = warp_incl_scan(nr);
+        // its primitive: the first whose items end after i
+        int p = 0;
+#pragma unroll
+        for (int d = 16; d > 0; d >>= 1)
+            if (__shfl_sync(0xFFFFFFFFu, incl, p + d - 1) <= i) p += d;
+        const uint32_t first = __shfl_sync(0xFFFFFFFFu, incl - nr, p);
+        if (i >= __shfl_sync(0xFFFFFFFFu, incl, 31)) continue;
+        const uint32_t t = g * 32 + p;
+        const TriRec r = load_rec(recs + t, s.prim == EUC_PRIM_TRIANGLE_LIST ? kRecRaster : kRecAll);
+        raster_row(s, r, t, r.by0 + (i - first), vbuf, cnt, 0, nullptr, probe);
+    }
+    const uint32_t sum = warp_sum(cnt);
+    if (lane == 0 && sum) atomicAdd(&stats[0].candidates, (unsigned long long)sum);
 }
 
 // ---------------------------------------------------------------------------

@@ -359,3 +359,33 @@ def test_depths_at_the_edges_of_the_positive_class(gpu_ctx, strip_ctx, z, clear)
         a, b = ref["depth"].view(np.uint32), got["depth"].view(np.uint32)
         assert np.array_equal(a, b)
         assert np.array_equal(ref["color"], got["color"])
+
+
+@pytest.mark.parametrize("prims", [abi.PRIM_TRIANGLE_LIST, abi.PRIM_LINE_LIST])
+@pytest.mark.parametrize("n,w,h", [(1, 70, 33), (31, 64, 32), (33, 64, 33), (257, 97, 61), (1023, 1, 50), (4000, 255, 9),
+                                   (32768, 160, 90), (32769, 160, 90), (300, 1024, 1024), (300, 1024, 1025)])
+def test_frames_at_the_edges_of_the_small_scene_path(prims, n, w, h):
+    """Primitive groups, setup blocks and both limits of the three-launch path
+    (32768 primitives, 2^20 pixels), one scene more than fits included; three
+    calls: plain, recorded, replayed with other inputs."""
+    from euc_gb300 import capi
+    ctx = capi.Context(0)
+    try:
+        for seed in (80, 81, 82):
+            if prims == abi.PRIM_LINE_LIST:
+                make = lambda: scenes.lines_frame(seed=seed, width=w, height=h, nlines=n, len_hi=40.0)
+            else:
+                make = lambda: scenes.soup_frame(seed=seed, width=w, height=h, ntris=n, area_hi=60.0)
+            ref, ref_stats = run_oracle(make())
+            got, got_stats = run_gpu(ctx, make())
+            assert got_stats == ref_stats
+            assert_targets_match(make(), ref, got)
+        bad = make()
+        bad.passes[0].indices = bad.passes[0].indices.copy()
+        bad.passes[0].indices[-1] = bad.passes[0].nverts
+        got, got_stats = run_gpu(ctx, bad)
+        assert got_stats[0][0] == abi.ERR_INDEX_OOB
+        clean = bad.alloc_host_targets()
+        assert all(np.array_equal(got[k], clean[k]) for k in clean)
+    finally:
+        ctx.close()
