@@ -636,7 +636,7 @@ int run_batch(euc_ctx *ctx, const euc_scene *scenes, size_t n, cudaStream_t st, 
         if ((rc = grow(ctx->strip_off, (nstrips + 1) * sizeof(uint32_t)))) return rc;
         if ((rc = grow(ctx->strip_uoff, (nstrips + 1) * sizeof(uint32_t)))) return rc;
         if ((rc = grow(ctx->entries, entry_cap * sizeof(uint2)))) return rc;
-        if ((rc = grow(ctx->unit_strip, (nstrips + entry_cap / kStripUnit + 1) * sizeof(uint32_t)))) return rc;
+        if ((rc = grow(ctx->unit_strip, (nstrips + entry_cap / kStripUnitMin + 1) * sizeof(uint32_t)))) return rc;
         if ((rc = grow(ctx->bbox, tri * sizeof(uint4)))) return rc;
     }
     // staging: scene table | vtx bases | resolve bases | geometry bases |
@@ -735,6 +735,7 @@ int run_batch(euc_ctx *ctx, const euc_scene *scenes, size_t n, cudaStream_t st, 
                                                    (SceneStats *)ctx->stats.p, (uint4 *)ctx->cov.p,
                                                    (const uint8_t *)ctx->galive.p,
                                                    nstrips ? (uint4 *)ctx->bbox.p : nullptr);
+    const unsigned strip_grid = (unsigned)ctx->nsm * kStripBlocksPerSm;
     // binning blocks stride the setup chunks
     const unsigned bin_grid = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(nchunks, (uint64_t)ctx->nsm * 8));
     if (nstrips) {  // the strip path's routing and counts
@@ -750,7 +751,7 @@ int run_batch(euc_ctx *ctx, const euc_scene *scenes, size_t n, cudaStream_t st, 
     k_scan_plan<<<(unsigned)(nscan + 1 + nsblk), kBlock, 0, st>>>(
         (const uint32_t *)ctx->rows.p, (const uint2 *)ctx->chunk_sums.p, tri, (uint32_t *)ctx->live_tri.p,
         (uint64_t *)ctx->live_rowoff.p, (unsigned long long *)ctx->totals.p, (uint32_t)nscan, dsc, ns,
-        (const uint4 *)ctx->cov.p, ibase, rbase, (const uint32_t *)ctx->strip_cnt.p, (uint32_t)nstrips,
+        (const uint4 *)ctx->cov.p, ibase, rbase, (const uint32_t *)ctx->strip_cnt.p, (uint32_t)nstrips, strip_grid,
         (uint32_t *)ctx->strip_off.p, (uint32_t *)ctx->strip_uoff.p, (uint32_t *)ctx->unit_strip.p);
     cudaEvent_t e3 = prof_event(ctx, st);
     const euc_tuning &tu = ctx->tune;
@@ -789,7 +790,7 @@ int run_batch(euc_ctx *ctx, const euc_scene *scenes, size_t n, cudaStream_t st, 
     // with most of the GPU idle, and k_strip's blocks start there (48-scene
     // batch, a whole call: 578 us one after the other, 490 us with both)
     if (nstrips) {
-        CUDA_TRY(launch_beside(k_strip, (unsigned)ctx->nsm * kStripBlocksPerSm, kStripThreads, strip_smem, st, dsc, dsb,
+        CUDA_TRY(launch_beside(k_strip, strip_grid, kStripThreads, strip_smem, st, dsc, dsb,
                                ns, (const uint4 *)ctx->cov.p, (const uint32_t *)ctx->strip_off.p,
                                (const uint32_t *)ctx->strip_uoff.p, (const uint32_t *)ctx->unit_strip.p,
                                (const uint2 *)ctx->entries.p, (const TriRec *)ctx->recs.p, (const int *)ctx->err.p,
@@ -867,8 +868,10 @@ int run_batch(euc_ctx *ctx, const euc_scene *scenes, size_t n, cudaStream_t st, 
 // that launches, not work, set their time (k_front's comment has the figures).
 // kFramePrims bounds the groups a block scans; kFramePixels bounds the keys that k_front seeds beyond the
 // covered rectangle (12 bytes a pixel: 12.6 MB, some 2 us beside the setup);
-// kFrameVerts keeps a large unindexed buffer on the batch's path.  A batch, a
-// forced strip path and a profiled context take the other kernels.
+// kFrameVerts keeps unindexed soups of more than 21 k triangles on the batch's
+// path, whose strips pay there (640x480: 16 k triangles of up to 2000 px 58 us
+// here and 130 us on the strips, 32 k of up to 8000 px 229 and 126).  A batch,
+// a forced strip path and a profiled context take the other kernels.
 // ---------------------------------------------------------------------------
 constexpr uint64_t kFramePixels = 1ull << 20, kFrameVerts = 1ull << 16;
 
@@ -2040,7 +2043,7 @@ extern "C" int euc_render_noalloc(const euc_pipeline_desc *desc, const void *uni
     k_scan_plan<<<nscan + 1, kBlock, 0, st>>>((const uint32_t *)(a + kNaOffRows), (const uint2 *)(a + kNaOffChunks),
                                               tri, (uint32_t *)(a + kNaOffLiveTri), (uint64_t *)(a + kNaOffLiveOff),
                                               (unsigned long long *)(a + kNaOffTotals), nscan, dsc, 1,
-                                              (const uint4 *)(a + kNaOffCov), ibase, rbase, nullptr, 0, nullptr, nullptr,
+                                              (const uint4 *)(a + kNaOffCov), ibase, rbase, nullptr, 0, 1, nullptr, nullptr,
                                               nullptr);
     const uint64_t ichunks = (pix + kInitChunk - 1) / kInitChunk + 1;
     k_init<<<chunk_grid(ichunks, nsm), kBlock, 0, st>>>(dsc, ibase, 1, (const uint4 *)(a + kNaOffCov),

@@ -603,7 +603,9 @@ constexpr int kStripBlocksPerSm = 2;          // k_strip blocks resident per SM 
 constexpr uint32_t kStripMaxRows = 16;        // rows of a strip at most
 constexpr size_t kStripKeyBytes = 96 * 1024;  // a strip's keys in shared memory at most
 constexpr uint32_t kRowsBinned = 0x80000000u; // rows[t]: the primitive went to the strips
-constexpr uint32_t kStripUnit = 1024;         // entries of one strip a k_strip block takes at once at most
+constexpr uint32_t kStripUnit = 1024;         // entries of one strip a k_strip block takes at once at most ...
+constexpr uint32_t kStripUnitMin = 128;       // ... and at least, where a launch has few of them (strip_unit)
+constexpr uint32_t kStripUnitsPerBlock = 3;   // units that each resident block should find
 constexpr uint32_t kStripClaim = 32;          // items a k_strip warp claims at a time
 constexpr uint64_t kStripOverdraw = 4;        // fragments per covered pixel that route a scene to the strips ...
 constexpr uint64_t kStripTriFrags = 16;       // ... when its triangles make this many fragments each on average
@@ -619,6 +621,19 @@ __host__ __device__ inline uint32_t strip_rows(uint32_t W, uint32_t H) {
     if (W == 0 || H == 0 || H >= (1u << 24) || 8ull * strip_pitch(W) > kStripKeyBytes) return 0;
     const uint64_t r = kStripKeyBytes / (8ull * strip_pitch(W));
     return (uint32_t)(r < kStripMaxRows ? r : kStripMaxRows);
+}
+
+// Entries per unit of a launch with `entries` of them for `blocks` resident
+// blocks.  A full unit keeps a block some 100 us, so a launch of fewer than a
+// few hundred units would leave most of the GPU idle at its end (or from its
+// start): smaller units then, whose own sort and merge cost a few us each.
+// 48-scene batch, a whole call: 472 us with 1024 entries always, 455 / 441 /
+// 440 / 456 us with 2 / 3 / 4 / 8 units a block; 192 served requests 4.88 ms,
+// 4.90 with 3, 4.93 with 4, 5.11 with 8; one 640x480 soup of 32768 triangles
+// 102 -> 72 us.
+__host__ __device__ inline uint32_t strip_unit(unsigned long long entries, uint32_t blocks) {
+    const unsigned long long u = (entries / ((unsigned long long)blocks * kStripUnitsPerBlock) + 31ull) & ~31ull;
+    return u < kStripUnitMin ? kStripUnitMin : u > kStripUnit ? kStripUnit : (uint32_t)u;
 }
 
 // Width bucket of a k_strip entry (the span w of its middle row in the
@@ -1692,7 +1707,7 @@ EUC_DEV uint32_t strip_block_scan(uint32_t v, uint32_t *smem /* >= kStripThreads
 }
 
 // ---------------------------------------------------------------------------
-// k_strip: one unit (up to kStripUnit entries of one strip) at a time per
+// k_strip: one unit (up to strip_unit entries of one strip) at a time per
 // block, claimed from a work counter (totals[7]).  sbase: the first strip of
 // each scene (nsc + 1 entries).  The unit's keys over the strip's rows inside
 // the scene's covered rectangle start at ~0 in shared memory; the warps
@@ -1728,7 +1743,7 @@ __global__ void __launch_bounds__(kStripThreads, kStripBlocksPerSm) k_strip(cons
     static_assert(offsetof(TriRec, bx0) == 48, "k_strip reads the bbox width from 8-byte word 6 of a record");
     const int tid = threadIdx.x, lane = tid & 31;
     const uint32_t nstrips = (uint32_t)sbase[nsc];
-    const uint32_t nunits = strip_uoff[nstrips];
+    const uint32_t nunits = strip_uoff[nstrips], unit = strip_unit(totals[6], gridDim.x);
     const uint32_t keys_saddr = (uint32_t)__cvta_generic_to_shared(s_keys);
     uint32_t key_bytes;  // the launch's dynamic shared memory
     asm("mov.u32 %0, %%dynamic_smem_size;" : "=r"(key_bytes));
@@ -1752,8 +1767,8 @@ __global__ void __launch_bounds__(kStripThreads, kStripBlocksPerSm) k_strip(cons
         const bool empty = r0 >= r1 || cx0 >= cx1;  // never for a strip with entries
         const uint32_t wc = empty ? 0u : cx1 - cx0, area = empty ? 0u : (r1 - r0) * strip_pitch(wc);
         const uint32_t pitch = strip_pitch(wc);
-        const uint32_t e_begin = strip_off[g] + (u - strip_uoff[g]) * kStripUnit;
-        const int nload = (int)(min(e_begin + kStripUnit, strip_off[g + 1]) - e_begin);
+        const uint32_t e_begin = strip_off[g] + (u - strip_uoff[g]) * unit;
+        const int nload = (int)(min(e_begin + unit, strip_off[g + 1]) - e_begin);
         // the unit's entries, two per thread, ordered by the span of their
         // middle row in the strip, widest first (a counting sort over
         // kWidthBuckets): the rows a warp walks together have about the same
@@ -2048,10 +2063,10 @@ EUC_DEV void plan_chunks(const SceneDev *__restrict__ sc, int nsc, const uint4 *
 }
 
 // Exclusive scans of the strips' entry counts into their list offsets, and
-// of their units (ceil(count / kStripUnit)) into unit offsets (nstrips + 1
-// entries each), and the strip of every unit.  Block b covers strips
+// of their units (ceil(count / unit)) into unit offsets (nstrips + 1 entries
+// each), and the strip of every unit.  Block b covers strips
 // [b*kScanBlock, (b+1)*kScanBlock) and sums the strips before them itself.
-EUC_DEV void strip_scan_block(uint32_t b, const uint32_t *__restrict__ cnt, uint32_t nstrips,
+EUC_DEV void strip_scan_block(uint32_t b, const uint32_t *__restrict__ cnt, uint32_t nstrips, uint32_t unit,
                               uint32_t *__restrict__ off, uint32_t *__restrict__ uoff,
                               uint32_t *__restrict__ unit_strip) {
     __shared__ uint32_t s_a[kBlock / 32 + 1];
@@ -2060,7 +2075,7 @@ EUC_DEV void strip_scan_block(uint32_t b, const uint32_t *__restrict__ cnt, uint
     uint32_t pre = 0, preu = 0;
     for (uint64_t j = threadIdx.x; j < g0; j += kBlock) {
         pre += cnt[j];
-        preu += (cnt[j] + kStripUnit - 1) / kStripUnit;
+        preu += (cnt[j] + unit - 1) / unit;
     }
     uint32_t tp, tu;
     block_excl_scan<uint32_t>(pre, s_a, &tp);
@@ -2076,14 +2091,14 @@ EUC_DEV void strip_scan_block(uint32_t b, const uint32_t *__restrict__ cnt, uint
     for (int k = 0; k < kScanPer; ++k) {
         c[k] = q0 + k < nstrips ? cnt[q0 + k] : 0u;
         mine += c[k];
-        mineu += (c[k] + kStripUnit - 1) / kStripUnit;
+        mineu += (c[k] + unit - 1) / unit;
     }
     uint32_t bt, btu;
     uint32_t o = s_pre[0] + block_excl_scan<uint32_t>(mine, s_a, &bt);
     uint32_t ou = s_pre[1] + block_excl_scan<uint32_t>(mineu, s_a, &btu);
 #pragma unroll
     for (int k = 0; k < kScanPer; ++k) {
-        const uint32_t nu = (c[k] + kStripUnit - 1) / kStripUnit;
+        const uint32_t nu = (c[k] + unit - 1) / unit;
         if (q0 + k < nstrips) {
             off[q0 + k] = o;
             uoff[q0 + k] = ou;
@@ -2110,11 +2125,12 @@ __global__ void __launch_bounds__(kBlock) k_scan_plan(const uint32_t *__restrict
                                                       const SceneDev *__restrict__ sc, int nsc,
                                                       const uint4 *__restrict__ cov, uint64_t *__restrict__ ibase,
                                                       uint64_t *__restrict__ rbase, const uint32_t *__restrict__ strip_cnt,
-                                                      uint32_t nstrips, uint32_t *__restrict__ strip_off,
+                                                      uint32_t nstrips, uint32_t strip_blocks,
+                                                      uint32_t *__restrict__ strip_off,
                                                       uint32_t *__restrict__ strip_uoff, uint32_t *__restrict__ unit_strip) {
     if (blockIdx.x == nscan) plan_chunks(sc, nsc, cov, ibase, rbase);
     else if (blockIdx.x > nscan)
-        strip_scan_block(blockIdx.x - nscan - 1, strip_cnt, nstrips, strip_off, strip_uoff, unit_strip);
+        strip_scan_block(blockIdx.x - nscan - 1, strip_cnt, nstrips, strip_unit(totals[6], strip_blocks), strip_off, strip_uoff, unit_strip);
     else scan_block(rows, chunk_sums, ntri, live_tri, live_rowoff, totals, nscan);
 }
 

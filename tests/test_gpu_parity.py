@@ -389,3 +389,14 @@ def test_frames_at_the_edges_of_the_small_scene_path(prims, n, w, h):
         assert all(np.array_equal(got[k], clean[k]) for k in clean)
     finally:
         ctx.close()
+
+
+@pytest.mark.parametrize("n,area", [(40, 30000.0), (700, 3000.0), (9000, 900.0), (60000, 120.0)])
+def test_strip_units_of_every_size(strip_ctx, n, area):
+    """Few entries (units of kStripUnitMin) to many (full units): the unit
+    size follows from the launch's entry count."""
+    make = _soup(seed=90, w=300, h=200, n=n, hi=area)
+    ref, ref_stats = run_oracle(make())
+    got, got_stats = run_gpu(strip_ctx, make())
+    assert got_stats == ref_stats
+    assert_targets_match(make(), ref, got)
