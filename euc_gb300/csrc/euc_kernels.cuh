@@ -2304,7 +2304,7 @@ EUC_DEV void resolve_chunk(const SceneDev &s, const uint4 &cv, const ChunkGeom &
     const uint32_t L = s.level;
     for (uint32_t j = lane; j < njobs; j += 32) {
         const int slot = s_job[j] >> 2, c = s_job[j] & 3;
-        const TriRec &r = recs[s_t[slot]];  // (field loads here: the vector copy costs this path registers)
+        const TriRec r = load_rec(recs + s_t[slot], s.prim == EUC_PRIM_TRIANGLE_LIST ? kRecShade : kRecAll);
         float xf, yf;
         if (L == 0) {
             xf = (float)s_xy[slot][0];
