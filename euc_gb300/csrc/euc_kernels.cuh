@@ -1030,6 +1030,31 @@ __host__ __device__ inline uint64_t rect_area(const uint4 &c) {
 // is spent on pixels that no primitive reaches.
 constexpr int kChunkGroup = 16;
 
+// The covered rectangle cut into segments of at most kSeg pixels of one row,
+// one a warp (chunk lb of kBlock / 32 segments): a lane's pixels are 32 apart
+// in the segment, so the row's addresses are computed once and a pixel costs
+// no division or wrap.  256 spheres of 640x480 (86 k pixels of the rectangle
+// each): k_init 71 -> 57 us (45 -> 24 M instructions), k_resolve<GouraudFn>
+// 214 -> 203 us (130 -> 108 M; what bounds it now is L1, 84 % busy).
+template <int kSeg>
+struct RowSegment {
+    uint32_t y, x, xend;  // the row, this lane's first pixel, the end of the row or segment
+    EUC_DEV RowSegment(const uint4 &cv, uint32_t lb) {
+        const uint32_t nseg = (~cv.z - cv.x + kSeg - 1) / kSeg;
+        const uint32_t u = lb * (kBlock / 32) + (threadIdx.x >> 5), row = u / nseg;
+        y = cv.y + row;
+        const uint32_t x0 = cv.x + (u - row * nseg) * kSeg;
+        xend = y < ~cv.w ? min(x0 + kSeg, ~cv.z) : 0u;  // (a warp beyond the last segment has none)
+        x = x0 + (threadIdx.x & 31);
+    }
+};
+template <int kSeg>
+__host__ __device__ inline uint64_t segment_chunks(const uint4 &cv) {
+    if (rect_area(cv) == 0) return 0;
+    const uint64_t nseg = (~cv.z - cv.x + kSeg - 1) / kSeg;
+    return (nseg * (~cv.w - cv.y) + kBlock / 32 - 1) / (kBlock / 32);
+}
+
 // Entries i0, i0 + kBlock, i0 + 2 kBlock, ... of a row-major rectangle rw
 // wide, as (column, row): one division for the first entry and one for the
 // step, then a fixed quotient and remainder per step (the column wraps at
@@ -1052,11 +1077,10 @@ struct RectWalk {
     }
 };
 
-// Each thread of k_init initialises kInitPer entries of the covered rectangle,
-// kBlock apart, so that every load and store instruction of a warp covers 32
-// consecutive entries and the kInitPer depth loads are in flight together; a
-// chunk is kBlock * kInitPer entries.
+// A lane of k_init initialises kInitPer entries of a row segment, its depth
+// loads in flight together.  kInitChunk: entries of a chunk at most.
 constexpr int kInitPer = 8;
+constexpr int kInitSeg = 32 * kInitPer;
 constexpr int kInitChunk = kBlock * kInitPer;
 
 // Scene of chunk `c` given the scene of an earlier chunk of the same group.
@@ -1077,43 +1101,44 @@ __global__ void __launch_bounds__(kBlock) k_init(const SceneDev *__restrict__ sc
         __syncthreads();
         if (threadIdx.x == 0) s_scene = find_scene(ibase, nsc, c0);
         __syncthreads();
+        const uint64_t c1 = min(c0 + group, nchunks);
         int si = s_scene;
-        for (uint64_t c = c0; c < c0 + group && c < nchunks; ++c) {
-            si = advance_scene(ibase, nsc, si, c);
-            const SceneDev &s = sc[si];
+        for (uint64_t c = c0; c < c1; ++si) {  // a scene's chunks of the group
+            const uint64_t first = ibase[si], end = min(ibase[si + 1], c1);
+            if (c >= end) continue;
             // pixel and entry indices within a scene fit 32 bits (plan_scene)
-            const uint32_t i0 = (uint32_t)(c - ibase[si]) * kInitChunk + threadIdx.x;
-            unsigned long long *row0 = vbuf + s.pix_base;
+            const SceneDev &s = sc[si];
+            uint32_t lb = (uint32_t)(c - first);
+            const uint32_t lend = (uint32_t)(end - first);
+            c = end;
+            unsigned long long *const keys = vbuf + s.pix_base;
             if (s.keytype == KEY_ORDERED) {
                 // every entry, padding included (the pixel scan sums them all):
                 // no fragment yet, cursor 0
                 const uint32_t lim = (s.W * s.H + kBlock - 1) / kBlock * kBlock;
+                for (; lb < lend; ++lb) {
+                    const uint32_t i0 = lb * kInitChunk + threadIdx.x;
 #pragma unroll
-                for (int k = 0; k < kInitPer; ++k)
-                    if (i0 + k * kBlock < lim) row0[i0 + k * kBlock] = 0ull;
+                    for (int k = 0; k < kInitPer; ++k)
+                        if (i0 + k * kBlock < lim) keys[i0 + k * kBlock] = 0ull;
+                }
                 continue;
             }
-            // entries i0, i0 + kBlock, ... of the covered rectangle, row by row
             const uint4 cv = cov[si];
-            const uint32_t area = (uint32_t)rect_area(cv);
-            if (i0 >= area) continue;
-            RectWalk rk(i0, ~cv.z - cv.x);
-            uint32_t px[kInitPer];
-            float d[kInitPer];
+            const uint32_t W = s.W, dpitch = s.dpitch;
+            const uint8_t *const depth = s.depth;
+            const bool kmin = s.keytype == KEY_MIN, greater = s.depth_test == EUC_TEST_GREATER;
+            for (; lb < lend; ++lb) {
+                const RowSegment<kInitSeg> g(cv, lb);
+                unsigned long long *key = keys + (uint64_t)g.y * W + g.x;
+                const float *d0 = reinterpret_cast<const float *>(depth + (uint64_t)g.y * dpitch) + g.x;
+                float d[kInitPer];
 #pragma unroll
-            for (int k = 0; k < kInitPer; ++k, rk.next()) {
-                const uint32_t i = i0 + k * kBlock;
-                const bool live = i < area;
-                const uint32_t x = cv.x + rk.rx, y = cv.y + rk.ry;
-                px[k] = live ? y * s.W + x : 0xFFFFFFFFu;
-                d[k] = (live && s.keytype == KEY_MIN)
-                           ? *reinterpret_cast<const float *>(s.depth + (uint64_t)y * s.dpitch + 4ull * x)
-                           : 0.0f;
+                for (int k = 0; k < kInitPer; ++k) d[k] = kmin && g.x + 32 * k < g.xend ? d0[32 * k] : 0.0f;
+#pragma unroll
+                for (int k = 0; k < kInitPer; ++k)
+                    if (g.x + 32 * k < g.xend) key[32 * k] = kmin ? init_key_min(d[k], greater) : ~0ull;
             }
-#pragma unroll
-            for (int k = 0; k < kInitPer; ++k)
-                if (px[k] != 0xFFFFFFFFu)
-                    row0[px[k]] = s.keytype == KEY_MIN ? init_key_min(d[k], s.depth_test == EUC_TEST_GREATER) : ~0ull;
         }
     }
 }
@@ -1908,13 +1933,12 @@ EUC_DEV void get_v_data(const TriRec &r, const float *__restrict__ vd0, const fl
 // The winner's vertex outputs at (xf, yf): get_v_data for a triangle,
 // weighted_sum2 of the two ends for a line (lines.rs:98-110).
 template <class F>
-EUC_DEV void vdata_at(const SceneDev &s, const TriRec &r, const float *__restrict__ vb, float xf, float yf,
-                      float *out) {
+EUC_DEV void vdata_at(bool line, const TriRec &r, const float *__restrict__ vb, float xf, float yf, float *out) {
     constexpr int S = vd_stride(F::NV);
     float a0[S], a1[S];
     load_vd<F>(vb + (uint64_t)r.v[0] * S, a0);
     load_vd<F>(vb + (uint64_t)r.v[1] * S, a1);
-    if (s.prim != EUC_PRIM_TRIANGLE_LIST) {
+    if (line) {
         const float frac = ((r.flags & kLineUseX) ? xf - r.o[0] : yf - r.o[1]) * r.o[2];
 #pragma unroll
         for (int i = 0; i < F::NV; ++i) out[i] = a0[i] * (1.0f - frac) + a1[i] * frac;
@@ -1926,13 +1950,13 @@ EUC_DEV void vdata_at(const SceneDev &s, const TriRec &r, const float *__restric
 }
 
 // Decodes a visibility key; false when no fragment passed at this pixel.
-EUC_DEV bool decode_key(const SceneDev &s, unsigned long long key, uint32_t &t, float &z) {
-    if (s.keytype == KEY_MIN) {
+EUC_DEV bool decode_key(bool kmin, bool greater, unsigned long long key, uint32_t &t, float &z) {
+    if (kmin) {
         const uint32_t low = (uint32_t)key;
         if (low == 0) return false;
         t = (low >> 1) - 1u;
         uint32_t o = (uint32_t)(key >> 32);
-        if (s.depth_test == EUC_TEST_GREATER) o = ~o;
+        if (greater) o = ~o;
         z = (low & 1u) ? -0.0f : unord_f32(o);
         return true;
     }
@@ -1943,11 +1967,10 @@ EUC_DEV bool decode_key(const SceneDev &s, unsigned long long key, uint32_t &t, 
 }
 
 template <class F>
-EUC_DEV void store_pixel(const SceneDev &s, uint32_t x, uint32_t y, const float *frag) {
+EUC_DEV void store_pixel(uint8_t *p, uint32_t pfmt, uint32_t x, const float *frag) {  // p: pixel 0 of the row
     const float c0 = frag[0], c1 = F::NF > 1 ? frag[F::NF > 1 ? 1 : 0] : 0.0f;
     const float c2 = F::NF > 2 ? frag[F::NF > 2 ? 2 : 0] : 0.0f, c3 = F::NF > 3 ? frag[F::NF > 3 ? 3 : 0] : 0.0f;
-    uint8_t *p = s.pixel + (uint64_t)y * s.ppitch;
-    if (s.pfmt == EUC_FMT_RGBA32F) {  // the fragment as it is (no pack)
+    if (pfmt == EUC_FMT_RGBA32F) {  // the fragment as it is (no pack)
         float *q = reinterpret_cast<float *>(p) + 4ull * x;
         q[0] = c0;
         q[1] = c1;
@@ -1956,9 +1979,9 @@ EUC_DEV void store_pixel(const SceneDev &s, uint32_t x, uint32_t y, const float 
         return;
     }
     const uint32_t r8 = sat_u8(F::pack(c0)), g8 = sat_u8(F::pack(c1)), b8 = sat_u8(F::pack(c2)), a8 = sat_u8(F::pack(c3));
-    if (s.pfmt == EUC_FMT_RGBA8) {
+    if (pfmt == EUC_FMT_RGBA8) {
         reinterpret_cast<uint32_t *>(p)[x] = r8 | (g8 << 8) | (b8 << 16) | (a8 << 24);
-    } else if (s.pfmt == EUC_FMT_BGRA8) {
+    } else if (pfmt == EUC_FMT_BGRA8) {
         reinterpret_cast<uint32_t *>(p)[x] = b8 | (g8 << 8) | (r8 << 16) | (a8 << 24);
     } else {  // RGB8: two stores, the 2-byte one on its even address
         p += 3ull * x;
@@ -1995,18 +2018,19 @@ constexpr uint32_t kDirectShaders = (FlatFn::kDirect ? 1u << EUC_SHADER_FLAT : 0
 // Scenes resolved kDirectPer pixels per thread with no shared memory: depth
 // only, or a cheap shader without MSAA.
 constexpr int kDirectPer = 4;
+constexpr int kDirectSeg = 32 * kDirectPer;
 __host__ __device__ inline bool resolve_direct(const SceneDev &s) {
     return s.keytype != KEY_ORDERED &&
            (!s.pixel_write || (s.level == 0 && ((kDirectShaders >> s.shader) & 1u)));
 }
 
-// k_resolve chunks (blocks of work) of a scene: kBlock pixels of the covered
-// rectangle, or kBlock/32 warp tiles of 16x2 pixels over the row pairs and
+// k_resolve chunks (blocks of work) of a scene: kBlock / 32 row segments or
+// kBlock pixels of the covered rectangle, or kBlock/32 warp tiles of 16x2 pixels over the row pairs and
 // 16-pixel columns that meet it.
 __host__ __device__ inline uint64_t resolve_chunks(const SceneDev &s, const uint4 &cv) {
     const uint64_t area = rect_area(cv);
     if (area == 0) return 0;
-    if (resolve_direct(s)) return (area + kBlock * kDirectPer - 1) / (kBlock * kDirectPer);
+    if (resolve_direct(s)) return segment_chunks<kDirectSeg>(cv);
     if (resolve_by_quads(s)) {
         const uint64_t pairs = pair_of_row(~cv.w - 1, s.gr) - pair_of_row(cv.y, s.gr) + 1;
         const uint64_t cols = ((~cv.z - 1) >> 4) - (cv.x >> 4) + 1;
@@ -2042,7 +2066,7 @@ EUC_DEV void plan_chunks(const SceneDev *__restrict__ sc, int nsc, const uint4 *
                 const uint64_t lim = ((uint64_t)s.W * s.H + kBlock - 1) / kBlock * kBlock;
                 ni = (lim + kInitChunk - 1) / kInitChunk;
             } else {
-                ni = (rect_area(cv) + kInitChunk - 1) / kInitChunk;
+                ni = segment_chunks<kInitSeg>(cv);
                 nr = resolve_chunks(s, cv);
             }
         }
@@ -2159,41 +2183,41 @@ struct ResolveSmem {
     float frag[32][4][F::NF];
 };
 
-// Chunk `lb` of a resolve_direct scene: kBlock * kDirectPer pixels of the
-// covered rectangle, each thread taking kDirectPer of them kBlock apart (the
-// key loads of a thread are in flight together).
+// Chunk `lb` of a resolve_direct scene: a warp's row segment, kDirectPer
+// pixels a lane (their key loads, and then their record and varyings gathers,
+// are in flight together).  The scene's fields are read once, ahead of the
+// stores: behind one, the compiler has to read them again (20 loads a pixel,
+// twice what the shading itself needs).
 template <class F>
 EUC_DEV void resolve_direct_chunk(const SceneDev &s, const uint4 &cv, uint64_t lb, const TriRec *__restrict__ recs,
                                   const float *__restrict__ vdata, const unsigned long long *__restrict__ vbuf) {
-    const uint32_t area = (uint32_t)rect_area(cv);  // pixel indices fit 32 bits
-    const uint32_t i0 = (uint32_t)lb * (kBlock * kDirectPer) + threadIdx.x;
-    RectWalk rk(i0, ~cv.z - cv.x);
-    uint32_t px[kDirectPer], py[kDirectPer];
+    const RowSegment<kDirectSeg> g(cv, (uint32_t)lb);
+    const bool kmin = s.keytype == KEY_MIN, greater = s.depth_test == EUC_TEST_GREATER;
+    const unsigned long long *keys = vbuf + s.pix_base + (uint64_t)g.y * s.W + g.x;
     unsigned long long key[kDirectPer];
 #pragma unroll
-    for (int k = 0; k < kDirectPer; ++k, rk.next()) {
-        const uint32_t i = i0 + k * kBlock;
-        px[k] = cv.x + rk.rx;
-        py[k] = i < area ? cv.y + rk.ry : 0xFFFFFFFFu;
-        key[k] = i < area ? vbuf[s.pix_base + (uint64_t)py[k] * s.W + px[k]] : 0ull;
-    }
-    // unrolled: the record and varyings gathers of the pixels overlap
+    for (int k = 0; k < kDirectPer; ++k) key[k] = g.x + 32 * k < g.xend ? keys[32 * k] : kmin ? 0ull : ~0ull;
+    float *const drow = s.depth_write ? reinterpret_cast<float *>(s.depth + (uint64_t)g.y * s.dpitch) : nullptr;
+    uint8_t *const prow = s.pixel_write ? s.pixel + (uint64_t)g.y * s.ppitch : nullptr;
+    const uint32_t pfmt = s.pfmt, words = s.prim == EUC_PRIM_TRIANGLE_LIST ? kRecShade : kRecAll;
+    const bool line = s.prim != EUC_PRIM_TRIANGLE_LIST;
+    const float *const vb = vdata + (s.geom ? s.gvd_base : s.vd_base);
+    const typename F::U &u = *reinterpret_cast<const typename F::U *>(s.uniforms);
+    const float yf = (float)g.y;
 #pragma unroll
     for (int k = 0; k < kDirectPer; ++k) {
         uint32_t t;
         float z;
-        if (py[k] == 0xFFFFFFFFu || !decode_key(s, key[k], t, z)) continue;
-        const uint32_t x = px[k], y = py[k];
-        if (s.depth_write) *reinterpret_cast<float *>(s.depth + (uint64_t)y * s.dpitch + 4ull * x) = z;
-        if (!s.pixel_write) continue;
+        if (!decode_key(kmin, greater, key[k], t, z)) continue;
+        const uint32_t x = g.x + 32 * k;
+        if (drow) drow[x] = z;
+        if (!prow) continue;
         if constexpr (F::kDirect) {
-            const typename F::U &u = *reinterpret_cast<const typename F::U *>(s.uniforms);
-            const float *vb = vdata + (s.geom ? s.gvd_base : s.vd_base);
-            const TriRec r = load_rec(recs + t, s.prim == EUC_PRIM_TRIANGLE_LIST ? kRecShade : kRecAll);
+            const TriRec r = load_rec(recs + t, words);
             float vd[F::NV], frag[F::NF];
-            vdata_at<F>(s, r, vb, (float)x, (float)y, vd);
+            vdata_at<F>(line, r, vb, (float)x, yf, vd);
             F::fragment(u, vd, frag);
-            store_pixel<F>(s, x, y, frag);
+            store_pixel<F>(prow, pfmt, x, frag);
         }
     }
 }
@@ -2251,7 +2275,9 @@ EUC_DEV void resolve_chunk(const SceneDev &s, const uint4 &cv, const ChunkGeom &
     const bool inside = chunk_pixel(s, cv, geo, lb, x, y, lo);
     uint32_t t = 0xFFFFFFFFu;
     float z = 0.0f;
-    const bool win = inside && decode_key(s, vbuf[s.pix_base + (uint64_t)y * s.W + x], t, z);
+    const bool line = s.prim != EUC_PRIM_TRIANGLE_LIST;
+    const bool win = inside && decode_key(s.keytype == KEY_MIN, s.depth_test == EUC_TEST_GREATER,
+                                          vbuf[s.pix_base + (uint64_t)y * s.W + x], t, z);
     if (win && s.depth_write) *reinterpret_cast<float *>(s.depth + (uint64_t)y * s.dpitch + 4ull * x) = z;
     if (!s.pixel_write) return;  // uniform over the block (one scene)
 
@@ -2315,7 +2341,7 @@ EUC_DEV void resolve_chunk(const SceneDev &s, const uint4 &cv, const ChunkGeom &
             yf = (float)(slo + ((((sy - slo) >> L) + (uint32_t)(c >> 1)) << L));
         }
         float vd[F::NV];
-        vdata_at<F>(s, r, vb, xf, yf, vd);
+        vdata_at<F>(line, r, vb, xf, yf, vd);
         F::fragment(u, vd, s_frag[slot][c]);
     }
     __syncwarp();
@@ -2341,7 +2367,7 @@ EUC_DEV void resolve_chunk(const SceneDev &s, const uint4 &cv, const ChunkGeom &
             frag[i] = a0 * (1.0f - fx) + a1 * fx;
         }
     }
-    store_pixel<F>(s, x, y, frag);
+    store_pixel<F>(s.pixel + (uint64_t)y * s.ppitch, s.pfmt, x, frag);
 }
 
 // Blocks walk groups of `group` chunks (grid-strided) of the scenes
@@ -2797,9 +2823,10 @@ __global__ void __launch_bounds__(kBlock) k_oscan(unsigned long long *__restrict
 template <class F>
 EUC_DEV void shade_at(const SceneDev &s, const typename F::U &u, const TriRec &r, const float *__restrict__ vb,
                       uint32_t x, uint32_t y, float *frag) {
+    const bool line = s.prim != EUC_PRIM_TRIANGLE_LIST;
     float vd[F::NV];
     if (s.level == 0) {
-        vdata_at<F>(s, r, vb, (float)x, (float)y, vd);
+        vdata_at<F>(line, r, vb, (float)x, (float)y, vd);
         F::fragment(u, vd, frag);
         return;
     }
@@ -2810,8 +2837,8 @@ EUC_DEV void shade_at(const SceneDev &s, const typename F::U &u, const TriRec &r
     float t[4][F::NF];
 #pragma unroll
     for (int c = 0; c < 4; ++c) {
-        vdata_at<F>(s, r, vb, (float)((px + (uint32_t)(c & 1)) << L), (float)(lo + ((py + (uint32_t)(c >> 1)) << L)),
-                    vd);
+        vdata_at<F>(line, r, vb, (float)((px + (uint32_t)(c & 1)) << L),
+                    (float)(lo + ((py + (uint32_t)(c >> 1)) << L)), vd);
         F::fragment(u, vd, t[c]);
     }
 #pragma unroll

@@ -400,3 +400,20 @@ def test_strip_units_of_every_size(strip_ctx, n, area):
     got, got_stats = run_gpu(strip_ctx, make())
     assert got_stats == ref_stats
     assert_targets_match(make(), ref, got)
+
+
+@pytest.mark.parametrize("fmt", [abi.FMT_RGBA8, abi.FMT_RGB8])
+@pytest.mark.parametrize("w,h", [(1, 1), (31, 7), (32, 8), (33, 9), (127, 3), (128, 16), (129, 17), (255, 5), (256, 8), (257, 9),
+                                 (700, 1)])
+def test_row_segments_at_their_edges(gpu_ctx, strip_ctx, w, h, fmt):
+    """Targets covered whole, at the edges of the 128- and 256-pixel row
+    segments of the resolve and the key seeds; the batch's kernels (strip_ctx
+    keeps off the small-scene path) and the frame's."""
+    def make():
+        f = _layers(5, w=w, h=h, blend=abi.BLEND_REPLACE, pixel_fmt=fmt)()
+        return f
+    ref, ref_stats = run_oracle(make())
+    for ctx in (gpu_ctx, strip_ctx):
+        got, got_stats = run_gpu(ctx, make())
+        assert got_stats == ref_stats
+        assert_targets_match(make(), ref, got)

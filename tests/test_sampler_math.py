@@ -101,3 +101,27 @@ def test_byte_table_equals_division(tmp_path):
 
 def test_wrap_fmod_equals_fmod(tmp_path):
     _run(tmp_path, "wrap_fmod", FMOD_SRC)
+
+
+BYTE_SRC = r"""
+#include <cstdio>
+#include <cstring>
+#include "euc_device.cuh"
+int main() {
+    volatile float div = 255.0f;  // a run-time division, not folded
+    int bad = 0;
+    for (unsigned i = 0; i < 256; ++i) {
+        const float q = (float)i / div, p = eucg::byte_over_255(i);
+        if (std::memcmp(&q, &p, 4)) {
+            std::printf("byte %u: %a, division %a\n", i, p, q);
+            ++bad;
+        }
+    }
+    std::printf("%d mismatches\n", bad);
+    return bad != 0;
+}
+"""
+
+
+def test_byte_over_255_equals_the_division(tmp_path):
+    _run(tmp_path, "byte_over_255", BYTE_SRC)
