@@ -1808,7 +1808,7 @@ int euc_render_host_batch(euc_ctx *ctx, const euc_scene *scenes, size_t n, int t
 // whole device.  An euc_ctx grows its scratch buffers on demand, so such a
 // caller cannot use euc_render.  This entry point takes the same inputs and
 // outputs but keeps all of its scratch in one fixed array of this file,
-// g_noalloc_scratch (kNaBytes, about 21.0 MiB).  Every GPU that loads this
+// g_noalloc_scratch (kNaBytes, about 20.0 MiB).  Every GPU that loads this
 // library holds that array until the process exits.
 //
 // Limits: at most kNaMaxVerts vertices, kNaMaxGroups primitive slots (one

@@ -130,9 +130,13 @@ struct SceneDev {
     float ndc_x, ndc_y;
 };
 
-// Per-primitive record written by k_setup (128 bytes, 16-byte aligned).
-// The fields are ordered so that a triangle's raster walk needs the first six
-// 16-byte words and its shading words 0-2 and 6 (load_rec).
+// Per-primitive record written by the setup (112 bytes, 16-byte aligned): a
+// raster walk needs its first six 16-byte words (load_rec), the shading of a
+// pixel words 0, 1 and 6 (load_shade; dy[2] is in both).  The stride of seven
+// words matters: neighbouring pixels' and rows' primitives differ, their loads
+// meet in L1, and at a stride of 128 bytes the same word of every primitive
+// lies in the same bank (256 spheres: k_resolve<GouraudFn> 203 -> 188 us,
+// with one word of four less).
 struct __align__(16) TriRec {
     float o[3];    // w_hom_origin   (triangles.rs:143)
     float dx[3];   // w_hom_dx       (triangles.rs:144)
@@ -142,12 +146,12 @@ struct __align__(16) TriRec {
     float vby[6];  // screen vertices ordered by y (triangles.rs:148-171)
     uint32_t scene;
     uint32_t flags;               // a triangle's kTri* bits or a line's kLine* bits
+    float dy2;                    // dy[2] again
     uint32_t v[3];                // vertex ids after the winding reversal
-    uint32_t pad[5];
 };
-static_assert(sizeof(TriRec) == 128, "TriRec must stay 128 bytes");
-static_assert(offsetof(TriRec, bx0) == 48 && offsetof(TriRec, scene) == 88 && offsetof(TriRec, v) == 96,
-              "load_rec reads the record by 16-byte words");
+static_assert(sizeof(TriRec) == 112, "seven 16-byte words");
+static_assert(offsetof(TriRec, bx0) == 48 && offsetof(TriRec, scene) == 88 && offsetof(TriRec, dy2) == 96,
+              "load_rec and load_shade read the record by 16-byte words");
 
 // The 16-byte words of record *p that `words` selects (bit k: word k) as a
 // local TriRec, one vector load each instead of a load per field: rows and
@@ -155,9 +159,9 @@ static_assert(offsetof(TriRec, bx0) == 48 && offsetof(TriRec, scene) == 88 && of
 // is their count.  Unselected fields are left unset.
 EUC_DEV TriRec load_rec(const TriRec *__restrict__ p, uint32_t words) {
     const uint4 *q = reinterpret_cast<const uint4 *>(p);
-    uint4 w[8];
+    uint4 w[6];
 #pragma unroll
-    for (int k = 0; k < 8; ++k) w[k] = (words >> k) & 1u ? __ldg(q + k) : make_uint4(0u, 0u, 0u, 0u);
+    for (int k = 0; k < 6; ++k) w[k] = (words >> k) & 1u ? __ldg(q + k) : make_uint4(0u, 0u, 0u, 0u);
     TriRec r;
     r.o[0] = __uint_as_float(w[0].x); r.o[1] = __uint_as_float(w[0].y); r.o[2] = __uint_as_float(w[0].z);
     r.dx[0] = __uint_as_float(w[0].w); r.dx[1] = __uint_as_float(w[1].x); r.dx[2] = __uint_as_float(w[1].y);
@@ -168,18 +172,31 @@ EUC_DEV TriRec load_rec(const TriRec *__restrict__ p, uint32_t words) {
     r.vby[2] = __uint_as_float(w[4].z); r.vby[3] = __uint_as_float(w[4].w);
     r.vby[4] = __uint_as_float(w[5].x); r.vby[5] = __uint_as_float(w[5].y);
     r.scene = w[5].z; r.flags = w[5].w;
-    r.v[0] = w[6].x; r.v[1] = w[6].y; r.v[2] = w[6].z; r.pad[0] = w[6].w;
-    r.pad[1] = w[7].x; r.pad[2] = w[7].y; r.pad[3] = w[7].z; r.pad[4] = w[7].w;
     return r;
 }
+
+// What the shading of a pixel needs of a record.
+struct ShadeRec {
+    float o[3], dx[3], dy[3];
+    uint32_t v[3];
+};
+EUC_DEV ShadeRec load_shade(const TriRec *__restrict__ p) {
+    const uint4 *q = reinterpret_cast<const uint4 *>(p);
+    const uint4 a = __ldg(q), b = __ldg(q + 1), c = __ldg(q + 6);
+    ShadeRec r;
+    r.o[0] = __uint_as_float(a.x); r.o[1] = __uint_as_float(a.y); r.o[2] = __uint_as_float(a.z);
+    r.dx[0] = __uint_as_float(a.w); r.dx[1] = __uint_as_float(b.x); r.dx[2] = __uint_as_float(b.y);
+    r.dy[0] = __uint_as_float(b.z); r.dy[1] = __uint_as_float(b.w); r.dy[2] = __uint_as_float(c.x);
+    r.v[0] = c.y; r.v[1] = c.z; r.v[2] = c.w;
+    return r;
+}
+constexpr int kRecWords = sizeof(TriRec) / 16;
+constexpr uint32_t kRecRaster = 0x3Fu;  // words 0-5: weights, z, bbox, vertices by y, scene, flags
 // Triangle flags (k_setup).
 constexpr uint32_t kTriNoClip = 1u;   // all vertices pass the z clip
 constexpr uint32_t kTriFullRows = 2u; // every row spans the whole bbox
 constexpr uint32_t kTriOneBand = 4u;  // every row lies in one band
 constexpr uint32_t kTriZPos = 8u;     // kTriNoClip and no vertex z has its sign bit set
-constexpr uint32_t kRecRaster = 0x3Fu;  // words 0-5: weights, z, bbox, vertices by y, scene, flags
-constexpr uint32_t kRecShade = 0x47u;   // words 0-2 and 6: weights, z, vertex ids
-constexpr uint32_t kRecAll = 0xFFu;
 
 struct SceneStats {
     unsigned long long culled;
@@ -428,10 +445,11 @@ __global__ void __launch_bounds__(kBlock) k_geometry(const SceneDev *__restrict_
 
 // ---------------------------------------------------------------------------
 // Lines (lines.rs:30-119).  A line record reuses TriRec's storage:
-//   o = {screen x0, screen y0, norm}, zc = {euclidean z0, z1},
-//   ln = {major start a1, minor start b1, |dmajor|, |dminor|, first step},
-//   bx0 / bx1 = the window's minor-axis range (inclusive), by0 = 0,
-//   by1 = steps in the window's major range, v = {vertex 0, vertex 1},
+//   o = {screen x0, screen y0, norm}, dx[0] = the bits of flags (for the
+//   shading), zc = {euclidean z0, z1}, vby = the bits of {major start a1, minor
+//   start b1, |dmajor|, |dminor|, first step}, bx0 / bx1 = the window's
+//   minor-axis range (inclusive), by0 = 0, by1 = steps in the window's major
+//   range, v = {vertex 0, vertex 1, vertex 1},
 //   flags: kLineUseX (frac along x), kLineXMajor, kLineNegMaj, kLineNegMin.
 // ---------------------------------------------------------------------------
 constexpr uint32_t kLineUseX = 4u, kLineXMajor = 8u, kLineNegMaj = 16u, kLineNegMin = 32u;
@@ -548,13 +566,13 @@ EUC_DEV void setup_line(const SceneDev &s, int si, uint64_t lt, uint64_t t, Clip
     r.zc[2] = 0.0f;
 #pragma unroll
     for (int k = 0; k < 3; ++k) r.dx[k] = r.dy[k] = 0.0f;
-#pragma unroll
-    for (int k = 0; k < 6; ++k) r.vby[k] = 0.0f;
-    r.pad[0] = (uint32_t)(int32_t)a1;
-    r.pad[1] = (uint32_t)(int32_t)b1;
-    r.pad[2] = (uint32_t)amaj;
-    r.pad[3] = (uint32_t)amin;
-    r.pad[4] = (uint32_t)i_lo;
+    r.dy2 = 0.0f;
+    r.vby[0] = __int_as_float((int32_t)a1);
+    r.vby[1] = __int_as_float((int32_t)b1);
+    r.vby[2] = __uint_as_float((uint32_t)amaj);
+    r.vby[3] = __uint_as_float((uint32_t)amin);
+    r.vby[4] = __uint_as_float((uint32_t)i_lo);
+    r.vby[5] = 0.0f;
     r.bx0 = (uint32_t)wb1;
     r.bx1 = (uint32_t)wb2;
     r.by0 = 0;
@@ -565,10 +583,11 @@ EUC_DEV void setup_line(const SceneDev &s, int si, uint64_t lt, uint64_t t, Clip
     r.scene = (uint32_t)si;
     r.flags = (use_x ? kLineUseX : 0u) | (xmaj ? kLineXMajor : 0u) | (dmaj < 0 ? kLineNegMaj : 0u) |
               (dmin < 0 ? kLineNegMin : 0u);
+    r.dx[0] = __uint_as_float(r.flags);
     const float4 *src = reinterpret_cast<const float4 *>(&r);
     float4 *dst = reinterpret_cast<float4 *>(recs + t);
 #pragma unroll
-    for (int k = 0; k < 8; ++k) dst[k] = src[k];
+    for (int k = 0; k < kRecWords; ++k) dst[k] = src[k];
     out.nrows = r.by1;
     out.cx0 = (uint32_t)wx1;
     out.cx1 = (uint32_t)wx2;
@@ -648,7 +667,7 @@ __host__ __device__ inline uint32_t width_bucket(uint32_t w) {
 // Primitive setup: triangles.rs:55-199, once per primitive (euc repeats it per
 // band; only the bbox clamp depends on the band and that is applied per row).
 // Primitive t of scene si, by one thread; clip_of(v) is vertex v's clip
-// position.  A triangle's record is staged in the warp's 4 KB (store_records);
+// position.  A triangle's record is staged by the warp (store_records);
 // bbox (null when the batch has no strips) receives the bbox of every triangle
 // with rows: the binning reads those 16 bytes instead of the record's line.
 // ---------------------------------------------------------------------------
@@ -805,8 +824,7 @@ EUC_DEV void setup_prim(const SceneDev &s, int si, uint64_t t, ClipOf clip_of, T
                                                       __float_as_uint(h[2][2])) >= 0;
                 r.flags = (noclip ? kTriNoClip : 0u) | (full_rows ? kTriFullRows : 0u) |
                           (one_band ? kTriOneBand : 0u) | (zpos ? kTriZPos : 0u);
-#pragma unroll
-                for (int k = 0; k < 5; ++k) r.pad[k] = 0;
+                r.dy2 = r.dy[2];
                 out.nrows = bx1 > bx0 ? by1 - by0 : 0u;
                 // NDC area |winding| / 2 is (W / 2) x (H / 2) pixels per unit
                 out.frag_est = fminf(fabsf(winding) * (size_x * size_y * 0.125f), (float)(bx1 - bx0) * (float)(by1 - by0));
@@ -835,7 +853,7 @@ EUC_DEV void setup_prim(const SceneDev &s, int si, uint64_t t, ClipOf clip_of, T
                     // keeps exactly those)
                     const uint4 *src = reinterpret_cast<const uint4 *>(&r);
 #pragma unroll
-                    for (int k = 0; k < 8; ++k) stage[lane * 8 + (k ^ (lane & 7))] = src[k];
+                    for (int k = 0; k < kRecWords; ++k) stage[lane * kRecWords + k] = src[k];
                     staged = true;
                     if (bbox) bbox[t] = make_uint4(bx0, bx1, by0, by1);  // the binning's copy
                     out.cx0 = bx0;
@@ -848,19 +866,19 @@ EUC_DEV void setup_prim(const SceneDev &s, int si, uint64_t t, ClipOf clip_of, T
     }
 }
 
-// The records a warp staged, out as 512-byte stores: 16-byte word k of lane
-// l's record sits at l * 8 + (k ^ (l & 7)), which keeps both the staging and
-// the copy-out at the minimum four wavefronts.  warp_recs: lane 0's record.
+// The records a warp staged, out as 512-byte stores (an odd stride of words:
+// no bank conflicts on either side).  warp_recs: lane 0's record.
 EUC_DEV void store_records(const uint4 *stage, bool staged, TriRec *__restrict__ warp_recs) {
-    const int lane = threadIdx.x & 31;
+    static_assert(kRecWords % 2 == 1, "an odd stride");
+    const uint32_t lane = threadIdx.x & 31;
     const uint32_t live = __ballot_sync(0xFFFFFFFFu, staged);
     __syncwarp();
     if (live) {
         uint4 *dst = reinterpret_cast<uint4 *>(warp_recs);
 #pragma unroll
-        for (int k = 0; k < 8; ++k) {
-            const int c = k * 32 + lane, owner = c >> 3;
-            if ((live >> owner) & 1u) dst[c] = stage[owner * 8 + ((c & 7) ^ (owner & 7))];
+        for (uint32_t k = 0; k < kRecWords; ++k) {
+            const uint32_t c = k * 32 + lane;
+            if ((live >> (c / kRecWords)) & 1u) dst[c] = stage[c];
         }
     }
 }
@@ -916,7 +934,7 @@ __global__ void __launch_bounds__(kBlock) k_setup(const SceneDev *__restrict__ s
                                                   int *__restrict__ err, SceneStats *__restrict__ stats,
                                                   uint4 *__restrict__ cov, const uint8_t *__restrict__ galive,
                                                   uint4 *__restrict__ bbox) {
-    __shared__ uint4 s_rec[kBlock / 32][32 * 8];
+    __shared__ uint4 s_rec[kBlock / 32][32 * kRecWords];
     uint4 *stage = s_rec[threadIdx.x >> 5];
     bool staged = false;
     const uint64_t t = (uint64_t)blockIdx.x * kBlock + threadIdx.x;
@@ -1151,12 +1169,12 @@ __global__ void __launch_bounds__(kBlock) k_init(const SceneDev *__restrict__ sc
 EUC_DEV void raster_line_step(const SceneDev &s, const TriRec &r, uint32_t t, uint32_t k,
                               unsigned long long *__restrict__ vbuf, uint32_t &cnt, int phase,
                               uint2 *__restrict__ frags, bool probe) {
-    const uint64_t i = (uint64_t)r.pad[4] + k;
-    const uint64_t amaj = r.pad[2], amin = r.pad[3];
+    const uint64_t i = (uint64_t)__float_as_uint(r.vby[4]) + k;
+    const uint64_t amaj = __float_as_uint(r.vby[2]), amin = __float_as_uint(r.vby[3]);
     // |dmajor|, |dminor| < 2^31: the numerator stays below 2^64
     const uint64_t m = amaj ? (2 * amin * i + amaj - 1) / (2 * amaj) : 0;
-    const long long a = (long long)(int32_t)r.pad[0] + ((r.flags & kLineNegMaj) ? -(long long)i : (long long)i);
-    const long long b = (long long)(int32_t)r.pad[1] + ((r.flags & kLineNegMin) ? -(long long)m : (long long)m);
+    const long long a = (long long)__float_as_int(r.vby[0]) + ((r.flags & kLineNegMaj) ? -(long long)i : (long long)i);
+    const long long b = (long long)__float_as_int(r.vby[1]) + ((r.flags & kLineNegMin) ? -(long long)m : (long long)m);
     if (b < (long long)r.bx0 || b > (long long)r.bx1) return;  // outside the window's minor range
     const uint32_t x = (uint32_t)((r.flags & kLineXMajor) ? a : b), y = (uint32_t)((r.flags & kLineXMajor) ? b : a);
     const float frac = ((r.flags & kLineUseX) ? (float)x - r.o[0] : (float)y - r.o[1]) * r.o[2];
@@ -1477,10 +1495,9 @@ __global__ void __launch_bounds__(kBlock, 4) k_raster(const SceneDev *__restrict
             const uint64_t i = i0 + lane;
             if (i >= nitems) continue;
             const uint32_t t = live_tri[l0 + a];
-            TriRec r = load_rec(recs + t, kRecRaster);
+            const TriRec r = load_rec(recs + t, kRecRaster);
             const uint32_t scene = r.scene;
             if (err[scene]) continue;
-            if (sc[scene].prim != EUC_PRIM_TRIANGLE_LIST) r = load_rec(recs + t, kRecAll);  // a line's walk state
             if (phase == 1 && sc[scene].keytype != KEY_ORDERED) continue;  // the fill pass is for ordered scenes
             uint32_t cnt = 0;
             raster_row(sc[scene], r, t, r.by0 + (uint32_t)(i - off[a]), vbuf, cnt, phase, frags, probe);
@@ -1765,7 +1782,6 @@ __global__ void __launch_bounds__(kStripThreads, kStripBlocksPerSm) k_strip(cons
     static_assert(2 * kStripThreads == kStripUnit && kStripMaxRows <= 255, "two entries per thread, rows in 8 bits");
     static_assert(kStripMaxRows < 32 && kStripClaim % 32 == 0 && kStripUnit <= 65536,
                   "one table slot per entry at most, claims start at a slot, entries in 16 bits");
-    static_assert(offsetof(TriRec, bx0) == 48, "k_strip reads the bbox width from 8-byte word 6 of a record");
     const int tid = threadIdx.x, lane = tid & 31;
     const uint32_t nstrips = (uint32_t)sbase[nsc];
     const uint32_t nunits = strip_uoff[nstrips], unit = strip_unit(totals[6], gridDim.x);
@@ -1918,7 +1934,7 @@ __global__ void __launch_bounds__(kStripThreads, kStripBlocksPerSm) k_strip(cons
 // k_resolve<F>: shade the winner of every pixel and write colour / depth.
 // ---------------------------------------------------------------------------
 template <class F>
-EUC_DEV void get_v_data(const TriRec &r, const float *__restrict__ vd0, const float *__restrict__ vd1,
+EUC_DEV void get_v_data(const ShadeRec &r, const float *__restrict__ vd0, const float *__restrict__ vd1,
                         const float *__restrict__ vd2, float xf, float yf, float *out) {  // triangles.rs:274-294
     float w[3];
 #pragma unroll
@@ -1933,13 +1949,13 @@ EUC_DEV void get_v_data(const TriRec &r, const float *__restrict__ vd0, const fl
 // The winner's vertex outputs at (xf, yf): get_v_data for a triangle,
 // weighted_sum2 of the two ends for a line (lines.rs:98-110).
 template <class F>
-EUC_DEV void vdata_at(bool line, const TriRec &r, const float *__restrict__ vb, float xf, float yf, float *out) {
+EUC_DEV void vdata_at(bool line, const ShadeRec &r, const float *__restrict__ vb, float xf, float yf, float *out) {
     constexpr int S = vd_stride(F::NV);
     float a0[S], a1[S];
     load_vd<F>(vb + (uint64_t)r.v[0] * S, a0);
     load_vd<F>(vb + (uint64_t)r.v[1] * S, a1);
     if (line) {
-        const float frac = ((r.flags & kLineUseX) ? xf - r.o[0] : yf - r.o[1]) * r.o[2];
+        const float frac = ((__float_as_uint(r.dx[0]) & kLineUseX) ? xf - r.o[0] : yf - r.o[1]) * r.o[2];
 #pragma unroll
         for (int i = 0; i < F::NV; ++i) out[i] = a0[i] * (1.0f - frac) + a1[i] * frac;
         return;
@@ -2199,7 +2215,7 @@ EUC_DEV void resolve_direct_chunk(const SceneDev &s, const uint4 &cv, uint64_t l
     for (int k = 0; k < kDirectPer; ++k) key[k] = g.x + 32 * k < g.xend ? keys[32 * k] : kmin ? 0ull : ~0ull;
     float *const drow = s.depth_write ? reinterpret_cast<float *>(s.depth + (uint64_t)g.y * s.dpitch) : nullptr;
     uint8_t *const prow = s.pixel_write ? s.pixel + (uint64_t)g.y * s.ppitch : nullptr;
-    const uint32_t pfmt = s.pfmt, words = s.prim == EUC_PRIM_TRIANGLE_LIST ? kRecShade : kRecAll;
+    const uint32_t pfmt = s.pfmt;
     const bool line = s.prim != EUC_PRIM_TRIANGLE_LIST;
     const float *const vb = vdata + (s.geom ? s.gvd_base : s.vd_base);
     const typename F::U &u = *reinterpret_cast<const typename F::U *>(s.uniforms);
@@ -2213,7 +2229,7 @@ EUC_DEV void resolve_direct_chunk(const SceneDev &s, const uint4 &cv, uint64_t l
         if (drow) drow[x] = z;
         if (!prow) continue;
         if constexpr (F::kDirect) {
-            const TriRec r = load_rec(recs + t, words);
+            const ShadeRec r = load_shade(recs + t);
             float vd[F::NV], frag[F::NF];
             vdata_at<F>(line, r, vb, (float)x, yf, vd);
             F::fragment(u, vd, frag);
@@ -2330,7 +2346,7 @@ EUC_DEV void resolve_chunk(const SceneDev &s, const uint4 &cv, const ChunkGeom &
     const uint32_t L = s.level;
     for (uint32_t j = lane; j < njobs; j += 32) {
         const int slot = s_job[j] >> 2, c = s_job[j] & 3;
-        const TriRec r = load_rec(recs + s_t[slot], s.prim == EUC_PRIM_TRIANGLE_LIST ? kRecShade : kRecAll);
+        const ShadeRec r = load_shade(recs + s_t[slot]);
         float xf, yf;
         if (L == 0) {
             xf = (float)s_xy[slot][0];
@@ -2469,7 +2485,7 @@ struct FrontArgs {
 
 template <class F>
 __global__ void __launch_bounds__(kBlock) k_front(const __grid_constant__ FrontArgs a) {
-    __shared__ uint4 s_rec[kBlock / 32][32 * 8];
+    __shared__ uint4 s_rec[kBlock / 32][32 * kRecWords];
     launch_next();  // k_frame_raster, which waits for this kernel before its first read
     const SceneDev &s = a.d;
     const typename F::U &u = *reinterpret_cast<const typename F::U *>(a.uni);
@@ -2600,7 +2616,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_frame_raster(const SceneDev *__re
         const uint32_t first = __shfl_sync(0xFFFFFFFFu, incl - nr, p);
         if (i >= __shfl_sync(0xFFFFFFFFu, incl, 31)) continue;
         const uint32_t t = g * 32 + p;
-        const TriRec r = load_rec(recs + t, s.prim == EUC_PRIM_TRIANGLE_LIST ? kRecRaster : kRecAll);
+        const TriRec r = load_rec(recs + t, kRecRaster);
         raster_row(s, r, t, r.by0 + (i - first), vbuf, cnt, 0, nullptr, probe);
     }
     const uint32_t sum = warp_sum(cnt);
@@ -2821,7 +2837,7 @@ __global__ void __launch_bounds__(kBlock) k_oscan(unsigned long long *__restrict
 
 // Fragment of primitive `r` at pixel (x, y): plain or coarse-grid MSAA.
 template <class F>
-EUC_DEV void shade_at(const SceneDev &s, const typename F::U &u, const TriRec &r, const float *__restrict__ vb,
+EUC_DEV void shade_at(const SceneDev &s, const typename F::U &u, const ShadeRec &r, const float *__restrict__ vb,
                       uint32_t x, uint32_t y, float *frag) {
     const bool line = s.prim != EUC_PRIM_TRIANGLE_LIST;
     float vd[F::NV];
@@ -2971,9 +2987,7 @@ __global__ void __launch_bounds__(kBlock, F::NV > 4 ? 2 : 3) k_resolve_ordered(c
         if (!s.pixel_write) continue;
         for (uint32_t k = 0; k < npass; ++k) {
             float frag[F::NF];
-            shade_at<F>(s, u, load_rec(recs + s_pass[k][threadIdx.x],
-                                       s.prim == EUC_PRIM_TRIANGLE_LIST ? kRecShade : kRecAll),
-                        vb, x, y, frag);
+            shade_at<F>(s, u, load_shade(recs + s_pass[k][threadIdx.x]), vb, x, y, frag);
             float c[4] = {frag[0], F::NF > 1 ? frag[F::NF > 1 ? 1 : 0] : 0.0f,
                           F::NF > 2 ? frag[F::NF > 2 ? 2 : 0] : 0.0f, F::NF > 3 ? frag[F::NF > 3 ? 3 : 0] : 0.0f};
             if (s.blend == EUC_BLEND_ALPHA) {  // src-over on the unpacked old pixel

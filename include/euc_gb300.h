@@ -416,7 +416,7 @@ int euc_sample_nearest(const void *texels, uint32_t ndim, const uint32_t *size, 
  * euc: it exists for callers that may not allocate device memory, such as an
  * engine or plugin host that owns a fixed device-memory budget, or a render
  * thread that cannot pay for cudaMalloc/cudaFree (both synchronise the whole
- * device).  Scratch lives in one fixed array inside the library (about 21.0
+ * device).  Scratch lives in one fixed array inside the library (about 20.0
  * MiB per device that loads it, held until exit).  Limits: 65,536 vertices,
  * 65,536 primitive slots (one per triangle, one per line, three per triangle
  * of a LineTriangleList), 1,048,576 target pixels; larger scenes return
