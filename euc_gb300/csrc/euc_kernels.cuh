@@ -208,13 +208,19 @@ struct SceneStats {
 // ---------------------------------------------------------------------------
 // Small helpers
 // ---------------------------------------------------------------------------
-EUC_DEV int find_scene(const uint64_t *base, int n, uint64_t pos) {
-    int lo = 0, hi = n;  // largest i with base[i] <= pos
-    while (hi - lo > 1) {
-        int mid = (lo + hi) >> 1;
-        if (base[mid] <= pos) lo = mid; else hi = mid;
+// The largest i < n with base[i] <= pos (base[0] <= pos), by the whole warp:
+// 32-way steps, so that 1024 scenes are two dependent loads away and not ten.
+EUC_DEV int find_scene(const uint64_t *__restrict__ base, int n, uint64_t pos) {
+    const int lane = threadIdx.x & 31;
+    int lo = 0, hi = n;
+    while (hi - lo > 32) {
+        const int step = (hi - lo + 31) / 32, at = lo + lane * step;
+        const bool le = at < hi && base[at] <= pos;
+        lo += (31 - __clz(__ballot_sync(0xFFFFFFFFu, le))) * step;  // lane 0 always qualifies
+        hi = min(lo + step, hi);
     }
-    return lo;
+    const bool le = lo + lane < hi && base[lo + lane] <= pos;
+    return lo + 31 - __clz(__ballot_sync(0xFFFFFFFFu, le));
 }
 
 // Order-preserving map of a non-NaN float onto uint32.
@@ -321,11 +327,8 @@ __global__ void __launch_bounds__(kBlock) k_vertex(const SceneDev *__restrict__ 
                                                    float *__restrict__ vdata, const PrepArgs prep) {
     for (uint64_t i = (uint64_t)blockIdx.x * kBlock + threadIdx.x; i < prep.n; i += (uint64_t)gridDim.x * kBlock)
         prep_clear(prep, i);
-    __shared__ int s_scene;
     const uint64_t pos = (blk_begin + blockIdx.x) * (uint64_t)kBlock;
-    if (threadIdx.x == 0) s_scene = s_begin + find_scene(vtx_base + s_begin, s_end - s_begin, pos);
-    __syncthreads();
-    const SceneDev &s = sc[s_scene];
+    const SceneDev &s = sc[s_begin + find_scene(vtx_base + s_begin, s_end - s_begin, pos)];
     const uint64_t v = pos + threadIdx.x - s.vtx_base;
     if (v >= s.nverts) return;
     const typename F::U &u = *reinterpret_cast<const typename F::U *>(s.uniforms);
@@ -395,11 +398,8 @@ __global__ void __launch_bounds__(kBlock) k_geometry(const SceneDev *__restrict_
                                                      int s_begin, int s_end, uint64_t blk_begin, float4 *__restrict__ clip,
                                                      float *__restrict__ vdata, uint8_t *__restrict__ galive,
                                                      int *__restrict__ err) {
-    __shared__ int s_scene;
     const uint64_t pos = (blk_begin + blockIdx.x) * (uint64_t)kBlock;
-    if (threadIdx.x == 0) s_scene = s_begin + find_scene(gin_base + s_begin, s_end - s_begin, pos);
-    __syncthreads();
-    const int si = s_scene;
+    const int si = s_begin + find_scene(gin_base + s_begin, s_end - s_begin, pos);
     const SceneDev &s = sc[si];
     const uint64_t g = pos + threadIdx.x - gin_base[si];
     if (g >= s.ngin) return;
@@ -1111,16 +1111,12 @@ EUC_DEV int advance_scene(const uint64_t *base, int nsc, int si, uint64_t c) {
 __global__ void __launch_bounds__(kBlock) k_init(const SceneDev *__restrict__ sc, const uint64_t *__restrict__ ibase,
                                                  int nsc, const uint4 *__restrict__ cov,
                                                  unsigned long long *__restrict__ vbuf, uint32_t group) {
-    __shared__ int s_scene;
     launch_next();  // k_bin, which reads nothing this kernel writes
     const uint64_t nchunks = ibase[nsc];
     for (uint64_t g = blockIdx.x; g * group < nchunks; g += gridDim.x) {
         const uint64_t c0 = g * group;
-        __syncthreads();
-        if (threadIdx.x == 0) s_scene = find_scene(ibase, nsc, c0);
-        __syncthreads();
         const uint64_t c1 = min(c0 + group, nchunks);
-        int si = s_scene;
+        int si = find_scene(ibase, nsc, c0);
         for (uint64_t c = c0; c < c1; ++si) {  // a scene's chunks of the group
             const uint64_t first = ibase[si], end = min(ibase[si + 1], c1);
             if (c >= end) continue;
@@ -2895,17 +2891,15 @@ __global__ void __launch_bounds__(kBlock, F::NV > 4 ? 2 : 3) k_resolve_ordered(c
                                                             const uint2 *__restrict__ frags, uint64_t frag_cap,
                                                             const unsigned long long *__restrict__ totals,
                                                             const uint4 *__restrict__ cov) {
-    __shared__ int s_scene;
     __shared__ uint32_t s_pass[kOWindow][kBlock];  // the passing primitives of each thread's window
     if (totals[4] > frag_cap) return;  // the lists were not filled: the host grows them and comes back
     const uint64_t blk = blk_begin + blockIdx.x;
-    if (threadIdx.x == 0) s_scene = s_begin + find_scene(res_base + s_begin, s_end - s_begin, blk);
-    __syncthreads();
-    const SceneDev &s = sc[s_scene];
-    const uint64_t q = (blk - res_base[s_scene]) * kBlock + threadIdx.x;
+    const int si = s_begin + find_scene(res_base + s_begin, s_end - s_begin, blk);
+    const SceneDev &s = sc[si];
+    const uint64_t q = (blk - res_base[si]) * kBlock + threadIdx.x;
     if (q >= (uint64_t)s.W * s.H) return;
     const uint32_t y = (uint32_t)q / s.W, x = (uint32_t)q - y * s.W;
-    if (!covered(cov[s_scene], x, y)) return;
+    if (!covered(cov[si], x, y)) return;
     const unsigned long long e = vbuf[s.pix_base + q];
     const uint2 *list = frags + (uint32_t)e;
     const uint32_t n = (uint32_t)(e >> 32);
