@@ -243,10 +243,18 @@ EUC_DEV unsigned long long init_key_min(float d0, bool greater) {
 
 // Programmatic dependent launch: a kernel launched with it in stream order
 // starts once every block of the kernel before it has called launch_next (or
-// ended), and calls wait_previous before it ends, so that what follows it in
-// the stream still comes after both.
+// ended).  begin_stage: the stage waits for the one before it (and so for
+// everything earlier), with its blocks already on the SMs that stage leaves
+// idle at its end, and lets the next stage come in the same way.  A stage that
+// needs nothing of the one before it (k_bin, k_strip) calls launch_next first
+// and wait_previous only before it ends: it runs beside that stage, everything
+// before which has ended, and what follows in the stream comes after both.
 EUC_DEV void launch_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 EUC_DEV void wait_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+EUC_DEV void begin_stage() {
+    wait_previous();
+    launch_next();
+}
 
 template <typename T>
 EUC_DEV T warp_incl_scan(T v) {
@@ -325,6 +333,7 @@ template <class F>
 __global__ void __launch_bounds__(kBlock) k_vertex(const SceneDev *__restrict__ sc, const uint64_t *__restrict__ vtx_base,
                                                    int s_begin, int s_end, uint64_t blk_begin, float4 *__restrict__ clip,
                                                    float *__restrict__ vdata, const PrepArgs prep) {
+    begin_stage();
     for (uint64_t i = (uint64_t)blockIdx.x * kBlock + threadIdx.x; i < prep.n; i += (uint64_t)gridDim.x * kBlock)
         prep_clear(prep, i);
     const uint64_t pos = (blk_begin + blockIdx.x) * (uint64_t)kBlock;
@@ -398,6 +407,7 @@ __global__ void __launch_bounds__(kBlock) k_geometry(const SceneDev *__restrict_
                                                      int s_begin, int s_end, uint64_t blk_begin, float4 *__restrict__ clip,
                                                      float *__restrict__ vdata, uint8_t *__restrict__ galive,
                                                      int *__restrict__ err) {
+    begin_stage();
     const uint64_t pos = (blk_begin + blockIdx.x) * (uint64_t)kBlock;
     const int si = s_begin + find_scene(gin_base + s_begin, s_end - s_begin, pos);
     const SceneDev &s = sc[si];
@@ -935,6 +945,7 @@ __global__ void __launch_bounds__(kBlock) k_setup(const SceneDev *__restrict__ s
                                                   uint4 *__restrict__ cov, const uint8_t *__restrict__ galive,
                                                   uint4 *__restrict__ bbox) {
     __shared__ uint4 s_rec[kBlock / 32][32 * kRecWords];
+    begin_stage();
     uint4 *stage = s_rec[threadIdx.x >> 5];
     bool staged = false;
     const uint64_t t = (uint64_t)blockIdx.x * kBlock + threadIdx.x;
@@ -1111,7 +1122,7 @@ EUC_DEV int advance_scene(const uint64_t *base, int nsc, int si, uint64_t c) {
 __global__ void __launch_bounds__(kBlock) k_init(const SceneDev *__restrict__ sc, const uint64_t *__restrict__ ibase,
                                                  int nsc, const uint4 *__restrict__ cov,
                                                  unsigned long long *__restrict__ vbuf, uint32_t group) {
-    launch_next();  // k_bin, which reads nothing this kernel writes
+    begin_stage();  // (k_bin, which reads nothing this kernel writes, runs beside it)
     const uint64_t nchunks = ibase[nsc];
     for (uint64_t g = blockIdx.x; g * group < nchunks; g += gridDim.x) {
         const uint64_t c0 = g * group;
@@ -1430,7 +1441,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_raster(const SceneDev *__restrict
                                                    uint2 *__restrict__ frags, uint64_t frag_cap, int witems,
                                                    bool probe) {
     __shared__ uint64_t s_off[kBlock / 32][kWarpItems];
-    launch_next();  // k_strip: its keys and this kernel's meet in order-free reductions
+    begin_stage();  // (k_strip runs beside it: their keys meet in order-free reductions)
     if (phase == 1 && totals[4] > frag_cap) return;  // the lists do not fit: the host grows them and comes back
     const int lane = threadIdx.x & 31;
     uint64_t *off = s_off[threadIdx.x >> 5];
@@ -1538,6 +1549,7 @@ __global__ void __launch_bounds__(kBlock) k_bin_count(const SceneDev *__restrict
                                                       unsigned long long *__restrict__ nentries, uint64_t entry_cap,
                                                       uint32_t strip_mode) {
     __shared__ uint32_t s_hist[kBinHist];
+    begin_stage();
     const int lane = threadIdx.x & 31;
     for (uint64_t c = blockIdx.x; c < nchunks; c += gridDim.x) {  // uniform over the block
         const int si = chunk_scene ? (int)chunk_scene[c] : 0;
@@ -1594,6 +1606,7 @@ __global__ void __launch_bounds__(kBlock) k_bin(const SceneDev *__restrict__ sc,
                                                 const uint32_t *__restrict__ strip_off, uint32_t *__restrict__ strip_fill,
                                                 uint2 *__restrict__ entries, uint32_t strip_mode) {
     __shared__ uint32_t s_cnt[kBinHist], s_base[kBinHist];
+    launch_next();
     for (uint64_t c = blockIdx.x; c < nchunks; c += gridDim.x) {  // uniform over the block
         const int si = chunk_scene ? (int)chunk_scene[c] : 0;
         const SceneDev &s = sc[si];
@@ -1778,6 +1791,7 @@ __global__ void __launch_bounds__(kStripThreads, kStripBlocksPerSm) k_strip(cons
     static_assert(2 * kStripThreads == kStripUnit && kStripMaxRows <= 255, "two entries per thread, rows in 8 bits");
     static_assert(kStripMaxRows < 32 && kStripClaim % 32 == 0 && kStripUnit <= 65536,
                   "one table slot per entry at most, claims start at a slot, entries in 16 bits");
+    launch_next();
     const int tid = threadIdx.x, lane = tid & 31;
     const uint32_t nstrips = (uint32_t)sbase[nsc];
     const uint32_t nunits = strip_uoff[nstrips], unit = strip_unit(totals[6], gridDim.x);
@@ -2164,6 +2178,7 @@ __global__ void __launch_bounds__(kBlock) k_scan_plan(const uint32_t *__restrict
                                                       uint32_t nstrips, uint32_t strip_blocks,
                                                       uint32_t *__restrict__ strip_off,
                                                       uint32_t *__restrict__ strip_uoff, uint32_t *__restrict__ unit_strip) {
+    begin_stage();
     if (blockIdx.x == nscan) plan_chunks(sc, nsc, cov, ibase, rbase);
     else if (blockIdx.x > nscan)
         strip_scan_block(blockIdx.x - nscan - 1, strip_cnt, nstrips, strip_unit(totals[6], strip_blocks), strip_off, strip_uoff, unit_strip);
@@ -2172,6 +2187,7 @@ __global__ void __launch_bounds__(kBlock) k_scan_plan(const uint32_t *__restrict
 
 // The clears of prep_clear as a launch of their own (n threads).
 __global__ void __launch_bounds__(kBlock) k_prep(const PrepArgs prep) {
+    begin_stage();
     const uint64_t i = (uint64_t)blockIdx.x * kBlock + threadIdx.x;
     if (i < prep.n) prep_clear(prep, i);
 }
@@ -2394,6 +2410,7 @@ __global__ void __launch_bounds__(kBlock, F::kResolveBlocks) k_resolve(const Sce
                                                     const uint4 *__restrict__ cov) {
     // warps work independently: each has its own job list and no block barrier
     __shared__ ResolveSmem<F> s_warp[kBlock / 32];
+    begin_stage();
     ResolveSmem<F> &sm = s_warp[threadIdx.x >> 5];
     const uint64_t *base = rbase + s_begin;
     const int n = s_end - s_begin;
@@ -2550,7 +2567,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_frame_raster(const SceneDev *__re
                                                            unsigned long long *__restrict__ vbuf, bool probe) {
     __shared__ uint32_t s_a[kBlock / 32 + 1];
     __shared__ __align__(16) uint32_t s_pref[kFrameGroups];
-    wait_previous();
+    begin_stage();
     const SceneDev &s = sc[0];
     const int lane = threadIdx.x & 31;
     const uint32_t ngroups = (s.ngroups + 31u) >> 5;
@@ -2800,6 +2817,7 @@ __global__ void __launch_bounds__(kBlock) k_oscan(unsigned long long *__restrict
                                                   volatile unsigned long long *__restrict__ host_total) {
     __shared__ unsigned long long s_a[kBlock / 32 + 1];
     __shared__ unsigned long long s_base;
+    begin_stage();
     static_assert(kOScanPer == 8 && kBlock % kOScanPer == 0, "four 16-byte words a thread, ranges in whole blocks");
     const uint64_t q0 = p0 + (uint64_t)blockIdx.x * kOScanBlock + (uint64_t)threadIdx.x * kOScanPer;
     const bool live = q0 < p1;  // p0 and p1 are multiples of kBlock
@@ -2892,6 +2910,7 @@ __global__ void __launch_bounds__(kBlock, F::NV > 4 ? 2 : 3) k_resolve_ordered(c
                                                             const unsigned long long *__restrict__ totals,
                                                             const uint4 *__restrict__ cov) {
     __shared__ uint32_t s_pass[kOWindow][kBlock];  // the passing primitives of each thread's window
+    begin_stage();
     if (totals[4] > frag_cap) return;  // the lists were not filled: the host grows them and comes back
     const uint64_t blk = blk_begin + blockIdx.x;
     const int si = s_begin + find_scene(res_base + s_begin, s_end - s_begin, blk);
