@@ -378,7 +378,7 @@ int raster_blocks_per_sm() {
     static int n = 0;
     if (n == 0) {
         int b = 0;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_raster, kBlock, 0) != cudaSuccess || b < 1) {
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_raster<RASTER_KEYS>, kBlock, 0) != cudaSuccess || b < 1) {
             (void)cudaGetLastError();
             b = 4;
         }
@@ -551,6 +551,36 @@ struct StageOverride {
     void *dev = nullptr;
     size_t need = 0;
 };
+
+// The ordered scenes' lists, their counts being in the entries [p0, p1) of
+// vbuf: the counts become list offsets (k_oscan), then `fill(cap)` enqueues the
+// second raster pass and `resolve(cap)` the resolves.  Both are enqueued
+// against the fragment buffer as it is (`cap` fragments), and do nothing when
+// the lists do not fit it; the host waits for the number of fragments alone
+// (while they run), and enqueues them again after growing the buffer.
+template <class Fill, class Resolve>
+int ordered_lists(euc_ctx *ctx, uint64_t p0, uint64_t p1, cudaStream_t st, Fill fill, Resolve resolve) {
+    int rc;
+    const uint64_t nb = (p1 - p0 + kOScanBlock - 1) / kOScanBlock;
+    if ((rc = ensure_host_words(ctx))) return rc;
+    if (!ctx->total_ready) CUDA_TRY(cudaEventCreateWithFlags(&ctx->total_ready, cudaEventDisableTiming));
+    // a first guess: four fragments a pixel, 512 MB at most
+    if ((rc = grow(ctx->frags, std::min<uint64_t>(4 * p1, 1ull << 26) * sizeof(uint2)))) return rc;
+    CUDA_TRY(launch_stage(ctx, k_oscan, (unsigned)nb, kBlock, 0, st, (unsigned long long *)ctx->vbuf.p, p0, p1,
+                          (unsigned long long *)ctx->totals.p, ctx->h_words));
+    CUDA_TRY(cudaEventRecord(ctx->total_ready, st));
+    ctx->launches += 1;
+    for (;;) {
+        const uint64_t cap = std::min<uint64_t>(ctx->frags.cap / sizeof(uint2), 0xFFFFFFFEull);
+        CUDA_TRY(fill(cap));
+        resolve(cap);
+        CUDA_TRY(cudaEventSynchronize(ctx->total_ready));
+        const unsigned long long nfrag = *(volatile unsigned long long *)ctx->h_words;
+        if (nfrag <= cap) return EUC_OK;
+        if (nfrag >= 0xFFFFFFFFull) return EUC_ERR_CAPACITY;  // list offsets are 32-bit
+        if ((rc = grow(ctx->frags, nfrag * sizeof(uint2)))) return rc;  // (waits for the passes above)
+    }
+}
 
 int run_batch(euc_ctx *ctx, const euc_scene *scenes, size_t n, cudaStream_t st, StageOverride *so = nullptr) {
     std::vector<Plan> plans;
@@ -795,12 +825,18 @@ int run_batch(euc_ctx *ctx, const euc_scene *scenes, size_t n, cudaStream_t st, 
         1, std::min<uint64_t>(busy, (uint64_t)ctx->nsm * (tu.raster_blocks_per_sm ? tu.raster_blocks_per_sm
                                                                                    : (uint32_t)ctx->raster_blocks)));
     const bool probe = tu.raster_probe == 1;
-    CUDA_TRY(launch_stage(ctx, k_raster, rgrid, kBlock, 0, st, dsc, (const TriRec *)ctx->recs.p,
-                          (const uint32_t *)ctx->live_tri.p, (const uint64_t *)ctx->live_rowoff.p,
-                          (unsigned long long *)ctx->totals.p, (const int *)ctx->err.p,
-                          (unsigned long long *)ctx->vbuf.p, (SceneStats *)ctx->stats.p, 0, nullptr, 0, witems,
-                          probe));
-    ctx->launches += 4;
+    int first_ordered = ns;
+    while (first_ordered > 0 && plans[first_ordered - 1].d.keytype == KEY_ORDERED) --first_ordered;
+    auto raster = [&](auto kernel, uint64_t cap) {
+        ctx->launches += 1;
+        return launch_stage(ctx, kernel, rgrid, kBlock, 0, st, dsc, (const TriRec *)ctx->recs.p,
+                            (const uint32_t *)ctx->live_tri.p, (const uint64_t *)ctx->live_rowoff.p,
+                            (unsigned long long *)ctx->totals.p, (const int *)ctx->err.p,
+                            (unsigned long long *)ctx->vbuf.p, (SceneStats *)ctx->stats.p, (uint2 *)ctx->frags.p, cap,
+                            witems, probe);
+    };
+    if (first_ordered > 0) CUDA_TRY(raster(k_raster<RASTER_KEYS>, 0));
+    ctx->launches += 3;
     // the strips, beside the item queue: k_raster's last warps walk long rows
     // with most of the GPU idle, and k_strip's blocks start there (48-scene
     // batch, a whole call: 578 us one after the other, 490 us with both)
@@ -813,46 +849,21 @@ int run_batch(euc_ctx *ctx, const euc_scene *scenes, size_t n, cudaStream_t st, 
                                (unsigned long long *)ctx->totals.p));
         ctx->launches += 1;
     }
-    // ordered scenes: the per-pixel counts become list offsets, then the lists
-    // are filled in a second raster pass and resolved.  Both passes are
-    // enqueued against the fragment buffer as it is, and do nothing when the
-    // lists do not fit it; the host waits for the number of fragments alone
-    // (while they run), and enqueues them again after growing the buffer.
-    int first_ordered = ns;
-    while (first_ordered > 0 && plans[first_ordered - 1].d.keytype == KEY_ORDERED) --first_ordered;
     if (first_ordered < ns) {
-        const uint64_t p0 = plans[first_ordered].d.pix_base, p1 = pix;
-        const uint64_t nb = (p1 - p0 + kOScanBlock - 1) / kOScanBlock;
-        if ((rc = ensure_host_words(ctx))) return rc;
-        if (!ctx->total_ready) CUDA_TRY(cudaEventCreateWithFlags(&ctx->total_ready, cudaEventDisableTiming));
-        // a first guess: four fragments a pixel, 512 MB at most
-        if ((rc = grow(ctx->frags, std::min<uint64_t>(4 * pix, 1ull << 26) * sizeof(uint2)))) return rc;
-        unsigned long long *totals = (unsigned long long *)ctx->totals.p;
-        CUDA_TRY(launch_stage(ctx, k_oscan, (unsigned)nb, kBlock, 0, st, (unsigned long long *)ctx->vbuf.p, p0, p1,
-                              totals, ctx->h_words));
-        CUDA_TRY(cudaEventRecord(ctx->total_ready, st));
-        ctx->launches += 1;
-        for (;;) {
-            const uint64_t cap = std::min<uint64_t>(ctx->frags.cap / sizeof(uint2), 0xFFFFFFFEull);
-            CUDA_TRY(launch_stage(ctx, k_raster, rgrid, kBlock, 0, st, dsc, (const TriRec *)ctx->recs.p,
-                                  (const uint32_t *)ctx->live_tri.p, (const uint64_t *)ctx->live_rowoff.p, totals,
-                                  (const int *)ctx->err.p, (unsigned long long *)ctx->vbuf.p,
-                                  (SceneStats *)ctx->stats.p, 1, (uint2 *)ctx->frags.p, cap, witems, probe));
-            ctx->launches += 1;
-            for (int a = first_ordered; a < ns;) {
-                int b = a;
-                while (b < ns && group_of(plans[b]) == group_of(plans[a])) ++b;
-                const uint64_t blk0 = res_base[a], blk1 = b < ns ? res_base[b] : res;
-                dispatch_resolve_ordered(plans[a].d.shader, dsc, drb, a, b, blk0, blk1 - blk0, cap, ctx, st);
-                ctx->launches += blk1 > blk0;
-                a = b;
-            }
-            CUDA_TRY(cudaEventSynchronize(ctx->total_ready));
-            const unsigned long long nfrag = *(volatile unsigned long long *)ctx->h_words;
-            if (nfrag <= cap) break;
-            if (nfrag >= 0xFFFFFFFFull) return EUC_ERR_CAPACITY;  // list offsets are 32-bit
-            if ((rc = grow(ctx->frags, nfrag * sizeof(uint2)))) return rc;  // (waits for the passes above)
-        }
+        CUDA_TRY(raster(k_raster<RASTER_COUNT>, 0));
+        rc = ordered_lists(
+            ctx, plans[first_ordered].d.pix_base, pix, st, [&](uint64_t cap) { return raster(k_raster<RASTER_FILL>, cap); },
+            [&](uint64_t cap) {
+                for (int a = first_ordered; a < ns;) {
+                    int b = a;
+                    while (b < ns && group_of(plans[b]) == group_of(plans[a])) ++b;
+                    const uint64_t blk0 = res_base[a], blk1 = b < ns ? res_base[b] : res;
+                    dispatch_resolve_ordered(plans[a].d.shader, dsc, drb, a, b, blk0, blk1 - blk0, cap, ctx, st);
+                    ctx->launches += blk1 > blk0;
+                    a = b;
+                }
+            });
+        if (rc) return rc;
     }
     cudaEvent_t e5 = prof_event(ctx, st);
     for (int a = 0; a < first_ordered;) {  // the ordered scenes are done
@@ -892,8 +903,7 @@ int run_batch(euc_ctx *ctx, const euc_scene *scenes, size_t n, cudaStream_t st, 
 constexpr uint64_t kFramePixels = 1ull << 20, kFrameVerts = 1ull << 16;
 
 bool frame_path(const euc_ctx *ctx, const Plan &p) {
-    return p.d.keytype != KEY_ORDERED && p.d.geom == EUC_GEOM_NONE && p.d.ngroups >= 1 && p.d.ngroups <= kFramePrims &&
-           p.d.nverts <= kFrameVerts && (uint64_t)p.d.W * p.d.H <= kFramePixels && ctx->tune.strip_path != 2 &&
+    return p.d.geom == EUC_GEOM_NONE && p.d.ngroups >= 1 && p.d.ngroups <= kFramePrims && p.d.nverts <= kFrameVerts && (uint64_t)p.d.W * p.d.H <= kFramePixels && ctx->tune.strip_path != 2 &&
            !ctx->profiling;
 }
 
@@ -909,6 +919,7 @@ int fill_front(euc_ctx *ctx, const Plan &p, FrontArgs &a) {
     if ((rc = grow(ctx->stats, sizeof(SceneStats)))) return rc;
     if ((rc = grow(ctx->cov, sizeof(uint4)))) return rc;
     if ((rc = grow(ctx->plan, 4 * sizeof(uint64_t)))) return rc;
+    if ((rc = grow(ctx->totals, 8 * sizeof(unsigned long long)))) return rc;
     if ((rc = grow(ctx->front, sizeof(FrontScratch)))) return rc;
     constexpr size_t off_u = (sizeof(SceneDev) + 15) / 16 * 16;
     static_assert(sizeof(euc_phong_uniforms) <= sizeof(FrontArgs::uni), "uniform copies hold any shader's struct");
@@ -952,13 +963,31 @@ int launch_frame(euc_ctx *ctx, const FrontArgs &a, cudaStream_t st, int *host_er
     const uint64_t items = (uint64_t)a.d.ngroups * ((uint64_t)std::max(a.d.W, a.d.H) + 2);
     const uint64_t busy = items / kBlock + a.nsb;
     const unsigned grid = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(busy, (uint64_t)ctx->nsm * ctx->raster_blocks));
-    CUDA_TRY(launch_beside(true, k_frame_raster, grid, kBlock, 0, st, (const SceneDev *)a.stage_scene,
-                           (const TriRec *)a.recs, (const uint32_t *)a.rows, (const FrontScratch *)a.front, a.nsb,
-                           (int *)ctx->err.p, host_err, (SceneStats *)ctx->stats.p, (uint4 *)ctx->cov.p,
-                           (uint64_t *)ctx->plan.p, a.vbuf, ctx->tune.raster_probe == 1));
-    dispatch_resolve(a.d.shader, a.stage_scene, (uint64_t *)ctx->plan.p, 0, 1, resolve_blocks(a.d), ctx, st);
+    const SceneDev *const sc = a.stage_scene;
+    auto raster = [&](auto kernel, bool beside, uint64_t cap) {
+        ctx->launches += 1;
+        return launch_beside(beside, kernel, grid, kBlock, 0, st, sc, (const TriRec *)a.recs, (const uint32_t *)a.rows,
+                             (const FrontScratch *)a.front, a.nsb, (int *)ctx->err.p, host_err,
+                             (SceneStats *)ctx->stats.p, (uint4 *)ctx->cov.p, (uint64_t *)ctx->plan.p, a.vbuf,
+                             (unsigned long long *)ctx->totals.p, (uint2 *)ctx->frags.p, cap,
+                             ctx->tune.raster_probe == 1);
+    };
+    const uint64_t nblk = resolve_blocks(a.d);
+    ctx->launches += 2;
+    if (a.d.keytype == KEY_ORDERED) {
+        CUDA_TRY(raster(k_frame_raster<RASTER_COUNT>, true, 0));
+        const uint64_t pix = pad_up((uint64_t)a.d.W * a.d.H, kBlock);
+        int rc = ordered_lists(
+            ctx, 0, pix, st, [&](uint64_t cap) { return raster(k_frame_raster<RASTER_FILL>, true, cap); },
+            [&](uint64_t cap) {
+                dispatch_resolve_ordered(a.d.shader, sc, (uint64_t *)ctx->plan.p, 0, 1, 0, nblk, cap, ctx, st);
+            });
+        if (rc) return rc;
+    } else {
+        CUDA_TRY(raster(k_frame_raster<RASTER_KEYS>, true, 0));
+        dispatch_resolve(a.d.shader, sc, (uint64_t *)ctx->plan.p, 0, 1, nblk, ctx, st);
+    }
     CUDA_TRY(cudaGetLastError());
-    ctx->launches += 3;
     return EUC_OK;
 }
 
@@ -1368,7 +1397,9 @@ ShapeGraph *shape_record(euc_ctx *ctx, const euc_scene &s, const Plan &p, std::v
 int render_one(euc_ctx *ctx, const euc_scene &s, cudaStream_t st) {
     Plan p;
     if (int rc = plan_scene(s, p)) return rc;
-    if (ctx->profiling || p.skip || p.d.keytype == KEY_ORDERED) return run_batch(ctx, &s, 1, st);
+    if (ctx->profiling || p.skip) return run_batch(ctx, &s, 1, st);
+    if (p.d.keytype == KEY_ORDERED)  // (waits for a fragment count: not recorded)
+        return frame_path(ctx, p) ? run_frame(ctx, p, st) : run_batch(ctx, &s, 1, st);
     std::vector<unsigned char> key = shape_key(ctx, p);
     ShapeGraph *g = nullptr;
     size_t at = 0;
@@ -2065,10 +2096,10 @@ extern "C" int euc_render_noalloc(const euc_pipeline_desc *desc, const void *uni
     k_init<<<chunk_grid(ichunks, nsm), kBlock, 0, st>>>(dsc, ibase, 1, (const uint4 *)(a + kNaOffCov),
                                                          (unsigned long long *)(a + kNaOffVbuf),
                                                          chunk_group(ichunks, nsm));
-    k_raster<<<(unsigned)(nsm * raster_blocks_per_sm()), kBlock, 0, st>>>(
+    k_raster<RASTER_KEYS><<<(unsigned)(nsm * raster_blocks_per_sm()), kBlock, 0, st>>>(
         dsc, (const TriRec *)(a + kNaOffRecs), (const uint32_t *)(a + kNaOffLiveTri), (const uint64_t *)(a + kNaOffLiveOff),
         (unsigned long long *)(a + kNaOffTotals), (const int *)(a + kNaOffErr),
-        (unsigned long long *)(a + kNaOffVbuf), (SceneStats *)(a + kNaOffStats), 0, nullptr, 0, kWarpItems, false);
+        (unsigned long long *)(a + kNaOffVbuf), (SceneStats *)(a + kNaOffStats), nullptr, 0, kWarpItems, false);
     na_dispatch(false, d.shader, dsc, rbase, resolve_blocks(d), a, st);
     if (device_status)
         CUDA_TRY(cudaMemcpyAsync(device_status, a + kNaOffErr, sizeof(int), cudaMemcpyDeviceToDevice, st));

@@ -1031,8 +1031,8 @@ EUC_DEV void scan_block(const uint32_t *__restrict__ rows, const uint2 *__restri
     if (blockIdx.x == nscan - 1 && threadIdx.x == kBlock - 1) {
         totals[0] = base_l + bl;
         totals[1] = base_r + br;
-        totals[2] = 0;  // work counter of k_raster, phase 0
-        totals[3] = 0;  // work counter of k_raster, phase 1 (ordered scenes)
+        totals[2] = 0;  // work counter of k_raster<RASTER_KEYS>
+        totals[3] = 0;  // ... of RASTER_COUNT, and of RASTER_FILL (k_oscan clears it in between)
         totals[4] = totals[5] = 0;  // k_oscan: fragments, finished blocks
     }
 }
@@ -1171,11 +1171,17 @@ __global__ void __launch_bounds__(kBlock) k_init(const SceneDev *__restrict__ sc
 // ---------------------------------------------------------------------------
 // k_raster: one (primitive, row) at a time per thread, warp-scheduled.
 // ---------------------------------------------------------------------------
+// What a raster launch does: the keys of the scenes that have them, the ordered
+// scenes' candidate counts (low word of each pixel's entry), or their lists
+// ((primitive, z) at offset, low word, + cursor, high word).
+enum RasterMode : int { RASTER_KEYS = 0, RASTER_COUNT = 1, RASTER_FILL = 2 };
+
 // Step k (in the window's major range) of line t: its pixel, then the same
 // candidate handling as a triangle's pixel (lines.rs:79-97).
+template <int kMode>
 EUC_DEV void raster_line_step(const SceneDev &s, const TriRec &r, uint32_t t, uint32_t k,
-                              unsigned long long *__restrict__ vbuf, uint32_t &cnt, int phase,
-                              uint2 *__restrict__ frags, bool probe) {
+                              unsigned long long *__restrict__ vbuf, uint32_t &cnt, uint2 *__restrict__ frags,
+                              bool probe) {
     const uint64_t i = (uint64_t)__float_as_uint(r.vby[4]) + k;
     const uint64_t amaj = __float_as_uint(r.vby[2]), amin = __float_as_uint(r.vby[3]);
     // |dmajor|, |dminor| < 2^31: the numerator stays below 2^64
@@ -1188,15 +1194,14 @@ EUC_DEV void raster_line_step(const SceneDev &s, const TriRec &r, uint32_t t, ui
     const float z = r.zc[0] + frac * (r.zc[1] - r.zc[0]);
     if (s.zclip && !(s.zmin <= z && z <= s.zmax)) return;  // CoordinateMode::passes_z_clip
     unsigned long long *key = vbuf + s.pix_base + (uint64_t)y * s.W + x;
-    if (s.keytype == KEY_ORDERED) {
-        unsigned int *e = reinterpret_cast<unsigned int *>(key);
-        if (phase == 0) {
-            ++cnt;
-            atomicAdd(e, 1u);
-        } else {
-            const unsigned long long old = atomicAdd(key, 1ull << 32);  // offset | cursor
-            frags[(uint32_t)old + (uint32_t)(old >> 32)] = make_uint2(t, __float_as_uint(z));
-        }
+    if constexpr (kMode == RASTER_COUNT) {
+        ++cnt;
+        atomicAdd(reinterpret_cast<unsigned int *>(key), 1u);
+        return;
+    }
+    if constexpr (kMode == RASTER_FILL) {
+        const unsigned long long old = atomicAdd(key, 1ull << 32);  // offset | cursor
+        frags[(uint32_t)old + (uint32_t)(old >> 32)] = make_uint2(t, __float_as_uint(z));
         return;
     }
     ++cnt;
@@ -1232,10 +1237,10 @@ EUC_DEV uint32_t zpos_order(float z) { return __float_as_uint(z) | 0x80000000u; 
 
 // The pixel span [xs, xe) of row y of triangle r: the whole band-clamped
 // bbox row when the extent is below 128, else the edge intersections
-// (triangles.rs:219-253).  False when it is empty.
-EUC_DEV bool row_span(const SceneDev &s, const TriRec &r, uint32_t y, uint32_t &xs, uint32_t &xe) {
+// (triangles.rs:219-253; `full`: which).  False when it is empty.
+EUC_DEV bool row_span(const SceneDev &s, const TriRec &r, uint32_t y, uint32_t &xs, uint32_t &xe, bool &full) {
     const float yf = (float)y;
-    bool full = r.flags & kTriFullRows;  // one band, extent < 128 (k_setup)
+    full = r.flags & kTriFullRows;  // one band, extent < 128 (k_setup)
     if (!full && !(r.flags & kTriOneBand)) {  // rows in several bands
         // band of this row and the band-clamped bbox (pipeline.rs:341-360, triangles.rs:114-139)
         const uint32_t lo = (y / s.gr) * s.gr;
@@ -1263,15 +1268,16 @@ EUC_DEV bool row_span(const SceneDev &s, const TriRec &r, uint32_t y, uint32_t &
     return xs < xe;
 }
 
+template <int kMode>
 EUC_DEV void raster_row(const SceneDev &s, const TriRec &r, uint32_t t, uint32_t y,
-                        unsigned long long *__restrict__ vbuf, uint32_t &cnt, int phase, uint2 *__restrict__ frags,
-                        bool probe) {
+                        unsigned long long *__restrict__ vbuf, uint32_t &cnt, uint2 *__restrict__ frags, bool probe) {
     if (s.prim != EUC_PRIM_TRIANGLE_LIST) {  // lines: `y` is the step within the window
-        raster_line_step(s, r, t, y, vbuf, cnt, phase, frags, probe);
+        raster_line_step<kMode>(s, r, t, y, vbuf, cnt, frags, probe);
         return;
     }
     uint32_t xs, xe;
-    if (!row_span(s, r, y, xs, xe)) return;
+    bool full;
+    if (!row_span(s, r, y, xs, xe, full)) return;
     // row-start weights, then the serial walk (triangles.rs:257-301)
     const float yf = (float)y;
     const float xsf = (float)xs;
@@ -1286,7 +1292,7 @@ EUC_DEV void raster_row(const SceneDev &s, const TriRec &r, uint32_t t, uint32_t
     const bool kmin = s.keytype == KEY_MIN, greater = s.depth_test == EUC_TEST_GREATER;
     const uint32_t tmin = (t + 1u) << 1;
     const unsigned long long tlast = (unsigned long long)(~t) << 32;
-    if (kmin && !probe) {
+    if (kMode == RASTER_KEYS && kmin && !probe) {
         // Less / Greater with depth writes, fire-and-forget reductions: each
         // candidate is keyed and reduced where the walk finds it
         if (!greater && (r.flags & kTriZPos)) {
@@ -1326,11 +1332,51 @@ EUC_DEV void raster_row(const SceneDev &s, const TriRec &r, uint32_t t, uint32_t
         }
         return;
     }
+    // The ordered passes between two edges, where nearly every pixel is a
+    // candidate: no branch, the others add 0.  (A branch around an atomic costs
+    // the walk some 45 cycles a pixel.  Kept off the keys, whose launches are
+    // not bound by their longest rows: 256 spheres 606 us against 614.)
+    if (kMode == RASTER_COUNT && noclip && !full) {
+#pragma unroll 4
+        for (uint32_t x = xs; x < xe; ++x) {
+            const float wu2 = (w2 - w0) - w1;
+            const uint32_t in = (w0 >= 0.0f) & (w1 >= 0.0f) & (wu2 >= 0.0f) ? 1u : 0u;
+            cnt += in;
+            atomicAdd(reinterpret_cast<unsigned int *>(row_keys + x), in);
+            w0 = w0 + d0;
+            w1 = w1 + d1;
+            w2 = w2 + d2;
+        }
+        return;
+    }
+    if (kMode == RASTER_FILL && noclip && !full) {
+        // eight cursors in flight; a pixel that is no candidate moves none
+        constexpr int kFill = 8;
+        for (uint32_t x = xs; x < xe; x += kFill) {
+            unsigned long long e[kFill];
+            float zz[kFill];
+            bool in[kFill];
+#pragma unroll
+            for (int k = 0; k < kFill; ++k) {
+                const float wu2 = (w2 - w0) - w1;
+                in[k] = (w0 >= 0.0f) & (w1 >= 0.0f) & (wu2 >= 0.0f) & (x + k < xe);
+                zz[k] = (z0 * w0 + z1 * w1) + z2 * wu2;
+                e[k] = atomicAdd(row_keys + min(x + k, xe - 1u), in[k] ? 1ull << 32 : 0ull);
+                w0 = w0 + d0;
+                w1 = w1 + d1;
+                w2 = w2 + d2;
+            }
+#pragma unroll
+            for (int k = 0; k < kFill; ++k)
+                if (in[k]) frags[(uint32_t)e[k] + (uint32_t)(e[k] >> 32)] = make_uint2(t, __float_as_uint(zz[k]));
+        }
+        return;
+    }
     // The walk advances pixel by pixel exactly as euc's loop does; candidates
-    // are gathered kWalk at a time so that their key loads are in flight
-    // together instead of one L2 round trip per pixel.
-    constexpr int kWalk = 4;
-    static_assert(kWalk == 4, "the empty-group test below names four candidates");
+    // are gathered kWalk at a time so that their key loads (eight cursors in
+    // the fill pass: 56 -> 45 us for 960x540 and 2.2 M fragments) are in
+    // flight together instead of one L2 round trip per pixel.
+    constexpr int kWalk = kMode == RASTER_FILL ? 8 : 4;
     for (uint32_t x = xs; x < xe; x += kWalk) {
         float zz[kWalk];
         bool cand[kWalk];
@@ -1354,28 +1400,28 @@ EUC_DEV void raster_row(const SceneDev &s, const TriRec &r, uint32_t t, uint32_t
         }
         // most groups of a full-bbox row (extent < 128) hold no candidate:
         // only the weight additions above are needed there
-        if (!(cand[0] | cand[1] | cand[2] | cand[3])) continue;
-        if (s.keytype == KEY_ORDERED) {
-            // phase 0 counts each pixel's candidates (low word of its entry);
-            // phase 1 appends (primitive, z) at offset (low word, set by the
-            // pixel scan) + cursor (high word): one 64-bit atomic returns both,
-            // and the group's are all in flight before the first store
-            if (phase == 0) {
+        bool any = false;
 #pragma unroll
-                for (int k = 0; k < kWalk; ++k) {
-                    if (!cand[k]) continue;
-                    ++cnt;
-                    atomicAdd(reinterpret_cast<unsigned int *>(row_keys + x + k), 1u);
-                }
-            } else {
-                unsigned long long e[kWalk];
+        for (int k = 0; k < kWalk; ++k) any |= cand[k];
+        if (!any) continue;
+        if constexpr (kMode == RASTER_COUNT) {
 #pragma unroll
-                for (int k = 0; k < kWalk; ++k)
-                    e[k] = cand[k] ? atomicAdd(row_keys + x + k, 1ull << 32) : 0ull;
-#pragma unroll
-                for (int k = 0; k < kWalk; ++k)
-                    if (cand[k]) frags[(uint32_t)e[k] + (uint32_t)(e[k] >> 32)] = make_uint2(t, __float_as_uint(zz[k]));
+            for (int k = 0; k < kWalk; ++k) {
+                if (!cand[k]) continue;
+                ++cnt;
+                atomicAdd(reinterpret_cast<unsigned int *>(row_keys + x + k), 1u);
             }
+            continue;
+        }
+        if constexpr (kMode == RASTER_FILL) {
+            // one 64-bit atomic returns offset and cursor, and the group's are
+            // all in flight before the first store
+            unsigned long long e[kWalk];
+#pragma unroll
+            for (int k = 0; k < kWalk; ++k) e[k] = cand[k] ? atomicAdd(row_keys + x + k, 1ull << 32) : 0ull;
+#pragma unroll
+            for (int k = 0; k < kWalk; ++k)
+                if (cand[k]) frags[(uint32_t)e[k] + (uint32_t)(e[k] >> 32)] = make_uint2(t, __float_as_uint(zz[k]));
             continue;
         }
         unsigned long long key[kWalk];
@@ -1432,17 +1478,18 @@ EUC_DEV void raster_row(const SceneDev &s, const TriRec &r, uint32_t t, uint32_t
 // kWarpItems (a launch-shape choice; results do not depend on it).
 constexpr int kWarpItems = 256;
 
+template <int kMode>
 __global__ void __launch_bounds__(kBlock, 4) k_raster(const SceneDev *__restrict__ sc, const TriRec *__restrict__ recs,
                                                    const uint32_t *__restrict__ live_tri,
                                                    const uint64_t *__restrict__ live_rowoff,
                                                    unsigned long long *__restrict__ totals,
                                                    const int *__restrict__ err, unsigned long long *__restrict__ vbuf,
-                                                   SceneStats *__restrict__ stats, int phase,
-                                                   uint2 *__restrict__ frags, uint64_t frag_cap, int witems,
-                                                   bool probe) {
+                                                   SceneStats *__restrict__ stats, uint2 *__restrict__ frags,
+                                                   uint64_t frag_cap, int witems, bool probe) {
+    constexpr int kCounter = kMode == RASTER_KEYS ? 2 : 3;  // the launch's work counter in totals
     __shared__ uint64_t s_off[kBlock / 32][kWarpItems];
     begin_stage();  // (k_strip runs beside it: their keys meet in order-free reductions)
-    if (phase == 1 && totals[4] > frag_cap) return;  // the lists do not fit: the host grows them and comes back
+    if (kMode == RASTER_FILL && totals[4] > frag_cap) return;  // the lists do not fit: the host grows them and comes back
     const int lane = threadIdx.x & 31;
     uint64_t *off = s_off[threadIdx.x >> 5];
     const uint64_t nlive = totals[0], nitems = totals[1];
@@ -1460,7 +1507,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_raster(const SceneDev *__restrict
     if (gwarp * witems >= nitems) return;
     for (;;) {
         unsigned long long base = 0;
-        if (lane == 0) base = atomicAdd(totals + 2 + phase, (unsigned long long)witems);
+        if (lane == 0) base = atomicAdd(totals + kCounter, (unsigned long long)witems);
         base = __shfl_sync(0xFFFFFFFFu, base, 0);
         if (base >= nitems) break;
         // largest l with live_rowoff[l] <= base; invariant off(lo) <= base < off(hi)
@@ -1505,9 +1552,9 @@ __global__ void __launch_bounds__(kBlock, 4) k_raster(const SceneDev *__restrict
             const TriRec r = load_rec(recs + t, kRecRaster);
             const uint32_t scene = r.scene;
             if (err[scene]) continue;
-            if (phase == 1 && sc[scene].keytype != KEY_ORDERED) continue;  // the fill pass is for ordered scenes
+            if ((sc[scene].keytype == KEY_ORDERED) != (kMode != RASTER_KEYS)) continue;  // another launch's scene
             uint32_t cnt = 0;
-            raster_row(sc[scene], r, t, r.by0 + (uint32_t)(i - off[a]), vbuf, cnt, phase, frags, probe);
+            raster_row<kMode>(sc[scene], r, t, r.by0 + (uint32_t)(i - off[a]), vbuf, cnt, frags, probe);
             if (scene0 == 0xFFFFFFFFu) scene0 = scene;
             if (scene == scene0) cnt0 += cnt;
             else if (cnt) atomicAdd(&stats[scene].candidates, (unsigned long long)cnt);
@@ -1842,7 +1889,8 @@ __global__ void __launch_bounds__(kStripThreads, kStripBlocksPerSm) k_strip(cons
                 uint32_t xs = rs.bx0, xe = rs.bx1;
                 if (!(rs.flags & kTriFullRows)) {
                     const uint32_t ya = ev[h].y >> 16, yb = ev[h].y & 0xFFFFu;
-                    if (!row_span(s, rs, s0 + ((ya + yb) >> 1), xs, xe)) xe = xs;
+                    bool full;
+                    if (!row_span(s, rs, s0 + ((ya + yb) >> 1), xs, xe, full)) xe = xs;
                 }
                 bk[h] = kWidthBuckets - 1u - width_bucket(xe - xs);  // widest first
             }
@@ -1908,7 +1956,8 @@ __global__ void __launch_bounds__(kStripThreads, kStripBlocksPerSm) k_strip(cons
                     const uint32_t y = s0 + s_ya[a] + (i - s_pref[a]);
                     const TriRec r = load_rec(recs + t, kRecRaster);
                     uint32_t xs, xe;
-                    if (!row_span(s, r, y, xs, xe)) continue;
+                    bool full;
+                    if (!row_span(s, r, y, xs, xe, full)) continue;
                     strip_walk_row(s, r, t, y, xs, xe, keys_saddr + 8u * ((y - r0) * pitch) - 8u * cx0, cnt);
                 }
             }
@@ -2448,8 +2497,9 @@ __global__ void __launch_bounds__(kBlock, F::kResolveBlocks) k_resolve(const Sce
 
 // ---------------------------------------------------------------------------
 // The frame path: one small scene (at most kFramePrims primitive slots, no
-// geometry stage, no ordered blend) in three launches instead of seven.  Such a
-// scene is bound by the latency of its dependent launches, not by their work,
+// geometry stage) in three launches instead of seven (an ordered blend's two
+// raster passes, scan and resolve in five instead of eight).  Such a scene is
+// bound by the latency of its dependent launches, not by their work,
 // so the stages that need nothing of each other share one:
 //   k_front<F>      the scene's table and uniforms (its parameter) out to the
 //                   staging that the next two read; the setup of 256
@@ -2536,6 +2586,13 @@ __global__ void __launch_bounds__(kBlock) k_front(const __grid_constant__ FrontA
         }
     } else if (b < a.nsb + a.nib) {
         const uint32_t area = s.W * s.H, i0 = (b - a.nsb) * kInitChunk + threadIdx.x;
+        if (s.keytype == KEY_ORDERED) {  // no fragment yet, cursor 0; the padding too (k_oscan sums it)
+            const uint32_t lim = (area + kBlock - 1) / kBlock * kBlock;
+#pragma unroll
+            for (int k = 0; k < kInitPer; ++k)
+                if (i0 + k * kBlock < lim) a.vbuf[i0 + k * kBlock] = 0ull;
+            return;
+        }
         RectWalk rk(i0, s.W);
         float d[kInitPer];
 #pragma unroll
@@ -2557,6 +2614,7 @@ __global__ void __launch_bounds__(kBlock) k_front(const __grid_constant__ FrontA
     }
 }
 
+template <int kMode>
 __global__ void __launch_bounds__(kBlock, 4) k_frame_raster(const SceneDev *__restrict__ sc,
                                                            const TriRec *__restrict__ recs,
                                                            const uint32_t *__restrict__ rows,
@@ -2564,10 +2622,13 @@ __global__ void __launch_bounds__(kBlock, 4) k_frame_raster(const SceneDev *__re
                                                            int *__restrict__ err, volatile int *__restrict__ host_err,
                                                            SceneStats *__restrict__ stats, uint4 *__restrict__ cov,
                                                            uint64_t *__restrict__ rbase,
-                                                           unsigned long long *__restrict__ vbuf, bool probe) {
+                                                           unsigned long long *__restrict__ vbuf,
+                                                           unsigned long long *__restrict__ totals,
+                                                           uint2 *__restrict__ frags, uint64_t frag_cap, bool probe) {
     __shared__ uint32_t s_a[kBlock / 32 + 1];
     __shared__ __align__(16) uint32_t s_pref[kFrameGroups];
     begin_stage();
+    if (kMode == RASTER_FILL && totals[4] > frag_cap) return;  // the lists do not fit: the host grows them
     const SceneDev &s = sc[0];
     const int lane = threadIdx.x & 31;
     const uint32_t ngroups = (s.ngroups + 31u) >> 5;
@@ -2578,7 +2639,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_frame_raster(const SceneDev *__re
 #pragma unroll
     for (uint32_t k = 0; k < 4; ++k) steps[k] = 4 * threadIdx.x + k < ngroups ? (steps[k] + 31u) >> 5 : 0u;
     const int bad = __syncthreads_or(threadIdx.x < nsb && front->blk[threadIdx.x].bad);
-    if (blockIdx.x == 0 && threadIdx.x < 32) {
+    if (kMode != RASTER_FILL && blockIdx.x == 0 && threadIdx.x < 32) {
         FrontBlock q;
         q.cov = make_uint4(0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu);
         q.culled = 0;
@@ -2602,6 +2663,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_frame_raster(const SceneDev *__re
             stats[0].culled = q.culled;
             rbase[0] = 0;
             rbase[1] = bad ? 0ull : resolve_chunks(s, q.cov);  // a scene with a bad index draws nothing
+            if (kMode == RASTER_COUNT) totals[4] = totals[5] = 0;  // k_oscan: fragments, finished blocks
         }
     }
     if (bad) return;
@@ -2630,7 +2692,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_frame_raster(const SceneDev *__re
         if (i >= __shfl_sync(0xFFFFFFFFu, incl, 31)) continue;
         const uint32_t t = g * 32 + p;
         const TriRec r = load_rec(recs + t, kRecRaster);
-        raster_row(s, r, t, r.by0 + (i - first), vbuf, cnt, 0, nullptr, probe);
+        raster_row<kMode>(s, r, t, r.by0 + (i - first), vbuf, cnt, frags, probe);
     }
     const uint32_t sum = warp_sum(cnt);
     if (lane == 0 && sum) atomicAdd(&stats[0].candidates, (unsigned long long)sum);
@@ -2843,6 +2905,7 @@ __global__ void __launch_bounds__(kBlock) k_oscan(unsigned long long *__restrict
     if (threadIdx.x == 0) {
         __threadfence();
         if (atomicAdd(totals + 5, 1ull) == gridDim.x - 1) {
+            totals[3] = 0;  // the fill pass's work counter
             *host_total = atomicAdd(totals + 4, 0ull);
             __threadfence_system();
         }
@@ -2889,16 +2952,27 @@ EUC_DEV void order_frags(unsigned long long &a, unsigned long long &b) {
 
 constexpr int kOWindow = 8;  // fragments of a pixel ordered at a time, in registers
 
+// A warp's windows in k_resolve_ordered: the passing primitives of each lane,
+// the lanes' pixels, their evaluations as one list, and the results.
+struct OrderedSmem {
+    uint32_t pass[kOWindow][32];
+    uint32_t xy[32][2];
+    uint8_t job[kOWindow * 32];  // lane << 3 | k
+    float4 frag[kOWindow * 32];
+};
+
 // Replays each pixel's fragments in submission order with euc's sequential
 // depth test (pipeline.rs:519-526) and blend-into-the-current-pixel
 // (pipeline.rs:574-576).  A pixel takes its list in windows of kOWindow
 // fragments: a list that fits is ordered by Batcher's odd-even merge network
 // (19 exchanges), a longer one is read through once per window, keeping the
-// next kOWindow primitives.  The depth test then runs over the window alone
-// and leaves the passing primitives in shared memory, so that a warp shades
-// as often as its pixel with the most of them and not as often as the longest
-// list: with a scan of the list per fragment and the shading inside that loop
-// 960x540 with 8000 triangles (4.3 fragments a pixel) took 83 us here.
+// next kOWindow primitives.  The depth test then runs over the window alone,
+// and the fragments that pass are shaded by the warp together, whichever
+// pixels they are of, before each lane blends its own in order: what a
+// fragment waits for (record, varyings, texels) is waited for once per 32 of
+// them, not once per fragment of the pixel with the most.  960x540, 8000
+// triangles, 4.3 fragments a pixel: 83 us with a scan of the list per fragment
+// and the shading inside it, 53 with the windows, 49 with the shared list.
 template <class F>
 __global__ void __launch_bounds__(kBlock, F::NV > 4 ? 2 : 3) k_resolve_ordered(const SceneDev *__restrict__ sc,
                                                             const uint64_t *__restrict__ res_base, int s_begin,
@@ -2909,32 +2983,34 @@ __global__ void __launch_bounds__(kBlock, F::NV > 4 ? 2 : 3) k_resolve_ordered(c
                                                             const uint2 *__restrict__ frags, uint64_t frag_cap,
                                                             const unsigned long long *__restrict__ totals,
                                                             const uint4 *__restrict__ cov) {
-    __shared__ uint32_t s_pass[kOWindow][kBlock];  // the passing primitives of each thread's window
+    __shared__ OrderedSmem s_warp[kBlock / 32];
     begin_stage();
     if (totals[4] > frag_cap) return;  // the lists were not filled: the host grows them and comes back
+    OrderedSmem &sm = s_warp[threadIdx.x >> 5];
+    const uint32_t lane = threadIdx.x & 31;
     const uint64_t blk = blk_begin + blockIdx.x;
     const int si = s_begin + find_scene(res_base + s_begin, s_end - s_begin, blk);
     const SceneDev &s = sc[si];
     const uint64_t q = (blk - res_base[si]) * kBlock + threadIdx.x;
-    if (q >= (uint64_t)s.W * s.H) return;
     const uint32_t y = (uint32_t)q / s.W, x = (uint32_t)q - y * s.W;
-    if (!covered(cov[si], x, y)) return;
-    const unsigned long long e = vbuf[s.pix_base + q];
+    const bool inside = q < (uint64_t)s.W * s.H && covered(cov[si], x, y);
+    const unsigned long long e = inside ? vbuf[s.pix_base + q] : 0ull;
     const uint2 *list = frags + (uint32_t)e;
-    const uint32_t n = (uint32_t)(e >> 32);
-    if (n == 0) return;
+    const uint32_t n = (uint32_t)(e >> 32);  // 0: a lane that only helps to shade
+    if (!__any_sync(0xFFFFFFFFu, n)) return;
+    const bool write = s.pixel_write, depth_write = s.depth_write, alpha = s.blend == EUC_BLEND_ALPHA;
+    const uint32_t test = s.depth_test;
     float *dp = s.depth ? reinterpret_cast<float *>(s.depth + (uint64_t)y * s.dpitch + 4ull * x) : nullptr;
     const bool f32 = s.pfmt == EUC_FMT_RGBA32F;  // the pixel kept as four floats
     uint8_t *pp = s.pixel ? s.pixel + (uint64_t)y * s.ppitch +
                                 (uint64_t)x * (f32 ? 16u : s.pfmt == EUC_FMT_RGB8 ? 3u : 4u)
                           : nullptr;
-    const bool uses_depth = s.depth_test != EUC_TEST_NONE || s.depth_write;
-    float D = uses_depth ? *dp : 0.0f;
+    float D = n && (test != EUC_TEST_NONE || depth_write) ? *dp : 0.0f;
     const int ri = s.pfmt == EUC_FMT_BGRA8 ? 2 : 0, bi = s.pfmt == EUC_FMT_BGRA8 ? 0 : 2;
     const int nch = s.pfmt == EUC_FMT_RGB8 ? 3 : 4;
     uint32_t ch[4] = {0, 0, 0, 255};
     float pf[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-    if (s.pixel_write) {
+    if (write && n) {
         if (f32)
             for (int i = 0; i < 4; ++i) pf[i] = reinterpret_cast<const float *>(pp)[i];
         else
@@ -2942,10 +3018,12 @@ __global__ void __launch_bounds__(kBlock, F::NV > 4 ? 2 : 3) k_resolve_ordered(c
     }
     const typename F::U &u = *reinterpret_cast<const typename F::U *>(s.uniforms);
     const float *vb = vdata + (s.geom ? s.gvd_base : s.vd_base);
+    sm.xy[lane][0] = x;
+    sm.xy[lane][1] = y;
     uint32_t last = 0;  // 1 + the last primitive of the windows before
-    for (uint32_t done = 0; done < n; done += kOWindow) {
+    for (uint32_t done = 0; __any_sync(0xFFFFFFFFu, done < n); done += kOWindow) {
         uint32_t npass = 0;
-        {
+        if (done < n) {
             unsigned long long w[kOWindow];  // the next kOWindow primitives, in order (~0: none)
             if (n <= kOWindow) {
 #pragma unroll
@@ -2989,29 +3067,40 @@ __global__ void __launch_bounds__(kBlock, F::NV > 4 ? 2 : 3) k_resolve_ordered(c
                 if (done + k >= n) break;
                 const float z = __uint_as_float((uint32_t)w[k]);
                 bool pass = true;
-                if (s.depth_test == EUC_TEST_LESS) pass = z < D;
-                else if (s.depth_test == EUC_TEST_EQUAL) pass = z == D;
-                else if (s.depth_test == EUC_TEST_GREATER) pass = z > D;
+                if (test == EUC_TEST_LESS) pass = z < D;
+                else if (test == EUC_TEST_EQUAL) pass = z == D;
+                else if (test == EUC_TEST_GREATER) pass = z > D;
                 if (!pass) continue;
-                if (s.depth_write) D = z;
-                s_pass[npass++][threadIdx.x] = (uint32_t)(w[k] >> 32);
+                if (depth_write) D = z;
+                sm.pass[npass++][lane] = (uint32_t)(w[k] >> 32);
             }
         }
-        if (!s.pixel_write) continue;
-        for (uint32_t k = 0; k < npass; ++k) {
+        // the warp's list of evaluations
+        const uint32_t inc = warp_incl_scan(npass), off = inc - npass, njobs = __shfl_sync(0xFFFFFFFFu, inc, 31);
+        if (!write || !njobs) continue;
+        for (uint32_t k = 0; k < npass; ++k) sm.job[off + k] = (uint8_t)(lane << 3 | k);
+        __syncwarp();
+        for (uint32_t j = lane; j < njobs; j += 32) {
+            const uint32_t slot = sm.job[j] >> 3, k = sm.job[j] & 7u;
             float frag[F::NF];
-            shade_at<F>(s, u, load_shade(recs + s_pass[k][threadIdx.x]), vb, x, y, frag);
-            float c[4] = {frag[0], F::NF > 1 ? frag[F::NF > 1 ? 1 : 0] : 0.0f,
-                          F::NF > 2 ? frag[F::NF > 2 ? 2 : 0] : 0.0f, F::NF > 3 ? frag[F::NF > 3 ? 3 : 0] : 0.0f};
-            if (s.blend == EUC_BLEND_ALPHA) {  // src-over on the unpacked old pixel
+            shade_at<F>(s, u, load_shade(recs + sm.pass[k][slot]), vb, sm.xy[slot][0], sm.xy[slot][1], frag);
+            sm.frag[j] = make_float4(frag[0], F::NF > 1 ? frag[F::NF > 1 ? 1 : 0] : 0.0f,
+                                     F::NF > 2 ? frag[F::NF > 2 ? 2 : 0] : 0.0f,
+                                     F::NF > 3 ? frag[F::NF > 3 ? 3 : 0] : 0.0f);
+        }
+        __syncwarp();
+        for (uint32_t k = 0; k < npass; ++k) {
+            const float4 v = sm.frag[off + k];
+            float c[4] = {v.x, v.y, v.z, v.w};
+            if (alpha) {  // src-over on the unpacked old pixel
                 float old[4];
                 if (f32) {
                     for (int i = 0; i < 4; ++i) old[i] = pf[i];
                 } else {
-                    old[0] = (float)ch[ri] / 255.0f;
-                    old[1] = (float)ch[1] / 255.0f;
-                    old[2] = (float)ch[bi] / 255.0f;
-                    old[3] = nch == 3 ? 1.0f : (float)ch[3] / 255.0f;
+                    old[0] = byte_over_255(ch[ri]);
+                    old[1] = byte_over_255(ch[1]);
+                    old[2] = byte_over_255(ch[bi]);
+                    old[3] = nch == 3 ? 1.0f : byte_over_255(ch[3]);
                 }
                 const float a = c[3];
 #pragma unroll
@@ -3026,9 +3115,11 @@ __global__ void __launch_bounds__(kBlock, F::NV > 4 ? 2 : 3) k_resolve_ordered(c
             ch[bi] = sat_u8(F::pack(c[2]));
             if (nch == 4) ch[3] = sat_u8(F::pack(c[3]));
         }
+        __syncwarp();  // the next window reuses the warp's shared memory
     }
-    if (s.depth_write) *dp = D;
-    if (s.pixel_write) {
+    if (!n) return;
+    if (depth_write) *dp = D;
+    if (write) {
         if (f32)
             for (int i = 0; i < 4; ++i) reinterpret_cast<float *>(pp)[i] = pf[i];
         else

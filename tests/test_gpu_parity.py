@@ -417,3 +417,32 @@ def test_row_segments_at_their_edges(gpu_ctx, strip_ctx, w, h, fmt):
         got, got_stats = run_gpu(ctx, make())
         assert got_stats == ref_stats
         assert_targets_match(make(), ref, got)
+
+
+@pytest.mark.parametrize("w,h", [(1, 1), (33, 7), (64, 4), (257, 5), (190, 101)])
+@pytest.mark.parametrize("kind", ["soup", "perspective", "phong", "lines"])
+def test_ordered_frames_on_both_paths(gpu_ctx, strip_ctx, kind, w, h):
+    """src-over scenes through the small-scene path and through the batch's
+    kernels (strip_ctx keeps off the former): rows at the edges of 32 lanes
+    and of the pixel scan's blocks, rectangles smaller than the target, runs
+    of uneven lists whose fragments the warp shades together, rows with and
+    without the guard tests, and a shader of every record size."""
+    if kind == "soup":
+        make = _soup(seed=95, w=w, h=h, n=700, hi=0.2 * w * h + 20.0, alpha=True)
+    elif kind == "lines":
+        make = lambda: scenes.lines_frame(seed=95, width=w, height=h, nlines=300, len_hi=40.0)
+    elif kind == "phong":
+        make = _knot(0, w=w, h=h, shadow=64)
+    else:
+        make = _sphere(width=w, height=h)
+    base = make
+    def make():
+        f = base()
+        f.passes[-1].desc.blend = abi.BLEND_ALPHA
+        return f
+    ref, ref_stats = run_oracle(make())
+    for ctx in (gpu_ctx, strip_ctx):
+        got, got_stats = run_gpu(ctx, make())
+        assert [s[:2] for s in got_stats] == [s[:2] for s in ref_stats]
+        # a Phong byte may be one step off, and so may the blend's rounding of it
+        assert_targets_match(make(), ref, got, 2 if kind == "phong" else 0)
