@@ -895,12 +895,13 @@ int run_batch(euc_ctx *ctx, const euc_scene *scenes, size_t n, cudaStream_t st, 
 // that launches, not work, set their time (k_front's comment has the figures).
 // kFramePrims bounds the groups a block scans; kFramePixels bounds the keys that k_front seeds beyond the
 // covered rectangle (12 bytes a pixel: 12.6 MB, some 2 us beside the setup);
-// kFrameVerts keeps unindexed soups of more than 21 k triangles on the batch's
-// path, whose strips pay there (640x480: 16 k triangles of up to 2000 px 58 us
-// here and 130 us on the strips, 32 k of up to 8000 px 229 and 126).  A batch,
-// a forced strip path and a profiled context take the other kernels.
+// kFrameVerts is above three vertices a primitive, so that it is the primitives
+// that decide (640x480 triangle soups, here and on the batch's path, whose
+// strips take them, clears and host included: 32 k of up to 500 px 69 and 83 us,
+// of up to 2000 px 74 and 102, of up to 8000 px 122 and 135).  A
+// batch, a forced strip path and a profiled context take the other kernels.
 // ---------------------------------------------------------------------------
-constexpr uint64_t kFramePixels = 1ull << 20, kFrameVerts = 1ull << 16;
+constexpr uint64_t kFramePixels = 1ull << 20, kFrameVerts = 1ull << 17;
 
 bool frame_path(const euc_ctx *ctx, const Plan &p) {
     return p.d.geom == EUC_GEOM_NONE && p.d.ngroups >= 1 && p.d.ngroups <= kFramePrims && p.d.nverts <= kFrameVerts && (uint64_t)p.d.W * p.d.H <= kFramePixels && ctx->tune.strip_path != 2 &&

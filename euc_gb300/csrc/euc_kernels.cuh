@@ -1268,11 +1268,27 @@ EUC_DEV bool row_span(const SceneDev &s, const TriRec &r, uint32_t y, uint32_t &
     return xs < xe;
 }
 
+// Lanes that share a row of a primitive (raster_row).  Four: their pixels lie in
+// one 32-byte sector of keys, which halves what the reductions cost (22 M 64-bit
+// ones, by scattered lanes 164 us, by fours 85, by whole warps 65; 32-bit counts
+// 110, 31, 17), and the longest row of a step takes a quarter of the time.  Each
+// lane adds the weights of all four pixels, so it pays where rows are long or
+// few: a small scene's launches (960x540, 8000 triangles: count 32 -> 22 us, fill
+// 45 -> 31; 640x480, 20 k triangles of up to 8000 px 149 -> 91 us; eight lanes 24
+// and 56, two 27 and 37) and the ordered passes, not the item queue's keys (256
+// spheres 190 us by single lanes, 209 by fours).
 template <int kMode>
+constexpr int kRowLanes = kMode == RASTER_KEYS ? 1 : 4;
+constexpr int kFrameLanes = 4;
+
+// One row of a primitive by kLanes lanes, of which this is lane q: lane q takes
+// the pixels xs + q, xs + q + kLanes, ..., and adds the weights of the others
+// on the way (the sums are euc's serial ones).
+template <int kMode, int kLanes>
 EUC_DEV void raster_row(const SceneDev &s, const TriRec &r, uint32_t t, uint32_t y,
-                        unsigned long long *__restrict__ vbuf, uint32_t &cnt, uint2 *__restrict__ frags, bool probe) {
+                        unsigned long long *__restrict__ vbuf, uint32_t &cnt, uint2 *__restrict__ frags, bool probe, int q) {
     if (s.prim != EUC_PRIM_TRIANGLE_LIST) {  // lines: `y` is the step within the window
-        raster_line_step<kMode>(s, r, t, y, vbuf, cnt, frags, probe);
+        if (q == 0) raster_line_step<kMode>(s, r, t, y, vbuf, cnt, frags, probe);
         return;
     }
     uint32_t xs, xe;
@@ -1285,6 +1301,20 @@ EUC_DEV void raster_row(const SceneDev &s, const TriRec &r, uint32_t t, uint32_t
     float w1 = (r.o[1] + r.dy[1] * yf) + r.dx[1] * xsf;
     float w2 = (r.o[2] + r.dy[2] * yf) + r.dx[2] * xsf;
     const float d0 = r.dx[0], d1 = r.dx[1], d2 = r.dx[2];
+    const auto advance = [&](int pixels) {
+#pragma unroll
+        for (int k = 0; k < pixels; ++k) {
+            w0 = w0 + d0;
+            w1 = w1 + d1;
+            w2 = w2 + d2;
+        }
+    };
+    if (kLanes > 1) {
+#pragma unroll
+        for (int k = 0; k < kLanes - 1; ++k)
+            if (k < q) advance(1);
+        xs += q;
+    }
     const float z0 = r.zc[0], z1 = r.zc[1], z2 = r.zc[2];
     const bool noclip = r.flags & kTriNoClip;
     unsigned long long *row_keys = vbuf + s.pix_base + (uint64_t)y * s.W;
@@ -1297,22 +1327,20 @@ EUC_DEV void raster_row(const SceneDev &s, const TriRec &r, uint32_t t, uint32_t
         // candidate is keyed and reduced where the walk finds it
         if (!greater && (r.flags & kTriZPos)) {
 #pragma unroll 4
-            for (uint32_t x = xs; x < xe; ++x) {
+            for (uint32_t x = xs; x < xe; x += kLanes) {
                 const float wu2 = (w2 - w0) - w1;
                 if (w0 >= 0.0f && w1 >= 0.0f && wu2 >= 0.0f) {
                     const float z = (z0 * w0 + z1 * w1) + z2 * wu2;
                     ++cnt;
                     atomicMin(row_keys + x, ((unsigned long long)zpos_order(z) << 32) | tmin);
                 }
-                w0 = w0 + d0;
-                w1 = w1 + d1;
-                w2 = w2 + d2;
+                advance(kLanes);
             }
             return;
         }
         const uint32_t flip = greater ? 0xFFFFFFFFu : 0u;
 #pragma unroll 4
-        for (uint32_t x = xs; x < xe; ++x) {
+        for (uint32_t x = xs; x < xe; x += kLanes) {
             const float wu2 = (w2 - w0) - w1;
             if (w0 >= 0.0f && w1 >= 0.0f && wu2 >= 0.0f) {
                 const float z = (z0 * w0 + z1 * w1) + z2 * wu2;
@@ -1326,45 +1354,39 @@ EUC_DEV void raster_row(const SceneDev &s, const TriRec &r, uint32_t t, uint32_t
                     }
                 }
             }
-            w0 = w0 + d0;
-            w1 = w1 + d1;
-            w2 = w2 + d2;
+            advance(kLanes);
         }
         return;
     }
     // The ordered passes between two edges, where nearly every pixel is a
     // candidate: no branch, the others add 0.  (A branch around an atomic costs
-    // the walk some 45 cycles a pixel.  Kept off the keys, whose launches are
-    // not bound by their longest rows: 256 spheres 606 us against 614.)
+    // the walk some 45 cycles a pixel.  Kept off the keys: 256 spheres 606 us
+    // against 614.)
     if (kMode == RASTER_COUNT && noclip && !full) {
 #pragma unroll 4
-        for (uint32_t x = xs; x < xe; ++x) {
+        for (uint32_t x = xs; x < xe; x += kLanes) {
             const float wu2 = (w2 - w0) - w1;
             const uint32_t in = (w0 >= 0.0f) & (w1 >= 0.0f) & (wu2 >= 0.0f) ? 1u : 0u;
             cnt += in;
             atomicAdd(reinterpret_cast<unsigned int *>(row_keys + x), in);
-            w0 = w0 + d0;
-            w1 = w1 + d1;
-            w2 = w2 + d2;
+            advance(kLanes);
         }
         return;
     }
     if (kMode == RASTER_FILL && noclip && !full) {
-        // eight cursors in flight; a pixel that is no candidate moves none
-        constexpr int kFill = 8;
-        for (uint32_t x = xs; x < xe; x += kFill) {
+        // four cursors in flight; a pixel that is no candidate moves none
+        constexpr int kFill = 4;
+        for (uint32_t x = xs; x < xe; x += kFill * kLanes) {
             unsigned long long e[kFill];
             float zz[kFill];
             bool in[kFill];
 #pragma unroll
             for (int k = 0; k < kFill; ++k) {
                 const float wu2 = (w2 - w0) - w1;
-                in[k] = (w0 >= 0.0f) & (w1 >= 0.0f) & (wu2 >= 0.0f) & (x + k < xe);
+                in[k] = (w0 >= 0.0f) & (w1 >= 0.0f) & (wu2 >= 0.0f) & (x + k * kLanes < xe);
                 zz[k] = (z0 * w0 + z1 * w1) + z2 * wu2;
-                e[k] = atomicAdd(row_keys + min(x + k, xe - 1u), in[k] ? 1ull << 32 : 0ull);
-                w0 = w0 + d0;
-                w1 = w1 + d1;
-                w2 = w2 + d2;
+                e[k] = atomicAdd(row_keys + min(x + k * kLanes, xe - 1u), in[k] ? 1ull << 32 : 0ull);
+                advance(kLanes);
             }
 #pragma unroll
             for (int k = 0; k < kFill; ++k)
@@ -1373,18 +1395,17 @@ EUC_DEV void raster_row(const SceneDev &s, const TriRec &r, uint32_t t, uint32_t
         return;
     }
     // The walk advances pixel by pixel exactly as euc's loop does; candidates
-    // are gathered kWalk at a time so that their key loads (eight cursors in
-    // the fill pass: 56 -> 45 us for 960x540 and 2.2 M fragments) are in
+    // are gathered kWalk at a time so that their key loads and cursors are in
     // flight together instead of one L2 round trip per pixel.
-    constexpr int kWalk = kMode == RASTER_FILL ? 8 : 4;
-    for (uint32_t x = xs; x < xe; x += kWalk) {
+    constexpr int kWalk = 4;
+    for (uint32_t x = xs; x < xe; x += kWalk * kLanes) {
         float zz[kWalk];
         bool cand[kWalk];
 #pragma unroll
         for (int k = 0; k < kWalk; ++k) {
             cand[k] = false;
             zz[k] = 0.0f;
-            if (x + k < xe) {
+            if (x + k * kLanes < xe) {
                 const float wu2 = (w2 - w0) - w1;
                 if (w0 >= 0.0f && w1 >= 0.0f && wu2 >= 0.0f) {
                     const float z = (z0 * w0 + z1 * w1) + z2 * wu2;
@@ -1393,9 +1414,7 @@ EUC_DEV void raster_row(const SceneDev &s, const TriRec &r, uint32_t t, uint32_t
                         zz[k] = z;
                     }
                 }
-                w0 = w0 + d0;
-                w1 = w1 + d1;
-                w2 = w2 + d2;
+                advance(kLanes);
             }
         }
         // most groups of a full-bbox row (extent < 128) hold no candidate:
@@ -1409,7 +1428,7 @@ EUC_DEV void raster_row(const SceneDev &s, const TriRec &r, uint32_t t, uint32_t
             for (int k = 0; k < kWalk; ++k) {
                 if (!cand[k]) continue;
                 ++cnt;
-                atomicAdd(reinterpret_cast<unsigned int *>(row_keys + x + k), 1u);
+                atomicAdd(reinterpret_cast<unsigned int *>(row_keys + x + k * kLanes), 1u);
             }
             continue;
         }
@@ -1418,7 +1437,7 @@ EUC_DEV void raster_row(const SceneDev &s, const TriRec &r, uint32_t t, uint32_t
             // all in flight before the first store
             unsigned long long e[kWalk];
 #pragma unroll
-            for (int k = 0; k < kWalk; ++k) e[k] = cand[k] ? atomicAdd(row_keys + x + k, 1ull << 32) : 0ull;
+            for (int k = 0; k < kWalk; ++k) e[k] = cand[k] ? atomicAdd(row_keys + x + k * kLanes, 1ull << 32) : 0ull;
 #pragma unroll
             for (int k = 0; k < kWalk; ++k)
                 if (cand[k]) frags[(uint32_t)e[k] + (uint32_t)(e[k] >> 32)] = make_uint2(t, __float_as_uint(zz[k]));
@@ -1429,7 +1448,7 @@ EUC_DEV void raster_row(const SceneDev &s, const TriRec &r, uint32_t t, uint32_t
         float old[kWalk];
         if (!kmin && s.depth_test != EUC_TEST_NONE) {
 #pragma unroll
-            for (int k = 0; k < kWalk; ++k) old[k] = cand[k] ? row_depth[x + k] : 0.0f;
+            for (int k = 0; k < kWalk; ++k) old[k] = cand[k] ? row_depth[x + k * kLanes] : 0.0f;
         }
 #pragma unroll
         for (int k = 0; k < kWalk; ++k) {
@@ -1455,15 +1474,15 @@ EUC_DEV void raster_row(const SceneDev &s, const TriRec &r, uint32_t t, uint32_t
             // depth complexity: most candidates lose)
             unsigned long long cur[kWalk];
 #pragma unroll
-            for (int k = 0; k < kWalk; ++k) cur[k] = pass[k] ? __ldcg(row_keys + x + k) : 0ull;
+            for (int k = 0; k < kWalk; ++k) cur[k] = pass[k] ? __ldcg(row_keys + x + k * kLanes) : 0ull;
 #pragma unroll
             for (int k = 0; k < kWalk; ++k)
-                if (pass[k] && key[k] < cur[k]) atomicMin(row_keys + x + k, key[k]);
+                if (pass[k] && key[k] < cur[k]) atomicMin(row_keys + x + k * kLanes, key[k]);
         } else {
             // fire-and-forget reductions: the walk never waits on memory
 #pragma unroll
             for (int k = 0; k < kWalk; ++k)
-                if (pass[k]) atomicMin(row_keys + x + k, key[k]);
+                if (pass[k]) atomicMin(row_keys + x + k * kLanes, key[k]);
         }
     }
 }
@@ -1487,6 +1506,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_raster(const SceneDev *__restrict
                                                    SceneStats *__restrict__ stats, uint2 *__restrict__ frags,
                                                    uint64_t frag_cap, int witems, bool probe) {
     constexpr int kCounter = kMode == RASTER_KEYS ? 2 : 3;  // the launch's work counter in totals
+    constexpr int kLanes = kRowLanes<kMode>, kItems = 32 / kLanes;  // items of a step
     __shared__ uint64_t s_off[kBlock / 32][kWarpItems];
     begin_stage();  // (k_strip runs beside it: their keys meet in order-free reductions)
     if (kMode == RASTER_FILL && totals[4] > frag_cap) return;  // the lists do not fit: the host grows them and comes back
@@ -1528,25 +1548,25 @@ __global__ void __launch_bounds__(kBlock, 4) k_raster(const SceneDev *__restrict
         for (int j = lane; j < witems; j += 32) off[j] = l0 + j < nlive ? live_rowoff[l0 + j] : ~0ull;
         __syncwarp();
         uint32_t scene0 = 0xFFFFFFFFu, cnt0 = 0;
-        // The 32 items of a step are consecutive, so their primitives are a
+        // The items of a step are consecutive, so their primitives are a
         // run of the window from a0 (the primitive of the step's first item):
         // lane j marks where primitive a0 + 1 + j starts within the step, and
         // each lane counts the starts at or before its own item.
         int a0 = 0;  // window entry 0 is the primitive of item `base`
-        for (int s = 0; s < witems / 32; ++s) {
-            const uint64_t i0 = base + (uint64_t)s * 32;
+        for (int s = 0; s < witems / kItems; ++s) {
+            const uint64_t i0 = base + (uint64_t)s * kItems;
             if (i0 >= nitems) break;
             const int c = a0 + 1 + lane;
             uint32_t bit = 0;
-            if (lane < 31 && c < witems) {
+            if (lane < kItems - 1 && c < witems) {
                 const uint64_t o = off[c];
-                if (o > i0 && o < i0 + 32) bit = 1u << (uint32_t)(o - i0);
+                if (o > i0 && o < i0 + kItems) bit = 1u << (uint32_t)(o - i0);
             }
             const uint32_t starts = __reduce_or_sync(0xFFFFFFFFu, bit);
-            const int a = a0 + __popc(starts & ((2u << lane) - 1u));
+            const int a = a0 + __popc(starts & ((2u << lane / kLanes) - 1u));
             const int alast = a0 + __popc(starts);  // the primitive of the step's last item
-            a0 = (alast + 1 < witems && off[alast + 1] == i0 + 32) ? alast + 1 : alast;
-            const uint64_t i = i0 + lane;
+            a0 = (alast + 1 < witems && off[alast + 1] == i0 + kItems) ? alast + 1 : alast;
+            const uint64_t i = i0 + lane / kLanes;
             if (i >= nitems) continue;
             const uint32_t t = live_tri[l0 + a];
             const TriRec r = load_rec(recs + t, kRecRaster);
@@ -1554,7 +1574,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_raster(const SceneDev *__restrict
             if (err[scene]) continue;
             if ((sc[scene].keytype == KEY_ORDERED) != (kMode != RASTER_KEYS)) continue;  // another launch's scene
             uint32_t cnt = 0;
-            raster_row<kMode>(sc[scene], r, t, r.by0 + (uint32_t)(i - off[a]), vbuf, cnt, frags, probe);
+            raster_row<kMode, kLanes>(sc[scene], r, t, r.by0 + (uint32_t)(i - off[a]), vbuf, cnt, frags, probe, lane % kLanes);
             if (scene0 == 0xFFFFFFFFu) scene0 = scene;
             if (scene == scene0) cnt0 += cnt;
             else if (cnt) atomicAdd(&stats[scene].candidates, (unsigned long long)cnt);
@@ -2509,9 +2529,10 @@ __global__ void __launch_bounds__(kBlock, F::kResolveBlocks) k_resolve(const Sce
 //                   varyings of 256 vertices a block; the keys of
 //                   kInitChunk pixels a block, over the whole target
 //                   (the covered rectangle is not known yet)
-//   k_frame_raster  32 items a warp step, spread evenly over the grid from the
-//                   row sums of the 32-primitive groups, which every block
-//                   scans for itself; block 0 also finishes the scene's
+//   k_frame_raster  eight rows a warp step, four lanes each (32 steps of lines),
+//                   spread evenly over the grid from the row sums of the
+//                   32-primitive groups, which every block scans for itself;
+//                   block 0 also finishes the scene's
 //                   covered rectangle, error and culled count for
 //   k_resolve<F>    as in a batch
 // Nothing is cleared ahead: the setup blocks store their own sums.  640x480
@@ -2632,12 +2653,14 @@ __global__ void __launch_bounds__(kBlock, 4) k_frame_raster(const SceneDev *__re
     const SceneDev &s = sc[0];
     const int lane = threadIdx.x & 31;
     const uint32_t ngroups = (s.ngroups + 31u) >> 5;
-    // four consecutive groups a thread: their steps of 32 items
+    // four consecutive groups a thread: their steps
     static_assert(kFrameGroups == 4 * kBlock && kFrameBlocks <= kBlock, "four groups a thread, one setup block a thread");
     const uint4 gr = *reinterpret_cast<const uint4 *>(front->group_rows + 4 * threadIdx.x);
     uint32_t steps[4] = {gr.x, gr.y, gr.z, gr.w};
+    // a step is a warp's: rows by kFrameLanes lanes each, a line's steps by one
+    const uint32_t per = s.prim == EUC_PRIM_TRIANGLE_LIST ? 32u / kFrameLanes : 32u;
 #pragma unroll
-    for (uint32_t k = 0; k < 4; ++k) steps[k] = 4 * threadIdx.x + k < ngroups ? (steps[k] + 31u) >> 5 : 0u;
+    for (uint32_t k = 0; k < 4; ++k) steps[k] = 4 * threadIdx.x + k < ngroups ? (steps[k] + per - 1) / per : 0u;
     const int bad = __syncthreads_or(threadIdx.x < nsb && front->blk[threadIdx.x].bad);
     if (kMode != RASTER_FILL && blockIdx.x == 0 && threadIdx.x < 32) {
         FrontBlock q;
@@ -2681,7 +2704,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_frame_raster(const SceneDev *__re
         static_assert(kFrameGroups == 32 * 32, "a two-level search, 32 ways each");
         const uint32_t g32 = 32u * (uint32_t)(__popc(__ballot_sync(0xFFFFFFFFu, s_pref[32 * lane] <= st)) - 1);
         const uint32_t g = g32 + (uint32_t)__popc(__ballot_sync(0xFFFFFFFFu, s_pref[g32 + lane] <= st)) - 1u;
-        const uint32_t i = (st - s_pref[g]) * 32 + lane;  // this lane's item in the group
+        const uint32_t i = (st - s_pref[g]) * per + (per == 32 ? lane : lane / kFrameLanes);  // this lane's item in the group
         const uint32_t nr = rows[g * 32 + lane], incl = warp_incl_scan(nr);
         // its primitive: the first whose items end after i
         int p = 0;
@@ -2692,7 +2715,10 @@ __global__ void __launch_bounds__(kBlock, 4) k_frame_raster(const SceneDev *__re
         if (i >= __shfl_sync(0xFFFFFFFFu, incl, 31)) continue;
         const uint32_t t = g * 32 + p;
         const TriRec r = load_rec(recs + t, kRecRaster);
-        raster_row<kMode>(s, r, t, r.by0 + (i - first), vbuf, cnt, frags, probe);
+        if (s.prim != EUC_PRIM_TRIANGLE_LIST)
+            raster_line_step<kMode>(s, r, t, r.by0 + (i - first), vbuf, cnt, frags, probe);
+        else
+            raster_row<kMode, kFrameLanes>(s, r, t, r.by0 + (i - first), vbuf, cnt, frags, probe, lane % kFrameLanes);
     }
     const uint32_t sum = warp_sum(cnt);
     if (lane == 0 && sum) atomicAdd(&stats[0].candidates, (unsigned long long)sum);
