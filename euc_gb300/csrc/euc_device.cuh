@@ -269,11 +269,26 @@ struct PhongFn {  // examples/teapot.rs:69-141 with a surface texture
     static constexpr int kResolveBlocks = 4;  // k_resolve blocks per SM: at 5 its registers spill (12 % slower)
     using U = euc_phong_uniforms;
     static EUC_DEV void vertex(const U &u, const euc_vertex_layout &l, const uint8_t *v, float clip[4], float *vd) {
-        const float p[4] = {ld_f32(v + l.position), ld_f32(v + l.position + 4), ld_f32(v + l.position + 8), 1.0f};
+        // position, normal and texture coordinates packed in eight aligned words: two
+        // loads for eight (k_vertex has the figures)
+        float at[8];
+        if (l.position == 0 && l.normal == 12 && l.uv == 24 && (((uintptr_t)v | l.stride) & 15) == 0) {
+            const float4 a = *reinterpret_cast<const float4 *>(v), b = *reinterpret_cast<const float4 *>(v + 16);
+            at[0] = a.x, at[1] = a.y, at[2] = a.z, at[3] = a.w;
+            at[4] = b.x, at[5] = b.y, at[6] = b.z, at[7] = b.w;
+        } else {
+#pragma unroll
+            for (int i = 0; i < 3; ++i) {
+                at[i] = ld_f32(v + l.position + 4 * i);
+                at[3 + i] = ld_f32(v + l.normal + 4 * i);
+            }
+#pragma unroll
+            for (int i = 0; i < 2; ++i) at[6 + i] = l.uv >= 0 ? ld_f32(v + l.uv + 4 * i) : 0.0f;
+        }
+        const float p[4] = {at[0], at[1], at[2], 1.0f};
         float wpos[4];
         mat4_vec4(u.model, p, wpos);
-        const float n4[4] = {ld_f32(v + l.normal) * u.normal_sign, ld_f32(v + l.normal + 4) * u.normal_sign,
-                             ld_f32(v + l.normal + 8) * u.normal_sign, 0.0f};
+        const float n4[4] = {at[3] * u.normal_sign, at[4] * u.normal_sign, at[5] * u.normal_sign, 0.0f};
         float wnorm[4];
         mat4_vec4(u.model, n4, wnorm);
         const float wp1[4] = {wpos[0], wpos[1], wpos[2], 1.0f};
@@ -290,13 +305,8 @@ struct PhongFn {  // examples/teapot.rs:69-141 with a surface texture
         vd[6] = lvp[0] / lvp[3];
         vd[7] = lvp[1] / lvp[3];
         vd[8] = lvp[2] / lvp[3];
-        if (l.uv >= 0) {
-            vd[9] = ld_f32(v + l.uv);
-            vd[10] = ld_f32(v + l.uv + 4);
-        } else {
-            vd[9] = 0.0f;
-            vd[10] = 0.0f;
-        }
+        vd[9] = at[6];
+        vd[10] = at[7];
     }
     static EUC_DEV void fragment(const U &u, const float *vd, float *f) {
         float n[3], cam_dir[3], light_dir[3], t[3];

@@ -446,3 +446,56 @@ def test_ordered_frames_on_both_paths(gpu_ctx, strip_ctx, kind, w, h):
         assert [s[:2] for s in got_stats] == [s[:2] for s in ref_stats]
         # a Phong byte may be one step off, and so may the blend's rounding of it
         assert_targets_match(make(), ref, got, 2 if kind == "phong" else 0)
+
+
+@pytest.mark.parametrize("order,pad,shift", [("pnu", 0, 0), ("pnu", 1, 0), ("pnu", 4, 0), ("pnu", 0, 4), ("pnu", 4, 8),
+                                             ("pun", 0, 0), ("npu", 0, 0), ("pn", 0, 0), ("pn", 2, 0)])
+def test_phong_vertices_of_every_layout(gpu_ctx, strip_ctx, order, pad, shift):
+    """Packed vertices on 16-byte boundaries take two loads: the same values
+    with padding between them, on other boundaries, in another order and
+    without texture coordinates give the oracle's image, and the layouts that
+    hold the same attributes the packed one's bytes."""
+    import torch
+    from euc_gb300 import frames
+    base = _knot(0, w=97, h=61, shadow=64)()
+    spec = base.passes[-1]
+    words = np.frombuffer(spec.vertices.tobytes(), dtype=np.float32).reshape(-1, 8)
+    attrs = {"p": words[:, 0:3], "n": words[:, 3:6], "u": words[:, 6:8]}
+
+    def images(order, pad, shift):
+        cols, at, offs = [], 0, {"u": -1}
+        for c in order:
+            offs[c] = 4 * at
+            cols.append(attrs[c])
+            at += attrs[c].shape[1]
+        cols.append(np.full((len(words), pad), 7.0, dtype=np.float32))
+        f = _knot(0, w=97, h=61, shadow=64)()
+        p = f.passes[-1]
+        p.vertices = np.ascontiguousarray(np.concatenate(cols, axis=1)).view(np.uint8).reshape(-1)
+        p.layout = scenes.layout(4 * (at + pad), position=offs["p"], normal=offs["n"], uv=offs["u"])
+        ref, _ = run_oracle(f)
+        got = []
+        for ctx in (gpu_ctx, strip_ctx):
+            df = frames.DeviceFrame(f, "cuda:0")
+            df.clear()
+            for k, q in enumerate(f.passes):
+                desc, uni, keep = df.bound_pass(k)
+                v, i, _ = df.passes[k]
+                if q is p:
+                    v = torch.cat([torch.zeros(shift, dtype=torch.uint8, device=v.device), v])
+                px = frames.tensor_target(df.targets[q.pixel] if q.pixel else None,
+                                          f.target(q.pixel).fmt if q.pixel else abi.FMT_NONE)
+                dp = frames.tensor_target(df.targets[q.depth] if q.depth else None, abi.FMT_R32F)
+                assert ctx.render(desc.desc, uni, desc.layout, v.data_ptr() + (shift if q is p else 0), q.nverts,
+                                  i.data_ptr(), i.numel(), px, dp, frames._stream_ptr(None)) == abi.OK
+                torch.cuda.synchronize()
+                del keep
+            got.append(df.to_host())
+            assert_targets_match(f, ref, got[-1], 1)
+        return got
+
+    got = images(order, pad, shift)
+    if "u" in order:
+        for a, b in zip(got, images("pnu", 0, 0)):
+            for name in a:
+                assert np.array_equal(a[name].view(np.uint8), b[name].view(np.uint8)), name
