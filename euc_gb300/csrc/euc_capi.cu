@@ -1,8 +1,9 @@
 // euc_capi.cu — host runtime and C ABI of the GB300 triangle pipeline.
 //
 // A render is a batch of one scene; a batch runs every scene through the same
-// six launches (vertex per shader kind, setup, scan, init, raster, resolve per
-// shader kind) on one stream.  Scratch buffers live in the context and grow
+// launches (vertex per shader kind, setup, strip counts, scan, init, binning,
+// raster, strips, resolve per shader kind) on one stream; a small scene of its
+// own takes three (run_frame).  Scratch buffers live in the context and grow
 // on demand (euc_ctx_reserve pre-sizes them).  Scene tables and uniforms go
 // up through a ring of pinned staging slots, each guarded by an event.
 
@@ -1255,13 +1256,13 @@ void graph_free(euc_graph *g) {
 }  // namespace
 
 // ---------------------------------------------------------------------------
-// euc_render's recorded shapes.  A plain render is eight dependent stream
-// operations (the scene-table copy and seven launches), and for a small
+// euc_render's recorded shapes.  A plain render is three (a small scene) to
+// ten dependent stream operations, and for a small
 // scene their latencies, not the kernels, set the time per call.  So
 // euc_render records the launches of a scene shape as a CUDA graph the
 // second time it sees that shape, and from then on a call of the same shape
 // fills the scene table and uniforms into the parameter of the graph's first
-// kernel (k_stage_param, which writes them to the shape's device staging)
+// kernel (k_front, or k_stage_param, which write them to device staging)
 // and replays the graph: one parameter update and one graph launch.  The
 // staging travels with the launch, so the host keeps no ring of page-locked
 // slots and never waits for one; on GB300 the former copy of a page-locked

@@ -1,6 +1,7 @@
 // euc_kernels.cuh — the GB300 triangle pipeline kernels.
 //
-// Stages (all scenes of a batch go through each stage in one launch):
+// Stages (all scenes of a batch go through each stage in one launch; a small
+// scene of its own takes k_front, k_frame_raster and k_resolve instead):
 //   k_vertex<F>   one thread per unique vertex: the vertex functor
 //                 (pipeline.rs:273-276; shading once per vertex instead of once
 //                 per index gives the same bits because the functor is pure)
@@ -15,6 +16,9 @@
 //                 primitives that cover at least one row; one more block
 //                 plans the init / resolve chunks of every scene
 //   k_init        per pixel: the visibility key of the depth already in place
+//   k_bin_count, k_bin, k_strip
+//                 overdrawn scenes: entries per strip of rows, and their walk
+//                 with the strip's keys in shared memory
 //   k_raster      one thread per (primitive, row): euc's serial f32 weight
 //                 walk along the row span (triangles.rs:219-303), inside test,
 //                 z, z-clip and the depth test against a 64-bit visibility
@@ -22,6 +26,8 @@
 //   k_resolve<F>  per pixel: the winning primitive is shaded once
 //                 (get_v_data, fragment, coarse-grid MSAA, blend) and the
 //                 colour and depth are written (pipeline.rs:529-578)
+// and for blends that read the old pixel k_raster<RASTER_COUNT>, k_oscan,
+// k_raster<RASTER_FILL> and k_resolve_ordered<F>.
 //
 // Why an arg-min is exact.  With a blend that ignores the old pixel (every
 // blend in euc's examples), euc's sequential loop leaves in each pixel the
