@@ -909,6 +909,17 @@ bool frame_path(const euc_ctx *ctx, const Plan &p) {
            !ctx->profiling;
 }
 
+// The scratch of a size that no scene changes (some 8 KB), there from the
+// context's creation: a render whose other scratch is large enough allocates
+// nothing, inside a caller's stream capture for instance.
+constexpr size_t kFrameUni = (sizeof(SceneDev) + 15) / 16 * 16;  // the uniforms' place in frame_stage
+static_assert(sizeof(euc_phong_uniforms) <= sizeof(FrontArgs::uni), "uniform copies hold any shader's struct");
+
+int grow_front(euc_ctx *ctx) {
+    if (int rc = grow(ctx->front, sizeof(FrontScratch))) return rc;
+    return grow(ctx->frame_stage, kFrameUni + sizeof(FrontArgs::uni));
+}
+
 // Sizes the scratch and fills k_front's parameter for a planned scene.
 int fill_front(euc_ctx *ctx, const Plan &p, FrontArgs &a) {
     const uint64_t tri = pad_up(p.d.ngroups, kBlock), pix = pad_up((uint64_t)p.d.W * p.d.H, kBlock);
@@ -922,14 +933,11 @@ int fill_front(euc_ctx *ctx, const Plan &p, FrontArgs &a) {
     if ((rc = grow(ctx->cov, sizeof(uint4)))) return rc;
     if ((rc = grow(ctx->plan, 4 * sizeof(uint64_t)))) return rc;
     if ((rc = grow(ctx->totals, 8 * sizeof(unsigned long long)))) return rc;
-    if ((rc = grow(ctx->front, sizeof(FrontScratch)))) return rc;
-    constexpr size_t off_u = (sizeof(SceneDev) + 15) / 16 * 16;
-    static_assert(sizeof(euc_phong_uniforms) <= sizeof(FrontArgs::uni), "uniform copies hold any shader's struct");
-    if ((rc = grow(ctx->frame_stage, off_u + sizeof(FrontArgs::uni)))) return rc;
+    if ((rc = grow_front(ctx))) return rc;
     a.d = p.d;
     a.d.vtx_base = a.d.vd_base = a.d.tri_base = a.d.pix_base = 0;
     a.stage_scene = (SceneDev *)ctx->frame_stage.p;
-    a.stage_uni = (unsigned char *)ctx->frame_stage.p + off_u;
+    a.stage_uni = (unsigned char *)ctx->frame_stage.p + kFrameUni;
     a.d.uniforms = a.stage_uni;
     std::memcpy(a.uni, p.uniforms, p.usize);
     a.usize = (uint32_t)pad_up(p.usize, 4);
@@ -1052,6 +1060,10 @@ int euc_ctx_create(int device, euc_ctx **out) {
         (void)cudaGetLastError();
         delete c;
         return EUC_ERR_CUDA;
+    }
+    if (int rc = grow_front(c)) {
+        euc_ctx_destroy(c);
+        return rc;
     }
     *out = c;
     return EUC_OK;

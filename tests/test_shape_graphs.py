@@ -87,3 +87,35 @@ def test_ordered_scenes_repeat_on_the_plain_path():
             _check(ctx, scenes.soup_frame(seed=5, width=128, height=80, ntris=600, area_hi=900.0, alpha=True))
     finally:
         ctx.close()
+
+
+def test_a_warm_context_renders_a_small_scene_inside_a_capture():
+    """After a larger render (of the batch's kernels: more than 2^20 pixels)
+    a small scene's first render allocates nothing, so that a caller may
+    record it: the recording's replay gives the oracle's image."""
+    import torch
+    from euc_gb300 import frames
+    ctx = capi.Context(0)
+    try:
+        _check(ctx, scenes.sphere_frame(seed=1, width=1100, height=1000))
+        f = scenes.sphere_frame(seed=2, width=200, height=150)
+        df = frames.DeviceFrame(f, "cuda:0")
+        p, uni, keep = df.bound_pass(0)
+        v, i, _ = df.passes[0]
+        pt = frames.tensor_target(df.targets[p.pixel], f.target(p.pixel).fmt)
+        dt = frames.tensor_target(df.targets[p.depth], abi.FMT_R32F)
+        torch.cuda.synchronize()
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g):
+            df.clear()
+            rc = ctx.render(p.desc, uni, p.layout, v.data_ptr(), p.nverts, i.data_ptr(), i.numel(), pt, dt,
+                            frames._stream_ptr(None))
+        assert rc == abi.OK
+        g.replay()
+        g.replay()
+        torch.cuda.synchronize()
+        ref, _ = run_oracle(f)
+        assert_targets_match(f, ref, df.to_host())
+        del keep
+    finally:
+        ctx.close()
