@@ -1915,8 +1915,10 @@ __global__ void __launch_bounds__(kStripThreads, kStripBlocksPerSm) k_strip(cons
     const uint32_t keys_saddr = (uint32_t)__cvta_generic_to_shared(s_keys);
     uint32_t key_bytes;  // the launch's dynamic shared memory
     asm("mov.u32 %0, %%dynamic_smem_size;" : "=r"(key_bytes));
-    for (uint32_t i = tid; i < key_bytes / 8; i += kStripThreads) s_keys[i] = ~0ull;
-    for (;;) {
+    // (no unit: the scenes all went to the item queue.  Leaving the keys alone
+    // then gives k_raster its SMs sooner: 500 k triangle knot 196.3 -> 194.0 us.)
+    for (uint32_t i = tid; nunits && i < key_bytes / 8; i += kStripThreads) s_keys[i] = ~0ull;
+    while (nunits) {
         if (tid == 0) {
             s_u = (uint32_t)atomicAdd(totals + 7, 1ull);
             s_next = 0;
