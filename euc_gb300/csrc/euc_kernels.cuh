@@ -648,12 +648,17 @@ constexpr uint32_t kTinyPixels = 4;
 // a strip), go through k_raster's item queue after the strips.  Which way a
 // primitive goes changes no result: the keys are order-free reductions.
 // ---------------------------------------------------------------------------
-constexpr int kStripThreads = 512;            // threads of a k_strip block
+// Threads of a k_strip block: two blocks of 24 warps, which 40 registers a
+// thread just allow, find more of the walk's issue slots than 2 x 16 (57
+// registers): 1080p soup 481 -> 460 us, 256 scenes 2176 -> 2069, 48 scenes 389
+// -> 382 (18 warps 455 / 2129 / 386, 20 458 / 2098 / 384, 22 462 / 2081 / 383).
+// The shared memory is full too: with 25 warps two blocks no longer fit.
+constexpr int kStripThreads = 768;
 constexpr int kStripBlocksPerSm = 2;          // k_strip blocks resident per SM (its grid)
 constexpr uint32_t kStripMaxRows = 16;        // rows of a strip at most
 constexpr size_t kStripKeyBytes = 96 * 1024;  // a strip's keys in shared memory at most
 constexpr uint32_t kRowsBinned = 0x80000000u; // rows[t]: the primitive went to the strips
-constexpr uint32_t kStripUnit = 1024;         // entries of one strip a k_strip block takes at once at most ...
+constexpr uint32_t kStripUnit = 2 * kStripThreads;  // entries of one strip a k_strip block takes at once at most ...
 constexpr uint32_t kStripUnitMin = 128;       // ... and at least, where a launch has few of them (strip_unit)
 constexpr uint32_t kStripUnitsPerBlock = 3;   // units that each resident block should find
 constexpr uint32_t kStripClaim = 32;          // items a k_strip warp claims at a time
