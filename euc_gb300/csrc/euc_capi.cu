@@ -555,12 +555,15 @@ struct StageOverride {
 
 // The ordered scenes' lists, their counts being in the entries [p0, p1) of
 // vbuf: the counts become list offsets (k_oscan), then `fill(cap)` enqueues the
-// second raster pass and `resolve(cap)` the resolves.  Both are enqueued
-// against the fragment buffer as it is (`cap` fragments), and do nothing when
-// the lists do not fit it; the host waits for the number of fragments alone
-// (while they run), and enqueues them again after growing the buffer.
+// second raster pass and `resolve(cap)` the resolves.  The host waits for the
+// number of fragments alone: the fill is enqueued against the fragment buffer
+// as it is (`cap` fragments), does nothing when the lists do not fit it, and is
+// enqueued again after the buffer has grown.  So are the ordered scenes'
+// resolves, unless they follow others in `resolve` (late): those come when the
+// lists are known to fit, while the fill runs, so that a batch that cannot be
+// drawn for want of list space draws nothing.
 template <class Fill, class Resolve>
-int ordered_lists(euc_ctx *ctx, uint64_t p0, uint64_t p1, cudaStream_t st, Fill fill, Resolve resolve) {
+int ordered_lists(euc_ctx *ctx, uint64_t p0, uint64_t p1, bool late, cudaStream_t st, Fill fill, Resolve resolve) {
     int rc;
     const uint64_t nb = (p1 - p0 + kOScanBlock - 1) / kOScanBlock;
     if ((rc = ensure_host_words(ctx))) return rc;
@@ -574,10 +577,13 @@ int ordered_lists(euc_ctx *ctx, uint64_t p0, uint64_t p1, cudaStream_t st, Fill 
     for (;;) {
         const uint64_t cap = std::min<uint64_t>(ctx->frags.cap / sizeof(uint2), 0xFFFFFFFEull);
         CUDA_TRY(fill(cap));
-        resolve(cap);
+        if (!late) resolve(cap);
         CUDA_TRY(cudaEventSynchronize(ctx->total_ready));
         const unsigned long long nfrag = *(volatile unsigned long long *)ctx->h_words;
-        if (nfrag <= cap) return EUC_OK;
+        if (nfrag <= cap) {
+            if (late) resolve(cap);
+            return EUC_OK;
+        }
         if (nfrag >= 0xFFFFFFFFull) return EUC_ERR_CAPACITY;  // list offsets are 32-bit
         if ((rc = grow(ctx->frags, nfrag * sizeof(uint2)))) return rc;  // (waits for the passes above)
     }
@@ -850,31 +856,30 @@ int run_batch(euc_ctx *ctx, const euc_scene *scenes, size_t n, cudaStream_t st, 
                                (unsigned long long *)ctx->totals.p));
         ctx->launches += 1;
     }
+    // the resolves, group by group: the ordered scenes' last, so that a blended
+    // scene that shares its targets with an opaque one is blended onto it
+    cudaEvent_t e5 = nullptr;
+    auto resolves = [&](uint64_t cap) {
+        if (!e5) e5 = prof_event(ctx, st);
+        for (int a = 0; a < ns;) {
+            int b = a;
+            while (b < ns && group_of(plans[b]) == group_of(plans[a])) ++b;
+            const uint64_t blk0 = res_base[a], blk1 = b < ns ? res_base[b] : res;
+            if (a >= first_ordered)
+                dispatch_resolve_ordered(plans[a].d.shader, dsc, drb, a, b, blk0, blk1 - blk0, cap, ctx, st);
+            else
+                dispatch_resolve(plans[a].d.shader, dsc, rbase, a, b, blk1 - blk0, ctx, st);
+            ctx->launches += blk1 > blk0;
+            a = b;
+        }
+    };
+    rc = EUC_OK;
     if (first_ordered < ns) {
         CUDA_TRY(raster(k_raster<RASTER_COUNT>, 0));
-        rc = ordered_lists(
-            ctx, plans[first_ordered].d.pix_base, pix, st, [&](uint64_t cap) { return raster(k_raster<RASTER_FILL>, cap); },
-            [&](uint64_t cap) {
-                for (int a = first_ordered; a < ns;) {
-                    int b = a;
-                    while (b < ns && group_of(plans[b]) == group_of(plans[a])) ++b;
-                    const uint64_t blk0 = res_base[a], blk1 = b < ns ? res_base[b] : res;
-                    dispatch_resolve_ordered(plans[a].d.shader, dsc, drb, a, b, blk0, blk1 - blk0, cap, ctx, st);
-                    ctx->launches += blk1 > blk0;
-                    a = b;
-                }
-            });
-        if (rc) return rc;
-    }
-    cudaEvent_t e5 = prof_event(ctx, st);
-    for (int a = 0; a < first_ordered;) {  // the ordered scenes are done
-        int b = a;
-        while (b < first_ordered && group_of(plans[b]) == group_of(plans[a])) ++b;
-        const uint64_t blk0 = res_base[a];
-        const uint64_t blk1 = b < ns ? res_base[b] : res;
-        dispatch_resolve(plans[a].d.shader, dsc, rbase, a, b, blk1 - blk0, ctx, st);
-        ctx->launches += blk1 > blk0;
-        a = b;
+        rc = ordered_lists(ctx, plans[first_ordered].d.pix_base, pix, first_ordered > 0, st,
+                           [&](uint64_t cap) { return raster(k_raster<RASTER_FILL>, cap); }, resolves);
+    } else {
+        resolves(0);
     }
     cudaEvent_t e6 = prof_event(ctx, st);
     prof_mark(ctx, EUC_STAGE_VERTEX, e0, e1);
@@ -888,7 +893,7 @@ int run_batch(euc_ctx *ctx, const euc_scene *scenes, size_t n, cudaStream_t st, 
         CUDA_TRY(cudaEventRecord(slot->done, st));
         slot->pending = true;
     }
-    return EUC_OK;
+    return rc;
 }
 
 // ---------------------------------------------------------------------------
@@ -988,7 +993,7 @@ int launch_frame(euc_ctx *ctx, const FrontArgs &a, cudaStream_t st, int *host_er
         CUDA_TRY(raster(k_frame_raster<RASTER_COUNT>, true, 0));
         const uint64_t pix = pad_up((uint64_t)a.d.W * a.d.H, kBlock);
         int rc = ordered_lists(
-            ctx, 0, pix, st, [&](uint64_t cap) { return raster(k_frame_raster<RASTER_FILL>, true, cap); },
+            ctx, 0, pix, false, st, [&](uint64_t cap) { return raster(k_frame_raster<RASTER_FILL>, true, cap); },
             [&](uint64_t cap) {
                 dispatch_resolve_ordered(a.d.shader, sc, (uint64_t *)ctx->plan.p, 0, 1, 0, nblk, cap, ctx, st);
             });

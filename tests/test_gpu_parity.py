@@ -499,3 +499,40 @@ def test_phong_vertices_of_every_layout(gpu_ctx, strip_ctx, order, pad, shift):
         for a, b in zip(got, images("pnu", 0, 0)):
             for name in a:
                 assert np.array_equal(a[name].view(np.uint8), b[name].view(np.uint8)), name
+
+
+@pytest.mark.parametrize("layers", [3, 41])
+@pytest.mark.parametrize("blended_first", [False, True])
+def test_a_batch_draws_its_blended_scenes_over_its_opaque_ones(layers, blended_first):
+    """An opaque and a src-over scene on the same targets and two more on
+    targets of their own, in one batch call: the blended scene lands on the
+    opaque image whatever the order in the call, with lists that fit the first
+    fragment buffer and with lists it has to grow for."""
+    import torch
+    from euc_gb300 import capi, frames
+
+    def make():
+        opaque, blended = _soup(seed=61, w=37, h=19, n=60, hi=150.0)(), _layers(layers)()
+        shared = scenes.FrameSpec("shared", opaque.targets, [opaque.passes[0], blended.passes[0]])
+        return [shared, _soup(seed=62, w=37, h=19, n=200, hi=90.0)(), _layers(layers, seed=63)()]
+    ctx = capi.Context(0)
+    try:
+        dfs = [frames.DeviceFrame(f, "cuda:0") for f in make()]
+        arr, keep = [], []
+        for df in dfs:
+            df.clear()
+            for k in range(len(df.frame.passes)):
+                s, kp = df.scene(k)
+                arr.append(s)
+                keep.append(kp)
+        assert ctx.render_batch(arr[::-1] if blended_first else arr, frames._stream_ptr(None)) == abi.OK
+        assert ctx.sync(frames._stream_ptr(None)) == abi.OK
+        candidates = ctx.stats(frames._stream_ptr(None)).candidates
+        total = 0
+        for f, df in zip(make(), dfs):
+            ref, ref_stats = run_oracle(f)
+            total += sum(s[1] for s in ref_stats)
+            assert_targets_match(f, ref, df.to_host())
+        assert candidates == total
+    finally:
+        ctx.close()
