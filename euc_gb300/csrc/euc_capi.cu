@@ -899,19 +899,11 @@ int run_batch(euc_ctx *ctx, const euc_scene *scenes, size_t n, cudaStream_t st, 
 // ---------------------------------------------------------------------------
 // The frame path (k_front, k_frame_raster, k_resolve): scenes small enough
 // that launches, not work, set their time (k_front's comment has the figures).
-// kFramePrims bounds the groups a block scans; kFramePixels bounds the keys that k_front seeds beyond the
-// covered rectangle (12 bytes a pixel: 12.6 MB, some 2 us beside the setup);
-// kFrameVerts is above three vertices a primitive, so that it is the primitives
-// that decide (640x480 triangle soups, here and on the batch's path, whose
-// strips take them, clears and host included: 32 k of up to 500 px 69 and 83 us,
-// of up to 2000 px 74 and 102, of up to 8000 px 122 and 135).  A
-// batch, a forced strip path and a profiled context take the other kernels.
+// frame_fits has the rule.  A batch, a forced strip path and a profiled context
+// take the other kernels.
 // ---------------------------------------------------------------------------
-constexpr uint64_t kFramePixels = 1ull << 20, kFrameVerts = 1ull << 17;
-
 bool frame_path(const euc_ctx *ctx, const Plan &p) {
-    return p.d.geom == EUC_GEOM_NONE && p.d.ngroups >= 1 && p.d.ngroups <= kFramePrims && p.d.nverts <= kFrameVerts && (uint64_t)p.d.W * p.d.H <= kFramePixels && ctx->tune.strip_path != 2 &&
-           !ctx->profiling;
+    return frame_fits(p.d) && ctx->tune.strip_path != 2 && !ctx->profiling;
 }
 
 // The scratch of a size that no scene changes (some 8 KB), there from the
@@ -974,8 +966,8 @@ int launch_frame(euc_ctx *ctx, const FrontArgs &a, cudaStream_t st, int *host_er
     case EUC_SHADER_PHONG: launch_front<PhongFn>(a, st); break;
     case EUC_SHADER_SHADOW: launch_front<ShadowFn>(a, st); break;
     }
-    // a warp takes 32 items a step; a primitive slot has at most max(W, H) + 2
-    const uint64_t items = (uint64_t)a.d.ngroups * ((uint64_t)std::max(a.d.W, a.d.H) + 2);
+    // a warp takes 32 items a step
+    const uint64_t items = a.d.ngroups * slot_items(a.d);
     const uint64_t busy = items / kBlock + a.nsb;
     const unsigned grid = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(busy, (uint64_t)ctx->nsm * ctx->raster_blocks));
     const SceneDev *const sc = a.stage_scene;

@@ -2600,6 +2600,26 @@ constexpr uint32_t kFrameGroups = 1024;                // 32-primitive groups at
 constexpr uint32_t kFramePrims = 32 * kFrameGroups;
 constexpr uint32_t kFrameBlocks = kFramePrims / kBlock;  // setup blocks at most
 
+constexpr uint64_t kFramePixels = 1ull << 20, kFrameVerts = 1ull << 17;
+
+// Rows (a line's steps) that a primitive slot of the scene has at most.
+__host__ __device__ inline uint64_t slot_items(const SceneDev &s) { return (uint64_t)(s.W > s.H ? s.W : s.H) + 2; }
+
+// The scenes that the frame path takes.  kFramePrims bounds the groups a block
+// scans; kFramePixels the keys that k_front seeds beyond the covered rectangle
+// (12 bytes a pixel: 12.6 MB, some 2 us beside the setup); kFrameVerts is above
+// three vertices a primitive, so that it is the primitives that decide (640x480
+// triangle soups, here and on the batch's path, whose strips take them, clears
+// and host included: 32 k of up to 500 px 69 and 83 us, of up to 2000 px 74 and
+// 102, of up to 8000 px 122 and 135).  kFrameItems: k_frame_raster counts its
+// steps in 32 bits and strides them by the grid's warps (a narrow target of
+// 2^20 rows under 32 k full-height triangles would have 2^32).
+constexpr uint64_t kFrameItems = 1ull << 31;
+__host__ __device__ inline bool frame_fits(const SceneDev &s) {
+    return s.geom == EUC_GEOM_NONE && s.ngroups >= 1 && s.ngroups <= kFramePrims && s.nverts <= kFrameVerts &&
+           (uint64_t)s.W * s.H <= kFramePixels && s.ngroups * slot_items(s) <= kFrameItems;
+}
+
 struct FrontBlock {  // a setup block's sums
     uint4 cov;       // min of (cx0, cy0, ~cx1, ~cy1)
     uint32_t culled, bad;
