@@ -672,7 +672,7 @@ int run_batch(euc_ctx *ctx, const euc_scene *scenes, size_t n, cudaStream_t st, 
     if ((rc = grow(ctx->chunk_sums, nchunks * sizeof(uint2)))) return rc;
     if ((rc = grow(ctx->live_tri, tri * sizeof(uint32_t)))) return rc;
     if ((rc = grow(ctx->live_rowoff, tri * sizeof(uint64_t)))) return rc;
-    if ((rc = grow(ctx->totals, 8 * sizeof(unsigned long long)))) return rc;
+    if ((rc = grow(ctx->totals, kTotals * sizeof(unsigned long long)))) return rc;
     if ((rc = grow(ctx->vbuf, pix * sizeof(unsigned long long)))) return rc;
     if ((rc = grow(ctx->err, ns * sizeof(int)))) return rc;
     if ((rc = grow(ctx->stats, ns * sizeof(SceneStats)))) return rc;
@@ -748,7 +748,7 @@ int run_batch(euc_ctx *ctx, const euc_scene *scenes, size_t n, cudaStream_t st, 
     prep.strip_cnt = (uint32_t *)ctx->strip_cnt.p;
     prep.strip_fill = (uint32_t *)ctx->strip_fill.p;
     prep.totals = (unsigned long long *)ctx->totals.p;
-    prep.n = std::max<uint64_t>((uint64_t)ns, std::max<uint64_t>(nstrips, 2));
+    prep.n = std::max<uint64_t>((uint64_t)ns, std::max<uint64_t>(nstrips, 4));
     prep.nsc = (uint32_t)ns;
     prep.nstrips = (uint32_t)nstrips;
     // vertex stage, one launch per shader kind; the first also does the clears
@@ -809,14 +809,16 @@ int run_batch(euc_ctx *ctx, const euc_scene *scenes, size_t n, cudaStream_t st, 
     const uint64_t ichunks = (pix + kInitChunk - 1) / kInitChunk + ns;  // bounds the chunks plan_chunks counts
     CUDA_TRY(launch_stage(ctx, k_init, chunk_grid(ichunks, ctx->nsm, tu.chunk_group, tu.chunk_blocks_per_sm), kBlock,
                           0, st, dsc, ibase, ns, (const uint4 *)ctx->cov.p, (unsigned long long *)ctx->vbuf.p,
-                          chunk_group(ichunks, ctx->nsm, tu.chunk_group, tu.chunk_blocks_per_sm)));
+                          chunk_group(ichunks, ctx->nsm, tu.chunk_group, tu.chunk_blocks_per_sm),
+                          (unsigned long long *)ctx->totals.p + kInitFlag));
     cudaEvent_t e4 = prof_event(ctx, st);
     // the strip lists, beside k_init (both need only the scans)
     if (nstrips) {
         CUDA_TRY(launch_beside(true, k_bin, bin_grid, kBlock, 0, st, dsc, dcs, nchunks, (const uint32_t *)ctx->rows.p,
                                (const uint4 *)ctx->bbox.p, (const uint4 *)ctx->cov.p, (const SceneStats *)ctx->stats.p,
                                (const uint32_t *)ctx->strip_off.p, (uint32_t *)ctx->strip_fill.p,
-                               (uint2 *)ctx->entries.p, strip_mode));
+                               (uint2 *)ctx->entries.p, strip_mode,
+                               (const unsigned long long *)ctx->totals.p + kInitFlag));
         ctx->launches += 1;
     }
     const int witems = tu.raster_warp_rows ? (int)tu.raster_warp_rows : kWarpItems;
@@ -929,7 +931,7 @@ int fill_front(euc_ctx *ctx, const Plan &p, FrontArgs &a) {
     if ((rc = grow(ctx->stats, sizeof(SceneStats)))) return rc;
     if ((rc = grow(ctx->cov, sizeof(uint4)))) return rc;
     if ((rc = grow(ctx->plan, 4 * sizeof(uint64_t)))) return rc;
-    if ((rc = grow(ctx->totals, 8 * sizeof(unsigned long long)))) return rc;
+    if ((rc = grow(ctx->totals, kTotals * sizeof(unsigned long long)))) return rc;
     if ((rc = grow_front(ctx))) return rc;
     a.d = p.d;
     a.d.vtx_base = a.d.vd_base = a.d.tri_base = a.d.pix_base = 0;
@@ -1104,7 +1106,7 @@ int euc_ctx_reserve(euc_ctx *ctx, uint64_t max_verts, uint64_t max_tris, uint64_
     if ((rc = grow(ctx->chunk_sums, (tri / kBlock + 1) * sizeof(uint2)))) return rc;
     if ((rc = grow(ctx->live_tri, tri * sizeof(uint32_t)))) return rc;
     if ((rc = grow(ctx->live_rowoff, tri * sizeof(uint64_t)))) return rc;
-    if ((rc = grow(ctx->totals, 8 * sizeof(unsigned long long)))) return rc;
+    if ((rc = grow(ctx->totals, kTotals * sizeof(unsigned long long)))) return rc;
     if ((rc = grow(ctx->vbuf, pix * sizeof(unsigned long long)))) return rc;
     if ((rc = grow(ctx->err, ns * sizeof(int)))) return rc;
     if ((rc = grow(ctx->stats, ns * sizeof(SceneStats)))) return rc;
@@ -1898,7 +1900,7 @@ constexpr size_t kNaStage = 4096;  // scene table, bases, uniforms
 constexpr size_t kNaOffErr = kNaStage;
 constexpr size_t kNaOffStats = kNaOffErr + 256;
 constexpr size_t kNaOffTotals = kNaOffStats + 256;
-constexpr size_t kNaOffCov = kNaOffTotals + 64;   // inside the 256-byte totals region
+constexpr size_t kNaOffCov = kNaOffTotals + 96;   // inside the 256-byte totals region
 constexpr size_t kNaOffPlan = kNaOffTotals + 128;  // plan_chunks's 2 x 2 chunk bases, same region
 constexpr size_t kNaOffClip = kNaOffTotals + 256;
 constexpr size_t kNaOffVdata = kNaOffClip + kNaMaxVerts * sizeof(float4);
@@ -1909,6 +1911,7 @@ constexpr size_t kNaOffLiveTri = kNaOffChunks + (kNaMaxGroups / kBlock) * sizeof
 constexpr size_t kNaOffLiveOff = kNaOffLiveTri + kNaMaxGroups * sizeof(uint32_t);
 constexpr size_t kNaOffVbuf = kNaOffLiveOff + kNaMaxGroups * sizeof(uint64_t);
 constexpr size_t kNaBytes = kNaOffVbuf + kNaMaxPixels * sizeof(unsigned long long);
+static_assert(kTotals * sizeof(unsigned long long) <= kNaOffCov - kNaOffTotals, "the rectangle follows the totals");
 static_assert(kNaOffClip % 256 == 0 && kNaOffVdata % 256 == 0 && kNaOffRecs % 256 == 0 && kNaOffRows % 256 == 0 &&
                   kNaOffChunks % 256 == 0 && kNaOffLiveTri % 256 == 0 && kNaOffLiveOff % 256 == 0 &&
                   kNaOffVbuf % 256 == 0,
@@ -2086,7 +2089,7 @@ extern "C" int euc_render_noalloc(const euc_pipeline_desc *desc, const void *uni
     prep.stats = (SceneStats *)(a + kNaOffStats);
     prep.cov = (uint4 *)(a + kNaOffCov);
     prep.totals = (unsigned long long *)(a + kNaOffTotals);
-    prep.n = 2;
+    prep.n = 4;
     prep.nsc = 1;
     k_prep<<<(unsigned)((prep.n + kBlock - 1) / kBlock), kBlock, 0, st>>>(prep);
     t_na_nsm = nsm;
@@ -2106,7 +2109,7 @@ extern "C" int euc_render_noalloc(const euc_pipeline_desc *desc, const void *uni
     const uint64_t ichunks = (pix + kInitChunk - 1) / kInitChunk + 1;
     k_init<<<chunk_grid(ichunks, nsm), kBlock, 0, st>>>(dsc, ibase, 1, (const uint4 *)(a + kNaOffCov),
                                                          (unsigned long long *)(a + kNaOffVbuf),
-                                                         chunk_group(ichunks, nsm));
+                                                         chunk_group(ichunks, nsm), nullptr);
     k_raster<RASTER_KEYS><<<(unsigned)(nsm * raster_blocks_per_sm()), kBlock, 0, st>>>(
         dsc, (const TriRec *)(a + kNaOffRecs), (const uint32_t *)(a + kNaOffLiveTri), (const uint64_t *)(a + kNaOffLiveOff),
         (unsigned long long *)(a + kNaOffTotals), (const int *)(a + kNaOffErr),

@@ -251,16 +251,34 @@ EUC_DEV unsigned long long init_key_min(float d0, bool greater) {
 // starts once every block of the kernel before it has called launch_next (or
 // ended).  begin_stage: the stage waits for the one before it (and so for
 // everything earlier), with its blocks already on the SMs that stage leaves
-// idle at its end, and lets the next stage come in the same way.  A stage that
-// needs nothing of the one before it (k_bin, k_strip) calls launch_next first
-// and wait_previous only before it ends: it runs beside that stage, everything
-// before which has ended, and what follows in the stream comes after both.
+// idle at its end, and lets the next stage come in the same way.
+//
+// A stage that needs nothing of the one before it (k_bin beside k_init, k_strip
+// beside k_raster) begins with begin_beside, lets the next stage come at once
+// and calls wait_previous only before it ends: it runs beside that stage, and
+// what follows in the stream comes after both.  What it reads was complete when
+// the stage beside it passed its own wait, but the wait makes it visible to that
+// grid alone.  So that grid's first thread, having waited, releases a flag, which
+// a thread of each block here acquires before the block's barrier: by causality
+// order all of the block then sees what that thread saw.  A flag that is not set
+// yet costs the overlap and nothing else: the block waits like any other stage.
+// (Flags are cleared with the batch's counters, before its first stage ends.)
 EUC_DEV void launch_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 EUC_DEV void wait_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-EUC_DEV void begin_stage() {
+EUC_DEV void begin_stage(unsigned long long *flag = nullptr) {
     wait_previous();
+    if (flag && blockIdx.x == 0 && threadIdx.x == 0)
+        asm volatile("st.release.gpu.global.u64 [%0], %1;" ::"l"(flag), "l"(1ull) : "memory");
     launch_next();
 }
+EUC_DEV void begin_beside(const unsigned long long *flag) {
+    launch_next();
+    unsigned long long set = 0;
+    if (threadIdx.x == 0) asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(set) : "l"(flag) : "memory");
+    if (!__syncthreads_or(set != 0)) wait_previous();
+}
+// The flags among totals[]: k_init's (read by k_bin), k_raster's (by k_strip).
+constexpr int kInitFlag = 8, kRasterFlag = 9, kTotals = 10;
 
 template <typename T>
 EUC_DEV T warp_incl_scan(T v) {
@@ -304,8 +322,9 @@ EUC_DEV T block_excl_scan(T v, T *smem /* >= kBlock/32 + 1 */, T *total) {
 // ---------------------------------------------------------------------------
 // The per-batch clears before k_setup: each scene's error, statistics and
 // covered rectangle, the strip counts and the strip path's counters
-// (totals[6]: entries taken, totals[7]: k_strip's work counter).  Entry i of
-// the n = max(scenes, strips, 2) covers index i of each.  The first vertex launch of a batch does them (nothing it reads or
+// (totals[6]: entries taken, totals[7]: k_strip's work counter, totals[8] and
+// [9]: the flags of begin_beside).  Entry i of the n = max(scenes, strips, 4)
+// covers index i of each.  The first vertex launch of a batch does them (nothing it reads or
 // writes is cleared), which saves a launch; k_prep does them when a batch has
 // no vertex launch, and on the no-allocation path.
 // ---------------------------------------------------------------------------
@@ -329,7 +348,7 @@ EUC_DEV void prep_clear(const PrepArgs &a, uint64_t i) {
         a.strip_cnt[i] = 0;
         a.strip_fill[i] = 0;
     }
-    if (i < 2) a.totals[6 + i] = 0;
+    if (i < 4) a.totals[6 + i] = 0;
 }
 
 // ---------------------------------------------------------------------------
@@ -1176,8 +1195,9 @@ EUC_DEV int advance_scene(const uint64_t *base, int nsc, int si, uint64_t c) {
 // ibase: the first k_init chunk of every scene (nsc + 1 entries, plan_chunks).
 __global__ void __launch_bounds__(kBlock) k_init(const SceneDev *__restrict__ sc, const uint64_t *__restrict__ ibase,
                                                  int nsc, const uint4 *__restrict__ cov,
-                                                 unsigned long long *__restrict__ vbuf, uint32_t group) {
-    begin_stage();  // (k_bin, which reads nothing this kernel writes, runs beside it)
+                                                 unsigned long long *__restrict__ vbuf, uint32_t group,
+                                                 unsigned long long *__restrict__ flag) {
+    begin_stage(flag);  // (k_bin, which reads nothing this kernel writes, runs beside it)
     const uint64_t nchunks = ibase[nsc];
     for (uint64_t g = blockIdx.x; g * group < nchunks; g += gridDim.x) {
         const uint64_t c0 = g * group;
@@ -1563,7 +1583,8 @@ __global__ void __launch_bounds__(kBlock, 4) k_raster(const SceneDev *__restrict
     constexpr int kCounter = kMode == RASTER_KEYS ? 2 : 3;  // the launch's work counter in totals
     constexpr int kLanes = kRowLanes<kMode>, kItems = 32 / kLanes;  // items of a step
     __shared__ uint64_t s_off[kBlock / 32][kWarpItems];
-    begin_stage();  // (k_strip runs beside it: their keys meet in order-free reductions)
+    // (k_strip runs beside the keys: theirs meet in order-free reductions)
+    begin_stage(kMode == RASTER_KEYS ? totals + kRasterFlag : nullptr);
     if (kMode == RASTER_FILL && totals[4] > frag_cap) return;  // the lists do not fit: the host grows them and comes back
     const int lane = threadIdx.x & 31;
     uint64_t *off = s_off[threadIdx.x >> 5];
@@ -1726,9 +1747,10 @@ __global__ void __launch_bounds__(kBlock) k_bin(const SceneDev *__restrict__ sc,
                                                 const uint4 *__restrict__ bbox, const uint4 *__restrict__ cov,
                                                 const SceneStats *__restrict__ stats,
                                                 const uint32_t *__restrict__ strip_off, uint32_t *__restrict__ strip_fill,
-                                                uint2 *__restrict__ entries, uint32_t strip_mode) {
+                                                uint2 *__restrict__ entries, uint32_t strip_mode,
+                                                const unsigned long long *__restrict__ flag) {
     __shared__ uint32_t s_cnt[kBinHist], s_base[kBinHist];
-    launch_next();
+    begin_beside(flag);
     for (uint64_t c = blockIdx.x; c < nchunks; c += gridDim.x) {  // uniform over the block
         const int si = chunk_scene ? (int)chunk_scene[c] : 0;
         const SceneDev &s = sc[si];
@@ -1913,7 +1935,7 @@ __global__ void __launch_bounds__(kStripThreads, kStripBlocksPerSm) k_strip(cons
     static_assert(2 * kStripThreads == kStripUnit && kStripMaxRows <= 255, "two entries per thread, rows in 8 bits");
     static_assert(kStripMaxRows < 32 && kStripClaim % 32 == 0 && kStripUnit <= 65536,
                   "one table slot per entry at most, claims start at a slot, entries in 16 bits");
-    launch_next();
+    begin_beside(totals + kRasterFlag);
     const int tid = threadIdx.x, lane = tid & 31;
     const uint32_t nstrips = (uint32_t)sbase[nsc];
     const uint32_t nunits = strip_uoff[nstrips], unit = strip_unit(totals[6], gridDim.x);
