@@ -792,7 +792,7 @@ int run_batch(euc_ctx *ctx, const euc_scene *scenes, size_t n, cudaStream_t st, 
         CUDA_TRY(launch_stage(ctx, k_bin_count, bin_grid, kBlock, 0, st, dsc, dcs, nchunks, (uint32_t *)ctx->rows.p,
                               (const uint4 *)ctx->bbox.p, (const uint4 *)ctx->cov.p, (const SceneStats *)ctx->stats.p,
                               (uint2 *)ctx->chunk_sums.p, (uint32_t *)ctx->strip_cnt.p,
-                              (unsigned long long *)ctx->totals.p + 6, entry_cap, strip_mode));
+                              (unsigned long long *)ctx->totals.p + kEntryCount, entry_cap, strip_mode));
         ctx->launches += 1;
     }
     cudaEvent_t e2 = prof_event(ctx, st);
@@ -810,7 +810,7 @@ int run_batch(euc_ctx *ctx, const euc_scene *scenes, size_t n, cudaStream_t st, 
     CUDA_TRY(launch_stage(ctx, k_init, chunk_grid(ichunks, ctx->nsm, tu.chunk_group, tu.chunk_blocks_per_sm), kBlock,
                           0, st, dsc, ibase, ns, (const uint4 *)ctx->cov.p, (unsigned long long *)ctx->vbuf.p,
                           chunk_group(ichunks, ctx->nsm, tu.chunk_group, tu.chunk_blocks_per_sm),
-                          (unsigned long long *)ctx->totals.p + kInitFlag));
+                          (unsigned long long *)ctx->totals.p));
     cudaEvent_t e4 = prof_event(ctx, st);
     // the strip lists, beside k_init (both need only the scans)
     if (nstrips) {
@@ -818,7 +818,7 @@ int run_batch(euc_ctx *ctx, const euc_scene *scenes, size_t n, cudaStream_t st, 
                                (const uint4 *)ctx->bbox.p, (const uint4 *)ctx->cov.p, (const SceneStats *)ctx->stats.p,
                                (const uint32_t *)ctx->strip_off.p, (uint32_t *)ctx->strip_fill.p,
                                (uint2 *)ctx->entries.p, strip_mode,
-                               (const unsigned long long *)ctx->totals.p + kInitFlag));
+                               (const unsigned long long *)ctx->totals.p));
         ctx->launches += 1;
     }
     const int witems = tu.raster_warp_rows ? (int)tu.raster_warp_rows : kWarpItems;

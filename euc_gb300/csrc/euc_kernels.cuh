@@ -163,11 +163,14 @@ static_assert(offsetof(TriRec, bx0) == 48 && offsetof(TriRec, scene) == 88 && of
 // local TriRec, one vector load each instead of a load per field: rows and
 // pixels of one primitive share it, so the loads hit L1 and what limits them
 // is their count.  Unselected fields are left unset.
-EUC_DEV TriRec load_rec(const TriRec *__restrict__ p, uint32_t words) {
+// kNew: by a kernel that was resident while the setup wrote it.
+template <bool kNew = false>
+EUC_DEV TriRec load_rec(const TriRec *p, uint32_t words) {
     const uint4 *q = reinterpret_cast<const uint4 *>(p);
     uint4 w[6];
 #pragma unroll
-    for (int k = 0; k < 6; ++k) w[k] = (words >> k) & 1u ? __ldg(q + k) : make_uint4(0u, 0u, 0u, 0u);
+    for (int k = 0; k < 6; ++k)
+        w[k] = !((words >> k) & 1u) ? make_uint4(0u, 0u, 0u, 0u) : kNew ? q[k] : __ldg(q + k);
     TriRec r;
     r.o[0] = __uint_as_float(w[0].x); r.o[1] = __uint_as_float(w[0].y); r.o[2] = __uint_as_float(w[0].z);
     r.dx[0] = __uint_as_float(w[0].w); r.dx[1] = __uint_as_float(w[1].x); r.dx[2] = __uint_as_float(w[1].y);
@@ -216,7 +219,7 @@ struct SceneStats {
 // ---------------------------------------------------------------------------
 // The largest i < n with base[i] <= pos (base[0] <= pos), by the whole warp:
 // 32-way steps, so that 1024 scenes are two dependent loads away and not ten.
-EUC_DEV int find_scene(const uint64_t *__restrict__ base, int n, uint64_t pos) {
+EUC_DEV int find_scene(const uint64_t *base, int n, uint64_t pos) {
     const int lane = threadIdx.x & 31;
     int lo = 0, hi = n;
     while (hi - lo > 32) {
@@ -261,24 +264,45 @@ EUC_DEV unsigned long long init_key_min(float d0, bool greater) {
 // grid alone.  So that grid's first thread, having waited, releases a flag, which
 // a thread of each block here acquires before the block's barrier: by causality
 // order all of the block then sees what that thread saw.  A flag that is not set
-// yet costs the overlap and nothing else: the block waits like any other stage.
-// (Flags are cleared with the batch's counters, before its first stage ends.)
+// yet costs the overlap and nothing else: the thread waits as in any other stage.
+// The flag is 1 + *count, the work there is for the stage beside, so that a
+// launch with none ends after this one load.  (Flags are cleared with the
+// batch's counters, before its first stage ends.)
+//
+// Read-only loads (__ldg, const __restrict__ parameters) are for data that does
+// not change while the kernel is resident.  A stage is resident while the one
+// before it, and a stage beside that one, still write: what those write is read
+// through plain pointers and loads, which stay behind the wait.
 EUC_DEV void launch_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 EUC_DEV void wait_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-EUC_DEV void begin_stage(unsigned long long *flag = nullptr) {
+EUC_DEV void begin_stage() {
+    wait_previous();
+    launch_next();
+}
+EUC_DEV void begin_stage(unsigned long long *flag, const unsigned long long *count) {
     wait_previous();
     if (flag && blockIdx.x == 0 && threadIdx.x == 0)
-        asm volatile("st.release.gpu.global.u64 [%0], %1;" ::"l"(flag), "l"(1ull) : "memory");
+        asm volatile("st.release.gpu.global.u64 [%0], %1;" ::"l"(flag), "l"(1ull + *count) : "memory");
     launch_next();
 }
-EUC_DEV void begin_beside(const unsigned long long *flag) {
+EUC_DEV unsigned long long begin_beside(const unsigned long long *flag, const unsigned long long *count) {
+    __shared__ unsigned long long s_set;
     launch_next();
-    unsigned long long set = 0;
-    if (threadIdx.x == 0) asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(set) : "l"(flag) : "memory");
-    if (!__syncthreads_or(set != 0)) wait_previous();
+    if (threadIdx.x == 0) {
+        unsigned long long set;
+        asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(set) : "l"(flag) : "memory");
+        if (!set) {
+            wait_previous();
+            set = 1ull + *count;
+        }
+        s_set = set;
+    }
+    __syncthreads();
+    return s_set - 1ull;
 }
-// The flags among totals[]: k_init's (read by k_bin), k_raster's (by k_strip).
-constexpr int kInitFlag = 8, kRasterFlag = 9, kTotals = 10;
+// Of a batch's counters totals[]: the entries that k_bin_count counted, k_strip's
+// units, and the flags of k_init (read by k_bin) and k_raster (by k_strip).
+constexpr int kEntryCount = 6, kInitFlag = 8, kRasterFlag = 9, kUnitCount = 10, kTotals = 11;
 
 template <typename T>
 EUC_DEV T warp_incl_scan(T v) {
@@ -348,7 +372,7 @@ EUC_DEV void prep_clear(const PrepArgs &a, uint64_t i) {
         a.strip_cnt[i] = 0;
         a.strip_fill[i] = 0;
     }
-    if (i < 4) a.totals[6 + i] = 0;
+    if (i < 4) a.totals[kEntryCount + i] = 0;
 }
 
 // ---------------------------------------------------------------------------
@@ -728,7 +752,7 @@ __host__ __device__ inline uint32_t width_bucket(uint32_t w) {
 // ---------------------------------------------------------------------------
 template <class ClipOf>
 EUC_DEV void setup_prim(const SceneDev &s, int si, uint64_t t, ClipOf clip_of, TriRec *__restrict__ recs,
-                        const uint8_t *__restrict__ galive, uint4 *__restrict__ bbox, uint4 *stage, bool &staged,
+                        const uint8_t *galive, uint4 *__restrict__ bbox, uint4 *stage, bool &staged,
                         SetupOut &out) {
     const int lane = threadIdx.x & 31;
     const uint64_t lt = t - s.tri_base;
@@ -987,10 +1011,10 @@ EUC_DEV SetupSums setup_block_sums(const SetupOut &o) {
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(kBlock, 5) k_setup(const SceneDev *__restrict__ sc,
                                                   const uint32_t *__restrict__ chunk_scene,
-                                                  const float4 *__restrict__ clip, TriRec *__restrict__ recs,
+                                                  const float4 *clip, TriRec *__restrict__ recs,
                                                   uint32_t *__restrict__ rows, uint2 *__restrict__ chunk_sums,
                                                   int *__restrict__ err, SceneStats *__restrict__ stats,
-                                                  uint4 *__restrict__ cov, const uint8_t *__restrict__ galive,
+                                                  uint4 *__restrict__ cov, const uint8_t *galive,
                                                   uint4 *__restrict__ bbox) {
     __shared__ uint4 s_rec[kBlock / 32][32 * kRecWords];
     begin_stage();
@@ -1038,7 +1062,7 @@ __global__ void __launch_bounds__(kBlock, 5) k_setup(const SceneDev *__restrict_
 // knot, 500 k triangles, 12.0 + 9.5 -> 9.9 + 7.7 us; 3.8 M primitives 24 -> 20,
 // where the earlier chunks' sums, read again by each block, are most of it).
 // ---------------------------------------------------------------------------
-EUC_DEV void scan_block(const uint32_t *__restrict__ rows, const uint2 *__restrict__ chunk_sums, uint64_t ntri,
+EUC_DEV void scan_block(const uint32_t *rows, const uint2 *chunk_sums, uint64_t ntri,
                         uint32_t *__restrict__ live_tri, uint64_t *__restrict__ live_rowoff,
                         unsigned long long *__restrict__ totals, uint32_t nscan) {
     constexpr int kWarps = kBlock / 32;
@@ -1193,11 +1217,12 @@ EUC_DEV int advance_scene(const uint64_t *base, int nsc, int si, uint64_t c) {
 }
 
 // ibase: the first k_init chunk of every scene (nsc + 1 entries, plan_chunks).
-__global__ void __launch_bounds__(kBlock) k_init(const SceneDev *__restrict__ sc, const uint64_t *__restrict__ ibase,
-                                                 int nsc, const uint4 *__restrict__ cov,
+__global__ void __launch_bounds__(kBlock) k_init(const SceneDev *__restrict__ sc, const uint64_t *ibase,
+                                                 int nsc, const uint4 *cov,
                                                  unsigned long long *__restrict__ vbuf, uint32_t group,
-                                                 unsigned long long *__restrict__ flag) {
-    begin_stage(flag);  // (k_bin, which reads nothing this kernel writes, runs beside it)
+                                                 unsigned long long *__restrict__ totals) {
+    // (k_bin, which reads nothing this kernel writes, runs beside it)
+    begin_stage(totals ? totals + kInitFlag : nullptr, totals + kEntryCount);
     const uint64_t nchunks = ibase[nsc];
     for (uint64_t g = blockIdx.x; g * group < nchunks; g += gridDim.x) {
         const uint64_t c0 = g * group;
@@ -1584,7 +1609,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_raster(const SceneDev *__restrict
     constexpr int kLanes = kRowLanes<kMode>, kItems = 32 / kLanes;  // items of a step
     __shared__ uint64_t s_off[kBlock / 32][kWarpItems];
     // (k_strip runs beside the keys: theirs meet in order-free reductions)
-    begin_stage(kMode == RASTER_KEYS ? totals + kRasterFlag : nullptr);
+    begin_stage(kMode == RASTER_KEYS ? totals + kRasterFlag : nullptr, totals + kUnitCount);
     if (kMode == RASTER_FILL && totals[4] > frag_cap) return;  // the lists do not fit: the host grows them and comes back
     const int lane = threadIdx.x & 31;
     uint64_t *off = s_off[threadIdx.x >> 5];
@@ -1685,9 +1710,9 @@ EUC_DEV bool strip_routed(const SceneDev &s, const SceneStats &st, const uint4 &
 
 __global__ void __launch_bounds__(kBlock) k_bin_count(const SceneDev *__restrict__ sc,
                                                       const uint32_t *__restrict__ chunk_scene, uint64_t nchunks,
-                                                      uint32_t *__restrict__ rows, const uint4 *__restrict__ bbox,
-                                                      const uint4 *__restrict__ cov,
-                                                      const SceneStats *__restrict__ stats,
+                                                      uint32_t *__restrict__ rows, const uint4 *bbox,
+                                                      const uint4 *cov,
+                                                      const SceneStats *stats,
                                                       uint2 *__restrict__ chunk_sums, uint32_t *__restrict__ strip_cnt,
                                                       unsigned long long *__restrict__ nentries, uint64_t entry_cap,
                                                       uint32_t strip_mode) {
@@ -1705,7 +1730,7 @@ __global__ void __launch_bounds__(kBlock) k_bin_count(const SceneDev *__restrict
         const uint32_t nr = rows[t];
         uint32_t q0 = 0, nst = 0;
         if (nr) {
-            const uint4 w3 = __ldg(bbox + t);  // bx0, bx1, by0, by1
+            const uint4 w3 = bbox[t];  // bx0, bx1, by0, by1
             q0 = w3.z / s.strip_h;
             nst = (w3.w - 1) / s.strip_h - q0 + 1;
         }
@@ -1748,10 +1773,10 @@ __global__ void __launch_bounds__(kBlock) k_bin(const SceneDev *__restrict__ sc,
                                                 const SceneStats *__restrict__ stats,
                                                 const uint32_t *__restrict__ strip_off, uint32_t *__restrict__ strip_fill,
                                                 uint2 *__restrict__ entries, uint32_t strip_mode,
-                                                const unsigned long long *__restrict__ flag) {
+                                                const unsigned long long *__restrict__ totals) {
     __shared__ uint32_t s_cnt[kBinHist], s_base[kBinHist];
-    begin_beside(flag);
-    for (uint64_t c = blockIdx.x; c < nchunks; c += gridDim.x) {  // uniform over the block
+    const bool any = begin_beside(totals + kInitFlag, totals + kEntryCount) != 0;
+    for (uint64_t c = blockIdx.x; any && c < nchunks; c += gridDim.x) {  // uniform over the block
         const int si = chunk_scene ? (int)chunk_scene[c] : 0;
         const SceneDev &s = sc[si];
         if (!strip_routed(s, stats[si], cov[si], strip_mode)) continue;
@@ -1935,10 +1960,9 @@ __global__ void __launch_bounds__(kStripThreads, kStripBlocksPerSm) k_strip(cons
     static_assert(2 * kStripThreads == kStripUnit && kStripMaxRows <= 255, "two entries per thread, rows in 8 bits");
     static_assert(kStripMaxRows < 32 && kStripClaim % 32 == 0 && kStripUnit <= 65536,
                   "one table slot per entry at most, claims start at a slot, entries in 16 bits");
-    begin_beside(totals + kRasterFlag);
+    const uint32_t nunits = (uint32_t)begin_beside(totals + kRasterFlag, totals + kUnitCount);
     const int tid = threadIdx.x, lane = tid & 31;
-    const uint32_t nstrips = (uint32_t)sbase[nsc];
-    const uint32_t nunits = strip_uoff[nstrips], unit = strip_unit(totals[6], gridDim.x);
+    const uint32_t unit = strip_unit(totals[kEntryCount], gridDim.x);
     const uint32_t keys_saddr = (uint32_t)__cvta_generic_to_shared(s_keys);
     uint32_t key_bytes;  // the launch's dynamic shared memory
     asm("mov.u32 %0, %%dynamic_smem_size;" : "=r"(key_bytes));
@@ -2226,7 +2250,7 @@ __host__ __device__ inline uint64_t resolve_blocks(const SceneDev &s) {
 
 // Chunk bases of k_init and k_resolve per scene, from the covered rectangles
 // (exclusive prefix sums, nsc + 1 entries each).  One block, any nsc.
-EUC_DEV void plan_chunks(const SceneDev *__restrict__ sc, int nsc, const uint4 *__restrict__ cov,
+EUC_DEV void plan_chunks(const SceneDev *__restrict__ sc, int nsc, const uint4 *cov,
                          uint64_t *__restrict__ ibase, uint64_t *__restrict__ rbase) {
     __shared__ uint64_t s_a[kBlock / 32 + 1];
     uint64_t ci = 0, cr = 0;
@@ -2264,9 +2288,9 @@ EUC_DEV void plan_chunks(const SceneDev *__restrict__ sc, int nsc, const uint4 *
 // of their units (ceil(count / unit)) into unit offsets (nstrips + 1 entries
 // each), and the strip of every unit.  Block b covers strips
 // [b*kScanBlock, (b+1)*kScanBlock) and sums the strips before them itself.
-EUC_DEV void strip_scan_block(uint32_t b, const uint32_t *__restrict__ cnt, uint32_t nstrips, uint32_t unit,
+EUC_DEV void strip_scan_block(uint32_t b, const uint32_t *cnt, uint32_t nstrips, uint32_t unit,
                               uint32_t *__restrict__ off, uint32_t *__restrict__ uoff,
-                              uint32_t *__restrict__ unit_strip) {
+                              uint32_t *__restrict__ unit_strip, unsigned long long *__restrict__ units) {
     __shared__ uint32_t s_a[kBlock / 32 + 1];
     __shared__ uint32_t s_pre[2];
     const uint64_t g0 = (uint64_t)b * kScanBlock;
@@ -2308,6 +2332,7 @@ EUC_DEV void strip_scan_block(uint32_t b, const uint32_t *__restrict__ cnt, uint
     if (g0 + kScanBlock >= nstrips && threadIdx.x == kBlock - 1) {
         off[nstrips] = s_pre[0] + bt;
         uoff[nstrips] = s_pre[1] + btu;
+        *units = s_pre[1] + btu;
     }
 }
 
@@ -2315,21 +2340,22 @@ EUC_DEV void strip_scan_block(uint32_t b, const uint32_t *__restrict__ cnt, uint
 // chunk plan of init / resolve (block nscan, plan_chunks) and the scans of
 // the strips (the blocks after, strip_scan_block): independent work after
 // k_setup, in one launch.
-__global__ void __launch_bounds__(kBlock) k_scan_plan(const uint32_t *__restrict__ rows,
-                                                      const uint2 *__restrict__ chunk_sums, uint64_t ntri,
+__global__ void __launch_bounds__(kBlock) k_scan_plan(const uint32_t *rows,
+                                                      const uint2 *chunk_sums, uint64_t ntri,
                                                       uint32_t *__restrict__ live_tri,
                                                       uint64_t *__restrict__ live_rowoff,
                                                       unsigned long long *__restrict__ totals, uint32_t nscan,
                                                       const SceneDev *__restrict__ sc, int nsc,
-                                                      const uint4 *__restrict__ cov, uint64_t *__restrict__ ibase,
-                                                      uint64_t *__restrict__ rbase, const uint32_t *__restrict__ strip_cnt,
+                                                      const uint4 *cov, uint64_t *__restrict__ ibase,
+                                                      uint64_t *__restrict__ rbase, const uint32_t *strip_cnt,
                                                       uint32_t nstrips, uint32_t strip_blocks,
                                                       uint32_t *__restrict__ strip_off,
                                                       uint32_t *__restrict__ strip_uoff, uint32_t *__restrict__ unit_strip) {
     begin_stage();
     if (blockIdx.x == nscan) plan_chunks(sc, nsc, cov, ibase, rbase);
     else if (blockIdx.x > nscan)
-        strip_scan_block(blockIdx.x - nscan - 1, strip_cnt, nstrips, strip_unit(totals[6], strip_blocks), strip_off, strip_uoff, unit_strip);
+        strip_scan_block(blockIdx.x - nscan - 1, strip_cnt, nstrips, strip_unit(totals[kEntryCount], strip_blocks),
+                         strip_off, strip_uoff, unit_strip, totals + kUnitCount);
     else scan_block(rows, chunk_sums, ntri, live_tri, live_rowoff, totals, nscan);
 }
 
@@ -2366,7 +2392,7 @@ struct ResolveSmem {
 // twice what the shading itself needs).
 template <class F>
 EUC_DEV void resolve_direct_chunk(const SceneDev &s, const uint4 &cv, uint64_t lb, const TriRec *__restrict__ recs,
-                                  const float *__restrict__ vdata, const unsigned long long *__restrict__ vbuf) {
+                                  const float *__restrict__ vdata, const unsigned long long *vbuf) {
     const RowSegment<kDirectSeg> g(cv, (uint32_t)lb);
     const bool kmin = s.keytype == KEY_MIN, greater = s.depth_test == EUC_TEST_GREATER;
     const unsigned long long *keys = vbuf + s.pix_base + (uint64_t)g.y * s.W + g.x;
@@ -2442,7 +2468,7 @@ EUC_DEV bool chunk_pixel(const SceneDev &s, const uint4 &cv, const ChunkGeom &g,
 template <class F>
 EUC_DEV void resolve_chunk(const SceneDev &s, const uint4 &cv, const ChunkGeom &geo, uint64_t lb,
                            const TriRec *__restrict__ recs,
-                           const float *__restrict__ vdata, const unsigned long long *__restrict__ vbuf,
+                           const float *__restrict__ vdata, const unsigned long long *vbuf,
                            ResolveSmem<F> &sm) {
     const int lane = threadIdx.x & 31;
     // 1. this thread's pixel
@@ -2551,11 +2577,11 @@ EUC_DEV void resolve_chunk(const SceneDev &s, const uint4 &cv, const ChunkGeom &
 // chunk of each.
 template <class F>
 __global__ void __launch_bounds__(kBlock, F::kResolveBlocks) k_resolve(const SceneDev *__restrict__ sc,
-                                                                    const uint64_t *__restrict__ rbase,
+                                                                    const uint64_t *rbase,
                                                     int s_begin, int s_end, uint32_t group,
                                                     const TriRec *__restrict__ recs, const float *__restrict__ vdata,
-                                                    const unsigned long long *__restrict__ vbuf,
-                                                    const uint4 *__restrict__ cov) {
+                                                    const unsigned long long *vbuf,
+                                                    const uint4 *cov) {
     // warps work independently: each has its own job list and no block barrier
     __shared__ ResolveSmem<F> s_warp[kBlock / 32];
     begin_stage();
@@ -2735,10 +2761,10 @@ __global__ void __launch_bounds__(kBlock) k_front(const __grid_constant__ FrontA
 }
 
 template <int kMode>
-__global__ void __launch_bounds__(kBlock, 4) k_frame_raster(const SceneDev *__restrict__ sc,
-                                                           const TriRec *__restrict__ recs,
-                                                           const uint32_t *__restrict__ rows,
-                                                           const FrontScratch *__restrict__ front, uint32_t nsb,
+__global__ void __launch_bounds__(kBlock, 4) k_frame_raster(const SceneDev *sc,
+                                                           const TriRec *recs,
+                                                           const uint32_t *rows,
+                                                           const FrontScratch *front, uint32_t nsb,
                                                            int *__restrict__ err, volatile int *__restrict__ host_err,
                                                            SceneStats *__restrict__ stats, uint4 *__restrict__ cov,
                                                            uint64_t *__restrict__ rbase,
@@ -2813,7 +2839,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_frame_raster(const SceneDev *__re
         const uint32_t first = __shfl_sync(0xFFFFFFFFu, incl - nr, p);
         if (i >= __shfl_sync(0xFFFFFFFFu, incl, 31)) continue;
         const uint32_t t = g * 32 + p;
-        const TriRec r = load_rec(recs + t, kRecRaster);
+        const TriRec r = load_rec<true>(recs + t, kRecRaster);
         if (s.prim != EUC_PRIM_TRIANGLE_LIST)
             raster_line_step<kMode>(s, r, t, r.by0 + (i - first), vbuf, cnt, frags, probe);
         else
@@ -3104,8 +3130,8 @@ __global__ void __launch_bounds__(kBlock, F::NV > 4 ? 2 : 3) k_resolve_ordered(c
                                                             int s_end, uint64_t blk_begin,
                                                             const TriRec *__restrict__ recs,
                                                             const float *__restrict__ vdata,
-                                                            const unsigned long long *__restrict__ vbuf,
-                                                            const uint2 *__restrict__ frags, uint64_t frag_cap,
+                                                            const unsigned long long *vbuf,
+                                                            const uint2 *frags, uint64_t frag_cap,
                                                             const unsigned long long *__restrict__ totals,
                                                             const uint4 *__restrict__ cov) {
     __shared__ OrderedSmem s_warp[kBlock / 32];
