@@ -836,9 +836,14 @@ int run_batch(euc_ctx *ctx, const euc_scene *scenes, size_t n, cudaStream_t st, 
     const bool probe = tu.raster_probe == 1;
     int first_ordered = ns;
     while (first_ordered > 0 && plans[first_ordered - 1].d.keytype == KEY_ORDERED) --first_ordered;
+    // A grid that leaves room on the GPU is launched as usual: blocks that come
+    // early are packed onto the SMs that the stage before leaves first, and stay
+    // there (two 640x480 triangles in a batch call 189 us early, 91 us after the
+    // stage before; 300 of 300 k pixels 873 and 327, 200 full targets 1040 and 399).
+    const bool wave = rgrid >= (unsigned)ctx->nsm * (unsigned)ctx->raster_blocks;
     auto raster = [&](auto kernel, uint64_t cap) {
         ctx->launches += 1;
-        return launch_stage(ctx, kernel, rgrid, kBlock, 0, st, dsc, (const TriRec *)ctx->recs.p,
+        return launch_beside(wave && !ctx->capturing, kernel, rgrid, kBlock, 0, st, dsc, (const TriRec *)ctx->recs.p,
                             (const uint32_t *)ctx->live_tri.p, (const uint64_t *)ctx->live_rowoff.p,
                             (unsigned long long *)ctx->totals.p, (const int *)ctx->err.p,
                             (unsigned long long *)ctx->vbuf.p, (SceneStats *)ctx->stats.p, (uint2 *)ctx->frags.p, cap,
