@@ -562,14 +562,18 @@ struct StageOverride {
 // resolves, unless they follow others in `resolve` (late): those come when the
 // lists are known to fit, while the fill runs, so that a batch that cannot be
 // drawn for want of list space draws nothing.
+constexpr uint64_t kFragGuess = 1ull << 23;
 template <class Fill, class Resolve>
 int ordered_lists(euc_ctx *ctx, uint64_t p0, uint64_t p1, bool late, cudaStream_t st, Fill fill, Resolve resolve) {
     int rc;
     const uint64_t nb = (p1 - p0 + kOScanBlock - 1) / kOScanBlock;
     if ((rc = ensure_host_words(ctx))) return rc;
     if (!ctx->total_ready) CUDA_TRY(cudaEventCreateWithFlags(&ctx->total_ready, cudaEventDisableTiming));
-    // a first guess: four fragments a pixel, 512 MB at most
-    if ((rc = grow(ctx->frags, std::min<uint64_t>(4 * p1, 1ull << 26) * sizeof(uint2)))) return rc;
+    // A first guess: four fragments for each pixel of the ordered scenes, 64 MB at
+    // most (1920x1080).  It only saves the first call a second fill: where the
+    // device has no room for it, what is there (nothing, then) is what there is.
+    if ((rc = grow(ctx->frags, std::min<uint64_t>(4 * (p1 - p0), kFragGuess) * sizeof(uint2))) && rc != EUC_ERR_OOM)
+        return rc;
     CUDA_TRY(launch_stage(ctx, k_oscan, (unsigned)nb, kBlock, 0, st, (unsigned long long *)ctx->vbuf.p, p0, p1,
                           (unsigned long long *)ctx->totals.p, ctx->h_words));
     CUDA_TRY(cudaEventRecord(ctx->total_ready, st));

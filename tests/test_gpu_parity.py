@@ -536,3 +536,26 @@ def test_a_batch_draws_its_blended_scenes_over_its_opaque_ones(layers, blended_f
         assert candidates == total
     finally:
         ctx.close()
+
+
+def test_the_fragment_buffer_is_sized_by_the_blended_scenes(gpu_ctx):
+    """A 64x64 blended scene beside large opaque ones takes list space for its
+    own pixels, not for the batch's (8.4 M: 268 MB at four fragments each)."""
+    import torch
+    from euc_gb300 import capi, frames
+    opaque = [scenes.soup_frame(seed=k, width=512, height=512, ntris=50, area_hi=500.0) for k in range(32)]
+    last = [scenes.soup_frame(seed=9, width=64, height=64, ntris=50, area_hi=500.0, alpha=a) for a in (False, True)]
+    batches = [frames.DeviceBatch(opaque + [f]) for f in last]
+    ctx = capi.Context(0)
+    try:
+        frames.render_batch(ctx, batches[0])  # the scratch of every scene, but for the lists
+        torch.cuda.synchronize()
+        before = torch.cuda.mem_get_info()[0]
+        frames.render_batch(ctx, batches[1])
+        torch.cuda.synchronize()
+        assert before - torch.cuda.mem_get_info()[0] < 32 << 20
+        got = batches[1].frames[-1].to_host()
+        ref, _ = run_oracle(last[1])
+        assert_targets_match(last[1], ref, got)
+    finally:
+        ctx.close()
