@@ -379,7 +379,7 @@ int raster_blocks_per_sm() {
     static int n = 0;
     if (n == 0) {
         int b = 0;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_raster<RASTER_KEYS>, kBlock, 0) != cudaSuccess || b < 1) {
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_raster<RASTER_KEYS, 1>, kBlock, 0) != cudaSuccess || b < 1) {
             (void)cudaGetLastError();
             b = 4;
         }
@@ -802,11 +802,15 @@ int run_batch(euc_ctx *ctx, const euc_scene *scenes, size_t n, cudaStream_t st, 
     cudaEvent_t e2 = prof_event(ctx, st);
     uint64_t *const ibase = (uint64_t *)ctx->plan.p, *const rbase = ibase + ns + 1;
     const uint64_t nsblk = (nstrips + kScanBlock - 1) / kScanBlock;
+    int first_ordered = ns;  // the ordered scenes come last
+    while (first_ordered > 0 && plans[first_ordered - 1].d.keytype == KEY_ORDERED) --first_ordered;
+    const bool mixed = first_ordered > 0 && first_ordered < ns;
     CUDA_TRY(launch_stage(ctx, k_scan_plan, (unsigned)(nscan + 1 + nsblk), kBlock, 0, st,
                           (const uint32_t *)ctx->rows.p, (const uint2 *)ctx->chunk_sums.p, tri,
                           (uint32_t *)ctx->live_tri.p, (uint64_t *)ctx->live_rowoff.p,
-                          (unsigned long long *)ctx->totals.p, (uint32_t)nscan, dsc, ns, (const uint4 *)ctx->cov.p,
-                          ibase, rbase, (const uint32_t *)ctx->strip_cnt.p, (uint32_t)nstrips, strip_grid,
+                          (unsigned long long *)ctx->totals.p, (uint32_t)nscan,
+                          mixed ? plans[first_ordered].d.tri_base : tri, dsc, ns, (const uint4 *)ctx->cov.p, ibase,
+                          rbase, (const uint32_t *)ctx->strip_cnt.p, (uint32_t)nstrips, strip_grid,
                           (uint32_t *)ctx->strip_off.p, (uint32_t *)ctx->strip_uoff.p, (uint32_t *)ctx->unit_strip.p));
     cudaEvent_t e3 = prof_event(ctx, st);
     const euc_tuning &tu = ctx->tune;
@@ -826,34 +830,32 @@ int run_batch(euc_ctx *ctx, const euc_scene *scenes, size_t n, cudaStream_t st, 
         ctx->launches += 1;
     }
     const int witems = tu.raster_warp_rows ? (int)tu.raster_warp_rows : kWarpItems;
-    // persistent blocks, but no more than the items can keep busy: a
-    // primitive slot has at most max(W, H) + 2 items (rows, or line steps)
-    uint64_t item_bound = 0;
-    for (int i = 0; i < ns; ++i) {
-        const uint64_t slots = (i + 1 < ns ? plans[i + 1].d.tri_base : tri) - plans[i].d.tri_base;
-        item_bound += slots * ((uint64_t)std::max(plans[i].d.W, plans[i].d.H) + 2);
-    }
-    const uint64_t busy = (item_bound + (uint64_t)witems * (kBlock / 32) - 1) / ((uint64_t)witems * (kBlock / 32));
-    const unsigned rgrid = (unsigned)std::max<uint64_t>(
-        1, std::min<uint64_t>(busy, (uint64_t)ctx->nsm * (tu.raster_blocks_per_sm ? tu.raster_blocks_per_sm
-                                                                                   : (uint32_t)ctx->raster_blocks)));
+    // persistent blocks, but no more than the items of the scenes [a, b) can keep
+    // busy: a primitive slot has at most slot_items of them
+    const uint64_t full = (uint64_t)ctx->nsm * (tu.raster_blocks_per_sm ? tu.raster_blocks_per_sm
+                                                                        : (uint32_t)ctx->raster_blocks);
+    auto slots_of = [&](int i) { return (i + 1 < ns ? plans[i + 1].d.tri_base : tri) - plans[i].d.tri_base; };
+    auto raster_grid = [&](int a, int b, uint64_t items_per_block) {
+        uint64_t items = 0;
+        for (int i = a; i < b; ++i) items += slots_of(i) * slot_items(plans[i].d);
+        return (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(full, (items + items_per_block - 1) / items_per_block));
+    };
     const bool probe = tu.raster_probe == 1;
-    int first_ordered = ns;
-    while (first_ordered > 0 && plans[first_ordered - 1].d.keytype == KEY_ORDERED) --first_ordered;
     // A grid that leaves room on the GPU is launched as usual: blocks that come
     // early are packed onto the SMs that the stage before leaves first, and stay
     // there (two 640x480 triangles in a batch call 189 us early, 91 us after the
     // stage before; 300 of 300 k pixels 873 and 327, 200 full targets 1040 and 399).
-    const bool wave = rgrid >= (unsigned)ctx->nsm * (unsigned)ctx->raster_blocks;
-    auto raster = [&](auto kernel, uint64_t cap) {
+    auto raster = [&](auto kernel, unsigned grid, uint64_t cap) {
+        const bool wave = grid >= (unsigned)ctx->nsm * (unsigned)ctx->raster_blocks;
         ctx->launches += 1;
-        return launch_beside(wave && !ctx->capturing, kernel, rgrid, kBlock, 0, st, dsc, (const TriRec *)ctx->recs.p,
+        return launch_beside(wave && !ctx->capturing, kernel, grid, kBlock, 0, st, dsc, (const TriRec *)ctx->recs.p,
                             (const uint32_t *)ctx->live_tri.p, (const uint64_t *)ctx->live_rowoff.p,
                             (unsigned long long *)ctx->totals.p, (const int *)ctx->err.p,
                             (unsigned long long *)ctx->vbuf.p, (SceneStats *)ctx->stats.p, (uint2 *)ctx->frags.p, cap,
-                            witems, probe);
+                            witems, probe, mixed);
     };
-    if (first_ordered > 0) CUDA_TRY(raster(k_raster<RASTER_KEYS>, 0));
+    if (first_ordered > 0)
+        CUDA_TRY(raster(k_raster<RASTER_KEYS, 1>, raster_grid(0, first_ordered, (uint64_t)witems * (kBlock / 32)), 0));
     ctx->launches += 3;
     // the strips, beside the item queue: k_raster's last warps walk long rows
     // with most of the GPU idle, and k_strip's blocks start there (48-scene
@@ -886,9 +888,21 @@ int run_batch(euc_ctx *ctx, const euc_scene *scenes, size_t n, cudaStream_t st, 
     };
     rc = EUC_OK;
     if (first_ordered < ns) {
-        CUDA_TRY(raster(k_raster<RASTER_COUNT>, 0));
-        rc = ordered_lists(ctx, plans[first_ordered].d.pix_base, pix, first_ordered > 0, st,
-                           [&](uint64_t cap) { return raster(k_raster<RASTER_FILL>, cap); }, resolves);
+        // four lanes a row, unless most of the primitives are lines, whose steps
+        // take one; a warp's claims go down to one step (32 / lanes items)
+        uint64_t lines = 0, tris = 0;
+        for (int i = first_ordered; i < ns; ++i)
+            (plans[i].d.prim == EUC_PRIM_TRIANGLE_LIST ? tris : lines) += plans[i].d.ngroups;
+        const bool wide = tris >= lines;
+        const unsigned grid = raster_grid(first_ordered, ns, wide ? kBlock / kOrderedLanes : kBlock);
+        CUDA_TRY(wide ? raster(k_raster<RASTER_COUNT, kOrderedLanes>, grid, 0) : raster(k_raster<RASTER_COUNT, 1>, grid, 0));
+        rc = ordered_lists(
+            ctx, plans[first_ordered].d.pix_base, pix, mixed, st,
+            [&](uint64_t cap) {
+                return wide ? raster(k_raster<RASTER_FILL, kOrderedLanes>, grid, cap)
+                            : raster(k_raster<RASTER_FILL, 1>, grid, cap);
+            },
+            resolves);
     } else {
         resolves(0);
     }
@@ -1909,7 +1923,7 @@ constexpr size_t kNaStage = 4096;  // scene table, bases, uniforms
 constexpr size_t kNaOffErr = kNaStage;
 constexpr size_t kNaOffStats = kNaOffErr + 256;
 constexpr size_t kNaOffTotals = kNaOffStats + 256;
-constexpr size_t kNaOffCov = kNaOffTotals + 96;   // inside the 256-byte totals region
+constexpr size_t kNaOffCov = kNaOffTotals + 112;   // inside the 256-byte totals region
 constexpr size_t kNaOffPlan = kNaOffTotals + 128;  // plan_chunks's 2 x 2 chunk bases, same region
 constexpr size_t kNaOffClip = kNaOffTotals + 256;
 constexpr size_t kNaOffVdata = kNaOffClip + kNaMaxVerts * sizeof(float4);
@@ -2112,17 +2126,17 @@ extern "C" int euc_render_noalloc(const euc_pipeline_desc *desc, const void *uni
     const uint32_t nscan = (uint32_t)((tri + kScanBlock - 1) / kScanBlock);
     k_scan_plan<<<nscan + 1, kBlock, 0, st>>>((const uint32_t *)(a + kNaOffRows), (const uint2 *)(a + kNaOffChunks),
                                               tri, (uint32_t *)(a + kNaOffLiveTri), (uint64_t *)(a + kNaOffLiveOff),
-                                              (unsigned long long *)(a + kNaOffTotals), nscan, dsc, 1,
+                                              (unsigned long long *)(a + kNaOffTotals), nscan, tri, dsc, 1,
                                               (const uint4 *)(a + kNaOffCov), ibase, rbase, nullptr, 0, 1, nullptr, nullptr,
                                               nullptr);
     const uint64_t ichunks = (pix + kInitChunk - 1) / kInitChunk + 1;
     k_init<<<chunk_grid(ichunks, nsm), kBlock, 0, st>>>(dsc, ibase, 1, (const uint4 *)(a + kNaOffCov),
                                                          (unsigned long long *)(a + kNaOffVbuf),
                                                          chunk_group(ichunks, nsm), nullptr);
-    k_raster<RASTER_KEYS><<<(unsigned)(nsm * raster_blocks_per_sm()), kBlock, 0, st>>>(
+    k_raster<RASTER_KEYS, 1><<<(unsigned)(nsm * raster_blocks_per_sm()), kBlock, 0, st>>>(
         dsc, (const TriRec *)(a + kNaOffRecs), (const uint32_t *)(a + kNaOffLiveTri), (const uint64_t *)(a + kNaOffLiveOff),
         (unsigned long long *)(a + kNaOffTotals), (const int *)(a + kNaOffErr),
-        (unsigned long long *)(a + kNaOffVbuf), (SceneStats *)(a + kNaOffStats), nullptr, 0, kWarpItems, false);
+        (unsigned long long *)(a + kNaOffVbuf), (SceneStats *)(a + kNaOffStats), nullptr, 0, kWarpItems, false, false);
     na_dispatch(false, d.shader, dsc, rbase, resolve_blocks(d), a, st);
     if (device_status)
         CUDA_TRY(cudaMemcpyAsync(device_status, a + kNaOffErr, sizeof(int), cudaMemcpyDeviceToDevice, st));

@@ -301,8 +301,10 @@ EUC_DEV unsigned long long begin_beside(const unsigned long long *flag, const un
     return s_set - 1ull;
 }
 // Of a batch's counters totals[]: the entries that k_bin_count counted, k_strip's
-// units, and the flags of k_init (read by k_bin) and k_raster (by k_strip).
-constexpr int kEntryCount = 6, kInitFlag = 8, kRasterFlag = 9, kUnitCount = 10, kTotals = 11;
+// units, the flags of k_init (read by k_bin) and k_raster (by k_strip), and the
+// live primitives and items before the first ordered scene's (mixed batches).
+constexpr int kEntryCount = 6, kInitFlag = 8, kRasterFlag = 9, kUnitCount = 10, kSplitLive = 11, kSplitItems = 12,
+              kTotals = 13;
 
 template <typename T>
 EUC_DEV T warp_incl_scan(T v) {
@@ -1061,10 +1063,12 @@ __global__ void __launch_bounds__(kBlock, 5) k_setup(const SceneDev *__restrict_
 // both sums are scanned in one word, and one barrier closes it (twelve before:
 // knot, 500 k triangles, 12.0 + 9.5 -> 9.9 + 7.7 us; 3.8 M primitives 24 -> 20,
 // where the earlier chunks' sums, read again by each block, are most of it).
+// tri_split: the first primitive of the ordered scenes, which come last (ntri
+// where there are none, or no others).
 // ---------------------------------------------------------------------------
 EUC_DEV void scan_block(const uint32_t *rows, const uint2 *chunk_sums, uint64_t ntri,
                         uint32_t *__restrict__ live_tri, uint64_t *__restrict__ live_rowoff,
-                        unsigned long long *__restrict__ totals, uint32_t nscan) {
+                        unsigned long long *__restrict__ totals, uint32_t nscan, uint64_t tri_split) {
     constexpr int kWarps = kBlock / 32;
     __shared__ unsigned long long s_l[kWarps], s_r[kWarps], s_w[kWarps];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -1117,6 +1121,10 @@ EUC_DEV void scan_block(const uint32_t *rows, const uint2 *chunk_sums, uint64_t 
     constexpr unsigned long long kLowMask = (1ull << kLow) - 1ull;
     unsigned long long ol = base_l + (before >> kLow), orr = base_r + (before & kLowMask);
     const unsigned long long bl = all >> kLow, br = all & kLowMask;
+    if (t0 == tri_split) {  // (a scene's first primitive: a multiple of kBlock)
+        totals[kSplitLive] = ol;
+        totals[kSplitItems] = orr;
+    }
 #pragma unroll
     for (int k = 0; k < kScanPer; ++k) {
         if (r[k]) {
@@ -1375,11 +1383,11 @@ EUC_DEV bool row_span(const SceneDev &s, const TriRec &r, uint32_t y, uint32_t &
 // lane adds the weights of all four pixels, so it pays where rows are long or
 // few: a small scene's launches (960x540, 8000 triangles: count 32 -> 22 us, fill
 // 45 -> 31; 640x480, 20 k triangles of up to 8000 px 149 -> 91 us; eight lanes 24
-// and 56, two 27 and 37) and the ordered passes, not the item queue's keys (256
-// spheres 190 us by single lanes, 209 by fours).
-template <int kMode>
-constexpr int kRowLanes = kMode == RASTER_KEYS ? 1 : 4;
-constexpr int kFrameLanes = 4;
+// and 56, two 27 and 37) and a batch's ordered passes, not the item queue's keys
+// (256 spheres 190 us by single lanes, 209 by fours).  A step of a line is one
+// pixel and takes one lane (four blended frames of 20 k lines: 186 us, 294 with
+// three lanes in four idle).
+constexpr int kFrameLanes = 4, kOrderedLanes = 4;
 
 // One row of a primitive by kLanes lanes, of which this is lane q: lane q takes
 // the pixels xs + q, xs + q + kLanes, ..., and adds the weights of the others
@@ -1597,42 +1605,49 @@ EUC_DEV void raster_row(const SceneDev &s, const TriRec &r, uint32_t t, uint32_t
 // kWarpItems (a launch-shape choice; results do not depend on it).
 constexpr int kWarpItems = 256;
 
-template <int kMode>
+// mixed: the batch has ordered and other scenes; each launch takes the items of
+// its own, the ordered ones being the last (64 spheres of 640x480 and a blended
+// scene of 64x64: 203 us a call, 300 with three walks over all items).
+template <int kMode, int kLanes>
 __global__ void __launch_bounds__(kBlock, 4) k_raster(const SceneDev *__restrict__ sc, const TriRec *__restrict__ recs,
                                                    const uint32_t *__restrict__ live_tri,
                                                    const uint64_t *__restrict__ live_rowoff,
                                                    unsigned long long *__restrict__ totals,
                                                    const int *__restrict__ err, unsigned long long *__restrict__ vbuf,
                                                    SceneStats *__restrict__ stats, uint2 *__restrict__ frags,
-                                                   uint64_t frag_cap, int witems, bool probe) {
+                                                   uint64_t frag_cap, int witems, bool probe, bool mixed) {
     constexpr int kCounter = kMode == RASTER_KEYS ? 2 : 3;  // the launch's work counter in totals
-    constexpr int kLanes = kRowLanes<kMode>, kItems = 32 / kLanes;  // items of a step
+    constexpr int kItems = 32 / kLanes;                     // items of a step
     __shared__ uint64_t s_off[kBlock / 32][kWarpItems];
     // (k_strip runs beside the keys: theirs meet in order-free reductions)
     begin_stage(kMode == RASTER_KEYS ? totals + kRasterFlag : nullptr, totals + kUnitCount);
     if (kMode == RASTER_FILL && totals[4] > frag_cap) return;  // the lists do not fit: the host grows them and comes back
     const int lane = threadIdx.x & 31;
     uint64_t *off = s_off[threadIdx.x >> 5];
-    const uint64_t nlive = totals[0], nitems = totals[1];
+    // this launch's live primitives [l_first, nlive) and items [first, nitems)
+    const bool keys = kMode == RASTER_KEYS;
+    const uint64_t nlive = mixed && keys ? totals[kSplitLive] : totals[0];
+    const uint64_t nitems = mixed && keys ? totals[kSplitItems] : totals[1];
+    const uint64_t l_first = mixed && !keys ? totals[kSplitLive] : 0, first = mixed && !keys ? totals[kSplitItems] : 0;
     // Few items for the grid (a small scene): smaller claims, down to one
     // step, so that every warp gets some instead of a few warps walking
     // many steps each (uniform over the grid: it depends on nitems alone)
     {
         const uint64_t nwarps = (uint64_t)gridDim.x * (kBlock / 32);
-        const uint64_t fair = (nitems + nwarps - 1) / nwarps;
-        if (fair < (uint64_t)witems) witems = (int)max((uint64_t)32, (fair + 31) / 32 * 32);
+        const uint64_t fair = (nitems - first + nwarps - 1) / nwarps;
+        if (fair < (uint64_t)witems) witems = (int)max((uint64_t)kItems, (fair + kItems - 1) / kItems * kItems);
     }
     // Warps beyond the number of chunks would only find the counter exhausted;
     // they leave at once instead of queueing on its atomic.
     const uint64_t gwarp = (uint64_t)blockIdx.x * (kBlock / 32) + (threadIdx.x >> 5);
-    if (gwarp * witems >= nitems) return;
+    if (gwarp * witems >= nitems - first) return;
     for (;;) {
         unsigned long long base = 0;
         if (lane == 0) base = atomicAdd(totals + kCounter, (unsigned long long)witems);
-        base = __shfl_sync(0xFFFFFFFFu, base, 0);
+        base = first + __shfl_sync(0xFFFFFFFFu, base, 0);
         if (base >= nitems) break;
         // largest l with live_rowoff[l] <= base; invariant off(lo) <= base < off(hi)
-        uint64_t lo = 0, hi = nlive;
+        uint64_t lo = l_first, hi = nlive;
         while (hi - lo > 32) {
             const uint64_t step = (hi - lo + 31) / 32;
             const uint64_t at = lo + lane * step;
@@ -1673,7 +1688,6 @@ __global__ void __launch_bounds__(kBlock, 4) k_raster(const SceneDev *__restrict
             const TriRec r = load_rec(recs + t, kRecRaster);
             const uint32_t scene = r.scene;
             if (err[scene]) continue;
-            if ((sc[scene].keytype == KEY_ORDERED) != (kMode != RASTER_KEYS)) continue;  // another launch's scene
             uint32_t cnt = 0;
             raster_row<kMode, kLanes>(sc[scene], r, t, r.by0 + (uint32_t)(i - off[a]), vbuf, cnt, frags, probe, lane % kLanes);
             if (scene0 == 0xFFFFFFFFu) scene0 = scene;
@@ -2345,7 +2359,7 @@ __global__ void __launch_bounds__(kBlock) k_scan_plan(const uint32_t *rows,
                                                       uint32_t *__restrict__ live_tri,
                                                       uint64_t *__restrict__ live_rowoff,
                                                       unsigned long long *__restrict__ totals, uint32_t nscan,
-                                                      const SceneDev *__restrict__ sc, int nsc,
+                                                      uint64_t tri_split, const SceneDev *__restrict__ sc, int nsc,
                                                       const uint4 *cov, uint64_t *__restrict__ ibase,
                                                       uint64_t *__restrict__ rbase, const uint32_t *strip_cnt,
                                                       uint32_t nstrips, uint32_t strip_blocks,
@@ -2356,7 +2370,7 @@ __global__ void __launch_bounds__(kBlock) k_scan_plan(const uint32_t *rows,
     else if (blockIdx.x > nscan)
         strip_scan_block(blockIdx.x - nscan - 1, strip_cnt, nstrips, strip_unit(totals[kEntryCount], strip_blocks),
                          strip_off, strip_uoff, unit_strip, totals + kUnitCount);
-    else scan_block(rows, chunk_sums, ntri, live_tri, live_rowoff, totals, nscan);
+    else scan_block(rows, chunk_sums, ntri, live_tri, live_rowoff, totals, nscan, tri_split);
 }
 
 // The clears of prep_clear as a launch of their own (n threads).

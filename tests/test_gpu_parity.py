@@ -559,3 +559,37 @@ def test_the_fragment_buffer_is_sized_by_the_blended_scenes(gpu_ctx):
         assert_targets_match(last[1], ref, got)
     finally:
         ctx.close()
+
+
+@pytest.mark.parametrize("parts", ["KO", "KkOo", "KkOoL", "KLL", "OoL", "EO", "KE", "KeL", "eK"])
+def test_batches_of_ordered_and_other_scenes(parts):
+    """Each raster launch of a mixed batch takes the items of its own scenes:
+    opaque ones (K, k), blended triangles (O, o) and lines (L), and scenes none
+    of whose primitives has a row (E opaque, e blended), in one call on a fresh
+    context, twice (the second with the buffers of the first)."""
+    from euc_gb300 import capi, frames
+    off = np.tile(np.array([5.0, 5.0, 0.5, 1.0], dtype=np.float32), (300, 1))
+    kinds = {
+        "K": lambda: scenes.soup_frame(seed=1, width=200, height=120, ntris=3000, area_hi=300.0),
+        "k": lambda: scenes.lines_frame(seed=2, width=97, height=61, nlines=300, len_hi=60.0),
+        "O": lambda: scenes.soup_frame(seed=3, width=150, height=90, ntris=700, area_hi=900.0, alpha=True),
+        "o": lambda: scenes.soup_frame(seed=4, width=33, height=17, ntris=257, area_hi=300.0, alpha=True),
+        "L": lambda: scenes.lines_frame(seed=5, width=128, height=65, nlines=2000, len_hi=90.0, alpha=True),
+        "E": lambda: scenes.clip_triangles_frame(off, np.zeros((300, 4), np.uint8), 64, 64),
+        "e": lambda: scenes.clip_triangles_frame(off, np.zeros((300, 4), np.uint8), 64, 64, blend=abi.BLEND_ALPHA),
+    }
+    ctx = capi.Context(0)
+    try:
+        for _ in range(2):
+            made = [kinds[c]() for c in parts]
+            dfs = [frames.DeviceFrame(f, "cuda:0") for f in made]
+            frames.render_batch(ctx, dfs)
+            assert ctx.sync(frames._stream_ptr(None)) == abi.OK
+            candidates, total = ctx.stats(frames._stream_ptr(None)).candidates, 0
+            for f, df in zip(made, dfs):
+                ref, ref_stats = run_oracle(f)
+                total += ref_stats[0][1]
+                assert_targets_match(f, ref, df.to_host())
+            assert candidates == total
+    finally:
+        ctx.close()
