@@ -302,8 +302,9 @@ enum euc_stage {
  * changes a result, only how work is spread over the GPU; 0 keeps the
  * default.  Set by an autotuner that times a batch under several shapes.   */
 typedef struct euc_tuning {
-    uint32_t raster_blocks_per_sm; /* persistent k_raster blocks per SM (default: occupancy limit) */
-    uint32_t raster_warp_rows;     /* (primitive, row) items a warp claims at once, 32..256, x32 (256) */
+    uint32_t raster_blocks_per_sm; /* persistent raster blocks per SM (default: occupancy limit)     */
+    uint32_t raster_warp_rows;     /* (primitive, row) items a warp claims at once, 32..256, x32 (256);
+                                    * a small scene's raster claims none: its warps stride the items  */
     uint32_t chunk_group;          /* 256-pixel chunks per scene lookup in init/resolve (adaptive)   */
     uint32_t chunk_blocks_per_sm;  /* init/resolve grid cap per SM (16)                              */
     uint32_t raster_probe;         /* 1: read a key before its atomicMin, 2: atomics only (default)  */
@@ -325,7 +326,8 @@ int euc_ctx_get_tuning(euc_ctx *ctx, euc_tuning *tuning);
 /* Profiling aid (no counterpart in euc): while enabled, each render records
  * CUDA events around its stages on its own stream.  euc_ctx_profile waits for
  * them, returns the summed milliseconds per stage and the number of kernel
- * launches issued since the last call, and resets both.                     */
+ * launches issued since the last call, and resets both.  A profiled context
+ * renders small scenes with the batch's kernels, whose stages are apart.    */
 int euc_ctx_set_profiling(euc_ctx *ctx, int enable);
 int euc_ctx_profile(euc_ctx *ctx, double ms[EUC_STAGE_COUNT], uint64_t *launches);
 
