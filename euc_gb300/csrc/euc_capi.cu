@@ -819,7 +819,8 @@ int run_batch(euc_ctx *ctx, const euc_scene *scenes, size_t n, cudaStream_t st, 
                           (uint32_t *)ctx->strip_off.p, (uint32_t *)ctx->strip_uoff.p, (uint32_t *)ctx->unit_strip.p));
     cudaEvent_t e3 = prof_event(ctx, st);
     const euc_tuning &tu = ctx->tune;
-    const uint64_t ichunks = (pix + kInitChunk - 1) / kInitChunk + ns;  // bounds the chunks plan_chunks counts
+    uint64_t ichunks = 0;  // bounds the chunks plan_chunks counts
+    for (const Plan &p : plans) ichunks += init_blocks(p.d);
     CUDA_TRY(launch_stage(ctx, k_init, chunk_grid(ichunks, ctx->nsm, tu.chunk_group, tu.chunk_blocks_per_sm), kBlock,
                           0, st, dsc, ibase, ns, (const uint4 *)ctx->cov.p, (unsigned long long *)ctx->vbuf.p,
                           chunk_group(ichunks, ctx->nsm, tu.chunk_group, tu.chunk_blocks_per_sm),
@@ -2140,7 +2141,7 @@ extern "C" int euc_render_noalloc(const euc_pipeline_desc *desc, const void *uni
                                               (unsigned long long *)(a + kNaOffTotals), nscan, tri, dsc, 1,
                                               (const uint4 *)(a + kNaOffCov), ibase, rbase, nullptr, 0, 1, nullptr, nullptr,
                                               nullptr);
-    const uint64_t ichunks = (pix + kInitChunk - 1) / kInitChunk + 1;
+    const uint64_t ichunks = init_blocks(d);
     k_init<<<chunk_grid(ichunks, nsm), kBlock, 0, st>>>(dsc, ibase, 1, (const uint4 *)(a + kNaOffCov),
                                                          (unsigned long long *)(a + kNaOffVbuf),
                                                          chunk_group(ichunks, nsm), nullptr);

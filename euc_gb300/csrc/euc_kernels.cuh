@@ -1165,29 +1165,52 @@ __host__ __device__ inline uint64_t rect_area(const uint4 &c) {
 // is spent on pixels that no primitive reaches.
 constexpr int kChunkGroup = 16;
 
-// The covered rectangle cut into segments of at most kSeg pixels of one row,
-// one a warp (chunk lb of kBlock / 32 segments): a lane's pixels are 32 apart
+// The covered rectangle cut into segments of at most 32 kPer pixels of one row,
+// one a warp (chunk lb of kBlock / 32 segments): a lane's kPer pixels are 32 apart
 // in the segment, so the row's addresses are computed once and a pixel costs
 // no division or wrap.  256 spheres of 640x480 (86 k pixels of the rectangle
 // each): k_init 71 -> 57 us (45 -> 24 M instructions), k_resolve<GouraudFn>
 // 214 -> 203 us (130 -> 108 M; what bounds it now is L1, 84 % busy).
-template <int kSeg>
+// A rectangle of at most 16 kPer columns gives a row as few lanes (a power of
+// two) as hold it, and a warp the next rows too: 4 x 100000 pixels 34 us a frame
+// against 62 with a warp a row, 16 x 32768 30 and 38, 64 x 8192 27 and 33.
+template <int kPer>
+__host__ __device__ inline bool narrow_rect(uint32_t w) { return w <= 16 * kPer; }
+template <int kPer>
+__host__ __device__ inline uint32_t segment_shift(uint32_t w) {  // log2 of a row's lanes, w > 0
+    uint32_t shift = 0;
+    for (uint32_t q = (w - 1) / kPer; q; q >>= 1) ++shift;
+    return shift;
+}
+template <int kPer>
 struct RowSegment {
     uint32_t y, x, xend;  // the row, this lane's first pixel, the end of the row or segment
+    uint32_t step;        // between this lane's pixels
     EUC_DEV RowSegment(const uint4 &cv, uint32_t lb) {
-        const uint32_t nseg = (~cv.z - cv.x + kSeg - 1) / kSeg;
-        const uint32_t u = lb * (kBlock / 32) + (threadIdx.x >> 5), row = u / nseg;
-        y = cv.y + row;
-        const uint32_t x0 = cv.x + (u - row * nseg) * kSeg;
-        xend = y < ~cv.w ? min(x0 + kSeg, ~cv.z) : 0u;  // (a warp beyond the last segment has none)
-        x = x0 + (threadIdx.x & 31);
+        const uint32_t w = ~cv.z - cv.x, u = lb * (kBlock / 32) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+        if (narrow_rect<kPer>(w)) {
+            const uint32_t shift = segment_shift<kPer>(w);
+            step = 1u << shift;
+            y = cv.y + ((u * 32 + lane) >> shift);
+            x = cv.x + (lane & (step - 1));
+            xend = y < ~cv.w ? ~cv.z : 0u;  // (a lane beyond the last row has none)
+        } else {
+            constexpr uint32_t kSeg = 32 * kPer;
+            const uint32_t nseg = (w + kSeg - 1) / kSeg, row = u / nseg, x0 = cv.x + (u - row * nseg) * kSeg;
+            step = 32;
+            y = cv.y + row;
+            x = x0 + lane;
+            xend = y < ~cv.w ? min(x0 + kSeg, ~cv.z) : 0u;  // (a warp beyond the last segment has none)
+        }
     }
 };
-template <int kSeg>
+template <int kPer>
 __host__ __device__ inline uint64_t segment_chunks(const uint4 &cv) {
     if (rect_area(cv) == 0) return 0;
-    const uint64_t nseg = (~cv.z - cv.x + kSeg - 1) / kSeg;
-    return (nseg * (~cv.w - cv.y) + kBlock / 32 - 1) / (kBlock / 32);
+    const uint64_t w = ~cv.z - cv.x, rows = ~cv.w - cv.y;
+    const uint64_t warps = narrow_rect<kPer>((uint32_t)w) ? ((rows << segment_shift<kPer>((uint32_t)w)) + 31) / 32
+                                                          : (w + 32 * kPer - 1) / (32 * kPer) * rows;
+    return (warps + kBlock / 32 - 1) / (kBlock / 32);
 }
 
 // Entries i0, i0 + kBlock, i0 + 2 kBlock, ... of a row-major rectangle rw
@@ -1215,8 +1238,15 @@ struct RectWalk {
 // A lane of k_init initialises kInitPer entries of a row segment, its depth
 // loads in flight together.  kInitChunk: entries of a chunk at most.
 constexpr int kInitPer = 8;
-constexpr int kInitSeg = 32 * kInitPer;
 constexpr int kInitChunk = kBlock * kInitPer;
+
+// k_init chunks of a scene: the row segments of its covered rectangle; every
+// entry, padding included, of an ordered one.
+__host__ __device__ inline uint64_t init_chunks(const SceneDev &s, const uint4 &cv) {
+    if (s.keytype != KEY_ORDERED) return segment_chunks<kInitPer>(cv);
+    const uint64_t lim = ((uint64_t)s.W * s.H + kBlock - 1) / kBlock * kBlock;
+    return (lim + kInitChunk - 1) / kInitChunk;
+}
 
 // Scene of chunk `c` given the scene of an earlier chunk of the same group.
 EUC_DEV int advance_scene(const uint64_t *base, int nsc, int si, uint64_t c) {
@@ -1262,15 +1292,15 @@ __global__ void __launch_bounds__(kBlock) k_init(const SceneDev *__restrict__ sc
             const uint8_t *const depth = s.depth;
             const bool kmin = s.keytype == KEY_MIN, greater = s.depth_test == EUC_TEST_GREATER;
             for (; lb < lend; ++lb) {
-                const RowSegment<kInitSeg> g(cv, lb);
+                const RowSegment<kInitPer> g(cv, lb);
                 unsigned long long *key = keys + (uint64_t)g.y * W + g.x;
                 const float *d0 = reinterpret_cast<const float *>(depth + (uint64_t)g.y * dpitch) + g.x;
                 float d[kInitPer];
 #pragma unroll
-                for (int k = 0; k < kInitPer; ++k) d[k] = kmin && g.x + 32 * k < g.xend ? d0[32 * k] : 0.0f;
+                for (int k = 0; k < kInitPer; ++k) d[k] = kmin && g.x + g.step * k < g.xend ? d0[g.step * k] : 0.0f;
 #pragma unroll
                 for (int k = 0; k < kInitPer; ++k)
-                    if (g.x + 32 * k < g.xend) key[32 * k] = kmin ? init_key_min(d[k], greater) : ~0ull;
+                    if (g.x + g.step * k < g.xend) key[g.step * k] = kmin ? init_key_min(d[k], greater) : ~0ull;
             }
         }
     }
@@ -2230,7 +2260,6 @@ constexpr uint32_t kDirectShaders = (FlatFn::kDirect ? 1u << EUC_SHADER_FLAT : 0
 // Scenes resolved kDirectPer pixels per thread with no shared memory: depth
 // only, or a cheap shader without MSAA.
 constexpr int kDirectPer = 4;
-constexpr int kDirectSeg = 32 * kDirectPer;
 __host__ __device__ inline bool resolve_direct(const SceneDev &s) {
     return s.keytype != KEY_ORDERED &&
            (!s.pixel_write || (s.level == 0 && ((kDirectShaders >> s.shader) & 1u)));
@@ -2242,7 +2271,7 @@ __host__ __device__ inline bool resolve_direct(const SceneDev &s) {
 __host__ __device__ inline uint64_t resolve_chunks(const SceneDev &s, const uint4 &cv) {
     const uint64_t area = rect_area(cv);
     if (area == 0) return 0;
-    if (resolve_direct(s)) return segment_chunks<kDirectSeg>(cv);
+    if (resolve_direct(s)) return segment_chunks<kDirectPer>(cv);
     if (resolve_by_quads(s)) {
         const uint64_t pairs = pair_of_row(~cv.w - 1, s.gr) - pair_of_row(cv.y, s.gr) + 1;
         const uint64_t cols = ((~cv.z - 1) >> 4) - (cv.x >> 4) + 1;
@@ -2251,16 +2280,18 @@ __host__ __device__ inline uint64_t resolve_chunks(const SceneDev &s, const uint
     return (area + kBlock - 1) / kBlock;
 }
 
-// Upper bound of resolve_chunks over every rectangle (the whole target), for
-// sizing launches on the host.
-__host__ __device__ inline uint64_t resolve_blocks(const SceneDev &s) {
+// Upper bounds of resolve_chunks and init_chunks over every rectangle (the whole
+// target), for sizing launches on the host.
+__host__ __device__ inline uint4 whole_target(const SceneDev &s) {
     uint4 full;
     full.x = 0;
     full.y = 0;
     full.z = ~s.W;
     full.w = ~s.H;
-    return resolve_chunks(s, full);
+    return full;
 }
+__host__ __device__ inline uint64_t resolve_blocks(const SceneDev &s) { return resolve_chunks(s, whole_target(s)); }
+__host__ __device__ inline uint64_t init_blocks(const SceneDev &s) { return init_chunks(s, whole_target(s)); }
 
 // Chunk bases of k_init and k_resolve per scene, from the covered rectangles
 // (exclusive prefix sums, nsc + 1 entries each).  One block, any nsc.
@@ -2274,13 +2305,8 @@ EUC_DEV void plan_chunks(const SceneDev *__restrict__ sc, int nsc, const uint4 *
         if (si < nsc) {
             const SceneDev &s = sc[si];
             const uint4 cv = cov[si];
-            if (s.keytype == KEY_ORDERED) {  // every entry; k_resolve_ordered sizes itself
-                const uint64_t lim = ((uint64_t)s.W * s.H + kBlock - 1) / kBlock * kBlock;
-                ni = (lim + kInitChunk - 1) / kInitChunk;
-            } else {
-                ni = segment_chunks<kInitSeg>(cv);
-                nr = resolve_chunks(s, cv);
-            }
+            ni = init_chunks(s, cv);
+            if (s.keytype != KEY_ORDERED) nr = resolve_chunks(s, cv);  // (k_resolve_ordered sizes itself)
         }
         uint64_t ti, tr;
         const uint64_t ei = block_excl_scan<uint64_t>(ni, s_a, &ti);
@@ -2407,12 +2433,12 @@ struct ResolveSmem {
 template <class F>
 EUC_DEV void resolve_direct_chunk(const SceneDev &s, const uint4 &cv, uint64_t lb, const TriRec *__restrict__ recs,
                                   const float *__restrict__ vdata, const unsigned long long *vbuf) {
-    const RowSegment<kDirectSeg> g(cv, (uint32_t)lb);
+    const RowSegment<kDirectPer> g(cv, (uint32_t)lb);
     const bool kmin = s.keytype == KEY_MIN, greater = s.depth_test == EUC_TEST_GREATER;
     const unsigned long long *keys = vbuf + s.pix_base + (uint64_t)g.y * s.W + g.x;
     unsigned long long key[kDirectPer];
 #pragma unroll
-    for (int k = 0; k < kDirectPer; ++k) key[k] = g.x + 32 * k < g.xend ? keys[32 * k] : kmin ? 0ull : ~0ull;
+    for (int k = 0; k < kDirectPer; ++k) key[k] = g.x + g.step * k < g.xend ? keys[g.step * k] : kmin ? 0ull : ~0ull;
     float *const drow = s.depth_write ? reinterpret_cast<float *>(s.depth + (uint64_t)g.y * s.dpitch) : nullptr;
     uint8_t *const prow = s.pixel_write ? s.pixel + (uint64_t)g.y * s.ppitch : nullptr;
     const uint32_t pfmt = s.pfmt;
@@ -2425,7 +2451,7 @@ EUC_DEV void resolve_direct_chunk(const SceneDev &s, const uint4 &cv, uint64_t l
         uint32_t t;
         float z;
         if (!decode_key(kmin, greater, key[k], t, z)) continue;
-        const uint32_t x = g.x + 32 * k;
+        const uint32_t x = g.x + g.step * k;
         if (drow) drow[x] = z;
         if (!prow) continue;
         if constexpr (F::kDirect) {

@@ -593,3 +593,28 @@ def test_batches_of_ordered_and_other_scenes(parts):
             assert candidates == total
     finally:
         ctx.close()
+
+
+@pytest.mark.parametrize("w,h", [(1, 700), (3, 401), (4, 64), (5, 333), (8, 33), (9, 100), (16, 257), (17, 65), (63, 40),
+                                 (64, 33), (65, 33), (127, 20), (128, 9), (129, 9)])
+@pytest.mark.parametrize("test,write", [(abi.TEST_LESS, 1), (abi.TEST_NONE, 0)])
+def test_narrow_targets(gpu_ctx, strip_ctx, w, h, test, write):
+    """Covered rectangles at the edges of the lanes that a row of the key seeds
+    (eight pixels a lane) and of the resolve (four) takes, at the target's left
+    edge and off it, on both raster paths."""
+    def make(k):
+        f = _layers(4, w=w + 5 * k, h=h, blend=abi.BLEND_REPLACE, depth_test=test, depth_write=write)()
+        if k:  # the last w columns of the target only
+            clip = np.zeros((6, 4), dtype=np.float32)
+            x0 = 2.0 * 5 / (w + 5) - 1.0
+            clip[:, :2] = [(x0, -1), (1, -1), (x0, 1), (1, -1), (1, 1), (x0, 1)]
+            clip[:, 2:] = [0.25, 1.0]
+            f = scenes.clip_triangles_frame(clip, np.arange(24, dtype=np.uint8).reshape(6, 4), w + 5, h,
+                                            depth_test=test, depth_write=write)
+        return f
+    for k in (0, 1):
+        ref, ref_stats = run_oracle(make(k))
+        for ctx in (gpu_ctx, strip_ctx):
+            got, got_stats = run_gpu(ctx, make(k))
+            assert got_stats == ref_stats
+            assert_targets_match(make(k), ref, got)
