@@ -867,10 +867,11 @@ int run_batch(euc_ctx *ctx, const euc_scene *scenes, size_t n, cudaStream_t st, 
     // with most of the GPU idle, and k_strip's blocks start there (48-scene
     // batch, a whole call: 578 us one after the other, 490 us with both)
     if (nstrips) {
-        CUDA_TRY(launch_beside(true, k_strip, strip_grid, kStripThreads, strip_smem, st, dsc, dsb, ns,
+        CUDA_TRY(launch_beside(true, k_strip<false>, strip_grid, kStripThreads, strip_smem, st, dsc, dsb, ns,
                                (const uint4 *)ctx->cov.p, (const uint32_t *)ctx->strip_off.p,
                                (const uint32_t *)ctx->strip_uoff.p, (const uint32_t *)ctx->unit_strip.p,
-                               (const uint2 *)ctx->entries.p, (const TriRec *)ctx->recs.p, (const int *)ctx->err.p,
+                               (const uint2 *)ctx->entries.p, nullptr, (const TriRec *)ctx->recs.p,
+                               (const int *)ctx->err.p,
                                (unsigned long long *)ctx->vbuf.p, (SceneStats *)ctx->stats.p,
                                (unsigned long long *)ctx->totals.p));
         ctx->launches += 1;
@@ -945,6 +946,18 @@ bool frame_path(const euc_ctx *ctx, const Plan &p) {
 constexpr size_t kFrameUni = (sizeof(SceneDev) + 15) / 16 * 16;  // the uniforms' place in frame_stage
 static_assert(sizeof(euc_phong_uniforms) <= sizeof(FrontArgs::uni), "uniform copies hold any shader's struct");
 
+// Whether k_strip<true> follows a scene's k_frame_raster, which leaves it the
+// work if there is enough of it (kFrameStripFrags).  The launch costs 2 us where
+// there is not (8192 triangles of 30 px 30.8 -> 32.7), so it is for the scenes that
+// a batch may send to its strips (kStripMinPixels), from kFrameStripPrims
+// primitives, and drawn without culling: what is culled by winding are the
+// closed meshes, whose front faces hardly cover a pixel more than a few times.
+bool frame_strips(const euc_ctx *ctx, const SceneDev &d) {
+    return d.prim == EUC_PRIM_TRIANGLE_LIST && d.keytype != KEY_ORDERED && d.cull == EUC_CULL_NONE &&
+           ctx->tune.strip_path == 0 && d.ngroups >= kFrameStripPrims &&
+           (uint64_t)d.ntris * kStripMinPixels >= (uint64_t)d.W * d.H;
+}
+
 int grow_front(euc_ctx *ctx) {
     if (int rc = grow(ctx->front, sizeof(FrontScratch))) return rc;
     return grow(ctx->frame_stage, kFrameUni + sizeof(FrontArgs::uni));
@@ -966,6 +979,8 @@ int fill_front(euc_ctx *ctx, const Plan &p, FrontArgs &a) {
     if ((rc = grow_front(ctx))) return rc;
     a.d = p.d;
     a.d.vtx_base = a.d.vd_base = a.d.tri_base = a.d.pix_base = 0;
+    a.d.strip_h = frame_strips(ctx, p.d) ? strip_rows(p.d.W, p.d.H) : 0u;
+    a.d.nstrips = (uint32_t)ctx->nsm * kStripBlocksPerSm;  // (k_strip<true>'s blocks)
     a.stage_scene = (SceneDev *)ctx->frame_stage.p;
     a.stage_uni = (unsigned char *)ctx->frame_stage.p + kFrameUni;
     a.d.uniforms = a.stage_uni;
@@ -1019,16 +1034,26 @@ int launch_frame(euc_ctx *ctx, const FrontArgs &a, cudaStream_t st, int *host_er
     const uint64_t nblk = resolve_blocks(a.d);
     ctx->launches += 2;
     if (a.d.keytype == KEY_ORDERED) {
-        CUDA_TRY(raster(k_frame_raster<RASTER_COUNT>, true, 0));
+        CUDA_TRY(raster(k_frame_raster<RASTER_COUNT, false>, true, 0));
         const uint64_t pix = pad_up((uint64_t)a.d.W * a.d.H, kBlock);
         int rc = ordered_lists(
-            ctx, 0, pix, false, st, [&](uint64_t cap) { return raster(k_frame_raster<RASTER_FILL>, true, cap); },
+            ctx, 0, pix, false, st, [&](uint64_t cap) { return raster(k_frame_raster<RASTER_FILL, false>, true, cap); },
             [&](uint64_t cap) {
                 dispatch_resolve_ordered(a.d.shader, sc, (uint64_t *)ctx->plan.p, 0, 1, 0, nblk, cap, ctx, st);
             });
         if (rc) return rc;
     } else {
-        CUDA_TRY(raster(k_frame_raster<RASTER_KEYS>, true, 0));
+        if (!a.d.strip_h) {
+            CUDA_TRY(raster(k_frame_raster<RASTER_KEYS, false>, true, 0));
+        } else {
+            CUDA_TRY(raster(k_frame_raster<RASTER_KEYS, true>, true, 0));
+            const size_t smem = (size_t)a.d.strip_h * strip_pitch(a.d.W) * sizeof(unsigned long long);
+            CUDA_TRY(launch_beside(true, k_strip<true>, a.d.nstrips, kStripThreads, smem, st, sc, nullptr, 1,
+                                   (const uint4 *)ctx->cov.p, nullptr, nullptr, nullptr, nullptr,
+                                   (const uint32_t *)a.rows, (const TriRec *)a.recs, (const int *)ctx->err.p, a.vbuf,
+                                   (SceneStats *)ctx->stats.p, (unsigned long long *)ctx->totals.p));
+            ctx->launches += 1;
+        }
         dispatch_resolve(a.d.shader, sc, (uint64_t *)ctx->plan.p, 0, 1, nblk, ctx, st);
     }
     CUDA_TRY(cudaGetLastError());
@@ -1090,7 +1115,8 @@ int euc_ctx_create(int device, euc_ctx **out) {
     }
     c->pageable = pageable != 0;
     // k_strip's keys: up to kStripKeyBytes of dynamic shared memory
-    if (cudaFuncSetAttribute(k_strip, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kStripKeyBytes) != cudaSuccess) {
+    if (cudaFuncSetAttribute(k_strip<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kStripKeyBytes) != cudaSuccess ||
+        cudaFuncSetAttribute(k_strip<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kStripKeyBytes) != cudaSuccess) {
         (void)cudaGetLastError();
         delete c;
         return EUC_ERR_CUDA;

@@ -710,6 +710,19 @@ constexpr uint32_t kStripClaim = 32;          // items a k_strip warp claims at 
 constexpr uint64_t kStripOverdraw = 4;        // fragments per covered pixel that route a scene to the strips ...
 constexpr uint64_t kStripTriFrags = 16;       // ... when its triangles make this many fragments each on average
 constexpr uint64_t kStripMinPixels = 64;      // target pixels per primitive above which a scene stays off them
+constexpr uint32_t kFrameGroups = 1024;       // 32-primitive groups of a small scene at most (frame_fits)
+constexpr uint32_t kFramePrims = 32 * kFrameGroups;
+// A small scene goes to the strips with this many fragments (its triangles'
+// screen areas) and more, the more the larger its target is, whose keys each
+// unit merges.  k_frame_raster and k_strip<true>, us a frame with clears: 640x480,
+// 16384 triangles of 1000 px 94 / 109, 2000 px 141 / 140, 5000 px 295 / 207, 30000
+// px 1430 / 596; 1024x1024, of 2000 px 151 / 167, 3000 px 199 / 190, 30000 px 1545
+// / 661; 320x240, 8192 of 2000 px 95 / 100, 3000 px 128 / 113, 30000 px 698 / 283.
+// (Through a batch's bins and strips those with 30000 px take 628, 690 and 296.)
+constexpr unsigned long long kFrameStripFrags = 16ull << 20, kFrameStripPerPixel = 28;
+// Fewer primitives than this stay with k_frame_raster, without the launch of
+// k_strip (4096 triangles of 30 px 29 us, of 30000 px 352 at 320x240).
+constexpr uint32_t kFrameStripPrims = 8192;
 constexpr uint32_t kBinHist = 1024;           // strips of a scene the binning kernels count in shared memory
 
 // Keys per row of a strip w pixels wide in shared memory: an odd count, so
@@ -1970,28 +1983,47 @@ EUC_DEV uint32_t strip_block_scan(uint32_t v, uint32_t *smem /* >= kStripThreads
     return r;
 }
 
+// The strips of a small scene that k_strip<true> walks (k_frame_raster leaves it
+// the scenes with kFrameStripFrags fragments or more): those that the covered
+// rectangle meets, each in as many ranges of primitives as give every resident
+// block kStripUnitsPerBlock units.  A unit finds its strip's primitives in its
+// range by itself, so that there are no lists to make.
+struct FrameStrips {
+    uint32_t first, strips, ranges;  // the first strip, how many, ranges of each
+    EUC_DEV FrameStrips(const SceneDev &s, const uint4 &cv, uint32_t blocks) {
+        first = cv.y / s.strip_h;
+        strips = (~cv.w - 1u) / s.strip_h - first + 1u;
+        ranges = (blocks * kStripUnitsPerBlock + strips - 1u) / strips;
+    }
+};
+
 // ---------------------------------------------------------------------------
 // k_strip: one unit (up to strip_unit entries of one strip) at a time per
-// block, claimed from a work counter (totals[7]).  sbase: the first strip of
-// each scene (nsc + 1 entries).  The unit's keys over the strip's rows inside
+// block, claimed from a work counter (totals[7]).  kFrame: a small scene's
+// (FrameStrips), whose unit is a strip and a range of primitives: it packs those
+// that meet the strip, up to kStripUnit of them at a time, and walks them until
+// the range is done.  sbase: the first strip of each scene (nsc + 1 entries).  The unit's keys over the strip's rows inside
 // the scene's covered rectangle start at ~0 in shared memory; the warps
 // claim runs of kStripClaim items of its entries from a shared counter and
 // walk them with shared-memory reductions; every key the unit lowered is
 // then merged into vbuf (which k_init seeded) with one 64-bit min and put
 // back to ~0 for the next unit.
 // ---------------------------------------------------------------------------
+template <bool kFrame>
 __global__ void __launch_bounds__(kStripThreads, kStripBlocksPerSm) k_strip(const SceneDev *__restrict__ sc,
                                                             const uint64_t *__restrict__ sbase, int nsc,
-                                                            const uint4 *__restrict__ cov,
+                                                            const uint4 *cov,
                                                             const uint32_t *__restrict__ strip_off,
                                                             const uint32_t *__restrict__ strip_uoff,
                                                             const uint32_t *__restrict__ unit_strip,
                                                             const uint2 *__restrict__ entries,
+                                                            const uint32_t *__restrict__ rows,
                                                             const TriRec *__restrict__ recs,
-                                                            const int *__restrict__ err,
+                                                            const int *err,
                                                             unsigned long long *__restrict__ vbuf,
                                                             SceneStats *__restrict__ stats,
-                                                            unsigned long long *__restrict__ totals) {
+                                                            unsigned long long *totals) {
+    static_assert(kFramePrims <= 1u << 15 && kStripMaxRows < 32, "a frame's entries are packed in a word");
     extern __shared__ unsigned long long s_keys[];  // rows [r0, r1) x columns [cx0, cx1) of the strip
     __shared__ uint32_t s_pref[kStripUnit];         // first item of each entry of the unit (in width order)
     __shared__ uint32_t s_t[kStripUnit];            // its primitive
@@ -2004,9 +2036,16 @@ __global__ void __launch_bounds__(kStripThreads, kStripBlocksPerSm) k_strip(cons
     static_assert(2 * kStripThreads == kStripUnit && kStripMaxRows <= 255, "two entries per thread, rows in 8 bits");
     static_assert(kStripMaxRows < 32 && kStripClaim % 32 == 0 && kStripUnit <= 65536,
                   "one table slot per entry at most, claims start at a slot, entries in 16 bits");
-    const uint32_t nunits = (uint32_t)begin_beside(totals + kRasterFlag, totals + kUnitCount);
+    uint32_t nunits;
+    if constexpr (kFrame) {
+        launch_next();
+        wait_previous();
+        nunits = (uint32_t)totals[kUnitCount];
+    } else {
+        nunits = (uint32_t)begin_beside(totals + kRasterFlag, totals + kUnitCount);
+    }
     const int tid = threadIdx.x, lane = tid & 31;
-    const uint32_t unit = strip_unit(totals[kEntryCount], gridDim.x);
+    const uint32_t unit = kFrame ? 0u : strip_unit(totals[kEntryCount], gridDim.x);
     const uint32_t keys_saddr = (uint32_t)__cvta_generic_to_shared(s_keys);
     uint32_t key_bytes;  // the launch's dynamic shared memory
     asm("mov.u32 %0, %%dynamic_smem_size;" : "=r"(key_bytes));
@@ -2021,115 +2060,156 @@ __global__ void __launch_bounds__(kStripThreads, kStripBlocksPerSm) k_strip(cons
         __syncthreads();
         const uint32_t u = s_u;
         if (u >= nunits) break;
-        const uint32_t g = unit_strip[u];
-        const int si = find_scene(sbase, nsc, g);
+        const uint32_t g = kFrame ? 0u : unit_strip[u];
+        const int si = kFrame ? 0 : find_scene(sbase, nsc, g);
         const SceneDev &s = sc[si];
         const uint4 cv = cov[si];
-        const uint32_t s0 = (g - s.strip_base) * s.strip_h;
+        uint32_t s0, pos = 0, end = 0;  // the strip's first row; a frame's primitives still to be looked at
+        if constexpr (kFrame) {
+            const FrameStrips f(s, cv, gridDim.x);
+            const uint32_t range = u / f.strips, per = (s.ngroups + f.ranges - 1) / f.ranges;
+            s0 = (f.first + (u - range * f.strips)) * s.strip_h;
+            pos = range * per;
+            end = min(pos + per, s.ngroups);
+        } else {
+            s0 = (g - s.strip_base) * s.strip_h;
+        }
         // every entry's rows lie in the strip and in the covered rectangle
         const uint32_t r0 = max(s0, cv.y), r1 = min(min(s0 + s.strip_h, s.H), ~cv.w);
         const uint32_t cx0 = cv.x, cx1 = ~cv.z;
         const bool empty = r0 >= r1 || cx0 >= cx1;  // never for a strip with entries
         const uint32_t wc = empty ? 0u : cx1 - cx0, area = empty ? 0u : (r1 - r0) * strip_pitch(wc);
         const uint32_t pitch = strip_pitch(wc);
-        const uint32_t e_begin = strip_off[g] + (u - strip_uoff[g]) * unit;
-        const int nload = (int)(min(e_begin + unit, strip_off[g + 1]) - e_begin);
-        // the unit's entries, two per thread, ordered by the span of their
-        // middle row in the strip, widest first (a counting sort over
-        // kWidthBuckets): the rows a warp walks together have about the same
-        // length, and the short ones come last, so that the warps reach the
-        // unit's closing barrier together
-        if (tid < (int)kWidthBuckets) s_bkt[tid] = 0;
-        uint2 ev[2];
-        uint32_t bk[2], rk[2];
-        __syncthreads();
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            const int k = 2 * tid + h;
-            ev[h] = make_uint2(0u, 0u);
-            bk[h] = 0xFFFFFFFFu;
-            if (k < nload) {
-                ev[h] = entries[e_begin + k];
-                // the span of the entry's middle row in this strip: the bbox
-                // width where every row spans it, else the edge intersections
-                TriRec rs = load_rec(recs + ev[h].x, 0x38u);  // words 3-5
-                uint32_t xs = rs.bx0, xe = rs.bx1;
-                if (!(rs.flags & kTriFullRows)) {
-                    const uint32_t ya = ev[h].y >> 16, yb = ev[h].y & 0xFFFFu;
-                    bool full;
-                    if (!row_span(s, rs, s0 + ((ya + yb) >> 1), xs, xe, full)) xe = xs;
-                }
-                bk[h] = kWidthBuckets - 1u - width_bucket(xe - xs);  // widest first
-            }
-            const uint32_t m = __match_any_sync(0xFFFFFFFFu, bk[h]);
-            const int leader = __ffs(m) - 1;
-            uint32_t base = 0;
-            if (bk[h] != 0xFFFFFFFFu && lane == leader) base = atomicAdd(s_bkt + bk[h], (uint32_t)__popc(m));
-            rk[h] = __shfl_sync(0xFFFFFFFFu, base, leader) + __popc(m & ((1u << lane) - 1u));
-        }
-        __syncthreads();
-        if (tid < 32) {  // bucket sizes -> first positions
-            static_assert(kWidthBuckets == 64, "two buckets per lane");
-            const uint32_t c0 = s_bkt[2 * lane], c1 = s_bkt[2 * lane + 1];
-            const uint32_t inc = warp_incl_scan(c0 + c1);
-            s_bkt[2 * lane] = inc - c0 - c1;
-            s_bkt[2 * lane + 1] = inc - c1;
-        }
-        __syncthreads();
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            if (bk[h] == 0xFFFFFFFFu) continue;
-            const uint32_t d = s_bkt[bk[h]] + rk[h];
-            s_t[d] = ev[h].x;
-            s_ya[d] = (uint8_t)(ev[h].y >> 16);
-            s_nr[d] = (uint8_t)((ev[h].y & 0xFFFFu) - (ev[h].y >> 16));
-        }
-        __syncthreads();
-        const uint32_t n0 = 2 * tid < nload ? s_nr[2 * tid] : 0u, n1 = 2 * tid + 1 < nload ? s_nr[2 * tid + 1] : 0u;
-        uint32_t total;
-        const uint32_t pre = strip_block_scan(n0 + n1, s_scan, &total);
-        s_pref[2 * tid] = pre;
-        s_pref[2 * tid + 1] = pre + n0;
-        // an entry has at most kStripMaxRows < 32 items, so at most one
-        // multiple of 32 falls in its range
-        if (n0 && ((pre + 31u) & ~31u) < pre + n0) s_first[(pre + 31u) >> 5] = (uint16_t)(2 * tid);
-        if (n1 && ((pre + n0 + 31u) & ~31u) < pre + n0 + n1) s_first[(pre + n0 + 31u) >> 5] = (uint16_t)(2 * tid + 1);
-        __syncthreads();
         uint32_t cnt = 0;
-        if (!err[si] && !empty) {  // a scene with a bad index draws nothing
-            for (;;) {
-                uint32_t i0 = 0;
-                if (lane == 0) i0 = atomicAdd(&s_next, kStripClaim);
-                i0 = __shfl_sync(0xFFFFFFFFu, i0, 0);
-                if (i0 >= total) break;
-                int a0 = s_first[i0 >> 5];  // the entry of item i0 (a multiple of kStripClaim)
-                const uint32_t iend = min(total, i0 + kStripClaim);
-                // 32 consecutive items at a time: their entries are a run from
-                // a0 (every entry has at least one row)
-                for (uint32_t j0 = i0; j0 < iend; j0 += 32) {
-                    const int c = a0 + 1 + lane;
-                    uint32_t bit = 0;
-                    if (lane < 31 && c < nload) {
-                        const uint32_t o = s_pref[c];
-                        if (o > j0 && o < j0 + 32) bit = 1u << (o - j0);
+        for (bool more = true; more;) {
+            uint32_t e_begin = 0;
+            int nload = 0;
+            if constexpr (kFrame) {
+                // the next primitives that meet the strip, up to a unit of them
+                while (pos < end && nload + kStripThreads <= (int)kStripUnit) {
+                    const uint32_t t = pos + tid;
+                    bool hit = t < end && rows[t];
+                    uint32_t ya = 0, yb = 0;
+                    if (hit) {
+                        const uint4 w3 = __ldg(reinterpret_cast<const uint4 *>(recs + t) + 3);  // bx0, bx1, by0, by1
+                        ya = max(w3.z, s0) - s0;
+                        yb = min(w3.w, s0 + s.strip_h) - s0;
+                        hit = w3.z < s0 + s.strip_h && w3.w > s0;
                     }
-                    const uint32_t starts = __reduce_or_sync(0xFFFFFFFFu, bit);
-                    const int a = a0 + __popc(starts & ((2u << lane) - 1u));
-                    const int alast = a0 + __popc(starts);
-                    a0 = (alast + 1 < nload && s_pref[alast + 1] == j0 + 32) ? alast + 1 : alast;
-                    const uint32_t i = j0 + lane;
-                    if (i >= iend) continue;
-                    const uint32_t t = s_t[a];
-                    const uint32_t y = s0 + s_ya[a] + (i - s_pref[a]);
-                    const TriRec r = load_rec(recs + t, kRecRaster);
-                    uint32_t xs, xe;
-                    bool full;
-                    if (!row_span(s, r, y, xs, xe, full)) continue;
-                    strip_walk_row(s, r, t, y, xs, xe, keys_saddr + 8u * ((y - r0) * pitch) - 8u * cx0, cnt);
+                    uint32_t found;
+                    const uint32_t at = strip_block_scan(hit ? 1u : 0u, s_scan, &found);
+                    if (hit) s_pref[nload + at] = t | ya << 15 | yb << 20;
+                    nload += (int)found;
+                    pos += kStripThreads;
+                }
+                more = pos < end;
+                if (tid == 0) s_next = 0;
+            } else {
+                e_begin = strip_off[g] + (u - strip_uoff[g]) * unit;
+                nload = (int)(min(e_begin + unit, strip_off[g + 1]) - e_begin);
+                more = false;
+            }
+            // the unit's entries, two per thread, ordered by the span of their
+            // middle row in the strip, widest first (a counting sort over
+            // kWidthBuckets): the rows a warp walks together have about the same
+            // length, and the short ones come last, so that the warps reach the
+            // unit's closing barrier together
+            if (tid < (int)kWidthBuckets) s_bkt[tid] = 0;
+            uint2 ev[2];
+            uint32_t bk[2], rk[2];
+            __syncthreads();
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int k = 2 * tid + h;
+                ev[h] = make_uint2(0u, 0u);
+                bk[h] = 0xFFFFFFFFu;
+                if (k < nload) {
+                    if constexpr (kFrame) {
+                        const uint32_t e = s_pref[k];
+                        ev[h] = make_uint2(e & 0x7FFFu, (e >> 15 & 31u) << 16 | e >> 20);
+                    } else {
+                        ev[h] = entries[e_begin + k];
+                    }
+                    // the span of the entry's middle row in this strip: the bbox
+                    // width where every row spans it, else the edge intersections
+                    TriRec rs = load_rec(recs + ev[h].x, 0x38u);  // words 3-5
+                    uint32_t xs = rs.bx0, xe = rs.bx1;
+                    if (!(rs.flags & kTriFullRows)) {
+                        const uint32_t ya = ev[h].y >> 16, yb = ev[h].y & 0xFFFFu;
+                        bool full;
+                        if (!row_span(s, rs, s0 + ((ya + yb) >> 1), xs, xe, full)) xe = xs;
+                    }
+                    bk[h] = kWidthBuckets - 1u - width_bucket(xe - xs);  // widest first
+                }
+                const uint32_t m = __match_any_sync(0xFFFFFFFFu, bk[h]);
+                const int leader = __ffs(m) - 1;
+                uint32_t base = 0;
+                if (bk[h] != 0xFFFFFFFFu && lane == leader) base = atomicAdd(s_bkt + bk[h], (uint32_t)__popc(m));
+                rk[h] = __shfl_sync(0xFFFFFFFFu, base, leader) + __popc(m & ((1u << lane) - 1u));
+            }
+            __syncthreads();
+            if (tid < 32) {  // bucket sizes -> first positions
+                static_assert(kWidthBuckets == 64, "two buckets per lane");
+                const uint32_t c0 = s_bkt[2 * lane], c1 = s_bkt[2 * lane + 1];
+                const uint32_t inc = warp_incl_scan(c0 + c1);
+                s_bkt[2 * lane] = inc - c0 - c1;
+                s_bkt[2 * lane + 1] = inc - c1;
+            }
+            __syncthreads();
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                if (bk[h] == 0xFFFFFFFFu) continue;
+                const uint32_t d = s_bkt[bk[h]] + rk[h];
+                s_t[d] = ev[h].x;
+                s_ya[d] = (uint8_t)(ev[h].y >> 16);
+                s_nr[d] = (uint8_t)((ev[h].y & 0xFFFFu) - (ev[h].y >> 16));
+            }
+            __syncthreads();
+            const uint32_t n0 = 2 * tid < nload ? s_nr[2 * tid] : 0u, n1 = 2 * tid + 1 < nload ? s_nr[2 * tid + 1] : 0u;
+            uint32_t total;
+            const uint32_t pre = strip_block_scan(n0 + n1, s_scan, &total);
+            s_pref[2 * tid] = pre;
+            s_pref[2 * tid + 1] = pre + n0;
+            // an entry has at most kStripMaxRows < 32 items, so at most one
+            // multiple of 32 falls in its range
+            if (n0 && ((pre + 31u) & ~31u) < pre + n0) s_first[(pre + 31u) >> 5] = (uint16_t)(2 * tid);
+            if (n1 && ((pre + n0 + 31u) & ~31u) < pre + n0 + n1) s_first[(pre + n0 + 31u) >> 5] = (uint16_t)(2 * tid + 1);
+            __syncthreads();
+            if (!err[si] && !empty) {  // a scene with a bad index draws nothing
+                for (;;) {
+                    uint32_t i0 = 0;
+                    if (lane == 0) i0 = atomicAdd(&s_next, kStripClaim);
+                    i0 = __shfl_sync(0xFFFFFFFFu, i0, 0);
+                    if (i0 >= total) break;
+                    int a0 = s_first[i0 >> 5];  // the entry of item i0 (a multiple of kStripClaim)
+                    const uint32_t iend = min(total, i0 + kStripClaim);
+                    // 32 consecutive items at a time: their entries are a run from
+                    // a0 (every entry has at least one row)
+                    for (uint32_t j0 = i0; j0 < iend; j0 += 32) {
+                        const int c = a0 + 1 + lane;
+                        uint32_t bit = 0;
+                        if (lane < 31 && c < nload) {
+                            const uint32_t o = s_pref[c];
+                            if (o > j0 && o < j0 + 32) bit = 1u << (o - j0);
+                        }
+                        const uint32_t starts = __reduce_or_sync(0xFFFFFFFFu, bit);
+                        const int a = a0 + __popc(starts & ((2u << lane) - 1u));
+                        const int alast = a0 + __popc(starts);
+                        a0 = (alast + 1 < nload && s_pref[alast + 1] == j0 + 32) ? alast + 1 : alast;
+                        const uint32_t i = j0 + lane;
+                        if (i >= iend) continue;
+                        const uint32_t t = s_t[a];
+                        const uint32_t y = s0 + s_ya[a] + (i - s_pref[a]);
+                        const TriRec r = load_rec(recs + t, kRecRaster);
+                        uint32_t xs, xe;
+                        bool full;
+                        if (!row_span(s, r, y, xs, xe, full)) continue;
+                        strip_walk_row(s, r, t, y, xs, xe, keys_saddr + 8u * ((y - r0) * pitch) - 8u * cx0, cnt);
+                    }
                 }
             }
+            __syncthreads();
         }
-        __syncthreads();
         // merge the keys this unit lowered (the padding column is never
         // written) and put them back to ~0; key i is at row i / pitch, column
         // i % pitch, stepped by kStripThreads without a division
@@ -2153,7 +2233,7 @@ __global__ void __launch_bounds__(kStripThreads, kStripBlocksPerSm) k_strip(cons
         if (lane == 0 && wsum) atomicAdd(&stats[si].candidates, (unsigned long long)wsum);
         __syncthreads();
     }
-    wait_previous();
+    if constexpr (!kFrame) wait_previous();
 }
 
 // ---------------------------------------------------------------------------
@@ -2680,12 +2760,12 @@ __global__ void __launch_bounds__(kBlock, F::kResolveBlocks) k_resolve(const Sce
 //                   block 0 also finishes the scene's
 //                   covered rectangle, error and culled count for
 //   k_resolve<F>    as in a batch
+// and between the last two, where a scene may be worth it (frame_strips), a
+// k_strip<true> that walks what k_frame_raster leaves it.
 // Nothing is cleared ahead: the setup blocks store their own sums.  640x480
 // sphere, 4 k triangles, back to back: 28.3 us a call as seven launches, 14.4
 // us as three (k_front 5.5, k_frame_raster 7.2, k_resolve 9.0 us each alone).
 // ---------------------------------------------------------------------------
-constexpr uint32_t kFrameGroups = 1024;                // 32-primitive groups at most
-constexpr uint32_t kFramePrims = 32 * kFrameGroups;
 constexpr uint32_t kFrameBlocks = kFramePrims / kBlock;  // setup blocks at most
 
 constexpr uint64_t kFramePixels = 1ull << 20, kFrameVerts = 1ull << 17;
@@ -2711,6 +2791,7 @@ __host__ __device__ inline bool frame_fits(const SceneDev &s) {
 struct FrontBlock {  // a setup block's sums
     uint4 cov;       // min of (cx0, cy0, ~cx1, ~cy1)
     uint32_t culled, bad;
+    unsigned long long walked;  // the fragments its triangles may make
 };
 struct FrontScratch {
     uint32_t group_rows[kFrameGroups];
@@ -2756,11 +2837,12 @@ __global__ void __launch_bounds__(kBlock) k_front(const __grid_constant__ FrontA
         const uint32_t wr = __reduce_add_sync(0xFFFFFFFFu, o.nrows);
         if ((threadIdx.x & 31) == 0) a.front->group_rows[t >> 5] = wr;
         const int bad = __syncthreads_or(o.bad);
-        const SetupSums q = setup_block_sums<false>(o);
+        const SetupSums q = s.strip_h ? setup_block_sums<true>(o) : setup_block_sums<false>(o);  // (k_strip<true> follows)
         if (threadIdx.x == 0) {
             a.front->blk[b].cov = make_uint4(q.x0, q.y0, q.nx1, q.ny1);
             a.front->blk[b].culled = q.culled;
             a.front->blk[b].bad = bad ? 1u : 0u;
+            a.front->blk[b].walked = q.walked;
         }
         if (b == 0) {  // (a scene has at least one setup block)
             const uint32_t *src = reinterpret_cast<const uint32_t *>(&a.d);
@@ -2800,7 +2882,8 @@ __global__ void __launch_bounds__(kBlock) k_front(const __grid_constant__ FrontA
     }
 }
 
-template <int kMode>
+// kStrips: k_strip<true> follows, which takes the scene if it has enough fragments.
+template <int kMode, bool kStrips>
 __global__ void __launch_bounds__(kBlock, 4) k_frame_raster(const SceneDev *sc,
                                                            const TriRec *recs,
                                                            const uint32_t *rows,
@@ -2813,6 +2896,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_frame_raster(const SceneDev *sc,
                                                            uint2 *__restrict__ frags, uint64_t frag_cap, bool probe) {
     __shared__ uint32_t s_a[kBlock / 32 + 1];
     __shared__ __align__(16) uint32_t s_pref[kFrameGroups];
+    __shared__ unsigned long long s_walked[kStrips ? kBlock / 32 : 1];
     begin_stage();
     if (kMode == RASTER_FILL && totals[4] > frag_cap) return;  // the lists do not fit: the host grows them
     const SceneDev &s = sc[0];
@@ -2826,7 +2910,18 @@ __global__ void __launch_bounds__(kBlock, 4) k_frame_raster(const SceneDev *sc,
     const uint32_t per = s.prim == EUC_PRIM_TRIANGLE_LIST ? 32u / kFrameLanes : 32u;
 #pragma unroll
     for (uint32_t k = 0; k < 4; ++k) steps[k] = 4 * threadIdx.x + k < ngroups ? (steps[k] + per - 1) / per : 0u;
+    if constexpr (kStrips) {
+        const unsigned long long w = warp_sum(threadIdx.x < nsb ? front->blk[threadIdx.x].walked : 0ull);
+        if (lane == 0) s_walked[threadIdx.x >> 5] = w;
+    }
     const int bad = __syncthreads_or(threadIdx.x < nsb && front->blk[threadIdx.x].bad);
+    bool strips = false;
+    if constexpr (kStrips) {
+        unsigned long long walked = 0;
+#pragma unroll
+        for (int w = 0; w < kBlock / 32; ++w) walked += s_walked[w];
+        strips = !bad && walked >= kFrameStripFrags + kFrameStripPerPixel * (s.W * s.H);
+    }
     if (kMode != RASTER_FILL && blockIdx.x == 0 && threadIdx.x < 32) {
         FrontBlock q;
         q.cov = make_uint4(0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu);
@@ -2852,9 +2947,14 @@ __global__ void __launch_bounds__(kBlock, 4) k_frame_raster(const SceneDev *sc,
             rbase[0] = 0;
             rbase[1] = bad ? 0ull : resolve_chunks(s, q.cov);  // a scene with a bad index draws nothing
             if (kMode == RASTER_COUNT) totals[4] = totals[5] = 0;  // k_oscan: fragments, finished blocks
+            if constexpr (kStrips) {
+                const FrameStrips f(s, q.cov, s.nstrips);  // (nstrips: k_strip's blocks)
+                totals[kUnitCount] = strips ? (unsigned long long)f.strips * f.ranges : 0ull;
+                totals[7] = 0;  // k_strip's work counter
+            }
         }
     }
-    if (bad) return;
+    if (bad || strips) return;
     uint32_t total;
     const uint32_t pre = block_excl_scan<uint32_t>((steps[0] + steps[1]) + (steps[2] + steps[3]), s_a, &total);
     *reinterpret_cast<uint4 *>(s_pref + 4 * threadIdx.x) =

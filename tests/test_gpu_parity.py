@@ -618,3 +618,33 @@ def test_narrow_targets(gpu_ctx, strip_ctx, w, h, test, write):
             got, got_stats = run_gpu(ctx, make(k))
             assert got_stats == ref_stats
             assert_targets_match(make(k), ref, got)
+
+
+@pytest.mark.parametrize("w,h,n,area", [(300, 200, 9000, 4000.0), (300, 200, 32768, 1500.0), (33, 700, 9001, 5000.0),
+                                        (1100, 60, 8192, 9000.0), (130, 97, 20000, 6000.0)])
+@pytest.mark.parametrize("desc", [dict(), dict(depth_test=abi.TEST_GREATER), dict(depth_test=abi.TEST_NONE, depth_write=0),
+                                  dict(depth_test=abi.TEST_LESS, depth_write=0), dict(aa_level=1, band_rows=11)])
+def test_overdrawn_small_scenes(gpu_ctx, w, h, n, area, desc):
+    """Small scenes with enough fragments for the strips: several strips and
+    ranges of primitives (the last one short), units packed in one and in
+    several goes, both kinds of keys, bands; and one with a bad index, which
+    draws nothing."""
+    def make(bad=False):
+        rng = np.random.default_rng(n)
+        clip = scenes.soup_triangles(rng, n, w, h, 0.9 * area, area, extent=0.8)
+        clip[:, 2] = rng.uniform(-0.1, 1.1, n * 3)
+        idx = rng.permutation(n * 3).astype(np.uint32)
+        if bad:
+            idx[-1] = n * 3
+        return scenes.clip_triangles_frame(clip, rng.integers(0, 256, (n * 3, 4), dtype=np.uint8), w, h, indices=idx,
+                                           depth_clear=0.5 if desc else 1.0, **desc)
+    ref, ref_stats = run_oracle(make(), threads=8)
+    for _ in range(3):  # plain, recorded, replayed
+        got, got_stats = run_gpu(gpu_ctx, make())
+        assert got_stats == ref_stats
+        assert_targets_match(make(), ref, got)
+    if not desc:
+        got, got_stats = run_gpu(gpu_ctx, make(bad=True))
+        assert got_stats[0][0] == abi.ERR_INDEX_OOB and got_stats[0][1] == 0
+        clean = make().alloc_host_targets()
+        assert all(np.array_equal(got[k], clean[k]) for k in clean)
