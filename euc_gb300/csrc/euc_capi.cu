@@ -468,12 +468,13 @@ void dispatch_geometry(uint32_t shader, const SceneDev *sc, const uint64_t *gb, 
     }
 }
 
+// narrow: one of the scenes is (narrow_scene<kDirectPer>)
 template <class F>
-void launch_resolve(const SceneDev *sc, const uint64_t *rbase, int s0, int s1, uint64_t nblk, euc_ctx *ctx,
+void launch_resolve(const SceneDev *sc, const uint64_t *rbase, int s0, int s1, uint64_t nblk, bool narrow, euc_ctx *ctx,
                     cudaStream_t st) {
     if (!nblk) return;
     const euc_tuning &tu = ctx->tune;
-    (void)launch_stage(ctx, k_resolve<F>, chunk_grid(nblk, ctx->nsm, tu.chunk_group, tu.chunk_blocks_per_sm), kBlock,
+    (void)launch_stage(ctx, narrow ? k_resolve<F, true> : k_resolve<F, false>, chunk_grid(nblk, ctx->nsm, tu.chunk_group, tu.chunk_blocks_per_sm), kBlock,
                        0, st, sc, rbase, s0, s1, chunk_group(nblk, ctx->nsm, tu.chunk_group, tu.chunk_blocks_per_sm),
                        (const TriRec *)ctx->recs.p, (const float *)ctx->vdata.p,
                        (const unsigned long long *)ctx->vbuf.p, (const uint4 *)ctx->cov.p);
@@ -492,14 +493,14 @@ void dispatch_vertex(uint32_t shader, const SceneDev *sc, const uint64_t *vb, in
 }
 
 void dispatch_resolve(uint32_t shader, const SceneDev *sc, const uint64_t *rbase, int s0, int s1, uint64_t nblk,
-                      euc_ctx *ctx, cudaStream_t st) {
+                      bool narrow, euc_ctx *ctx, cudaStream_t st) {
     switch (shader) {
-    case EUC_SHADER_FLAT: launch_resolve<FlatFn>(sc, rbase, s0, s1, nblk, ctx, st); break;
-    case EUC_SHADER_VCOLOR: launch_resolve<VColorFn>(sc, rbase, s0, s1, nblk, ctx, st); break;
-    case EUC_SHADER_GOURAUD: launch_resolve<GouraudFn>(sc, rbase, s0, s1, nblk, ctx, st); break;
-    case EUC_SHADER_TEXTURED: launch_resolve<TexturedFn>(sc, rbase, s0, s1, nblk, ctx, st); break;
-    case EUC_SHADER_PHONG: launch_resolve<PhongFn>(sc, rbase, s0, s1, nblk, ctx, st); break;
-    case EUC_SHADER_SHADOW: launch_resolve<ShadowFn>(sc, rbase, s0, s1, nblk, ctx, st); break;
+    case EUC_SHADER_FLAT: launch_resolve<FlatFn>(sc, rbase, s0, s1, nblk, narrow, ctx, st); break;
+    case EUC_SHADER_VCOLOR: launch_resolve<VColorFn>(sc, rbase, s0, s1, nblk, narrow, ctx, st); break;
+    case EUC_SHADER_GOURAUD: launch_resolve<GouraudFn>(sc, rbase, s0, s1, nblk, narrow, ctx, st); break;
+    case EUC_SHADER_TEXTURED: launch_resolve<TexturedFn>(sc, rbase, s0, s1, nblk, narrow, ctx, st); break;
+    case EUC_SHADER_PHONG: launch_resolve<PhongFn>(sc, rbase, s0, s1, nblk, narrow, ctx, st); break;
+    case EUC_SHADER_SHADOW: launch_resolve<ShadowFn>(sc, rbase, s0, s1, nblk, narrow, ctx, st); break;
     }
 }
 
@@ -888,7 +889,10 @@ int run_batch(euc_ctx *ctx, const euc_scene *scenes, size_t n, cudaStream_t st, 
             if (a >= first_ordered)
                 dispatch_resolve_ordered(plans[a].d.shader, dsc, drb, a, b, blk0, blk1 - blk0, cap, ctx, st);
             else
-                dispatch_resolve(plans[a].d.shader, dsc, rbase, a, b, blk1 - blk0, ctx, st);
+                dispatch_resolve(plans[a].d.shader, dsc, rbase, a, b, blk1 - blk0,
+                                 std::any_of(plans.begin() + a, plans.begin() + b,
+                                             [](const Plan &p) { return narrow_scene<kDirectPer>(p.d); }),
+                                 ctx, st);
             ctx->launches += blk1 > blk0;
             a = b;
         }
@@ -1054,7 +1058,7 @@ int launch_frame(euc_ctx *ctx, const FrontArgs &a, cudaStream_t st, int *host_er
                                    (SceneStats *)ctx->stats.p, (unsigned long long *)ctx->totals.p));
             ctx->launches += 1;
         }
-        dispatch_resolve(a.d.shader, sc, (uint64_t *)ctx->plan.p, 0, 1, nblk, ctx, st);
+        dispatch_resolve(a.d.shader, sc, (uint64_t *)ctx->plan.p, 0, 1, nblk, narrow_scene<kDirectPer>(a.d), ctx, st);
     }
     CUDA_TRY(cudaGetLastError());
     return EUC_OK;
@@ -2069,7 +2073,7 @@ void na_vertex_resolve(bool vertex, const SceneDev *sc, const uint64_t *base, ui
         k_vertex<F><<<(unsigned)nblk, kBlock, 0, st>>>(sc, base, 0, 1, 0, (float4 *)(a + kNaOffClip),
                                                        (float *)(a + kNaOffVdata), PrepArgs{});
     else
-        k_resolve<F><<<chunk_grid(nblk, t_na_nsm), kBlock, 0, st>>>(
+        k_resolve<F, true><<<chunk_grid(nblk, t_na_nsm), kBlock, 0, st>>>(
             sc, base, 0, 1, chunk_group(nblk, t_na_nsm), (const TriRec *)(a + kNaOffRecs),
             (const float *)(a + kNaOffVdata), (const unsigned long long *)(a + kNaOffVbuf), (const uint4 *)(a + kNaOffCov));
 }

@@ -221,7 +221,7 @@ struct VColorFn {  // examples/triangle.rs:14-25
 struct GouraudFn {
     static constexpr int NV = 3, NF = 4;
     static constexpr bool kDirect = true;  // shaded in place, without the job list of k_resolve
-    static constexpr int kResolveBlocks = 4;  // k_resolve blocks per SM: 5 spill; 256 spheres 601 us with 4, 605 with 5
+    static constexpr int kResolveBlocks = 5;  // k_resolve blocks per SM (12 bytes spilled): 256 spheres 603 us, 607 with 4
     using U = euc_gouraud_uniforms;
     static EUC_DEV void vertex(const U &u, const euc_vertex_layout &l, const uint8_t *v, float clip[4], float *vd) {
         const float p[4] = {ld_f32(v + l.position), ld_f32(v + l.position + 4), ld_f32(v + l.position + 8), 1.0f};

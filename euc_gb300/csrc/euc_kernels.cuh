@@ -1184,11 +1184,12 @@ constexpr int kChunkGroup = 16;
 // no division or wrap.  256 spheres of 640x480 (86 k pixels of the rectangle
 // each): k_init 71 -> 57 us (45 -> 24 M instructions), k_resolve<GouraudFn>
 // 214 -> 203 us (130 -> 108 M; what bounds it now is L1, 84 % busy).
-// A rectangle of at most 16 kPer columns gives a row as few lanes (a power of
-// two) as hold it, and a warp the next rows too: 4 x 100000 pixels 34 us a frame
-// against 62 with a warp a row, 16 x 32768 30 and 38, 64 x 8192 27 and 33.
+// Scenes whose targets have at most 16 kPer columns (narrow_scene) give a row as
+// few lanes (a power of two) as hold the rectangle's, and a warp the next rows
+// too: 4 x 100000 pixels 33 us a frame against 62 with a warp a row, 16 x 32768 30
+// and 38, 64 x 8192 27 and 33.
 template <int kPer>
-__host__ __device__ inline bool narrow_rect(uint32_t w) { return w <= 16 * kPer; }
+__host__ __device__ inline bool narrow_scene(const SceneDev &s) { return s.W <= 16 * kPer; }
 template <int kPer>
 __host__ __device__ inline uint32_t segment_shift(uint32_t w) {  // log2 of a row's lanes, w > 0
     uint32_t shift = 0;
@@ -1198,10 +1199,10 @@ __host__ __device__ inline uint32_t segment_shift(uint32_t w) {  // log2 of a ro
 template <int kPer>
 struct RowSegment {
     uint32_t y, x, xend;  // the row, this lane's first pixel, the end of the row or segment
-    uint32_t step;        // between this lane's pixels
-    EUC_DEV RowSegment(const uint4 &cv, uint32_t lb) {
+    uint32_t step;        // between this lane's pixels (32 where it is known that the scene is not narrow)
+    EUC_DEV RowSegment(const uint4 &cv, uint32_t lb, bool narrow) {
         const uint32_t w = ~cv.z - cv.x, u = lb * (kBlock / 32) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-        if (narrow_rect<kPer>(w)) {
+        if (narrow) {
             const uint32_t shift = segment_shift<kPer>(w);
             step = 1u << shift;
             y = cv.y + ((u * 32 + lane) >> shift);
@@ -1218,11 +1219,11 @@ struct RowSegment {
     }
 };
 template <int kPer>
-__host__ __device__ inline uint64_t segment_chunks(const uint4 &cv) {
+__host__ __device__ inline uint64_t segment_chunks(const SceneDev &s, const uint4 &cv) {
     if (rect_area(cv) == 0) return 0;
     const uint64_t w = ~cv.z - cv.x, rows = ~cv.w - cv.y;
-    const uint64_t warps = narrow_rect<kPer>((uint32_t)w) ? ((rows << segment_shift<kPer>((uint32_t)w)) + 31) / 32
-                                                          : (w + 32 * kPer - 1) / (32 * kPer) * rows;
+    const uint64_t warps = narrow_scene<kPer>(s) ? ((rows << segment_shift<kPer>((uint32_t)w)) + 31) / 32
+                                                 : (w + 32 * kPer - 1) / (32 * kPer) * rows;
     return (warps + kBlock / 32 - 1) / (kBlock / 32);
 }
 
@@ -1256,7 +1257,7 @@ constexpr int kInitChunk = kBlock * kInitPer;
 // k_init chunks of a scene: the row segments of its covered rectangle; every
 // entry, padding included, of an ordered one.
 __host__ __device__ inline uint64_t init_chunks(const SceneDev &s, const uint4 &cv) {
-    if (s.keytype != KEY_ORDERED) return segment_chunks<kInitPer>(cv);
+    if (s.keytype != KEY_ORDERED) return segment_chunks<kInitPer>(s, cv);
     const uint64_t lim = ((uint64_t)s.W * s.H + kBlock - 1) / kBlock * kBlock;
     return (lim + kInitChunk - 1) / kInitChunk;
 }
@@ -1304,8 +1305,9 @@ __global__ void __launch_bounds__(kBlock) k_init(const SceneDev *__restrict__ sc
             const uint32_t W = s.W, dpitch = s.dpitch;
             const uint8_t *const depth = s.depth;
             const bool kmin = s.keytype == KEY_MIN, greater = s.depth_test == EUC_TEST_GREATER;
+            const bool narrow = narrow_scene<kInitPer>(s);
             for (; lb < lend; ++lb) {
-                const RowSegment<kInitPer> g(cv, lb);
+                const RowSegment<kInitPer> g(cv, lb, narrow);
                 unsigned long long *key = keys + (uint64_t)g.y * W + g.x;
                 const float *d0 = reinterpret_cast<const float *>(depth + (uint64_t)g.y * dpitch) + g.x;
                 float d[kInitPer];
@@ -2351,7 +2353,7 @@ __host__ __device__ inline bool resolve_direct(const SceneDev &s) {
 __host__ __device__ inline uint64_t resolve_chunks(const SceneDev &s, const uint4 &cv) {
     const uint64_t area = rect_area(cv);
     if (area == 0) return 0;
-    if (resolve_direct(s)) return segment_chunks<kDirectPer>(cv);
+    if (resolve_direct(s)) return segment_chunks<kDirectPer>(s, cv);
     if (resolve_by_quads(s)) {
         const uint64_t pairs = pair_of_row(~cv.w - 1, s.gr) - pair_of_row(cv.y, s.gr) + 1;
         const uint64_t cols = ((~cv.z - 1) >> 4) - (cv.x >> 4) + 1;
@@ -2510,10 +2512,10 @@ struct ResolveSmem {
 // are in flight together).  The scene's fields are read once, ahead of the
 // stores: behind one, the compiler has to read them again (20 loads a pixel,
 // twice what the shading itself needs).
-template <class F>
+template <class F, bool kNarrow>
 EUC_DEV void resolve_direct_chunk(const SceneDev &s, const uint4 &cv, uint64_t lb, const TriRec *__restrict__ recs,
                                   const float *__restrict__ vdata, const unsigned long long *vbuf) {
-    const RowSegment<kDirectPer> g(cv, (uint32_t)lb);
+    const RowSegment<kDirectPer> g(cv, (uint32_t)lb, kNarrow && narrow_scene<kDirectPer>(s));
     const bool kmin = s.keytype == KEY_MIN, greater = s.depth_test == EUC_TEST_GREATER;
     const unsigned long long *keys = vbuf + s.pix_base + (uint64_t)g.y * s.W + g.x;
     unsigned long long key[kDirectPer];
@@ -2695,8 +2697,11 @@ EUC_DEV void resolve_chunk(const SceneDev &s, const uint4 &cv, const ChunkGeom &
 // Blocks walk groups of `group` chunks (grid-strided) of the scenes
 // [s_begin, s_end); rbase (global scene index, from plan_chunks) holds the first
 // chunk of each.
-template <class F>
-__global__ void __launch_bounds__(kBlock, F::kResolveBlocks) k_resolve(const SceneDev *__restrict__ sc,
+// kNarrow: the launch has narrow scenes (narrow_scene<kDirectPer>).  Without them
+// the step between a lane's pixels is a constant (640x480 sphere 25.0 us a frame
+// against 25.3), and GouraudFn's fifth block pays for its 12 bytes of spills.
+template <class F, bool kNarrow>
+__global__ void __launch_bounds__(kBlock, kNarrow && F::kResolveBlocks > 4 ? 4 : F::kResolveBlocks) k_resolve(const SceneDev *__restrict__ sc,
                                                                     const uint64_t *rbase,
                                                     int s_begin, int s_end, uint32_t group,
                                                     const TriRec *__restrict__ recs, const float *__restrict__ vdata,
@@ -2717,7 +2722,7 @@ __global__ void __launch_bounds__(kBlock, F::kResolveBlocks) k_resolve(const Sce
             si = advance_scene(base, n, si, c);
             const SceneDev &s = sc[s_begin + si];
             if (resolve_direct(s)) {  // uniform: one scene per chunk
-                resolve_direct_chunk<F>(s, cov[s_begin + si], c - base[si], recs, vdata, vbuf);
+                resolve_direct_chunk<F, kNarrow>(s, cov[s_begin + si], c - base[si], recs, vdata, vbuf);
             } else {
                 const uint4 cv = cov[s_begin + si];
                 if (si != gsi) {  // the block's chunks reached a new scene
