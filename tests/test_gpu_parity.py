@@ -648,3 +648,24 @@ def test_overdrawn_small_scenes(gpu_ctx, w, h, n, area, desc):
         assert got_stats[0][0] == abi.ERR_INDEX_OOB and got_stats[0][1] == 0
         clean = make().alloc_host_targets()
         assert all(np.array_equal(got[k], clean[k]) for k in clean)
+
+
+@pytest.mark.parametrize("n", [32, 33, 1024, 1025, 1500])
+def test_batches_of_many_tiny_scenes(n):
+    """Scene lookups by the whole warp, up to their third level (more than 1024
+    scenes): every scene's image is the oracle's."""
+    from euc_gb300 import capi, frames
+    made = [scenes.soup_frame(seed=k, width=7 + k % 5, height=6 + k % 3, ntris=1 + k % 4, area_hi=40.0) for k in range(n)]
+    batch = frames.DeviceBatch(made)
+    ctx = capi.Context(0)
+    try:
+        frames.render_batch(ctx, batch)
+        assert ctx.sync(frames._stream_ptr(None)) == abi.OK
+        candidates, total = ctx.stats(frames._stream_ptr(None)).candidates, 0
+        for f, df in zip(made, batch.frames):
+            ref, ref_stats = run_oracle(f)
+            total += ref_stats[0][1]
+            assert_targets_match(f, ref, df.to_host())
+        assert candidates == total
+    finally:
+        ctx.close()

@@ -116,3 +116,37 @@ def test_texture_ingest_tile_edges(fmt, ch, dtype, w, h, pad, off):
         assert (dst.cpu().numpy()[:, w:] == 0).all()
     finally:
         ctx.close()
+
+
+@pytest.mark.parametrize("fmt,ch,dtype", [(abi.SRC_RGBA8, 4, np.uint8), (abi.SRC_BGRA8, 4, np.uint8),
+                                          (abi.SRC_RGB8, 3, np.uint8), (abi.SRC_LUMA8, 1, np.uint8),
+                                          (abi.SRC_LUMA_ALPHA8, 2, np.uint8), (abi.SRC_R32F, 1, np.float32)])
+@pytest.mark.parametrize("w,h", [(1, 3), (2, 9), (3, 16), (5, 17), (127, 5), (129, 20), (130, 8), (515, 7)])
+def test_texture_ingest_word_rows_with_a_remainder(fmt, ch, dtype, w, h):
+    """Rows that start on whole words on both sides (source rows of a multiple
+    of 48 bytes, target rows of four texels) with widths that are no multiple of
+    four: the last texels of a row go one by one, and the padding of the target's
+    rows stays as it was."""
+    import torch
+    rng = np.random.default_rng(w * 11 + h + fmt)
+    img = (rng.standard_normal((h, w)).astype(np.float32) if dtype == np.float32
+           else rng.integers(0, 256, (h, w, ch) if ch > 1 else (h, w), dtype=np.uint8))
+    want = oracle.texture_ingest(img, fmt)
+    row = w * ch * img.itemsize
+    pitch = (row + 47) // 48 * 48
+    raw = np.full((h, pitch), 0xA5, dtype=np.uint8)
+    raw[:, :row] = np.ascontiguousarray(img).view(np.uint8).reshape(h, row)
+    src = torch.from_numpy(raw).cuda()
+    wide = (w + 3) // 4 * 4 + 4
+    ctx = capi.Context(0)
+    try:
+        dst = torch.full((h, wide, 4), 0x5A, dtype=torch.uint8, device="cuda")
+        assert src.data_ptr() % 16 == 0 and dst.data_ptr() % 16 == 0
+        assert capi.lib().euc_texture_ingest(ctx.handle, src.data_ptr(), w, h, pitch, fmt, dst.data_ptr(),
+                                             dst.stride(0), _stream()) == abi.OK
+        torch.cuda.synchronize()
+        got = dst.cpu().numpy()
+        assert np.array_equal(got[:, :w], want)
+        assert (got[:, w:] == 0x5A).all()
+    finally:
+        ctx.close()
