@@ -474,8 +474,9 @@ void launch_resolve(const SceneDev *sc, const uint64_t *rbase, int s0, int s1, u
                     cudaStream_t st) {
     if (!nblk) return;
     const euc_tuning &tu = ctx->tune;
-    (void)launch_stage(ctx, narrow ? k_resolve<F, true> : k_resolve<F, false>, chunk_grid(nblk, ctx->nsm, tu.chunk_group, tu.chunk_blocks_per_sm), kBlock,
-                       0, st, sc, rbase, s0, s1, chunk_group(nblk, ctx->nsm, tu.chunk_group, tu.chunk_blocks_per_sm),
+    (void)launch_stage(ctx, narrow ? k_resolve<F, true> : k_resolve<F, false>,
+                       chunk_grid(nblk, ctx->nsm, tu.chunk_group, tu.chunk_blocks_per_sm), kBlock, 0, st, sc, rbase, s0,
+                       s1, chunk_group(nblk, ctx->nsm, tu.chunk_group, tu.chunk_blocks_per_sm),
                        (const TriRec *)ctx->recs.p, (const float *)ctx->vdata.p,
                        (const unsigned long long *)ctx->vbuf.p, (const uint4 *)ctx->cov.p);
 }

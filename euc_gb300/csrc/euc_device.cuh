@@ -24,9 +24,8 @@ EUC_DEV float rmax(float a, float b) { return fmaxf(a, b); }
 
 // `v as usize` (saturating, NaN -> 0), further capped at 2^32 - 1.  Every use
 // clamps the result to a target extent below 2^32, so the cap changes nothing.
-// The hardware's conversion toward zero saturates at 0 and 2^32 - 1 and takes
-// a NaN to 0: one instruction, compared with the comparisons written out over
-// all 2^32 floats.
+// The conversion toward zero saturates at 0 and 2^32 - 1 and takes a NaN to 0
+// (PTX ISA, cvt from floating point to integer).
 EUC_DEV uint32_t sat_u32(float v) { return __float2uint_rz(v); }
 
 // `v as u8` (saturating, NaN -> 0).

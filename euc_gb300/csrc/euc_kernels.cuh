@@ -690,7 +690,7 @@ constexpr uint32_t kTinyPixels = 4;
 // fragments in shared memory, then merges every key it lowered into the keys
 // k_init seeded with one 64-bit min per pixel.  The other primitives, and the
 // scenes the path does not take (lines, ordered blends, targets too wide for
-// a strip), go through k_raster's item queue after the strips.  Which way a
+// a strip), go through k_raster's item queue beside them.  Which way a
 // primitive goes changes no result: the keys are order-free reductions.
 // ---------------------------------------------------------------------------
 // Threads of a k_strip block: two blocks of 24 warps, which 40 registers a
@@ -1021,8 +1021,8 @@ EUC_DEV SetupSums setup_block_sums(const SetupOut &o) {
 // k_setup: block b sets up primitives [b * kBlock, (b + 1) * kBlock), all of
 // scene chunk_scene[b] (null: scene 0).
 // Latency of the position gathers and of the stores: five blocks an SM (48
-// registers, 24 bytes spilled) hide more of it than four (62): 3.8 M primitives
-// 134 -> 119 us, 500 k 22.4 -> 20.9; six (40, 48 bytes spilled) 120 and 22.6.
+// registers, 8 bytes of spill stores) hide more of it than four (62): 3.8 M
+// primitives 134 -> 119 us, 500 k 22.4 -> 20.9; six (40, more spills) 120 and 22.6.
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(kBlock, 5) k_setup(const SceneDev *__restrict__ sc,
                                                   const uint32_t *__restrict__ chunk_scene,
@@ -2510,8 +2510,7 @@ struct ResolveSmem {
 // Chunk `lb` of a resolve_direct scene: a warp's row segment, kDirectPer
 // pixels a lane (their key loads, and then their record and varyings gathers,
 // are in flight together).  The scene's fields are read once, ahead of the
-// stores: behind one, the compiler has to read them again (20 loads a pixel,
-// twice what the shading itself needs).
+// stores: behind one, they would have to be read again.
 template <class F, bool kNarrow>
 EUC_DEV void resolve_direct_chunk(const SceneDev &s, const uint4 &cv, uint64_t lb, const TriRec *__restrict__ recs,
                                   const float *__restrict__ vdata, const unsigned long long *vbuf) {
@@ -2769,7 +2768,7 @@ __global__ void __launch_bounds__(kBlock, kNarrow && F::kResolveBlocks > 4 ? 4 :
 // k_strip<true> that walks what k_frame_raster leaves it.
 // Nothing is cleared ahead: the setup blocks store their own sums.  640x480
 // sphere, 4 k triangles, back to back: 28.3 us a call as seven launches, 14.4
-// us as three (k_front 5.5, k_frame_raster 7.2, k_resolve 9.0 us each alone).
+// us as three (k_front 5.5, k_frame_raster 8.7, k_resolve 9.1 us each alone).
 // ---------------------------------------------------------------------------
 constexpr uint32_t kFrameBlocks = kFramePrims / kBlock;  // setup blocks at most
 
@@ -3036,7 +3035,7 @@ __global__ void __launch_bounds__(kBlock) k_copy_pieces(const CopyPiece *__restr
 }
 
 // ---------------------------------------------------------------------------
-// Texture ingest: one thread per texel, image-crate layouts -> sampler layouts.
+// Texture ingest: image-crate layouts -> sampler layouts.
 // ---------------------------------------------------------------------------
 __host__ __device__ inline uint32_t src_bpp(uint32_t f) {
     switch (f) {
