@@ -565,11 +565,13 @@ struct StageOverride {
 // lists are known to fit, while the fill runs, so that a batch that cannot be
 // drawn for want of list space draws nothing.
 constexpr uint64_t kFragGuess = 1ull << 23;
-// Ordered scenes of more primitives than this may have long lists, which
-// k_resolve_ordered reads in windows, the faster the more a list is in order:
-// their raster passes keep to fewer warps where few suffice (200 triangles over
-// 64x64 pixels: 216 us a frame, 404 with a warp for each eight rows).
-constexpr uint32_t kShortLists = 64;
+// Scenes of at most this many primitives, which may be large for their number,
+// get a raster warp for each step of their rows.  With more, a warp for each 32
+// rows is as good or better: a 160x120 sphere of 224 triangles 22.4 us a frame, 23.1
+// with the larger grid; and ordered scenes' lists come out in better order, which
+// k_resolve_ordered's windows are the faster for (200 triangles over 64x64 pixels
+// 216 us, 404).
+constexpr uint32_t kFewPrims = 64;
 template <class Fill, class Resolve>
 int ordered_lists(euc_ctx *ctx, uint64_t p0, uint64_t p1, bool late, cudaStream_t st, Fill fill, Resolve resolve) {
     int rc;
@@ -907,7 +909,7 @@ int run_batch(euc_ctx *ctx, const euc_scene *scenes, size_t n, cudaStream_t st, 
             (plans[i].d.prim == EUC_PRIM_TRIANGLE_LIST ? tris : lines) += plans[i].d.ngroups;
         const bool wide = tris >= lines;
         bool dense = false;
-        for (int i = first_ordered; i < ns; ++i) dense = dense || plans[i].d.ngroups > kShortLists;
+        for (int i = first_ordered; i < ns; ++i) dense = dense || plans[i].d.ngroups > kFewPrims;
         const unsigned grid = raster_grid(first_ordered, ns, wide && !dense ? kBlock / kOrderedLanes : kBlock);
         CUDA_TRY(wide ? raster(k_raster<RASTER_COUNT, kOrderedLanes>, grid, 0) : raster(k_raster<RASTER_COUNT, 1>, grid, 0));
         rc = ordered_lists(
@@ -1022,8 +1024,8 @@ int launch_frame(euc_ctx *ctx, const FrontArgs &a, cudaStream_t st, int *host_er
     // a warp takes 32 / kFrameLanes rows a step, 32 steps of lines (with blocks
     // for 32 rows a warp, two triangles over 640x480 41 us a frame against 34,
     // ten 48 and 35, two over 1024x1024 70 and 49)
-    const bool dense = a.d.keytype == KEY_ORDERED && a.d.ngroups > kShortLists;
-    const uint32_t per_block = a.d.prim == EUC_PRIM_TRIANGLE_LIST && !dense ? kBlock / kFrameLanes : kBlock;
+    const bool few = a.d.ngroups <= kFewPrims && a.d.prim == EUC_PRIM_TRIANGLE_LIST;
+    const uint32_t per_block = few ? kBlock / kFrameLanes : kBlock;
     const uint64_t busy = a.d.ngroups * slot_items(a.d) / per_block + a.nsb;
     const uint32_t per_sm = ctx->tune.raster_blocks_per_sm ? ctx->tune.raster_blocks_per_sm : (uint32_t)ctx->raster_blocks;
     const unsigned grid = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(busy, (uint64_t)ctx->nsm * per_sm));
