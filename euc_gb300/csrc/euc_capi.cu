@@ -2069,27 +2069,27 @@ __global__ void k_na_stage(const NaStage st, unsigned char *__restrict__ a, uint
 }
 
 template <class F>
-void na_vertex_resolve(bool vertex, const SceneDev *sc, const uint64_t *base, uint64_t nblk, unsigned char *a,
-                       cudaStream_t st) {
+void na_vertex_resolve(bool vertex, const SceneDev *sc, const uint64_t *base, uint64_t nblk, bool narrow,
+                       unsigned char *a, cudaStream_t st) {
     if (!nblk) return;
     if (vertex)
         k_vertex<F><<<(unsigned)nblk, kBlock, 0, st>>>(sc, base, 0, 1, 0, (float4 *)(a + kNaOffClip),
                                                        (float *)(a + kNaOffVdata), PrepArgs{});
     else
-        k_resolve<F, true><<<chunk_grid(nblk, t_na_nsm), kBlock, 0, st>>>(
+        (narrow ? k_resolve<F, true> : k_resolve<F, false>)<<<chunk_grid(nblk, t_na_nsm), kBlock, 0, st>>>(
             sc, base, 0, 1, chunk_group(nblk, t_na_nsm), (const TriRec *)(a + kNaOffRecs),
             (const float *)(a + kNaOffVdata), (const unsigned long long *)(a + kNaOffVbuf), (const uint4 *)(a + kNaOffCov));
 }
 
-void na_dispatch(bool vertex, uint32_t shader, const SceneDev *sc, const uint64_t *base, uint64_t nblk,
+void na_dispatch(bool vertex, uint32_t shader, const SceneDev *sc, const uint64_t *base, uint64_t nblk, bool narrow,
                  unsigned char *a, cudaStream_t st) {
     switch (shader) {
-    case EUC_SHADER_FLAT: na_vertex_resolve<FlatFn>(vertex, sc, base, nblk, a, st); break;
-    case EUC_SHADER_VCOLOR: na_vertex_resolve<VColorFn>(vertex, sc, base, nblk, a, st); break;
-    case EUC_SHADER_GOURAUD: na_vertex_resolve<GouraudFn>(vertex, sc, base, nblk, a, st); break;
-    case EUC_SHADER_TEXTURED: na_vertex_resolve<TexturedFn>(vertex, sc, base, nblk, a, st); break;
-    case EUC_SHADER_PHONG: na_vertex_resolve<PhongFn>(vertex, sc, base, nblk, a, st); break;
-    case EUC_SHADER_SHADOW: na_vertex_resolve<ShadowFn>(vertex, sc, base, nblk, a, st); break;
+    case EUC_SHADER_FLAT: na_vertex_resolve<FlatFn>(vertex, sc, base, nblk, narrow, a, st); break;
+    case EUC_SHADER_VCOLOR: na_vertex_resolve<VColorFn>(vertex, sc, base, nblk, narrow, a, st); break;
+    case EUC_SHADER_GOURAUD: na_vertex_resolve<GouraudFn>(vertex, sc, base, nblk, narrow, a, st); break;
+    case EUC_SHADER_TEXTURED: na_vertex_resolve<TexturedFn>(vertex, sc, base, nblk, narrow, a, st); break;
+    case EUC_SHADER_PHONG: na_vertex_resolve<PhongFn>(vertex, sc, base, nblk, narrow, a, st); break;
+    case EUC_SHADER_SHADOW: na_vertex_resolve<ShadowFn>(vertex, sc, base, nblk, narrow, a, st); break;
     }
 }
 
@@ -2161,7 +2161,7 @@ extern "C" int euc_render_noalloc(const euc_pipeline_desc *desc, const void *uni
     prep.nsc = 1;
     k_prep<<<(unsigned)((prep.n + kBlock - 1) / kBlock), kBlock, 0, st>>>(prep);
     t_na_nsm = nsm;
-    na_dispatch(true, d.shader, dsc, zero_base, vtx / kBlock, a, st);
+    na_dispatch(true, d.shader, dsc, zero_base, vtx / kBlock, false, a, st);
     k_setup<<<(unsigned)(tri / kBlock), kBlock, 0, st>>>(dsc, nullptr, (const float4 *)(a + kNaOffClip),
                                                           (TriRec *)(a + kNaOffRecs), (uint32_t *)(a + kNaOffRows),
                                                           (uint2 *)(a + kNaOffChunks), (int *)(a + kNaOffErr),
@@ -2182,7 +2182,7 @@ extern "C" int euc_render_noalloc(const euc_pipeline_desc *desc, const void *uni
         dsc, (const TriRec *)(a + kNaOffRecs), (const uint32_t *)(a + kNaOffLiveTri), (const uint64_t *)(a + kNaOffLiveOff),
         (unsigned long long *)(a + kNaOffTotals), (const int *)(a + kNaOffErr),
         (unsigned long long *)(a + kNaOffVbuf), (SceneStats *)(a + kNaOffStats), nullptr, 0, kWarpItems, false, false);
-    na_dispatch(false, d.shader, dsc, rbase, resolve_blocks(d), a, st);
+    na_dispatch(false, d.shader, dsc, rbase, resolve_blocks(d), narrow_scene<kDirectPer>(d), a, st);
     if (device_status)
         CUDA_TRY(cudaMemcpyAsync(device_status, a + kNaOffErr, sizeof(int), cudaMemcpyDeviceToDevice, st));
     CUDA_TRY(cudaGetLastError());

@@ -133,3 +133,19 @@ def test_noalloc_reports_out_of_bounds_index_on_device():
     finally:
         ctx.close()
     assert np.any(df2.to_host()["depth"] < 1.0)
+
+
+@pytest.mark.parametrize("w,h", [(3, 200), (33, 70), (64, 33), (65, 33), (200, 40)])
+def test_noalloc_targets_of_every_width(w, h):
+    """Targets narrow enough for rows that share a warp, and just wider ones."""
+    import torch
+    f = scenes.soup_frame(seed=w, width=w, height=h, ntris=60, area_hi=0.3 * w * h + 2.0)
+    ref, _, codes = oracle.run_frame(f)
+    assert codes == [abi.OK]
+    df = frames.DeviceFrame(f, "cuda:0")
+    df.clear()
+    status = torch.full((1,), -1, dtype=torch.int32, device="cuda")
+    _render_noalloc(df, status)
+    torch.cuda.synchronize()
+    assert int(status.item()) == abi.OK
+    assert_targets_match(f, ref, df.to_host())
